@@ -7,6 +7,9 @@ Every value is computed here from its mathematical definition with Python's
 * pi/2 as a two-term double split (hi + lo) and 2/pi, for the Cody-Waite
   argument reduction of sin/cos;
 * the Taylor coefficients (-1)^k / (2k+1)! and (-1)^k / (2k)! of sin and cos;
+* the table (sin, cos)(j/64) over one turn and the short polynomials in the
+  remainder that go with it (the last cosine term economised, C. Lanczos,
+  "Applied Analysis", 1956);
 * ln 2 and, for F_j = 1 + j/64 (j = -19..27), the pairs (1/F_j, ln F_j) of a
   table-driven logarithm in the manner of P. T. P. Tang, "Table-driven
   implementation of the logarithm function in IEEE floating-point arithmetic",
@@ -103,32 +106,28 @@ def main() -> None:
         lg = dbl(F.ln()) if j != 0 else 0.0
         out.append(f"    {hexd(inv)}, {hexd(lg)},  /* j = {j} */ \\")
     out.append("")
-    # table-driven sincos: x = j*delta + r, delta = 2 pi / 256, |r| <= delta/2
-    n_sc = 256
-    delta = 2 * pi / n_sc
-    d_hi = dbl(delta)
-    d_lo = dbl(delta - Decimal(d_hi))
+    # table-driven sincos: x = j/64 + r, |r| <= 1/128 (both exact in Float32)
+    n_sc = 404                       # j/64 up to 403/64 > 2 pi
     out.append("")
     out.append(f"#define CLM_SC_N {n_sc}")
-    out.append(f"#define CLM_SC_DELTA_HI {hexd(d_hi)}")
-    out.append(f"#define CLM_SC_DELTA_LO {hexd(d_lo)}")
-    out.append(f"#define CLM_SC_INV_DELTA {hexd(dbl(1 / delta))}")
-    for n in (3, 5, 7):
+    for n in (3, 5):
         c = Decimal((-1) ** ((n - 1) // 2)) / Decimal(math.factorial(n))
         out.append(f"#define CLM_TS{n} {hexd(dbl(c))}")
-    for n in (2, 4, 6, 8):
-        c = Decimal((-1) ** (n // 2)) / Decimal(math.factorial(n))
-        out.append(f"#define CLM_TC{n} {hexd(dbl(c))}")
-    out.append("/* (sin, cos)(j * 2 pi / 256), j = 0..255; exact zeros where the value is 0 */")
+    # cos r - 1 = C2 r^2 + C4 r^4 + C6 r^6 economised to two terms: with t = r^2
+    # in [0, T], t^3 is replaced by the quadratic that leaves the least error
+    # (t^3 minus it is the cubic Chebyshev polynomial with its first root moved
+    # to t = 0), 0.0385 T^3 instead of T^3: 2^-56 of the result
+    T = Decimal(1) / Decimal(128 * 128)
+    root3 = Decimal(3).sqrt()
+    sc = T / (1 + root3 / 2)
+    c2, c4, c6 = Decimal(-1) / 2, Decimal(1) / 24, Decimal(-1) / 720
+    out.append(f"#define CLM_TC2 {hexd(dbl(c2 - c6 * (3 * sc * sc / 2)))}")
+    out.append(f"#define CLM_TC4 {hexd(dbl(c4 + c6 * (3 * root3 / 2 * sc)))}")
+    out.append("/* (sin, cos)(j / 64), j = 0..403 */")
     out.append("#define CLM_SC_TAB_INIT \\")
     for j in range(n_sc):
-        if j % 64 == 0:
-            sj, cj = (0.0, [1.0, 0.0, -1.0, 0.0][j // 64]) if j % 128 == 0 else (
-                [0.0, 1.0, 0.0, -1.0][j // 64], 0.0)
-        else:
-            sd, cd = d_sin_cos(delta * j)
-            sj, cj = dbl(sd), dbl(cd)
-        out.append(f"    {hexd(sj)}, {hexd(cj)},  /* j = {j} */ \\")
+        sd, cd = d_sin_cos(Decimal(j) / 64)
+        out.append(f"    {hexd(dbl(sd))}, {hexd(dbl(cd))},  /* j = {j} */ \\")
     out.append("")
     print("\n".join(out))
 
