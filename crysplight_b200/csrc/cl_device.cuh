@@ -69,23 +69,27 @@ __device__ __forceinline__ float u32_to_randu(uint32_t x)
 
 // A photon's uniform stream (PhiloxStream, src/philox.jl:34-62): key = seed,
 // counter = (pid lo, pid hi, block, 0).  The uniforms are buffered, already
-// converted by randu, in a per-lane ring of RING_LEN floats in shared memory:
-// word i of the lane at column `tid` sits at ring[(i % RING_LEN) * RING_STRIDE]
-// (every access is bank-conflict free).  Blocks are generated ahead of use, at
-// one convergent point of the warp loop; pop() consumes in order and peek(d)
-// looks d words ahead, so the sequence of uniforms is exactly the reference's.
-// 32 words (32 KB for 256 threads; rings of 28, 36, 40 and 48 words measured
-// 3-15% slower on the BGO+ESR scan)
-#ifndef CL_RING_LEN
-#define CL_RING_LEN 32
-#endif
-constexpr int RING_LEN = CL_RING_LEN;
-constexpr int RING_STRIDE = 256;      // columns: the largest block the kernels launch
+// converted by randu, in a per-lane ring of 32 floats in shared memory (rings
+// of 28, 36, 40 and 48 words measured 3-15% slower on the BGO+ESR scan): word i
+// of the lane at column tid sits in row i % 32, every access free of bank
+// conflicts.  Blocks are generated ahead of use, two at a time, at one
+// convergent point of the warp loop, and consumed in order, so the sequence of
+// uniforms is exactly the reference's.
+//
+// An iteration consumes at most 7 uniforms and reads them at fixed byte
+// offsets 0 .. 6 RING_ROW from its first one: rows 0..5 are stored a second
+// time in rows 32..37, so that no read wraps and an offset is an immediate of
+// the load instead of an add, a compare and a select per uniform.
+constexpr uint32_t RING_ROW = 1024;           // bytes: 256 columns, the largest block the kernels launch
+constexpr int RING_ROWS = 38;
+constexpr uint32_t RING_BYTES = RING_ROWS * RING_ROW;
+constexpr uint32_t RING_MASK = 32 * RING_ROW - 1;
+constexpr int DRAWS_PER_ITER = 7;
 
 struct Rng {
-    uint32_t pid_lo, pid_hi, block;
-    uint32_t head;   // index of the next unread word
-    int cnt;         // buffered words
+    uint32_t pid_lo, pid_hi;
+    uint32_t block;          // blocks generated (4 uniforms each)
+    uint32_t pos;            // uniforms consumed x RING_ROW + 4 tid: the next uniform is at pos & RING_MASK
 };
 
 __device__ __forceinline__ void rng_init(Rng& r, uint64_t pid)
@@ -93,107 +97,43 @@ __device__ __forceinline__ void rng_init(Rng& r, uint64_t pid)
     r.pid_lo = (uint32_t)pid;
     r.pid_hi = (uint32_t)(pid >> 32);
     r.block = 0;
-    r.head = 0;
-    r.cnt = 0;
+    r.pos = 4u * threadIdx.x;
 }
 
-// Two consecutive blocks at once (independent Philox chains interleave).
-// Requires cnt <= RING_LEN - 8.
-__device__ __forceinline__ void rng_fill2(Rng& r, float* ring, const uint32_t* rk)
+// Buffered uniforms x RING_ROW - 4 tid (0 <= 4 tid < RING_ROW); both counts
+// wrap, their difference does not.
+__device__ __forceinline__ int32_t rng_level(const Rng& r)
+{
+    return (int32_t)(r.block * (4u * RING_ROW) - r.pos);
+}
+__device__ __forceinline__ bool rng_short(const Rng& r) { return rng_level(r) <= (DRAWS_PER_ITER - 1) * (int32_t)RING_ROW; }
+__device__ __forceinline__ bool rng_room(const Rng& r) { return rng_level(r) <= 24 * (int32_t)RING_ROW; }
+__device__ __forceinline__ bool rng_under(const Rng& r) { return rng_level(r) <= -(int32_t)RING_ROW; }
+
+// Two consecutive blocks at once (independent Philox chains interleave); needs
+// rng_room.  The write row is a multiple of 8: the stores never wrap.
+__device__ __forceinline__ void rng_fill(Rng& r, unsigned char* ring, const uint32_t* rk)
 {
     const uint4 o = philox4x32_10_rk(make_uint4(r.pid_lo, r.pid_hi, r.block, 0u), rk);
     const uint4 q = philox4x32_10_rk(make_uint4(r.pid_lo, r.pid_hi, r.block + 1u, 0u), rk);
+    const uint32_t row = (r.block * (4u * RING_ROW)) & RING_MASK;
+    float* const p = reinterpret_cast<float*>(ring + row + 4u * threadIdx.x);
+    constexpr uint32_t S = RING_ROW / 4;
+    const float f[8] = {u32_to_randu(o.x), u32_to_randu(o.y), u32_to_randu(o.z), u32_to_randu(o.w),
+                        u32_to_randu(q.x), u32_to_randu(q.y), u32_to_randu(q.z), u32_to_randu(q.w)};
+#pragma unroll
+    for (int i = 0; i < 8; ++i) p[i * S] = f[i];
+    if (row == 0u) {
+#pragma unroll
+        for (int i = 0; i < RING_ROWS - 32; ++i) p[(32 + i) * S] = f[i];
+    }
     r.block += 2u;
-    const uint32_t w = r.head + (uint32_t)r.cnt;
-    ring[((w + 0u) % RING_LEN) * RING_STRIDE] = u32_to_randu(o.x);
-    ring[((w + 1u) % RING_LEN) * RING_STRIDE] = u32_to_randu(o.y);
-    ring[((w + 2u) % RING_LEN) * RING_STRIDE] = u32_to_randu(o.z);
-    ring[((w + 3u) % RING_LEN) * RING_STRIDE] = u32_to_randu(o.w);
-    ring[((w + 4u) % RING_LEN) * RING_STRIDE] = u32_to_randu(q.x);
-    ring[((w + 5u) % RING_LEN) * RING_STRIDE] = u32_to_randu(q.y);
-    ring[((w + 6u) % RING_LEN) * RING_STRIDE] = u32_to_randu(q.z);
-    ring[((w + 7u) % RING_LEN) * RING_STRIDE] = u32_to_randu(q.w);
-    r.cnt += 8;
 }
 
-// NB consecutive blocks at once.  Requires cnt <= RING_LEN - 4 * NB.
-template <int NB>
-__device__ __forceinline__ void rng_fill(Rng& r, float* ring, const uint32_t* rk)
+// The uniform `off` bytes (a multiple of RING_ROW) after the one at w.
+__device__ __forceinline__ float ring_word(const unsigned char* w, uint32_t off)
 {
-    uint4 o[NB];
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-        o[b] = philox4x32_10_rk(make_uint4(r.pid_lo, r.pid_hi, r.block + (uint32_t)b, 0u), rk);
-    r.block += (uint32_t)NB;
-    const uint32_t w = r.head + (uint32_t)r.cnt;
-    if (RING_LEN % (4 * NB) == 0 && (RING_LEN & (RING_LEN - 1)) == 0) {
-        // every fill writes 4*NB words and pops move head and cnt in step, so
-        // the write position head + cnt stays a multiple of 4*NB: the block
-        // never wraps and its stores sit at fixed offsets from its first word
-        float* blk = ring + (size_t)(w & (uint32_t)(RING_LEN - 1)) * RING_STRIDE;
-#pragma unroll
-        for (int b = 0; b < NB; ++b) {
-            blk[(4 * b + 0) * RING_STRIDE] = u32_to_randu(o[b].x);
-            blk[(4 * b + 1) * RING_STRIDE] = u32_to_randu(o[b].y);
-            blk[(4 * b + 2) * RING_STRIDE] = u32_to_randu(o[b].z);
-            blk[(4 * b + 3) * RING_STRIDE] = u32_to_randu(o[b].w);
-        }
-        r.cnt += 4 * NB;
-        return;
-    }
-#if CL_RING_WRAP
-    // w < 2 RING_LEN: one conditional subtraction wraps each index
-    auto at = [&](uint32_t k) -> float& {
-        const uint32_t i = w + k;
-        return ring[(i >= (uint32_t)RING_LEN ? i - (uint32_t)RING_LEN : i) * RING_STRIDE];
-    };
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-        at(4u * b + 0u) = u32_to_randu(o[b].x);
-        at(4u * b + 1u) = u32_to_randu(o[b].y);
-        at(4u * b + 2u) = u32_to_randu(o[b].z);
-        at(4u * b + 3u) = u32_to_randu(o[b].w);
-    }
-#else
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-        ring[((w + 4u * b + 0u) % RING_LEN) * RING_STRIDE] = u32_to_randu(o[b].x);
-        ring[((w + 4u * b + 1u) % RING_LEN) * RING_STRIDE] = u32_to_randu(o[b].y);
-        ring[((w + 4u * b + 2u) % RING_LEN) * RING_STRIDE] = u32_to_randu(o[b].z);
-        ring[((w + 4u * b + 3u) % RING_LEN) * RING_STRIDE] = u32_to_randu(o[b].w);
-    }
-#endif
-    r.cnt += 4 * NB;
-}
-
-#ifndef CL_RING_WRAP
-#define CL_RING_WRAP 1
-#endif
-
-__device__ __forceinline__ float rng_peek(const Rng& r, const float* ring, uint32_t d)
-{
-#if CL_RING_WRAP
-    uint32_t i = r.head + d;                   // head < RING_LEN, d < RING_LEN
-    i = i >= (uint32_t)RING_LEN ? i - (uint32_t)RING_LEN : i;
-    return ring[i * RING_STRIDE];
-#else
-    return ring[((r.head + d) % RING_LEN) * RING_STRIDE];
-#endif
-}
-
-// Pop the next uniform.  The warp loop keeps at least as many words buffered
-// as one iteration can consume (checked once per iteration through cnt).
-__device__ __forceinline__ float rng_pop(Rng& r, const float* ring)
-{
-#if CL_RING_WRAP
-    const float u = ring[r.head * RING_STRIDE];
-    r.head = r.head + 1u == (uint32_t)RING_LEN ? 0u : r.head + 1u;
-#else
-    const float u = ring[(r.head % RING_LEN) * RING_STRIDE];
-    r.head += 1u;
-#endif
-    r.cnt -= 1;
-    return u;
+    return *reinterpret_cast<const float*>(w + off);
 }
 
 // A register-only stream for the diagnostics kernel (same sequence).
@@ -356,6 +296,8 @@ struct Physics {
     uint32_t key0, key1;
     uint32_t rk[20];             // Philox round keys
     float qc2, qa2;              // (n_crystal/n_coupling)^2, (n_crystal/1)^2
+    float abs_rate, ray_rate;    // -log2(e) / length, NaN: no quick test (survive_below)
+    float fresnel_margin;        // error bound of the quick Fresnel test, +Inf: no quick test
     uint8_t abs_finite, ray_finite, wrap_specular, air_gap;
     uint8_t disc, sur_specular, two_sided, pad_;
 };
@@ -369,42 +311,68 @@ enum : int32_t {
 constexpr float TWO_PI_F = 6.2831854820251465f;   // 2f0*Float32(pi), exact doubling
 constexpr float C_MM_NS = 299.792458f;
 
-// fresnel, src/optics.jl:10-19.  Returns tir; R set when !tir.
-__device__ __forceinline__ bool fresnel(float n1, float n2, float cosi, float& R)
+__device__ __forceinline__ float rcp_approx(float x)
 {
-    const float q = n1 / n2;
-    const float sin2t = (q * q) * (1.0f - cosi * cosi);
-    if (sin2t >= 1.0f) { R = 1.0f; return true; }
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float sqrt_approx(float x)
+{
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float ex2_approx(float x)
+{
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// fresnel, src/optics.jl:10-19, where sin2t = (n1/n2)^2 (1 - cosi^2) < 1.
+__device__ __forceinline__ float fresnel_R(float n1, float n2, float sin2t, float cosi)
+{
     const float cost = sqrtf(1.0f - sin2t);
     const float a = (n1 * cosi - n2 * cost) / (n1 * cosi + n2 * cost);
     const float b = (n1 * cost - n2 * cosi) / (n1 * cost + n2 * cosi);
-    R = 0.5f * (a * a + b * b);
-    return false;
+    return 0.5f * (a * a + b * b);
 }
 
-// fresnel with (n1/n2)^2 precomputed (the same Float32 value the reference
-// computes each call).
-__device__ __forceinline__ bool fresnel_q2(float n1, float n2, float q2, float cosi, float& R)
+// u < R at an interface where sin2t < 1.  R is estimated with approximate
+// reciprocals and root: the estimate and the reference's rounded R each lie
+// within 2^-20 of the Fresnel formula in the same operands (a handful of
+// relative errors of 2^-22 at most in quotients of magnitude <= 1), so outside
+// fresnel_margin = 2^-17 the estimate decides; inside it (1.5e-5 of the
+// draws) the exact expression does.  Two IEEE divisions and a root less, each
+// with a branch of its own.
+__device__ __forceinline__ bool fresnel_reflects(const Physics& P, float n2, float sin2t, float cosi, float u)
 {
-    const float sin2t = q2 * (1.0f - cosi * cosi);
-    if (sin2t >= 1.0f) { R = 1.0f; return true; }
-    const float cost = sqrtf(1.0f - sin2t);
-    const float a = (n1 * cosi - n2 * cost) / (n1 * cosi + n2 * cost);
-    const float b = (n1 * cost - n2 * cosi) / (n1 * cost + n2 * cosi);
-    R = 0.5f * (a * a + b * b);
-    return false;
+    const float ct = sqrt_approx(1.0f - sin2t);
+    const float p = P.n_crystal * cosi, s = n2 * cosi;
+    const float a = __fmaf_rn(-n2, ct, p) * rcp_approx(__fmaf_rn(n2, ct, p));
+    const float b = __fmaf_rn(P.n_crystal, ct, -s) * rcp_approx(__fmaf_rn(P.n_crystal, ct, s));
+    const float over = __fmaf_rn(0.5f, __fmaf_rn(a, a, b * b), -u);      // R - u
+    if (fabsf(over) > P.fresnel_margin) return over > 0.0f;
+    return u < fresnel_R(P.n_crystal, n2, sin2t, cosi);
 }
 
-__device__ __forceinline__ int face_axis(int32_t face) { return face <= 2 ? 1 : (face <= 4 ? 2 : 3); }
-
-// specular, src/optics.jl:25-28.
-__device__ __forceinline__ void specular(float& ux, float& uy, float& uz, int32_t face)
+// A bound below exp(-d / length) (rate = -log2(e) / length): a uniform u below
+// it has -length log u > d in the reference's rounding too.  The exponent's
+// and ex2's errors and that of the Float32 product length * log u stay below
+// 2^-17 in log2 u wherever a uniform (>= 2^-24) can be below the bound; 2^-15
+// is taken off.
+__device__ __forceinline__ float survive_below(float d, float rate)
 {
-    const int a = face_axis(face);
-    // selects, not branches: a warp whose lanes hit different axes runs one path
-    ux = a == 1 ? -ux : ux;
-    uy = a == 2 ? -uy : uy;
-    uz = a == 3 ? -uz : uz;
+    return ex2_approx(__fmaf_rn(d, rate, -0x1p-15f));
+}
+
+// v > L ? L : (v < 0 ? 0 : v), NaN kept, in two instructions.
+__device__ __forceinline__ float clamp_to(float v, float L)
+{
+    float r;
+    asm("{\n\t.reg .f32 m;\n\tmin.NaN.f32 m, %1, %2;\n\tmax.NaN.f32 %0, m, 0f00000000;\n\t}" : "=f"(r) : "f"(v), "f"(L));
+    return r;
 }
 
 // Distance along one axis to the face the direction points at:
@@ -429,30 +397,62 @@ __device__ __forceinline__ int32_t wall_hit(const Physics& P, float x, float y, 
     return uz > 0.0f ? FACE_BACK : FACE_FRONT;
 }
 
+// wall_hit without its three IEEE divisions: the axis comes from approximate
+// quotients, and only the winner's is made exact.  Returns false where the
+// approximation does not decide (two axes within 2^-19 of each other, a
+// distance or direction component near zero, positions outside the crystal,
+// NaN): the caller then takes wall_hit.
+//
+// The quotient d = n/u: r = rcp(u) refined by one Newton step, q = n r, then
+// q + r (n - q u) with the residual exact in a fused multiply-add, which is the
+// correctly rounded quotient (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34
+// (1990)) when r is the correctly rounded reciprocal: so it is for every
+// Float32 mantissa but all-ones, which the theorem excludes and for which the
+// exact expression is taken.  With m > 2^-30 and |u| > 2^-40 nothing
+// under- or overflows.
+__device__ __forceinline__ bool wall_hit_fast(const Physics& P, float x, float y, float z, float ux, float uy,
+                                              float uz, float& d, int32_t& face, float& cosw)
+{
+    const float nx = (ux > 0.0f ? P.L0 : 0.0f) - x;
+    const float ny = (uy > 0.0f ? P.L1 : 0.0f) - y;
+    const float nz = (uz > 0.0f ? P.L2 : 0.0f) - z;
+    const float qx = nx * rcp_approx(ux), qy = ny * rcp_approx(uy), qz = nz * rcp_approx(uz);
+    const float lo = fminf(qx, qy), hi = fmaxf(qx, qy);
+    const float m = fminf(lo, qz), second = fminf(hi, fmaxf(lo, qz));
+    const bool on_x = qx == m, on_y = !on_x && qy == m;
+    const float u = on_x ? ux : (on_y ? uy : uz);
+    const float n = on_x ? nx : (on_y ? ny : nz);
+    const float au = fabsf(u);
+    float r = rcp_approx(u);
+    r = __fmaf_rn(r, __fmaf_rn(-u, r, 1.0f), r);
+    const float q = n * r;
+    d = __fmaf_rn(r, __fmaf_rn(-q, u, n), q);
+    face = (on_x ? 2 : (on_y ? 4 : 6)) - (u > 0.0f ? 1 : 0);
+    cosw = au;
+    return second > m * 1.000002f && m > 0x1p-30f && au > 0x1p-40f &&
+           (__float_as_uint(u) & 0x7fffffu) != 0x7fffffu;
+}
+
 // Direction about the inward normal of a face from cos(theta) = ct and the
-// azimuth's (sin, cos): the tail of lambertian_dir, src/optics.jl:119-137.
-__device__ __forceinline__ void lambertian_from(int32_t face, float ct, float sphi, float cphi,
+// other two components (a, b): the tail of lambertian_dir, src/optics.jl:119-137.
+__device__ __forceinline__ void lambertian_from(int32_t face, float ct, float a, float b,
                                                 float& ux, float& uy, float& uz)
 {
-    const float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
-    const float a = st * cphi, b = st * sphi;
     // the inward normal component on the face's axis, (a, b) on the other two
     // in axis order (XP: (-ct, a, b), YM: (a, ct, b), BACK: (a, b, -ct), ...),
     // by selects
-    const int ax = face_axis(face);
-    const float n = (face == FACE_XP || face == FACE_YP || face == FACE_BACK) ? -ct : ct;
-    ux = ax == 1 ? n : a;
-    uy = ax == 1 ? a : (ax == 2 ? n : b);
-    uz = ax == 3 ? n : b;
+    const float n = (face & 1) ? -ct : ct;
+    ux = face <= 2 ? n : a;
+    uy = face <= 2 ? a : (face <= 4 ? n : b);
+    uz = face > 4 ? n : b;
 }
 
 // The tail of rayleigh_dir, src/optics.jl:93-111: rotate u by the polar
-// cosine mu about itself with the azimuth's (sin, cos).
-__device__ __forceinline__ void rayleigh_rotate(float mu, float sphi, float cphi,
+// cosine mu about itself; (cb, sb) = sin(theta) (cos, sin) of the azimuth.
+__device__ __forceinline__ void rayleigh_rotate(float mu, float cb, float sb,
                                                 float& ux, float& uy, float& uz)
 {
-    const float st = sqrtf(fmaxf(0.0f, 1.0f - mu * mu));
-    const float cb = st * cphi, sb = st * sphi;
     // t1 = (-uy, ux, 0)/|(ux, uy)| if |uz| < 0.9, else (0, -uz, uy)/|(uy, uz)|:
     // the same operations on selected operands (one square root and division
     // for a warp whose lanes take both cases)

@@ -37,6 +37,8 @@
 namespace cl {
 
 constexpr unsigned FULL = 0xffffffffu;
+constexpr int GAUSS_OFF = 1 << 24;    // sqrt(-2 log u) after the 2^24 logs
+constexpr int N_COUNTERS = 10;        // cl_counters, then the photon-steps
 // The tables are replicated: entry e of copy c sits at [e * COPIES + c] and a
 // lane reads copy (lane % COPIES), so the 16-byte reads of the 8 lanes that
 // share a shared-memory wavefront hit distinct banks when COPIES = 8.
@@ -90,7 +92,7 @@ struct KArgs {
     unsigned long long* steps;
     unsigned int* done;
     unsigned int* err;
-    const float* logtab;  // log of every uniform (k+1)*2^-24 at [k], or NULL: compute
+    const float* logtab;  // log u and sqrt(-2 log u) of every uniform (logtab_fill), or NULL: compute
     unsigned long long budget_ns;   // device time budget of the launch, 0 = none
 };
 
@@ -141,30 +143,16 @@ __device__ __forceinline__ int64_t find_source(const int64_t* __restrict__ off, 
 // Per-lane transport states of the warp loop.  One loop iteration moves each
 // active lane one state forward; a whole wall interaction (move, UNIFIED try,
 // wrap) completes in one iteration, so an iteration is about one photon-step.
+// States from S_INIT on set a new direction from a polar cosine and an azimuth.
 enum : int32_t {
     S_IDLE = 0,   // no photon
-    S_INIT = 1,   // emission: direction and time (src/kernel.jl:173-180)
-    S_MOVE = 2,   // bulk competition + wall interaction (src/transport.jl:127-233)
-    S_UNI = 3,    // another UNIFIED try at the same wall (src/optics.jl:54-78)
+    S_MOVE = 1,   // bulk competition + wall interaction (src/transport.jl:127-233)
+    S_UNI = 2,    // another UNIFIED try at the same wall (src/optics.jl:54-78)
+    S_INIT = 3,   // emission: direction and time (src/kernel.jl:173-180)
     S_RAY = 4,    // Rayleigh rejection sampling + rotation (src/optics.jl:87-112)
     S_LAMB = 5,   // Lambertian re-injection (src/optics.jl:118-138)
 };
-// Uniforms one iteration can consume at most (move: abs, ray, 3 for the
-// UNIFIED try, Fresnel, wrap; a Rayleigh frame: two tries of 2 and the
-// azimuth).  The ring is topped up to this before the iteration's draws.
-constexpr int DRAWS_PER_ITER = 7;
-// Fresnel interfaces met in an iteration (one evaluation serves all three).
-enum : int32_t { FK_NONE = 0, FK_READOUT = 1, FK_POLISHED = 2, FK_FACET = 3 };
 
-#ifndef CL_FILL_JOIN
-#define CL_FILL_JOIN 1
-#endif
-#ifndef CL_FILL_BLOCKS
-#define CL_FILL_BLOCKS 2
-#endif
-#ifndef CL_USE_LOGTAB
-#define CL_USE_LOGTAB 1
-#endif
 #ifndef CL_DEFAULT_WARP_CHUNK
 #define CL_DEFAULT_WARP_CHUNK 0
 #endif
@@ -185,33 +173,60 @@ enum : int32_t { FK_NONE = 0, FK_READOUT = 1, FK_POLISHED = 2, FK_FACET = 3 };
 // CsI(Tl)+Teflon run files; SPEC_ANY reads every flag from the parameters.
 enum : int { SPEC_ANY = 0, SPEC_ESR = 1, SPEC_TEFLON = 2 };
 
+// log of a uniform u = k 2^-24 from the table (k in 1..2^24 at [k - 1]), or
+// evaluated where there is no table.
+__device__ __forceinline__ uint32_t uniform_index(float u) { return min((uint32_t)(u * 16777216.0f), 1u << 24); }
+__device__ __forceinline__ float uniform_log(const float* __restrict__ tab, float u, const double2* __restrict__ logtab)
+{
+    return tab ? __ldg(tab + (int)uniform_index(u) - 1) : cl_logf_u<LOG_COPIES>(u, logtab);
+}
+
+// The loop computes what decides a photon's next step exactly and everything
+// else it can do without: the bound is instruction issue (the state machine's
+// selects, moves and branches, not the arithmetic), so
+//   * the wall axis comes from approximate reciprocals and only the winning
+//     axis is divided; the bulk competition compares the uniforms with
+//     approximate survival probabilities; Fresnel compares its uniform with an
+//     approximate coefficient.  Each has an error bound, and a lane inside it
+//     (about 1e-5 of them; a bulk event always) takes the exact expressions,
+//     so every result has the reference's bits;
+//   * a lane's next uniforms are read at fixed offsets from one address (the
+//     ring is mirrored past its end), and the number consumed is added once;
+//   * outcomes are merged by selects into one flip / one new direction / one
+//     state change, not one branch each;
+//   * the tilt's sqrt(-2 log u) is looked up whole.
+// Measured on BGO+ESR (51.2M photons) and 3,001 CsI(Tl)+Teflon events: CL_LOOP_MS.
 template <int MODE, bool REC, bool TILE, int SPEC>
 __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(const __grid_constant__ KArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     double2 *s_tab, *s_sctab;
     load_tables(smem, s_tab, s_sctab);
-    float* s_ring = reinterpret_cast<float*>(smem + LOGTAB_BYTES);
-    uint32_t* s_counts = reinterpret_cast<uint32_t*>(s_ring + RING_LEN * RING_STRIDE);
+    unsigned char* const s_ring = smem + LOGTAB_BYTES;
+    uint32_t* s_counts = reinterpret_cast<uint32_t*>(s_ring + RING_BYTES);
     uint32_t* s_keys = s_counts + (TILE ? A.cells * A.bins_total : 0);
-    __shared__ unsigned long long s_cnt[10];
+    // per-warp counters (cl_counters order, then the steps); lane i owns entry i
+    __shared__ unsigned long long s_cnt[8][N_COUNTERS];
     __shared__ unsigned int s_last;
 
     const Physics& P = A.P;
     const int tid = threadIdx.x;
+    const int lane = tid & 31;
     if (TILE) {
         const int nt = A.cells * A.bins_total;
         for (int i = tid; i < nt; i += blockDim.x) s_counts[i] = 0u;
         for (int i = tid; i < A.cells; i += blockDim.x) s_keys[i] = INF_KEY;
     }
-    if (tid < 10) s_cnt[tid] = 0ull;
+    for (int i = tid; i < 8 * N_COUNTERS; i += blockDim.x) (&s_cnt[0][0])[i] = 0ull;
+    // every ring word holds a uniform from the start: lanes without a photon
+    // read them too, and their table lookups stay in range
+    for (int r = 0; r < RING_ROWS; ++r) *reinterpret_cast<float*>(s_ring + r * RING_ROW + 4 * tid) = 1.0f;
     __syncthreads();
 
     uint32_t* tile_counts = TILE ? s_counts : A.counts;
     uint32_t* tile_keys = TILE ? s_keys : A.keys;
-    float* ring = s_ring + tid;
+    unsigned long long* my_cnt = s_cnt[tid >> 5];
 
-    const int lane = tid & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     const double2* my_tab = s_tab + (lane % LOG_COPIES);
     const double2* my_sctab = s_sctab + (lane % SC_COPIES);
@@ -222,18 +237,17 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
     const bool ray_finite = SPEC != SPEC_ANY || P.ray_finite;
     const bool disc = SPEC == SPEC_ANY && P.disc;
     const bool two_sided = SPEC == SPEC_ANY && P.two_sided;
-    // states and interfaces a configuration never reaches (tests on them compile away)
+    // states a configuration never reaches (tests on them compile away)
     constexpr bool lamb_possible = SPEC != SPEC_ESR;      // Lambertian wrap or surround
-    constexpr bool polished_possible = SPEC == SPEC_ANY;  // back-painted face without roughness
     const float inf = __int_as_float(0x7f800000);
+    // uniforms a move draws for the bulk competition, as a byte offset in the ring
+    const uint32_t bulk_off = (abs_finite ? RING_ROW : 0) + (ray_finite ? RING_ROW : 0);
 
     // per-lane photon state
     float x = 0.f, y = 0.f, z = 0.f, ux = 0.f, uy = 0.f, uz = 0.f, t = 0.f;
-    float carry = 0.f;                 // uz (init), mu (Rayleigh), u1 (Lambertian)
-    int32_t bounces = 0, nscat = 0, st = S_IDLE, face = 0, tries = 0;
+    int32_t bounces = 0, nscat = 0, st = S_IDLE, face = 1, tries = 0;
     Rng rng;
     rng_init(rng, 0);
-    int64_t k = 0;
     int32_t seg = 0;
     // warp-uniform work pool
     int64_t pool_lo = 0, pool_hi = 0, pool_src = 0;
@@ -246,391 +260,342 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
     for (;;) {
         // ---- refill idle lanes from the warp's pool / the global queue ----
         const unsigned need = __ballot_sync(FULL, st == S_IDLE);
-        if (need != 0u && !exhausted) {
-            const int nneed = __popc(need);
-            const int rank = __popc(need & lt_mask);
-            int64_t my_k = -1;
-            int64_t my_hint = pool_src;
-            const int64_t avail = pool_hi - pool_lo;
-            const int64_t taken = avail < nneed ? avail : (int64_t)nneed;
-            if (st == S_IDLE && rank < taken) my_k = pool_lo + rank;
-            pool_lo += taken;
-            if (taken < nneed) {
-                unsigned long long base = 0;
-                if (lane == 0) base = atomicAdd(A.queue, (unsigned long long)A.warp_chunk);
-                base = __shfl_sync(FULL, base, 0);
-                if ((int64_t)base >= A.n) {
-                    exhausted = true;
-                } else {
-                    pool_lo = (int64_t)base;
-                    pool_hi = pool_lo + A.warp_chunk;
-                    if (pool_hi > A.n) pool_hi = A.n;
-                    if (MODE != 0) {
-                        int64_t s0 = 0;
-                        if (lane == 0) s0 = find_source(A.src_off, A.n_src, pool_src, pool_lo);
-                        pool_src = __shfl_sync(FULL, s0, 0);
+        if (need != 0u) {
+            if (!exhausted) {
+                const int nneed = __popc(need);
+                const int rank = __popc(need & lt_mask);
+                int64_t my_k = -1;
+                int64_t my_hint = pool_src;
+                const int64_t avail = pool_hi - pool_lo;
+                const int64_t taken = avail < nneed ? avail : (int64_t)nneed;
+                if (st == S_IDLE && rank < taken) my_k = pool_lo + rank;
+                pool_lo += taken;
+                if (taken < nneed) {
+                    unsigned long long base = 0;
+                    if (lane == 0) base = atomicAdd(A.queue, (unsigned long long)A.warp_chunk);
+                    base = __shfl_sync(FULL, base, 0);
+                    if ((int64_t)base >= A.n) {
+                        exhausted = true;
+                    } else {
+                        pool_lo = (int64_t)base;
+                        pool_hi = pool_lo + A.warp_chunk;
+                        if (pool_hi > A.n) pool_hi = A.n;
+                        if (MODE != 0) {
+                            int64_t s0 = 0;
+                            if (lane == 0) s0 = find_source(A.src_off, A.n_src, pool_src, pool_lo);
+                            pool_src = __shfl_sync(FULL, s0, 0);
+                        }
+                        const int64_t rem = nneed - taken;
+                        const int64_t avail2 = pool_hi - pool_lo;
+                        const int64_t taken2 = avail2 < rem ? avail2 : rem;
+                        if (st == S_IDLE && rank >= taken && rank - taken < taken2) {
+                            my_k = pool_lo + (rank - taken);
+                            my_hint = pool_src;
+                        }
+                        pool_lo += taken2;
                     }
-                    const int64_t rem = nneed - taken;
-                    const int64_t avail2 = pool_hi - pool_lo;
-                    const int64_t taken2 = avail2 < rem ? avail2 : rem;
-                    if (st == S_IDLE && rank >= taken && rank - taken < taken2) {
-                        my_k = pool_lo + (rank - taken);
-                        my_hint = pool_src;
+                }
+                if (my_k >= 0) {
+                    if (MODE == 0) {
+                        const int32_t j = A.npos == 1 ? 0 : (int32_t)((uint64_t)my_k % (uint64_t)A.npos);
+                        x = __ldg(A.px + j); y = __ldg(A.py + j); z = __ldg(A.pz + j);
+                        t = A.pt ? __ldg(A.pt + j) : 0.0f;
+                    } else {
+                        const int64_t s = find_source(A.src_off, A.n_src, my_hint, my_k);
+                        x = __ldg(A.px + s); y = __ldg(A.py + s); z = __ldg(A.pz + s);
+                        t = A.pt ? __ldg(A.pt + s) : 0.0f;
+                        seg = __ldg(A.src_seg + s);
                     }
-                    pool_lo += taken2;
+                    rng_init(rng, A.pid0 + (uint64_t)my_k + 1ull);
+                    bounces = 0; nscat = 0; tries = 0;
+                    st = S_INIT;
                 }
             }
-            if (my_k >= 0) {
-                k = my_k;
-                if (MODE == 0) {
-                    const int32_t j = A.npos == 1 ? 0 : (int32_t)((uint64_t)k % (uint64_t)A.npos);
-                    x = __ldg(A.px + j); y = __ldg(A.py + j); z = __ldg(A.pz + j);
-                    t = A.pt ? __ldg(A.pt + j) : 0.0f;
-                } else {
-                    const int64_t s = find_source(A.src_off, A.n_src, my_hint, k);
-                    x = __ldg(A.px + s); y = __ldg(A.py + s); z = __ldg(A.pz + s);
-                    t = A.pt ? __ldg(A.pt + s) : 0.0f;
-                    seg = __ldg(A.src_seg + s);
-                }
-                rng_init(rng, A.pid0 + (uint64_t)k + 1ull);
-                bounces = 0; nscat = 0; tries = 0;
-                st = S_INIT;
-            }
+            if (!__any_sync(FULL, st != S_IDLE)) break;
         }
-        if (!__any_sync(FULL, st != S_IDLE)) break;
         if (A.budget_ns != 0ull && ((++iter) & 255u) == 0u) {
             // photons still in flight are dropped; the host reports CL_ERR_TIMEOUT
             if (__any_sync(FULL, globaltimer_ns() - t_begin > A.budget_ns)) { timed_out = true; break; }
         }
 
         // ---- top up the uniform ring: one Philox call site for the warp ----
-        {
-            const bool want = st != S_IDLE && rng.cnt < DRAWS_PER_ITER;
-            if (__any_sync(FULL, want)) {
-#if CL_FILL_JOIN
-                // every lane with room tops up at this convergent point, so
-                // later iterations need the fill less often
-                if (st != S_IDLE && rng.cnt <= RING_LEN - 4 * CL_FILL_BLOCKS)
-                    rng_fill<CL_FILL_BLOCKS>(rng, ring, P.rk);
-#else
-                if (want) rng_fill2(rng, ring, P.rk);
-#endif
-            }
+        if (__any_sync(FULL, st != S_IDLE && rng_short(rng))) {
+            // every lane with room tops up at this convergent point, so later
+            // iterations need the fill less often
+            under |= rng_under(rng);
+            if (st != S_IDLE && rng_room(rng)) rng_fill(rng, s_ring, P.rk);
         }
 
-        // ---- pre: draw uniforms, stage arguments of the elementary functions ----
-        float a0 = 1.f, a1 = 1.f, a2 = 1.f, p0 = 1.f, p1 = 1.f;
-        bool nl0 = false, nl1 = false, nl2 = false, ns0 = false, ns1 = false;
-        bool ray_ok = false;
-        if (st == S_INIT) {
-            carry = 1.0f - 2.0f * rng_pop(rng, ring);       // uz
-            p1 = TWO_PI_F * rng_pop(rng, ring); ns1 = true;  // azimuth
-            if (P.tau > 0.0f) { a0 = rng_pop(rng, ring); nl0 = true; }
-        } else if (st == S_MOVE || st == S_UNI) {
-            if (st == S_MOVE) {
-                if (abs_finite) { a0 = rng_pop(rng, ring); nl0 = true; }
-                if (ray_finite) { a1 = rng_pop(rng, ring); nl1 = true; }
-            }
-            if (uni_possible) {
-                // speculative: the next three uniforms are the UNIFIED try's
-                // gaussian pair and facet azimuth if this step reaches a wrap
-                a2 = rng_peek(rng, ring, 0u); nl2 = true;
-                p0 = TWO_PI_F * rng_peek(rng, ring, 1u); ns0 = true;
-                p1 = TWO_PI_F * rng_peek(rng, ring, 2u); ns1 = true;
-            }
-        } else if (st == S_RAY) {
-            float mu = 1.0f - 2.0f * rng_pop(rng, ring);
-            ray_ok = 2.0f * rng_pop(rng, ring) <= 1.0f + mu * mu;
+        // ---- draws: this iteration's uniforms at fixed offsets ----
+        const unsigned char* const w = s_ring + (rng.pos & RING_MASK);
+        // the table lookup (tilt's gaussian, or the emission time's log) and the azimuth
+        uint32_t og = st == S_MOVE ? bulk_off : (st == S_INIT ? 2u * RING_ROW : 0u);
+        uint32_t oaz = st == S_MOVE ? bulk_off + 2u * RING_ROW : (st == S_UNI ? 2u * RING_ROW : RING_ROW);
+        float mu = 0.0f;
+        bool ray_ok = true;
+        if (st == S_RAY) {
+            // two rejection tries in one iteration (8 of 9 scatters end in it)
+            mu = 1.0f - 2.0f * ring_word(w, 0);
+            ray_ok = 2.0f * ring_word(w, RING_ROW) <= 1.0f + mu * mu;
+            oaz = 2u * RING_ROW;
             if (!ray_ok) {
-                // a second try in the same iteration (the reference's next
-                // draws, in order): 8 of 9 scatters end in one iteration
                 ++tries;
-                mu = 1.0f - 2.0f * rng_pop(rng, ring);
-                ray_ok = 2.0f * rng_pop(rng, ring) <= 1.0f + mu * mu;
+                mu = 1.0f - 2.0f * ring_word(w, 2u * RING_ROW);
+                ray_ok = 2.0f * ring_word(w, 3u * RING_ROW) <= 1.0f + mu * mu;
+                oaz = 4u * RING_ROW;
             }
-            carry = mu;
-            if (ray_ok) { p1 = TWO_PI_F * rng_pop(rng, ring); ns1 = true; }
-        } else if (lamb_possible && st == S_LAMB) {
-            carry = rng_pop(rng, ring);                       // u for cos(theta)
-            p1 = TWO_PI_F * rng_pop(rng, ring); ns1 = true;
         }
 
         // ---- elementary functions, once per warp (Float64, rounded once) ----
-        // Straight-line and unconditional: the five evaluations are independent,
-        // so their Float64 dependency chains interleave (lanes that need none of
-        // them get the harmless argument 1).
-        float L0, L1, L2, s0, c0, s1, c1;
+        // Straight-line and unconditional (a lane that needs none of them reads
+        // some other uniform), so that their latencies overlap.
+        const float ug = ring_word(w, og);
+        float G;                    // sqrt(-2 log u); for an emission the log itself
         if (A.logtab) {
-            // the logs' arguments are uniforms (k+1)*2^-24: look them up
-            // (issued before the sincos work so the loads overlap it)
-            // (the index is clamped into the table whatever the argument)
-            L0 = __ldg(A.logtab + min((uint32_t)(a0 * 16777216.0f) - 1u, 0xFFFFFFu));
-            L1 = __ldg(A.logtab + min((uint32_t)(a1 * 16777216.0f) - 1u, 0xFFFFFFu));
-            L2 = __ldg(A.logtab + min((uint32_t)(a2 * 16777216.0f) - 1u, 0xFFFFFFu));
+            G = __ldg(A.logtab + (int)uniform_index(ug) - 1 + (st == S_INIT ? 0 : GAUSS_OFF));
         } else {
-            L0 = cl_logf_u<LOG_COPIES>(a0, my_tab);
-            L1 = cl_logf_u<LOG_COPIES>(a1, my_tab);
-            L2 = cl_logf_u<LOG_COPIES>(a2, my_tab);
+            G = cl_logf_u<LOG_COPIES>(ug, my_tab);
+            if (st != S_INIT) G = sqrtf(-2.0f * G);
         }
-        cl_sincosf_core<SC_COPIES>(p0, my_sctab, &s0, &c0);
-        cl_sincosf_core<SC_COPIES>(p1, my_sctab, &s1, &c1);
-        (void)nl0; (void)nl1; (void)nl2; (void)ns0; (void)ns1;
+        float s0, c0, s1, c1;
+        cl_sincosf_core<SC_COPIES>(TWO_PI_F * ring_word(w, og + RING_ROW), my_sctab, &s0, &c0);
+        cl_sincosf_core<SC_COPIES>(TWO_PI_F * ring_word(w, oaz), my_sctab, &s1, &c1);
 
-        // ---- post, part 1 ----
-        int32_t status = ST_FLYING, idx = 0;
-        bool uni = false, wall_done = false, to_wrap = false;
-        int32_t fk = FK_NONE;                  // which Fresnel interface this lane meets
-        float fn2 = 1.0f, fq2 = 1.0f, fcos = 1.0f;
-        if (st == S_INIT) {
-            const float r = sqrtf(fmaxf(0.0f, 1.0f - carry * carry));
-            ux = r * c1; uy = r * s1; uz = carry;
-            if (P.tau > 0.0f) t += (-P.tau) * L0;
-            st = S_MOVE;
-        } else if (st == S_MOVE) {
-            float d;
-            const int32_t f = wall_hit(P, x, y, z, ux, uy, uz, d);
-            const float d_abs = abs_finite ? (-P.abs_len) * L0 : inf;
-            const float d_ray = ray_finite ? (-P.ray_len) * L1 : inf;
-            if (d_abs < d && d_abs <= d_ray) {
-                status = ST_ABS_BULK;
-            } else if (d_ray < d) {
-                x += d_ray * ux; y += d_ray * uy; z += d_ray * uz;
-                t += d_ray * P.inv_v;
-                st = S_RAY;
-                tries = 0;
+        int32_t status = ST_FLYING;
+        bool done = false;          // an interaction that counts as a bounce
+        if (st >= S_INIT) {
+            // ---- a new direction: emission, Rayleigh scatter, Lambertian lobe ----
+            float c = mu;
+            if (st == S_INIT) c = 1.0f - 2.0f * ring_word(w, 0);
+            if (lamb_possible && st == S_LAMB) c = sqrtf(ring_word(w, 0));
+            const float sn = sqrtf(fmaxf(0.0f, 1.0f - c * c));
+            const float a = sn * c1, b = sn * s1;
+            if (st == S_RAY) {
+                rng.pos += oaz + (ray_ok ? RING_ROW : 0u);
+                if (ray_ok || ++tries >= 4096) {
+                    overrun |= !ray_ok;
+                    rayleigh_rotate(c, a, b, ux, uy, uz);
+                    nscat += 1;
+                    done = true;
+                }
+            } else if (lamb_possible && st == S_LAMB) {
+                lambertian_from(face, c, a, b, ux, uy, uz);
+                rng.pos += 2u * RING_ROW;
+                done = true;
             } else {
-                // advance to the wall: clamp, then snap the hit axis (src/transport.jl:146-157)
-                const float nx_ = x + d * ux, ny_ = y + d * uy, nz_ = z + d * uz;
-                x = nx_ > P.L0 ? P.L0 : (nx_ < 0.0f ? 0.0f : nx_);
-                y = ny_ > P.L1 ? P.L1 : (ny_ < 0.0f ? 0.0f : ny_);
-                z = nz_ > P.L2 ? P.L2 : (nz_ < 0.0f ? 0.0f : nz_);
-                const int a = face_axis(f);
-                if (a == 1)      x = f == FACE_XP ? P.L0 : 0.0f;
-                else if (a == 2) y = f == FACE_YP ? P.L1 : 0.0f;
-                else             z = f == FACE_BACK ? P.L2 : 0.0f;
-                t += d * P.inv_v;
-                const float cosi = a == 1 ? fabsf(ux) : (a == 2 ? fabsf(uy) : fabsf(uz));
-                face = f;
-                if (f == FACE_BACK || (two_sided && f == FACE_FRONT)) {
-                    // readout face, src/transport.jl:161-185: Fresnel below
-                    fk = FK_READOUT; fn2 = P.n_coupling; fq2 = P.qc2; fcos = cosi;
-                } else if (!air_gap) {
+                ux = a; uy = b; uz = c;
+                rng.pos += 2u * RING_ROW;
+                if (P.tau > 0.0f) { t += (-P.tau) * G; rng.pos += RING_ROW; }
+                st = S_MOVE;
+            }
+        } else if (st != S_IDLE) {
+            bool hit = true;
+            float cosw = 1.0f;      // |cos| of the incidence on the wall
+            if (st == S_MOVE) {
+                // ---- the step to the wall ----
+                float d;
+                int32_t f;
+                const float u_abs = ring_word(w, 0);
+                const float u_ray = ring_word(w, abs_finite ? RING_ROW : 0);
+                if (!wall_hit_fast(P, x, y, z, ux, uy, uz, d, f, cosw)) {
+                    f = wall_hit(P, x, y, z, ux, uy, uz, d);
+                    cosw = fabsf(f <= 2 ? ux : (f <= 4 ? uy : uz));
+                }
+                rng.pos += bulk_off;
+                // no bulk interaction if each uniform is clearly below its
+                // survival probability exp(-d / length): the path length
+                // -length log u is then clearly above d
+                if (!((!abs_finite || u_abs < survive_below(d, P.abs_rate)) &&
+                      (!ray_finite || u_ray < survive_below(d, P.ray_rate)))) {
+                    const float d_abs = abs_finite ? (-P.abs_len) * uniform_log(A.logtab, u_abs, my_tab) : inf;
+                    const float d_ray = ray_finite ? (-P.ray_len) * uniform_log(A.logtab, u_ray, my_tab) : inf;
+                    if (d_abs < d && d_abs <= d_ray) {
+                        status = ST_ABS_BULK;
+                        hit = false;
+                    } else if (d_ray < d) {
+                        x += d_ray * ux; y += d_ray * uy; z += d_ray * uz;
+                        t += d_ray * P.inv_v;
+                        st = S_RAY;
+                        tries = 0;
+                        hit = false;
+                    }
+                }
+                if (hit) {
+                    // advance to the wall: clamp, then snap the hit axis (src/transport.jl:146-157)
+                    const float nx_ = x + d * ux, ny_ = y + d * uy, nz_ = z + d * uz;
+                    x = clamp_to(nx_, P.L0);
+                    y = clamp_to(ny_, P.L1);
+                    z = clamp_to(nz_, P.L2);
+                    if (f <= 2)      x = f == FACE_XP ? P.L0 : 0.0f;
+                    else if (f <= 4) y = f == FACE_YP ? P.L1 : 0.0f;
+                    else             z = f == FACE_BACK ? P.L2 : 0.0f;
+                    t += d * P.inv_v;
+                    face = f;
+                    tries = 0;
+                }
+            }
+            if (hit) {
+                // ---- the wall interaction; uniforms from w + og on ----
+                const unsigned char* const v = w + og;
+                const bool on_x = face <= 2, on_y = !on_x && face <= 4, on_z = face > 4;
+                const float sgn = (face & 1) ? 1.0f : -1.0f;      // outward normal component
+                const bool readout = face == FACE_BACK || (two_sided && face == FACE_FRONT);
+                bool flip = false, take = false, retry = false;
+                float rx = 0.f, ry = 0.f, rz = 0.f;
+                if (SPEC == SPEC_ANY && !readout && !air_gap) {
                     // front-painted wrap, src/transport.jl:186-198
-                    if (rng_pop(rng, ring) <= P.wrap_R) {
-                        if (wrap_specular) { specular(ux, uy, uz, f); wall_done = true; }
+                    rng.pos += RING_ROW;
+                    if (ring_word(v, 0) <= P.wrap_R) {
+                        if (wrap_specular) flip = true;
                         else st = S_LAMB;
                     } else {
                         status = ST_ABS_WALL;
                     }
-                } else if (uni_possible) {
-                    tries = 0;
-                    uni = true;                      // UNIFIED lobe, below
                 } else {
-                    // polished back-painted face, src/transport.jl:206-212: Fresnel below
-                    fk = FK_POLISHED; fn2 = 1.0f; fq2 = P.qa2; fcos = cosi;
-                }
-            }
-        } else if (st == S_UNI) {
-            uni = true;
-        } else if (st == S_RAY) {
-            if (ray_ok || ++tries >= 4096) {
-                overrun |= !ray_ok;
-                rayleigh_rotate(carry, s1, c1, ux, uy, uz);
-                nscat += 1;
-                bounces += 1;
-                if (bounces >= P.max_bounces) status = ST_CAP;
-                else st = S_MOVE;
-            }
-        } else if (lamb_possible && st == S_LAMB) {
-            lambertian_from(face, sqrtf(carry), s1, c1, ux, uy, uz);
-            wall_done = true;
-        }
-
-        // UNIFIED try, first half (src/optics.jl:55-56): the gaussian tilt
-        bool facet = false;
-        float alpha = 0.f;
-        if (uni) {
-            rng_pop(rng, ring);       // gaussian u1 (its log is L2)
-            rng_pop(rng, ring);       // gaussian u2 (its cos is c0)
-            alpha = P.sigma_alpha * fabsf(sqrtf(-2.0f * L2) * c0);
-            if (alpha >= 1.2f) {
-                if (++tries >= 20) { specular(ux, uy, uz, face); wall_done = true; st = S_MOVE; }
-                else st = S_UNI;
-            } else {
-                rng_pop(rng, ring);   // facet azimuth (its sincos is s1, c1)
-                facet = true;
-            }
-        }
-
-        // ---- facet tilt sin/cos, once per warp ----
-        float sa = 0.f, ca = 1.f;
-        if (__any_sync(FULL, facet)) {
-            cl_sincosf_core<SC_COPIES>(facet ? alpha : 1.0f, my_sctab, &sa, &ca);
-        }
-
-        // UNIFIED try, second half (src/optics.jl:57-66): the facet normal
-        float Nfx = 0.f, Nfy = 0.f, Nfz = 0.f;
-        bool retry = false;
-        if (facet) {
-            const int a = face_axis(face);
-            const float sgn = (face == FACE_XP || face == FACE_YP || face == FACE_BACK) ? 1.0f : -1.0f;
-            const float b = sa * c1, c = sa * s1;
-            Nfx = a == 1 ? ca * sgn : b;
-            Nfy = a == 2 ? ca * sgn : (a == 1 ? b : c);
-            Nfz = a == 3 ? ca * sgn : c;
-            const float cosi = ux * Nfx + uy * Nfy + uz * Nfz;
-            if (cosi <= 0.0f) retry = true;
-            else { fk = FK_FACET; fn2 = 1.0f; fq2 = P.qa2; fcos = cosi; }
-        }
-
-        // ---- Fresnel (src/optics.jl:10-19), one evaluation per warp ----
-        float R = 1.0f;
-        bool tir = true;
-        if (__any_sync(FULL, fk != FK_NONE)) {
-            if (fk != FK_NONE) tir = fresnel_q2(P.n_crystal, fn2, fq2, fcos, R);
-        }
-        if (fk != FK_NONE) {
-            const bool refl = tir || rng_pop(rng, ring) < R;
-            if (fk == FK_READOUT) {
-                if (refl) {
-                    specular(ux, uy, uz, face);
-                    wall_done = true;
-                } else if (!disc || (x - P.cx) * (x - P.cx) + (y - P.cy) * (y - P.cy) <= P.r2) {
-                    if (rng_pop(rng, ring) <= P.pde) {
-                        int32_t ii = 1 + (int32_t)(x / P.pitch);
-                        int32_t jj = 1 + (int32_t)(y / P.pitch);
-                        ii = ii < P.nx ? ii : P.nx;
-                        jj = jj < P.ny ? jj : P.ny;
-                        const int32_t lin = (jj - 1) * P.nx + ii;
-                        idx = face == FACE_FRONT ? -lin : lin;
-                        status = ST_DETECTED;
-                    } else {
-                        status = ST_ABS_SIPM;
+                    // UNIFIED facet (src/optics.jl:55-66); a readout lane computes
+                    // one too and does not use it
+                    const bool facet = uni_possible && !readout;
+                    float Nfx = 0.f, Nfy = 0.f, Nfz = 0.f, fcos = cosw;
+                    uint32_t fo = 0;             // offset of the Fresnel uniform
+                    if (uni_possible) {
+                        const float alpha = P.sigma_alpha * fabsf(G * c0);
+                        float sa, ca;
+                        cl_sincosf_core<SC_COPIES>(fminf(alpha, 1.2f), my_sctab, &sa, &ca);
+                        const float b = sa * c1, c = sa * s1, n = ca * sgn;
+                        Nfx = on_x ? n : b;
+                        Nfy = on_y ? n : (on_x ? b : c);
+                        Nfz = on_z ? n : c;
+                        const float cosi = ux * Nfx + uy * Nfy + uz * Nfz;
+                        if (facet) {
+                            fcos = cosi;
+                            // a tilt out of range is drawn again before its azimuth is
+                            retry = alpha >= 1.2f || cosi <= 0.0f;
+                            fo = alpha >= 1.2f ? 2u * RING_ROW : 3u * RING_ROW;
+                        }
                     }
-                } else if (rng_pop(rng, ring) <= P.sur_R) {
-                    if (P.sur_specular) { specular(ux, uy, uz, face); wall_done = true; }
-                    else st = S_LAMB;
-                } else {
-                    status = ST_ABS_SUR;
-                }
-            } else if (polished_possible && fk == FK_POLISHED) {
-                if (refl) { specular(ux, uy, uz, face); wall_done = true; }
-                else to_wrap = true;
-            } else {
-                // facet: reflect about the facet normal; keep it only if it
-                // points back into the crystal (src/optics.jl:68-77)
-                if (refl) {
-                    const int a = face_axis(face);
-                    const float sgn = (face == FACE_XP || face == FACE_YP || face == FACE_BACK) ? 1.0f : -1.0f;
-                    const float Nx = a == 1 ? sgn : 0.0f;
-                    const float Ny = a == 2 ? sgn : 0.0f;
-                    const float Nz = a == 3 ? sgn : 0.0f;
-                    const float rx = ux - (2.0f * fcos) * Nfx;
-                    const float ry = uy - (2.0f * fcos) * Nfy;
-                    const float rz = uz - (2.0f * fcos) * Nfz;
-                    if (rx * Nx + ry * Ny + rz * Nz < 0.0f) {
-                        ux = rx; uy = ry; uz = rz;
-                        wall_done = true;
-                        st = S_MOVE;
-                    } else {
-                        retry = true;
+                    // Fresnel (src/optics.jl:10-19)
+                    const float n2 = readout ? P.n_coupling : 1.0f;
+                    const float sin2t = (readout ? P.qc2 : P.qa2) * (1.0f - fcos * fcos);
+                    const float uf = ring_word(v, fo), un = ring_word(v, fo + RING_ROW);
+                    const bool tir = sin2t >= 1.0f;
+                    bool refl = tir;
+                    if (!tir) refl = fresnel_reflects(P, n2, sin2t, fcos, uf);
+                    rng.pos += fo + (retry || tir ? 0u : (refl ? RING_ROW : 2u * RING_ROW));
+                    // facet reflection, kept only if it points back into the
+                    // crystal (src/optics.jl:68-77)
+                    rx = ux - (2.0f * fcos) * Nfx;
+                    ry = uy - (2.0f * fcos) * Nfy;
+                    rz = uz - (2.0f * fcos) * Nfz;
+                    const bool inward = sgn * (on_x ? rx : (on_y ? ry : rz)) < 0.0f;
+                    const bool through = !refl && !retry;
+                    take = facet && refl && !retry && inward;
+                    retry |= facet && refl && !inward;
+                    flip = !facet && refl;
+                    if (through) {
+                        if (readout) {
+                            if (!disc || (x - P.cx) * (x - P.cx) + (y - P.cy) * (y - P.cy) <= P.r2) {
+                                status = un <= P.pde ? ST_DETECTED : ST_ABS_SIPM;
+                            } else if (un <= P.sur_R) {
+                                if (P.sur_specular) flip = true;
+                                else st = S_LAMB;
+                            } else {
+                                status = ST_ABS_SUR;
+                            }
+                        } else if (un <= P.wrap_R) {
+                            // the reflector behind the air gap (src/transport.jl:214-225)
+                            if (wrap_specular) flip = true;
+                            else st = S_LAMB;
+                        } else {
+                            status = ST_ABS_WALL;
+                        }
                     }
-                } else {
-                    to_wrap = true;
-                    st = S_MOVE;
+                    if (retry) {
+                        if (++tries >= 20) flip = true;
+                        else st = S_UNI;
+                    }
                 }
-            }
-        }
-        if (retry) {
-            if (++tries >= 20) { specular(ux, uy, uz, face); wall_done = true; st = S_MOVE; }
-            else st = S_UNI;
-        }
-
-        // transmitted into the air gap: the reflector (src/transport.jl:214-225)
-        if (to_wrap) {
-            if (rng_pop(rng, ring) <= P.wrap_R) {
-                if (wrap_specular) { specular(ux, uy, uz, face); wall_done = true; }
-                else st = S_LAMB;
-            } else {
-                status = ST_ABS_WALL;
+                ux = take ? rx : (flip && on_x ? -ux : ux);
+                uy = take ? ry : (flip && on_y ? -uy : uy);
+                uz = take ? rz : (flip && on_z ? -uz : uz);
+                done = take || flip;
             }
         }
 
-        under |= rng.cnt < 0;
-
-        // end of a wall interaction: count the bounce (src/transport.jl:228-232)
-        if (wall_done && status == ST_FLYING) {
+        // end of an interaction: count the bounce (src/transport.jl:228-232)
+        if (done) {
             bounces += 1;
             if (bounces >= P.max_bounces) status = ST_CAP;
-            else st = S_MOVE;
+            st = S_MOVE;
         }
 
-        // ---- detections: warp-aggregated atomics ----
-        const bool det = status == ST_DETECTED;
-        const unsigned dmask = __ballot_sync(FULL, det);
-        if (det) {
-            const int32_t lin = idx < 0 ? -idx : idx;
-            const int32_t cell = lin - 1;
-            const uint32_t key = float_key(t);
-            if (MODE == 0) {
-                const int32_t slot = cell + A.cells * time_bin0(t, P);
-                const unsigned g = __match_any_sync(dmask, slot);
-                // one atomic per distinct slot: the group's count and its earliest time
-                const uint32_t kmin = __reduce_min_sync(g, key);
-                if (lane == __ffs(g) - 1) {
-                    atomicAdd(tile_counts + slot, (uint32_t)__popc(g));
-                    atomicMin(tile_keys + cell, kmin);
-                }
-            } else {
-                // a segment id outside the maps (untrusted device input) drops the detection
-                const bool seg_ok = seg >= 0 && (int64_t)seg < A.n_seg;
-                const unsigned okmask = __ballot_sync(dmask, seg_ok);
-                if (seg_ok) {
-                    const unsigned long long slot =
-                        (unsigned long long)seg * (unsigned long long)A.cells + (unsigned long long)cell;
-                    const unsigned g = __match_any_sync(okmask, slot);
-                    const uint32_t kmin = __reduce_min_sync(g, key);
-                    if (lane == __ffs(g) - 1) {
-                        atomicAdd(A.maps + slot, (uint32_t)__popc(g));
-                        atomicMin(A.keys + slot, kmin);
-                    }
-                    if (MODE == 2) {
-                        // fixed-point time moments (exact integer sums, order-independent)
-                        const float tc = fminf(fmaxf(t, 0.0f), CL_MOMENT_T_MAX_NS);
-                        atomicAdd(A.tsum + slot, __float2ull_rn(tc * CL_MOMENT_T_SCALE));
-                        atomicAdd(A.tsum2 + slot, __float2ull_rn((tc * tc) * CL_MOMENT_T2_SCALE));
-                    }
-                } else {
-                    atomicOr(A.err, 16u);
-                }
-            }
-        }
-
-        // ---- terminal bookkeeping: warp-aggregated counters ----
+        // ---- terminal bookkeeping ----
         const bool term = status != ST_FLYING;
         const unsigned tmask = __ballot_sync(FULL, term);
         if (tmask != 0u) {
-            if (term) {
-                const unsigned g = __match_any_sync(tmask, status);
-                // counters[] order: ndet, ndet_front, bulk, wall, sipm, cap, sur
-                const int slot = status == ST_DETECTED ? 0 : (status == ST_ABS_SUR ? 6 : status);
-                if (lane == __ffs(g) - 1) atomicAdd(&s_cnt[slot], (unsigned long long)__popc(g));
-                if (REC) {
-                    if (A.r_status) A.r_status[k] = (uint8_t)status;
-                    if (A.r_idx) A.r_idx[k] = (int16_t)idx;
-                    if (A.r_t) A.r_t[k] = t;
-                    if (A.r_bounces) A.r_bounces[k] = bounces;
+            const bool det = status == ST_DETECTED;
+            int32_t idx = 0;
+            if (det) {
+                int32_t ii = 1 + (int32_t)(x / P.pitch);
+                int32_t jj = 1 + (int32_t)(y / P.pitch);
+                ii = ii < P.nx ? ii : P.nx;
+                jj = jj < P.ny ? jj : P.ny;
+                const int32_t lin = (jj - 1) * P.nx + ii;
+                idx = two_sided && face == FACE_FRONT ? -lin : lin;
+                const int32_t cell = lin - 1;
+                const uint32_t key = float_key(t);
+                // one reduction per photon: a warp seldom detects two photons in
+                // the same slot, and finding out costs more than it saves
+                if (MODE == 0) {
+                    atomicAdd(tile_counts + cell + A.cells * time_bin0(t, P), 1u);
+                    // the 64 keys are hot; most photons are later than the key
+                    // already there (which only ever falls)
+                    if (key < (TILE ? tile_keys[cell] : __ldcg(tile_keys + cell))) atomicMin(tile_keys + cell, key);
+                } else {
+                    // a segment id outside the maps (untrusted device input) drops the detection
+                    if (seg >= 0 && (int64_t)seg < A.n_seg) {
+                        const unsigned long long slot =
+                            (unsigned long long)seg * (unsigned long long)A.cells + (unsigned long long)cell;
+                        atomicAdd(A.maps + slot, 1u);
+                        atomicMin(A.keys + slot, key);
+                        if (MODE == 2) {
+                            // fixed-point time moments (exact integer sums, order-independent)
+                            const float tc = fminf(fmaxf(t, 0.0f), CL_MOMENT_T_MAX_NS);
+                            atomicAdd(A.tsum + slot, __float2ull_rn(tc * CL_MOMENT_T_SCALE));
+                            atomicAdd(A.tsum2 + slot, __float2ull_rn((tc * tc) * CL_MOMENT_T2_SCALE));
+                        }
+                    } else {
+                        atomicOr(A.err, 16u);
+                    }
                 }
             }
-            const unsigned front = __ballot_sync(FULL, det && idx < 0);
+            if (REC && term) {
+                const uint64_t k = (((uint64_t)rng.pid_hi << 32) | rng.pid_lo) - A.pid0 - 1ull;
+                if (A.r_status) A.r_status[k] = (uint8_t)status;
+                if (A.r_idx) A.r_idx[k] = (int16_t)idx;
+                if (A.r_t) A.r_t[k] = t;
+                if (A.r_bounces) A.r_bounces[k] = bounces;
+            }
+            // counters: the fates in five 6-bit fields of one reduction (the
+            // caps are what is left of the terminated lanes), the sums one each;
+            // lane i adds entry i of the warp's own counters
+            const uint32_t field = det ? 1u : (status == ST_ABS_SUR ? 1u << 24 : 1u << (6 * ((status - 1) & 3)));
+            const uint32_t fates = __reduce_add_sync(FULL, term && status != ST_CAP ? field : 0u);
+            const uint32_t front = two_sided ? (uint32_t)__popc(__ballot_sync(FULL, det && idx < 0)) : 0u;
             const uint32_t sb = __reduce_add_sync(FULL, det ? (uint32_t)bounces : 0u);
             const uint32_t sc = __reduce_add_sync(FULL, term ? (uint32_t)nscat : 0u);
             const uint32_t ss = __reduce_add_sync(FULL, term ? (uint32_t)(bounces + (status != ST_CAP)) : 0u);
-            if (lane == 0) {
-                if (front) atomicAdd(&s_cnt[1], (unsigned long long)__popc(front));
-                if (sc) atomicAdd(&s_cnt[7], (unsigned long long)sc);
-                if (sb) atomicAdd(&s_cnt[8], (unsigned long long)sb);
-                atomicAdd(&s_cnt[9], (unsigned long long)ss);
+            if (lane < N_COUNTERS) {
+                // ndet, ndet_front, bulk, wall, sipm, cap, sur, nscat, sum_bounces_det, steps
+                uint32_t add = fates & 63u;
+                if (lane == 1) add = front;
+                if (lane >= 2 && lane <= 4) add = (fates >> (6 * (lane - 1))) & 63u;
+                if (lane == 5) add = (uint32_t)__popc(tmask) - (fates & 63u) - ((fates >> 6) & 63u) -
+                                     ((fates >> 12) & 63u) - ((fates >> 18) & 63u) - (fates >> 24);
+                if (lane == 6) add = fates >> 24;
+                if (lane == 7) add = sc;
+                if (lane == 8) add = sb;
+                if (lane == 9) add = ss;
+                my_cnt[lane] += (unsigned long long)add;
             }
             if (term) st = S_IDLE;
         }
@@ -652,12 +617,10 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
             if (kk != INF_KEY) atomicMin(A.keys + i, kk);
         }
     }
-    if (tid < 9) {
-        const unsigned long long v = s_cnt[tid];
-        if (v) atomicAdd(A.counters + tid, v);
-    } else if (tid == 9) {
-        const unsigned long long v = s_cnt[9];
-        if (v) atomicAdd(A.steps, v);
+    if (tid < N_COUNTERS) {
+        unsigned long long v = 0;
+        for (int q = 0; q < 8; ++q) v += s_cnt[q][tid];
+        if (v) atomicAdd(tid < 9 ? A.counters + tid : A.steps, v);
     }
 
     if (MODE == 0) {
@@ -689,8 +652,9 @@ __global__ void init_kernel(uint32_t* counts, int64_t n_counts, uint32_t* keys, 
     if (i0 == 0) { *queue = 0ull; *steps = 0ull; *done = 0u; *err = 0u; }
 }
 
-// The log table of the uniforms: t[k] = cl_logf_u((k+1) * 2^-24), the same
-// function and rounding as the computed path, for k < 2^24.
+// The tables of the uniforms u = (k+1) 2^-24, k < 2^24: t[k] = log u and
+// t[GAUSS_OFF + k] = sqrt(-2 log u), the same functions and rounding as the
+// computed path.
 __global__ void logtab_fill(float* t)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -699,7 +663,11 @@ __global__ void logtab_fill(float* t)
     __syncthreads();
     const double2* my_tab = s_tab + (threadIdx.x % LOG_COPIES);
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < (1u << 24); k += gridDim.x * blockDim.x)
-        t[k] = cl_logf_u<LOG_COPIES>(u32_to_randu(k << 8), my_tab);
+    {
+        const float l = cl_logf_u<LOG_COPIES>(u32_to_randu(k << 8), my_tab);
+        t[k] = l;
+        t[GAUSS_OFF + k] = sqrtf(-2.0f * l);
+    }
 }
 
 // Segment mode: decode tmin keys in place and sum npe per segment.
@@ -786,7 +754,7 @@ struct cl_handle {
     int device = 0;
     int num_sms = 0;
     cudaStream_t stream = nullptr;
-    DevBuf logtab;                 // 2^24 floats, or empty: the kernels compute the logs
+    DevBuf logtab;                 // the tables of the uniforms, or empty: the kernels compute them
     char err[512] = {0};
     DevBuf src, out, rec, scratch, dbg;
     int ctas_per_sm = 0;
@@ -914,11 +882,10 @@ int cl_create(cl_handle** out, int device)
         delete h;
         return CL_ERR_OOM;
     }
-#if CL_USE_LOGTAB
-    // 64 MB table of the logs of all 2^24 uniforms; without it (allocation
-    // failure) the kernels evaluate the same function in place
-    if (cudaMalloc(&h->logtab.p, sizeof(float) << 24) == cudaSuccess) {
-        h->logtab.cap = sizeof(float) << 24;
+    // 128 MB: the logs of all 2^24 uniforms and their sqrt(-2 log u); without
+    // them (allocation failure) the kernels evaluate the same functions in place
+    if (cudaMalloc(&h->logtab.p, sizeof(float) << 25) == cudaSuccess) {
+        h->logtab.cap = sizeof(float) << 25;
         logtab_fill<<<h->num_sms * 4, 256, LOGTAB_BYTES, h->stream>>>((float*)h->logtab.p);
         if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(h->stream) != cudaSuccess) {
             cudaGetLastError();
@@ -929,7 +896,6 @@ int cl_create(cl_handle** out, int device)
         cudaGetLastError();
         h->logtab = DevBuf();
     }
-#endif
     *out = h;
     return CL_OK;
 }
@@ -1024,6 +990,15 @@ static Physics make_physics(const cl_box* box, const cl_optical_params* op, cons
         P.qc2 = qc * qc;
         P.qa2 = qa * qa;
     }
+    // rates of the bulk competition's quick test; NaN (no or a negative length)
+    // fails it, so those runs take the exact comparison
+    auto rate = [](float len) { return len > 0.0f ? (float)(-1.4426950408889634 / (double)len) : NAN; };
+    P.abs_rate = rate(op->abs_len_mm);
+    P.ray_rate = rate(op->rayleigh_mm);
+    // the quick Fresnel test's error bound holds for indices of this range
+    const bool plain = op->n_crystal >= 1e-3f && op->n_crystal <= 1e3f && op->n_coupling >= 1e-3f &&
+                       op->n_coupling <= 1e3f;
+    P.fresnel_margin = plain ? 0x1p-17f : INFINITY;
     P.abs_finite = std::isfinite(op->abs_len_mm) ? 1 : 0;
     P.ray_finite = std::isfinite(op->rayleigh_mm) ? 1 : 0;
     P.wrap_specular = op->wrap_specular ? 1 : 0;
@@ -1129,7 +1104,7 @@ static int enqueue_point(cl_handle* h, const Physics& P, const float* px, const 
     a.logtab = (const float*)h->logtab.p;
     a.budget_ns = h->budget_ns;
     const size_t tile_bytes = ((size_t)n_counts + cells) * sizeof(uint32_t);
-    const size_t base_bytes = LOGTAB_BYTES + (size_t)RING_LEN * RING_STRIDE * sizeof(float);
+    const size_t base_bytes = LOGTAB_BYTES + RING_BYTES;
     // the shared-memory histogram tile only where it still leaves room for 4
     // CTAs per SM: with fewer resident warps the loop issues less often, which
     // costs more than the tile saves in global atomics (10^6-photon point
@@ -1177,7 +1152,7 @@ static int enqueue_segments(cl_handle* h, const Physics& P, const float* sx, con
         a.queue = s.queue; a.steps = s.steps; a.done = s.done; a.err = s.err;
         a.logtab = (const float*)h->logtab.p;
         a.budget_ns = h->budget_ns;
-        const size_t smem = LOGTAB_BYTES + (size_t)RING_LEN * RING_STRIDE * sizeof(float);
+        const size_t smem = LOGTAB_BYTES + RING_BYTES;
         a.tsum = tsum; a.tsum2 = tsum2;
         const int rc = moments ? launch_transport<2, false, false>(h, a, smem, st)
                      : want_rec ? launch_transport<1, true, false>(h, a, smem, st)
