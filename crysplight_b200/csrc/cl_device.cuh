@@ -110,30 +110,36 @@ __device__ __forceinline__ bool rng_short(const Rng& r) { return rng_level(r) <=
 __device__ __forceinline__ bool rng_room(const Rng& r) { return rng_level(r) <= 24 * (int32_t)RING_ROW; }
 __device__ __forceinline__ bool rng_under(const Rng& r) { return rng_level(r) <= -(int32_t)RING_ROW; }
 
+// Ring accesses by 32-bit shared address (volatile: a read stays behind the
+// fill that stored it).
+__device__ __forceinline__ float ring_word(uint32_t a)
+{
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void ring_store(uint32_t a, float v)
+{
+    asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v));
+}
+
 // Two consecutive blocks at once (independent Philox chains interleave); needs
 // rng_room.  The write row is a multiple of 8: the stores never wrap.
-__device__ __forceinline__ void rng_fill(Rng& r, unsigned char* ring, const uint32_t* rk)
+__device__ __forceinline__ void rng_fill(Rng& r, uint32_t ring, const uint32_t* rk)
 {
     const uint4 o = philox4x32_10_rk(make_uint4(r.pid_lo, r.pid_hi, r.block, 0u), rk);
     const uint4 q = philox4x32_10_rk(make_uint4(r.pid_lo, r.pid_hi, r.block + 1u, 0u), rk);
     const uint32_t row = (r.block * (4u * RING_ROW)) & RING_MASK;
-    float* const p = reinterpret_cast<float*>(ring + row + 4u * threadIdx.x);
-    constexpr uint32_t S = RING_ROW / 4;
+    const uint32_t a = ring + row + 4u * threadIdx.x;
     const float f[8] = {u32_to_randu(o.x), u32_to_randu(o.y), u32_to_randu(o.z), u32_to_randu(o.w),
                         u32_to_randu(q.x), u32_to_randu(q.y), u32_to_randu(q.z), u32_to_randu(q.w)};
 #pragma unroll
-    for (int i = 0; i < 8; ++i) p[i * S] = f[i];
+    for (int i = 0; i < 8; ++i) ring_store(a + i * RING_ROW, f[i]);
     if (row == 0u) {
 #pragma unroll
-        for (int i = 0; i < RING_ROWS - 32; ++i) p[(32 + i) * S] = f[i];
+        for (int i = 0; i < RING_ROWS - 32; ++i) ring_store(a + (32 + i) * RING_ROW, f[i]);
     }
     r.block += 2u;
-}
-
-// The uniform `off` bytes (a multiple of RING_ROW) after the one at w.
-__device__ __forceinline__ float ring_word(const unsigned char* w, uint32_t off)
-{
-    return *reinterpret_cast<const float*>(w + off);
 }
 
 // A register-only stream for the diagnostics kernel (same sequence).
@@ -248,27 +254,29 @@ __device__ __forceinline__ float cl_logf_u(float x, const double2* __restrict__ 
 // be encoded and would first be moved into registers).
 static __constant__ double c_sc_coef[4] = {CLM_TS5, CLM_TS3, CLM_TC4, CLM_TC2};
 
-template <int STRIDE = 1>
-__device__ __forceinline__ void cl_sincosf_core(float x, const double2* __restrict__ sctab,
-                                                float* sp, float* cp)
+// 32-bit shared-memory addresses: through pointers the compiler derives the
+// window's base again at every use in the transport loop.
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void cl_sincosf_core(float x, uint32_t sctab, float* sp, float* cp)
 {
-    // j = rint(64 x) by the 1.5*2^23 shift; j sits in the low bits of the sum
+    // j = rint(64 x) by the 1.5*2^23 shift: the sum's bits are 0x4B400000 + j,
+    // and 16 times them (mod 2^32) the table offset plus a constant
     const float sh = __fmaf_rn(x, 64.0f, 12582912.0f);
     const float rf = __fmaf_rn(sh - 12582912.0f, -0.015625f, x);
-    const double2 sc = sctab[(__float_as_uint(sh) & 511u) * STRIDE];
+    double S, C;
+    asm("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(S), "=d"(C) : "r"(__float_as_uint(sh) * 16u + (sctab - 0xB4000000u)));
     const double r = (double)rf;
     const double r2 = r * r;
     const double sr = fma(r * r2, fma(c_sc_coef[0], r2, c_sc_coef[1]), r);    // sin r
     const double cm1 = r2 * fma(c_sc_coef[2], r2, c_sc_coef[3]);              // cos r - 1
-    *sp = __double2float_rn(fma(sc.y, sr, fma(sc.x, cm1, sc.x)));
-    *cp = __double2float_rn(fma(-sc.x, sr, fma(sc.y, cm1, sc.y)));
+    *sp = __double2float_rn(fma(C, sr, fma(S, cm1, S)));
+    *cp = __double2float_rn(fma(-S, sr, fma(C, cm1, C)));
 }
 
 // The same for any argument (diagnostics): outside the core's range, CUDA's
 // Float64 functions.
-template <int STRIDE = 1>
-__device__ __forceinline__ void cl_sincosf(float x, const double2* __restrict__ sctab,
-                                           float* sp, float* cp)
+__device__ __forceinline__ void cl_sincosf(float x, uint32_t sctab, float* sp, float* cp)
 {
     if (!(x >= 0.0f && x <= 6.2831855f)) {
         const float2 sc = slow_sincosf(x);
@@ -281,7 +289,7 @@ __device__ __forceinline__ void cl_sincosf(float x, const double2* __restrict__ 
         *cp = 1.0f;
         return;
     }
-    cl_sincosf_core<STRIDE>(x, sctab, sp, cp);
+    cl_sincosf_core(x, sctab, sp, cp);
 }
 
 // ---------------------------------------------------------------------------
@@ -330,6 +338,29 @@ __device__ __forceinline__ float ex2_approx(float x)
     return r;
 }
 
+// Correctly rounded square root and reciprocal of arguments well inside the
+// normal range (2^-40 .. 2^40; sqrt_mid also of 0), without the range tests and
+// slow paths of the general functions: an approximation refined by residuals
+// that are exact in a fused multiply-add (P. Markstein, "Computation of
+// elementary functions on the IBM RISC System/6000 processor", IBM J. Res.
+// Dev. 34 (1990)).  Both equal the IEEE operations for every Float32 mantissa
+// (tested over all of them).
+__device__ __forceinline__ float sqrt_mid(float x)
+{
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(fmaxf(x, 0x1p-60f)));
+    const float g = x * y, h = 0.5f * y;
+    const float e = __fmaf_rn(-h, g, 0.5f);
+    const float g1 = __fmaf_rn(g, e, g), h1 = __fmaf_rn(h, e, h);
+    return __fmaf_rn(__fmaf_rn(-g1, g1, x), h1, g1);
+}
+__device__ __forceinline__ float rcp_mid(float x)
+{
+    const float r = rcp_approx(x);
+    const float r1 = __fmaf_rn(r, __fmaf_rn(-x, r, 1.0f), r);
+    return __fmaf_rn(r1, __fmaf_rn(-x, r1, 1.0f), r1);
+}
+
 // fresnel, src/optics.jl:10-19, where sin2t = (n1/n2)^2 (1 - cosi^2) < 1.
 __device__ __forceinline__ float fresnel_R(float n1, float n2, float sin2t, float cosi)
 {
@@ -339,22 +370,30 @@ __device__ __forceinline__ float fresnel_R(float n1, float n2, float sin2t, floa
     return 0.5f * (a * a + b * b);
 }
 
-// u < R at an interface where sin2t < 1.  R is estimated with approximate
+// Reflection at an interface: total, or u < R.  R is estimated with approximate
 // reciprocals and root: the estimate and the reference's rounded R each lie
 // within 2^-20 of the Fresnel formula in the same operands (a handful of
 // relative errors of 2^-22 at most in quotients of magnitude <= 1), so outside
 // fresnel_margin = 2^-17 the estimate decides; inside it (1.5e-5 of the
 // draws) the exact expression does.  Two IEEE divisions and a root less, each
 // with a branch of its own.
+// The bound holds for indices in [1e-3, 1e3]; others always take the exact one.
+__host__ __device__ inline float fresnel_margin(float n1, float n2)
+{
+    const bool plain = n1 >= 1e-3f && n1 <= 1e3f && n2 >= 1e-3f && n2 <= 1e3f;
+    return plain ? 0x1p-17f : __builtin_inff();
+}
 __device__ __forceinline__ bool fresnel_reflects(const Physics& P, float n2, float sin2t, float cosi, float u)
 {
-    const float ct = sqrt_approx(1.0f - sin2t);
+    const bool tir = sin2t >= 1.0f;
+    const float ct = sqrt_approx(1.0f - sin2t);        // NaN beyond the critical angle
     const float p = P.n_crystal * cosi, s = n2 * cosi;
     const float a = __fmaf_rn(-n2, ct, p) * rcp_approx(__fmaf_rn(n2, ct, p));
     const float b = __fmaf_rn(P.n_crystal, ct, -s) * rcp_approx(__fmaf_rn(P.n_crystal, ct, s));
     const float over = __fmaf_rn(0.5f, __fmaf_rn(a, a, b * b), -u);      // R - u
-    if (fabsf(over) > P.fresnel_margin) return over > 0.0f;
-    return u < fresnel_R(P.n_crystal, n2, sin2t, cosi);
+    bool refl = tir || over > 0.0f;
+    if (!tir && !(fabsf(over) > P.fresnel_margin)) refl = u < fresnel_R(P.n_crystal, n2, sin2t, cosi);
+    return refl;
 }
 
 // A bound below exp(-d / length) (rate = -log2(e) / length): a uniform u below
@@ -362,6 +401,12 @@ __device__ __forceinline__ bool fresnel_reflects(const Physics& P, float n2, flo
 // and ex2's errors and that of the Float32 product length * log u stay below
 // 2^-17 in log2 u wherever a uniform (>= 2^-24) can be below the bound; 2^-15
 // is taken off.
+// A length that is not positive gives NaN, for which no uniform is below the
+// bound.
+__host__ __device__ inline float survive_rate(float len)
+{
+    return len > 0.0f ? (float)(-1.4426950408889634 / (double)len) : __builtin_nanf("");
+}
 __device__ __forceinline__ float survive_below(float d, float rate)
 {
     return ex2_approx(__fmaf_rn(d, rate, -0x1p-15f));
@@ -458,7 +503,8 @@ __device__ __forceinline__ void rayleigh_rotate(float mu, float cb, float sb,
     // for a warp whose lanes take both cases)
     const bool zlow = fabsf(uz) < 0.9f;
     const float pa = zlow ? ux : uy, pb = zlow ? uy : uz;
-    float inv = 1.0f / sqrtf(pa * pa + pb * pb);
+    // both sums of squares are those of a unit vector's components, >= 0.19
+    float inv = rcp_mid(sqrt_mid(pa * pa + pb * pb));
     const float t1x = zlow ? -pb * inv : 0.0f;
     const float t1y = zlow ? pa * inv : -pb * inv;
     const float t1z = zlow ? 0.0f : pa * inv;
@@ -468,7 +514,7 @@ __device__ __forceinline__ void rayleigh_rotate(float mu, float cb, float sb,
     const float vx = mu * ux + cb * t1x + sb * t2x;
     const float vy = mu * uy + cb * t1y + sb * t2y;
     const float vz = mu * uz + cb * t1z + sb * t2z;
-    inv = 1.0f / sqrtf(vx * vx + vy * vy + vz * vz);
+    inv = rcp_mid(sqrt_mid(vx * vx + vy * vy + vz * vz));
     ux = vx * inv; uy = vy * inv; uz = vz * inv;
 }
 

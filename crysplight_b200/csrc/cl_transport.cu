@@ -8,15 +8,15 @@
 //     its photon terminates, so long-bouncing photons never idle a warp;
 //   * parameters travel as a __grid_constant__ kernel argument (constant
 //     bank), the log table sits in shared memory;
-//   * point mode: the nx*ny*(nbins+1) count tile and the nx*ny first-time
-//     tile live in shared memory; detections are warp-aggregated with
-//     __match_any_sync (one shared atomic per distinct bin per warp step),
-//     first times use atomicMin on order-preserving uint32 keys; each CTA
-//     flushes its tile once with coalesced global atomics and the last CTA
-//     decodes the first-time keys in place;
+//   * point mode: where they fit, the nx*ny*(nbins+1) count tile and the nx*ny
+//     first-time tile live in shared memory; one atomic add per detection,
+//     first times by atomicMin on order-preserving uint32 keys where the
+//     photon is earlier than the key; each CTA flushes its tile once with
+//     coalesced global atomics and the last CTA decodes the first-time keys in
+//     place;
 //   * segment mode (scan points, 511 keV events): per-segment 8x8 maps and
-//     first-time keys are reduced with warp-aggregated global atomics;
-//     a finalize kernel decodes keys and sums npe.
+//     first-time keys are reduced with global atomics; a finalize kernel
+//     decodes keys and sums npe.
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -39,19 +39,8 @@ namespace cl {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int GAUSS_OFF = 1 << 24;    // sqrt(-2 log u) after the 2^24 logs
 constexpr int N_COUNTERS = 10;        // cl_counters, then the photon-steps
-// The tables are replicated: entry e of copy c sits at [e * COPIES + c] and a
-// lane reads copy (lane % COPIES), so the 16-byte reads of the 8 lanes that
-// share a shared-memory wavefront hit distinct banks when COPIES = 8.
-#ifndef CL_LOG_COPIES
-#define CL_LOG_COPIES 1
-#endif
-#ifndef CL_SC_COPIES
-#define CL_SC_COPIES 1
-#endif
-constexpr int LOG_COPIES = CL_LOG_COPIES;
-constexpr int SC_COPIES = CL_SC_COPIES;
-constexpr int SCTAB_BYTES = CLM_SC_N * 16 * SC_COPIES;
-constexpr int LOGTAB_BYTES = ((CLM_LOG_NTAB * 16 * LOG_COPIES + 127) / 128) * 128 + SCTAB_BYTES;  // both tables
+constexpr int SCTAB_BYTES = CLM_SC_N * 16;
+constexpr int LOGTAB_BYTES = ((CLM_LOG_NTAB * 16 + 127) / 128) * 128 + SCTAB_BYTES;  // both tables
 
 __constant__ double c_logtab[2 * CLM_LOG_NTAB] = { CLM_LOG_TAB_INIT };
 __constant__ double c_sctab[2 * CLM_SC_N] = { CLM_SC_TAB_INIT };
@@ -61,14 +50,10 @@ __device__ __forceinline__ void load_tables(unsigned char* smem, double2*& tab, 
 {
     sctab = reinterpret_cast<double2*>(smem);
     tab = reinterpret_cast<double2*>(smem + SCTAB_BYTES);
-    for (int i = threadIdx.x; i < CLM_SC_N * SC_COPIES; i += blockDim.x) {
-        const int e = i / SC_COPIES;
-        sctab[i] = make_double2(c_sctab[2 * e], c_sctab[2 * e + 1]);
-    }
-    for (int i = threadIdx.x; i < CLM_LOG_NTAB * LOG_COPIES; i += blockDim.x) {
-        const int e = i / LOG_COPIES;
-        tab[i] = make_double2(c_logtab[2 * e], c_logtab[2 * e + 1]);
-    }
+    for (int i = threadIdx.x; i < CLM_SC_N; i += blockDim.x)
+        sctab[i] = make_double2(c_sctab[2 * i], c_sctab[2 * i + 1]);
+    for (int i = threadIdx.x; i < CLM_LOG_NTAB; i += blockDim.x)
+        tab[i] = make_double2(c_logtab[2 * i], c_logtab[2 * i + 1]);
 }
 
 struct KArgs {
@@ -145,7 +130,7 @@ __device__ __forceinline__ int64_t find_source(const int64_t* __restrict__ off, 
 // wrap) completes in one iteration, so an iteration is about one photon-step.
 // States from S_INIT on set a new direction from a polar cosine and an azimuth.
 enum : int32_t {
-    S_IDLE = 0,   // no photon
+    S_IDLE = 0,   // no photon; below 0: minus the fate of a photon not yet booked
     S_MOVE = 1,   // bulk competition + wall interaction (src/transport.jl:127-233)
     S_UNI = 2,    // another UNIFIED try at the same wall (src/optics.jl:54-78)
     S_INIT = 3,   // emission: direction and time (src/kernel.jl:173-180)
@@ -175,10 +160,10 @@ enum : int { SPEC_ANY = 0, SPEC_ESR = 1, SPEC_TEFLON = 2 };
 
 // log of a uniform u = k 2^-24 from the table (k in 1..2^24 at [k - 1]), or
 // evaluated where there is no table.
-__device__ __forceinline__ uint32_t uniform_index(float u) { return min((uint32_t)(u * 16777216.0f), 1u << 24); }
+__device__ __forceinline__ int uniform_index(float u) { return (int)(u * 16777216.0f) - 1; }
 __device__ __forceinline__ float uniform_log(const float* __restrict__ tab, float u, const double2* __restrict__ logtab)
 {
-    return tab ? __ldg(tab + (int)uniform_index(u) - 1) : cl_logf_u<LOG_COPIES>(u, logtab);
+    return tab ? __ldg(tab + uniform_index(u)) : cl_logf_u(u, logtab);
 }
 
 // The loop computes what decides a photon's next step exactly and everything
@@ -195,7 +180,11 @@ __device__ __forceinline__ float uniform_log(const float* __restrict__ tab, floa
 //   * outcomes are merged by selects into one flip / one new direction / one
 //     state change, not one branch each;
 //   * the tilt's sqrt(-2 log u) is looked up whole.
-// Measured on BGO+ESR (51.2M photons) and 3,001 CsI(Tl)+Teflon events: CL_LOOP_MS.
+//   * booking an ended photon and starting the next one wait for a few free lanes.
+// Against the same states with exact expressions and a branch per outcome
+// (31.2 -> 20.4 warp instructions per photon-step): BGO+ESR scan of 51.2M
+// photons 143.9 -> 100.4 ms (49 G photon-steps/s), 3,001 CsI(Tl)+Teflon events
+// 32.6 -> 20.6 ms, 10^6-photon CsI(Tl) point 1.17 -> 0.79 ms.
 template <int MODE, bool REC, bool TILE, int SPEC>
 __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(const __grid_constant__ KArgs A)
 {
@@ -223,13 +212,18 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
     for (int r = 0; r < RING_ROWS; ++r) *reinterpret_cast<float*>(s_ring + r * RING_ROW + 4 * tid) = 1.0f;
     __syncthreads();
 
+    // free lanes that make a turnover worth its cost: 1 / 3 / 4 lanes took 105.5 /
+    // 100.5 / 101.0 ms on the scan (a photon ends every 97 steps); 1 / 4 / 8 / 10
+    // lanes 23.8 / 21.3 / 20.5 / 20.6 ms on the events (every 12 steps)
+    constexpr int TURNOVER = SPEC == SPEC_ESR ? 3 : 8;
+
     uint32_t* tile_counts = TILE ? s_counts : A.counts;
     uint32_t* tile_keys = TILE ? s_keys : A.keys;
     unsigned long long* my_cnt = s_cnt[tid >> 5];
 
     const unsigned lt_mask = (1u << lane) - 1u;
-    const double2* my_tab = s_tab + (lane % LOG_COPIES);
-    const double2* my_sctab = s_sctab + (lane % SC_COPIES);
+    const double2* my_tab = s_tab;
+    const uint32_t sc0 = smem_addr(smem), ring0 = sc0 + LOGTAB_BYTES;
     const bool air_gap = SPEC != SPEC_ANY || P.air_gap;
     const bool uni_possible = SPEC != SPEC_ANY || (P.air_gap && P.sigma_alpha > 0.0f);
     const bool wrap_specular = SPEC == SPEC_ESR || (SPEC == SPEC_ANY && P.wrap_specular);
@@ -258,10 +252,83 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
     const unsigned long long t_begin = A.budget_ns ? globaltimer_ns() : 0ull;
 
     for (;;) {
-        // ---- refill idle lanes from the warp's pool / the global queue ----
-        const unsigned need = __ballot_sync(FULL, st == S_IDLE);
-        if (need != 0u) {
+        // ---- turnover: book the ended photons, refill their lanes from the
+        // warp's pool / the global queue.  Both cost the same for one lane as
+        // for many, so lanes wait until TURNOVER of them are free.
+        if (__popc(__ballot_sync(FULL, st <= 0)) >= TURNOVER) {
+            const unsigned tmask = __ballot_sync(FULL, st < 0);
+            if (tmask != 0u) {
+                const int32_t status = st < 0 ? -st : ST_FLYING;
+                const bool det = status == ST_DETECTED;
+                int32_t idx = 0;
+                if (det) {
+                    int32_t ii = 1 + (int32_t)(x / P.pitch);
+                    int32_t jj = 1 + (int32_t)(y / P.pitch);
+                    ii = ii < P.nx ? ii : P.nx;
+                    jj = jj < P.ny ? jj : P.ny;
+                    const int32_t lin = (jj - 1) * P.nx + ii;
+                    idx = two_sided && face == FACE_FRONT ? -lin : lin;
+                    const int32_t cell = lin - 1;
+                    const uint32_t key = float_key(t);
+                    // one reduction per photon: a warp seldom detects two photons in
+                    // the same slot, and finding out costs more than it saves
+                    if (MODE == 0) {
+                        atomicAdd(tile_counts + cell + A.cells * time_bin0(t, P), 1u);
+                        // the cells' keys are hot; most photons are later than the
+                        // key already there (which only ever falls)
+                        if (key < (TILE ? tile_keys[cell] : __ldcg(tile_keys + cell))) atomicMin(tile_keys + cell, key);
+                    } else {
+                        // a segment id outside the maps (untrusted device input) drops the detection
+                        if (seg >= 0 && (int64_t)seg < A.n_seg) {
+                            const unsigned long long slot =
+                                (unsigned long long)seg * (unsigned long long)A.cells + (unsigned long long)cell;
+                            atomicAdd(A.maps + slot, 1u);
+                            atomicMin(A.keys + slot, key);
+                            if (MODE == 2) {
+                                // fixed-point time moments (exact integer sums, order-independent)
+                                const float tc = fminf(fmaxf(t, 0.0f), CL_MOMENT_T_MAX_NS);
+                                atomicAdd(A.tsum + slot, __float2ull_rn(tc * CL_MOMENT_T_SCALE));
+                                atomicAdd(A.tsum2 + slot, __float2ull_rn((tc * tc) * CL_MOMENT_T2_SCALE));
+                            }
+                        } else {
+                            atomicOr(A.err, 16u);
+                        }
+                    }
+                }
+                if (REC && st < 0) {
+                    const uint64_t k = (((uint64_t)rng.pid_hi << 32) | rng.pid_lo) - A.pid0 - 1ull;
+                    if (A.r_status) A.r_status[k] = (uint8_t)status;
+                    if (A.r_idx) A.r_idx[k] = (int16_t)idx;
+                    if (A.r_t) A.r_t[k] = t;
+                    if (A.r_bounces) A.r_bounces[k] = bounces;
+                }
+                // counters: the fates in five 6-bit fields of one reduction (the
+                // caps are what is left of the ended lanes), the sums one each;
+                // lane i adds entry i of the warp's own counters
+                const uint32_t field = st >= 0 || status == ST_CAP ? 0u
+                                       : (1u << (status == ST_DETECTED ? 0 : (status == ST_ABS_SUR ? 24 : 6 * (status - 1))));
+                const uint32_t fates = __reduce_add_sync(FULL, field);
+                const uint32_t front = two_sided ? (uint32_t)__popc(__ballot_sync(FULL, det && idx < 0)) : 0u;
+                const uint32_t sb = __reduce_add_sync(FULL, det ? (uint32_t)bounces : 0u);
+                const uint32_t sc = __reduce_add_sync(FULL, st < 0 ? (uint32_t)nscat : 0u);
+                const uint32_t ss = __reduce_add_sync(FULL, st < 0 ? (uint32_t)(bounces + (status != ST_CAP)) : 0u);
+                if (lane < N_COUNTERS) {
+                    // ndet, ndet_front, bulk, wall, sipm, cap, sur, nscat, sum_bounces_det, steps
+                    uint32_t add = fates & 63u;
+                    if (lane == 1) add = front;
+                    if (lane >= 2 && lane <= 4) add = (fates >> (6 * (lane - 1))) & 63u;
+                    if (lane == 5) add = (uint32_t)__popc(tmask) - (fates & 63u) - ((fates >> 6) & 63u) -
+                                         ((fates >> 12) & 63u) - ((fates >> 18) & 63u) - (fates >> 24);
+                    if (lane == 6) add = fates >> 24;
+                    if (lane == 7) add = sc;
+                    if (lane == 8) add = sb;
+                    if (lane == 9) add = ss;
+                    my_cnt[lane] += (unsigned long long)add;
+                }
+                if (st < 0) st = S_IDLE;
+            }
             if (!exhausted) {
+                const unsigned need = __ballot_sync(FULL, st == S_IDLE);
                 const int nneed = __popc(need);
                 const int rank = __popc(need & lt_mask);
                 int64_t my_k = -1;
@@ -311,37 +378,37 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                     st = S_INIT;
                 }
             }
-            if (!__any_sync(FULL, st != S_IDLE)) break;
+            if (!__any_sync(FULL, st > 0)) break;
         }
-        if (A.budget_ns != 0ull && ((++iter) & 255u) == 0u) {
+        if (((++iter) & 255u) == 0u && A.budget_ns != 0ull) {
             // photons still in flight are dropped; the host reports CL_ERR_TIMEOUT
             if (__any_sync(FULL, globaltimer_ns() - t_begin > A.budget_ns)) { timed_out = true; break; }
         }
 
         // ---- top up the uniform ring: one Philox call site for the warp ----
-        if (__any_sync(FULL, st != S_IDLE && rng_short(rng))) {
+        if (__any_sync(FULL, st > 0 && rng_short(rng))) {
             // every lane with room tops up at this convergent point, so later
             // iterations need the fill less often
             under |= rng_under(rng);
-            if (st != S_IDLE && rng_room(rng)) rng_fill(rng, s_ring, P.rk);
+            if (st > 0 && rng_room(rng)) rng_fill(rng, ring0, P.rk);
         }
 
         // ---- draws: this iteration's uniforms at fixed offsets ----
-        const unsigned char* const w = s_ring + (rng.pos & RING_MASK);
+        const uint32_t w = ring0 + (rng.pos & RING_MASK);
         // the table lookup (tilt's gaussian, or the emission time's log) and the azimuth
-        uint32_t og = st == S_MOVE ? bulk_off : (st == S_INIT ? 2u * RING_ROW : 0u);
+        const uint32_t og = st == S_MOVE ? bulk_off : (st == S_INIT ? 2u * RING_ROW : 0u);
         uint32_t oaz = st == S_MOVE ? bulk_off + 2u * RING_ROW : (st == S_UNI ? 2u * RING_ROW : RING_ROW);
         float mu = 0.0f;
         bool ray_ok = true;
         if (st == S_RAY) {
             // two rejection tries in one iteration (8 of 9 scatters end in it)
-            mu = 1.0f - 2.0f * ring_word(w, 0);
-            ray_ok = 2.0f * ring_word(w, RING_ROW) <= 1.0f + mu * mu;
+            mu = 1.0f - 2.0f * ring_word(w);
+            ray_ok = 2.0f * ring_word(w + RING_ROW) <= 1.0f + mu * mu;
             oaz = 2u * RING_ROW;
             if (!ray_ok) {
                 ++tries;
-                mu = 1.0f - 2.0f * ring_word(w, 2u * RING_ROW);
-                ray_ok = 2.0f * ring_word(w, 3u * RING_ROW) <= 1.0f + mu * mu;
+                mu = 1.0f - 2.0f * ring_word(w + 2u * RING_ROW);
+                ray_ok = 2.0f * ring_word(w + 3u * RING_ROW) <= 1.0f + mu * mu;
                 oaz = 4u * RING_ROW;
             }
         }
@@ -349,29 +416,31 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
         // ---- elementary functions, once per warp (Float64, rounded once) ----
         // Straight-line and unconditional (a lane that needs none of them reads
         // some other uniform), so that their latencies overlap.
-        const float ug = ring_word(w, og);
+        const uint32_t v = w + og;
+        const float ug = ring_word(v);
         float G;                    // sqrt(-2 log u); for an emission the log itself
         if (A.logtab) {
-            G = __ldg(A.logtab + (int)uniform_index(ug) - 1 + (st == S_INIT ? 0 : GAUSS_OFF));
+            G = __ldg(A.logtab + uniform_index(ug) + (st == S_INIT ? 0 : GAUSS_OFF));
         } else {
-            G = cl_logf_u<LOG_COPIES>(ug, my_tab);
+            G = cl_logf_u(ug, my_tab);
             if (st != S_INIT) G = sqrtf(-2.0f * G);
         }
         float s0, c0, s1, c1;
-        cl_sincosf_core<SC_COPIES>(TWO_PI_F * ring_word(w, og + RING_ROW), my_sctab, &s0, &c0);
-        cl_sincosf_core<SC_COPIES>(TWO_PI_F * ring_word(w, oaz), my_sctab, &s1, &c1);
+        cl_sincosf_core(TWO_PI_F * ring_word(v + RING_ROW), sc0, &s0, &c0);
+        cl_sincosf_core(TWO_PI_F * ring_word(w + oaz), sc0, &s1, &c1);
 
-        int32_t status = ST_FLYING;
         bool done = false;          // an interaction that counts as a bounce
         if (st >= S_INIT) {
             // ---- a new direction: emission, Rayleigh scatter, Lambertian lobe ----
             float c = mu;
-            if (st == S_INIT) c = 1.0f - 2.0f * ring_word(w, 0);
-            if (lamb_possible && st == S_LAMB) c = sqrtf(ring_word(w, 0));
-            const float sn = sqrtf(fmaxf(0.0f, 1.0f - c * c));
+            if (st != S_RAY) {
+                const float u = ring_word(w);
+                c = lamb_possible && st == S_LAMB ? sqrt_mid(u) : 1.0f - 2.0f * u;
+            }
+            const float sn = sqrt_mid(fmaxf(0.0f, 1.0f - c * c));
             const float a = sn * c1, b = sn * s1;
+            rng.pos += oaz + (ray_ok ? RING_ROW : 0u);
             if (st == S_RAY) {
-                rng.pos += oaz + (ray_ok ? RING_ROW : 0u);
                 if (ray_ok || ++tries >= 4096) {
                     overrun |= !ray_ok;
                     rayleigh_rotate(c, a, b, ux, uy, uz);
@@ -380,87 +449,77 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                 }
             } else if (lamb_possible && st == S_LAMB) {
                 lambertian_from(face, c, a, b, ux, uy, uz);
-                rng.pos += 2u * RING_ROW;
                 done = true;
             } else {
                 ux = a; uy = b; uz = c;
-                rng.pos += 2u * RING_ROW;
                 if (P.tau > 0.0f) { t += (-P.tau) * G; rng.pos += RING_ROW; }
                 st = S_MOVE;
             }
-        } else if (st != S_IDLE) {
+        } else if (st > 0) {
+            // ---- the step to the wall; another try (S_UNI) is a step of length 0
+            // at the wall it is on ----
+            float d, cosw;          // distance and |cos| of the incidence on the wall
+            int32_t f;
+            if (!wall_hit_fast(P, x, y, z, ux, uy, uz, d, f, cosw) && st == S_MOVE) {
+                f = wall_hit(P, x, y, z, ux, uy, uz, d);
+                cosw = fabsf(f <= 2 ? ux : (f <= 4 ? uy : uz));
+            }
+            if (st != S_MOVE) { d = 0.0f; f = face; }
+            else { tries = 0; face = f; }
+            const float u_abs = ring_word(w);
+            const float u_ray = ring_word(w + (abs_finite ? RING_ROW : 0u));
             bool hit = true;
-            float cosw = 1.0f;      // |cos| of the incidence on the wall
-            if (st == S_MOVE) {
-                // ---- the step to the wall ----
-                float d;
-                int32_t f;
-                const float u_abs = ring_word(w, 0);
-                const float u_ray = ring_word(w, abs_finite ? RING_ROW : 0);
-                if (!wall_hit_fast(P, x, y, z, ux, uy, uz, d, f, cosw)) {
-                    f = wall_hit(P, x, y, z, ux, uy, uz, d);
-                    cosw = fabsf(f <= 2 ? ux : (f <= 4 ? uy : uz));
-                }
-                rng.pos += bulk_off;
-                // no bulk interaction if each uniform is clearly below its
-                // survival probability exp(-d / length): the path length
-                // -length log u is then clearly above d
-                if (!((!abs_finite || u_abs < survive_below(d, P.abs_rate)) &&
-                      (!ray_finite || u_ray < survive_below(d, P.ray_rate)))) {
-                    const float d_abs = abs_finite ? (-P.abs_len) * uniform_log(A.logtab, u_abs, my_tab) : inf;
-                    const float d_ray = ray_finite ? (-P.ray_len) * uniform_log(A.logtab, u_ray, my_tab) : inf;
-                    if (d_abs < d && d_abs <= d_ray) {
-                        status = ST_ABS_BULK;
-                        hit = false;
-                    } else if (d_ray < d) {
-                        x += d_ray * ux; y += d_ray * uy; z += d_ray * uz;
-                        t += d_ray * P.inv_v;
-                        st = S_RAY;
-                        tries = 0;
-                        hit = false;
-                    }
-                }
-                if (hit) {
-                    // advance to the wall: clamp, then snap the hit axis (src/transport.jl:146-157)
-                    const float nx_ = x + d * ux, ny_ = y + d * uy, nz_ = z + d * uz;
-                    x = clamp_to(nx_, P.L0);
-                    y = clamp_to(ny_, P.L1);
-                    z = clamp_to(nz_, P.L2);
-                    if (f <= 2)      x = f == FACE_XP ? P.L0 : 0.0f;
-                    else if (f <= 4) y = f == FACE_YP ? P.L1 : 0.0f;
-                    else             z = f == FACE_BACK ? P.L2 : 0.0f;
-                    t += d * P.inv_v;
-                    face = f;
-                    tries = 0;
+            rng.pos += og;
+            // no bulk interaction if each uniform is clearly below its
+            // survival probability exp(-d / length): the path length
+            // -length log u is then clearly above d
+            if (!((!abs_finite || u_abs < survive_below(d, P.abs_rate)) &&
+                  (!ray_finite || u_ray < survive_below(d, P.ray_rate)))) {
+                const float d_abs = abs_finite ? (-P.abs_len) * uniform_log(A.logtab, u_abs, my_tab) : inf;
+                const float d_ray = ray_finite ? (-P.ray_len) * uniform_log(A.logtab, u_ray, my_tab) : inf;
+                if (d_abs < d && d_abs <= d_ray) {
+                    st = -ST_ABS_BULK;
+                    hit = false;
+                } else if (d_ray < d) {
+                    x += d_ray * ux; y += d_ray * uy; z += d_ray * uz;
+                    t += d_ray * P.inv_v;
+                    st = S_RAY;
+                    hit = false;
                 }
             }
             if (hit) {
-                // ---- the wall interaction; uniforms from w + og on ----
-                const unsigned char* const v = w + og;
-                const bool on_x = face <= 2, on_y = !on_x && face <= 4, on_z = face > 4;
-                const float sgn = (face & 1) ? 1.0f : -1.0f;      // outward normal component
-                const bool readout = face == FACE_BACK || (two_sided && face == FACE_FRONT);
-                bool flip = false, take = false, retry = false;
+                // advance to the wall: clamp, then snap the hit axis (src/transport.jl:146-157)
+                const bool on_x = f <= 2, on_y = !on_x && f <= 4, on_z = f > 4, outer = (f & 1) != 0;
+                const float nx_ = x + d * ux, ny_ = y + d * uy, nz_ = z + d * uz;
+                x = on_x ? (outer ? P.L0 : 0.0f) : clamp_to(nx_, P.L0);
+                y = on_y ? (outer ? P.L1 : 0.0f) : clamp_to(ny_, P.L1);
+                z = on_z ? (outer ? P.L2 : 0.0f) : clamp_to(nz_, P.L2);
+                t += d * P.inv_v;
+                // ---- the wall interaction; uniforms from v on ----
+                const float sgn = outer ? 1.0f : -1.0f;      // outward normal component
+                const bool readout = f == FACE_BACK || (two_sided && f == FACE_FRONT);
+                bool flip = false, take = false;
                 float rx = 0.f, ry = 0.f, rz = 0.f;
                 if (SPEC == SPEC_ANY && !readout && !air_gap) {
                     // front-painted wrap, src/transport.jl:186-198
                     rng.pos += RING_ROW;
-                    if (ring_word(v, 0) <= P.wrap_R) {
+                    if (ug <= P.wrap_R) {
                         if (wrap_specular) flip = true;
                         else st = S_LAMB;
                     } else {
-                        status = ST_ABS_WALL;
+                        st = -ST_ABS_WALL;
                     }
                 } else {
                     // UNIFIED facet (src/optics.jl:55-66); a readout lane computes
                     // one too and does not use it
                     const bool facet = uni_possible && !readout;
+                    bool retry = false;
                     float Nfx = 0.f, Nfy = 0.f, Nfz = 0.f, fcos = cosw;
                     uint32_t fo = 0;             // offset of the Fresnel uniform
                     if (uni_possible) {
                         const float alpha = P.sigma_alpha * fabsf(G * c0);
                         float sa, ca;
-                        cl_sincosf_core<SC_COPIES>(fminf(alpha, 1.2f), my_sctab, &sa, &ca);
+                        cl_sincosf_core(fminf(alpha, 1.2f), sc0, &sa, &ca);
                         const float b = sa * c1, c = sa * s1, n = ca * sgn;
                         Nfx = on_x ? n : b;
                         Nfy = on_y ? n : (on_x ? b : c);
@@ -474,42 +533,33 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                         }
                     }
                     // Fresnel (src/optics.jl:10-19)
-                    const float n2 = readout ? P.n_coupling : 1.0f;
                     const float sin2t = (readout ? P.qc2 : P.qa2) * (1.0f - fcos * fcos);
-                    const float uf = ring_word(v, fo), un = ring_word(v, fo + RING_ROW);
-                    const bool tir = sin2t >= 1.0f;
-                    bool refl = tir;
-                    if (!tir) refl = fresnel_reflects(P, n2, sin2t, fcos, uf);
-                    rng.pos += fo + (retry || tir ? 0u : (refl ? RING_ROW : 2u * RING_ROW));
+                    const float uf = ring_word(v + fo), un = ring_word(v + fo + RING_ROW);
+                    const bool refl = fresnel_reflects(P, readout ? P.n_coupling : 1.0f, sin2t, fcos, uf);
+                    rng.pos += fo + (retry || sin2t >= 1.0f ? 0u : (refl ? RING_ROW : 2u * RING_ROW));
                     // facet reflection, kept only if it points back into the
                     // crystal (src/optics.jl:68-77)
                     rx = ux - (2.0f * fcos) * Nfx;
                     ry = uy - (2.0f * fcos) * Nfy;
                     rz = uz - (2.0f * fcos) * Nfz;
                     const bool inward = sgn * (on_x ? rx : (on_y ? ry : rz)) < 0.0f;
-                    const bool through = !refl && !retry;
                     take = facet && refl && !retry && inward;
-                    retry |= facet && refl && !inward;
                     flip = !facet && refl;
-                    if (through) {
-                        if (readout) {
-                            if (!disc || (x - P.cx) * (x - P.cx) + (y - P.cy) * (y - P.cy) <= P.r2) {
-                                status = un <= P.pde ? ST_DETECTED : ST_ABS_SIPM;
-                            } else if (un <= P.sur_R) {
-                                if (P.sur_specular) flip = true;
-                                else st = S_LAMB;
-                            } else {
-                                status = ST_ABS_SUR;
-                            }
-                        } else if (un <= P.wrap_R) {
-                            // the reflector behind the air gap (src/transport.jl:214-225)
-                            if (wrap_specular) flip = true;
+                    if (!refl && !retry) {
+                        // through the interface: a SiPM or its surround, or the
+                        // reflector behind the air gap (src/transport.jl:161-225)
+                        const bool sipm = readout && (!disc || (x - P.cx) * (x - P.cx) + (y - P.cy) * (y - P.cy) <= P.r2);
+                        const bool kept = un <= (sipm ? P.pde : (SPEC == SPEC_ANY && readout ? P.sur_R : P.wrap_R));
+                        if (sipm) {
+                            st = kept ? -ST_DETECTED : -ST_ABS_SIPM;
+                        } else if (kept) {
+                            if (SPEC == SPEC_ANY && readout ? P.sur_specular : wrap_specular) flip = true;
                             else st = S_LAMB;
                         } else {
-                            status = ST_ABS_WALL;
+                            st = SPEC == SPEC_ANY && readout ? -ST_ABS_SUR : -ST_ABS_WALL;
                         }
                     }
-                    if (retry) {
+                    if (retry || (facet && refl && !inward)) {
                         if (++tries >= 20) flip = true;
                         else st = S_UNI;
                     }
@@ -524,80 +574,7 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
         // end of an interaction: count the bounce (src/transport.jl:228-232)
         if (done) {
             bounces += 1;
-            if (bounces >= P.max_bounces) status = ST_CAP;
-            st = S_MOVE;
-        }
-
-        // ---- terminal bookkeeping ----
-        const bool term = status != ST_FLYING;
-        const unsigned tmask = __ballot_sync(FULL, term);
-        if (tmask != 0u) {
-            const bool det = status == ST_DETECTED;
-            int32_t idx = 0;
-            if (det) {
-                int32_t ii = 1 + (int32_t)(x / P.pitch);
-                int32_t jj = 1 + (int32_t)(y / P.pitch);
-                ii = ii < P.nx ? ii : P.nx;
-                jj = jj < P.ny ? jj : P.ny;
-                const int32_t lin = (jj - 1) * P.nx + ii;
-                idx = two_sided && face == FACE_FRONT ? -lin : lin;
-                const int32_t cell = lin - 1;
-                const uint32_t key = float_key(t);
-                // one reduction per photon: a warp seldom detects two photons in
-                // the same slot, and finding out costs more than it saves
-                if (MODE == 0) {
-                    atomicAdd(tile_counts + cell + A.cells * time_bin0(t, P), 1u);
-                    // the 64 keys are hot; most photons are later than the key
-                    // already there (which only ever falls)
-                    if (key < (TILE ? tile_keys[cell] : __ldcg(tile_keys + cell))) atomicMin(tile_keys + cell, key);
-                } else {
-                    // a segment id outside the maps (untrusted device input) drops the detection
-                    if (seg >= 0 && (int64_t)seg < A.n_seg) {
-                        const unsigned long long slot =
-                            (unsigned long long)seg * (unsigned long long)A.cells + (unsigned long long)cell;
-                        atomicAdd(A.maps + slot, 1u);
-                        atomicMin(A.keys + slot, key);
-                        if (MODE == 2) {
-                            // fixed-point time moments (exact integer sums, order-independent)
-                            const float tc = fminf(fmaxf(t, 0.0f), CL_MOMENT_T_MAX_NS);
-                            atomicAdd(A.tsum + slot, __float2ull_rn(tc * CL_MOMENT_T_SCALE));
-                            atomicAdd(A.tsum2 + slot, __float2ull_rn((tc * tc) * CL_MOMENT_T2_SCALE));
-                        }
-                    } else {
-                        atomicOr(A.err, 16u);
-                    }
-                }
-            }
-            if (REC && term) {
-                const uint64_t k = (((uint64_t)rng.pid_hi << 32) | rng.pid_lo) - A.pid0 - 1ull;
-                if (A.r_status) A.r_status[k] = (uint8_t)status;
-                if (A.r_idx) A.r_idx[k] = (int16_t)idx;
-                if (A.r_t) A.r_t[k] = t;
-                if (A.r_bounces) A.r_bounces[k] = bounces;
-            }
-            // counters: the fates in five 6-bit fields of one reduction (the
-            // caps are what is left of the terminated lanes), the sums one each;
-            // lane i adds entry i of the warp's own counters
-            const uint32_t field = det ? 1u : (status == ST_ABS_SUR ? 1u << 24 : 1u << (6 * ((status - 1) & 3)));
-            const uint32_t fates = __reduce_add_sync(FULL, term && status != ST_CAP ? field : 0u);
-            const uint32_t front = two_sided ? (uint32_t)__popc(__ballot_sync(FULL, det && idx < 0)) : 0u;
-            const uint32_t sb = __reduce_add_sync(FULL, det ? (uint32_t)bounces : 0u);
-            const uint32_t sc = __reduce_add_sync(FULL, term ? (uint32_t)nscat : 0u);
-            const uint32_t ss = __reduce_add_sync(FULL, term ? (uint32_t)(bounces + (status != ST_CAP)) : 0u);
-            if (lane < N_COUNTERS) {
-                // ndet, ndet_front, bulk, wall, sipm, cap, sur, nscat, sum_bounces_det, steps
-                uint32_t add = fates & 63u;
-                if (lane == 1) add = front;
-                if (lane >= 2 && lane <= 4) add = (fates >> (6 * (lane - 1))) & 63u;
-                if (lane == 5) add = (uint32_t)__popc(tmask) - (fates & 63u) - ((fates >> 6) & 63u) -
-                                     ((fates >> 12) & 63u) - ((fates >> 18) & 63u) - (fates >> 24);
-                if (lane == 6) add = fates >> 24;
-                if (lane == 7) add = sc;
-                if (lane == 8) add = sb;
-                if (lane == 9) add = ss;
-                my_cnt[lane] += (unsigned long long)add;
-            }
-            if (term) st = S_IDLE;
+            st = bounces >= P.max_bounces ? -ST_CAP : S_MOVE;
         }
     }
     if (overrun) atomicOr(A.err, 1u);
@@ -661,10 +638,10 @@ __global__ void logtab_fill(float* t)
     double2 *s_tab, *s_sctab;
     load_tables(smem, s_tab, s_sctab);
     __syncthreads();
-    const double2* my_tab = s_tab + (threadIdx.x % LOG_COPIES);
+    const double2* my_tab = s_tab;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < (1u << 24); k += gridDim.x * blockDim.x)
     {
-        const float l = cl_logf_u<LOG_COPIES>(u32_to_randu(k << 8), my_tab);
+        const float l = cl_logf_u(u32_to_randu(k << 8), my_tab);
         t[k] = l;
         t[GAUSS_OFF + k] = sqrtf(-2.0f * l);
     }
@@ -703,13 +680,58 @@ __global__ void debug_math_kernel(int fn, const float* in, float* out, int64_t n
         const float x = in[i];
         float r;
         if (fn == 0) {
-            r = cl_logf<LOG_COPIES>(x, s_tab + (threadIdx.x % LOG_COPIES));
+            r = cl_logf(x, s_tab);
         } else {
             float sv, cv;
-            cl_sincosf<SC_COPIES>(x, s_sctab + (threadIdx.x % SC_COPIES), &sv, &cv);
+            cl_sincosf(x, smem_addr(s_sctab), &sv, &cv);
             r = fn == 1 ? sv : cv;
         }
         out[i] = r;
+    }
+}
+
+// The loop's quick decisions beside the exact expressions (items of `ni` input
+// and `no` output floats):
+//   7  x -> sqrt_mid(x)                       8  x -> rcp_mid(x)
+//   9  (x, y, z, ux, uy, uz, Lx, Ly, Lz) -> quick distance and face (0: undecided), exact distance and face
+//  10  (n1, n2, cosi, u) -> quick and exact "reflects" (total reflection included)
+//  11  (u, d, length) -> 1 if the quick test rules a bulk event out, exact -length log u
+__global__ void debug_step_kernel(int fn, const float* in, float* out, int64_t n)
+{
+    __shared__ __align__(16) unsigned char tabs[LOGTAB_BYTES];
+    double2 *s_tab, *s_sctab;
+    load_tables(tabs, s_tab, s_sctab);
+    __syncthreads();
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        if (fn == 7) out[i] = sqrt_mid(in[i]);
+        if (fn == 8) out[i] = rcp_mid(in[i]);
+        if (fn == 9) {
+            const float* q = in + 9 * i;
+            Physics P;
+            P.L0 = q[6]; P.L1 = q[7]; P.L2 = q[8];
+            float d, cosw;
+            int32_t f;
+            const bool ok = wall_hit_fast(P, q[0], q[1], q[2], q[3], q[4], q[5], d, f, cosw);
+            out[4 * i] = d;
+            out[4 * i + 1] = ok ? (float)f : 0.0f;
+            out[4 * i + 3] = (float)wall_hit(P, q[0], q[1], q[2], q[3], q[4], q[5], d);
+            out[4 * i + 2] = d;
+        }
+        if (fn == 10) {
+            const float* q = in + 4 * i;
+            Physics P;
+            P.n_crystal = q[0];
+            P.fresnel_margin = fresnel_margin(q[0], q[1]);
+            const float r = q[0] / q[1], sin2t = (r * r) * (1.0f - q[2] * q[2]);
+            out[2 * i] = fresnel_reflects(P, q[1], sin2t, q[2], q[3]) ? 1.0f : 0.0f;
+            out[2 * i + 1] = sin2t >= 1.0f || q[3] < fresnel_R(q[0], q[1], sin2t, q[2]) ? 1.0f : 0.0f;
+        }
+        if (fn == 11) {
+            const float* q = in + 3 * i;
+            out[2 * i] = q[0] < survive_below(q[1], survive_rate(q[2])) ? 1.0f : 0.0f;
+            out[2 * i + 1] = (-q[2]) * cl_logf_u(q[0], s_tab);
+        }
     }
 }
 
@@ -990,15 +1012,9 @@ static Physics make_physics(const cl_box* box, const cl_optical_params* op, cons
         P.qc2 = qc * qc;
         P.qa2 = qa * qa;
     }
-    // rates of the bulk competition's quick test; NaN (no or a negative length)
-    // fails it, so those runs take the exact comparison
-    auto rate = [](float len) { return len > 0.0f ? (float)(-1.4426950408889634 / (double)len) : NAN; };
-    P.abs_rate = rate(op->abs_len_mm);
-    P.ray_rate = rate(op->rayleigh_mm);
-    // the quick Fresnel test's error bound holds for indices of this range
-    const bool plain = op->n_crystal >= 1e-3f && op->n_crystal <= 1e3f && op->n_coupling >= 1e-3f &&
-                       op->n_coupling <= 1e3f;
-    P.fresnel_margin = plain ? 0x1p-17f : INFINITY;
+    P.abs_rate = survive_rate(op->abs_len_mm);
+    P.ray_rate = survive_rate(op->rayleigh_mm);
+    P.fresnel_margin = fresnel_margin(op->n_crystal, op->n_coupling);
     P.abs_finite = std::isfinite(op->abs_len_mm) ? 1 : 0;
     P.ray_finite = std::isfinite(op->rayleigh_mm) ? 1 : 0;
     P.wrap_specular = op->wrap_specular ? 1 : 0;
@@ -1499,7 +1515,7 @@ int cl_debug_eval(cl_handle* h, int fn, const void* in, void* out, int64_t n, ui
     if (!h) return CL_ERR_STATE;
     h->err[0] = 0;
     if (n < 0 || !out || (fn != 4 && fn != 6 && !in)) return set_err(h, CL_ERR_ARG, "bad debug arguments");
-    if (fn < 0 || fn > 6) return set_err(h, CL_ERR_ARG, "unknown debug function");
+    if (fn < 0 || fn > 11) return set_err(h, CL_ERR_ARG, "unknown debug function");
     if (fn == 4 && n_per < 1) return set_err(h, CL_ERR_ARG, "n_per must be >= 1");
     CK(h, cudaSetDevice(h->device), "cudaSetDevice");
     cudaStream_t st = h->stream;
@@ -1514,6 +1530,11 @@ int cl_debug_eval(cl_handle* h, int fn, const void* in, void* out, int64_t n, ui
     size_t in_b = 0, out_b = 0;
     if (fn <= 2) { in_b = 4 * (size_t)n; out_b = 4 * (size_t)n; }
     else if (fn == 3 || fn == 5) { in_b = 16 * (size_t)n; out_b = 16 * (size_t)n; }
+    else if (fn >= 7) {
+        constexpr size_t ni[5] = {1, 1, 9, 4, 3}, no[5] = {1, 1, 4, 2, 2};
+        in_b = 4 * ni[fn - 7] * (size_t)n;
+        out_b = 4 * no[fn - 7] * (size_t)n;
+    }
     else { out_b = 4 * (size_t)n * (size_t)n_per; }
     int rc = ensure(h, h->dbg, align256(in_b) + align256(out_b) + 256);
     if (rc != CL_OK) return rc;
@@ -1526,6 +1547,7 @@ int cl_debug_eval(cl_handle* h, int fn, const void* in, void* out, int64_t n, ui
         if (fn <= 2) debug_math_kernel<<<grid, 256, 0, st>>>(fn, (const float*)din, (float*)dout, n);
         else if (fn == 3 || fn == 5)
             debug_philox_kernel<<<grid, 256, 0, st>>>(fn == 5, (const uint32_t*)din, (uint32_t*)dout, n, k0, k1);
+        else if (fn >= 7) debug_step_kernel<<<grid, 256, 0, st>>>(fn, (const float*)din, (float*)dout, n);
         else debug_randu_kernel<<<grid, 256, 0, st>>>((float*)dout, n, n_per, k0, k1);
         CK(h, cudaGetLastError(), "debug kernel launch");
     }

@@ -251,6 +251,14 @@ class Engine:
         self._check(self.lib.cl_debug_eval(self.handle, 6, None, _ptr(out), int(n), 0, 0))
         return out
 
+    def eval_step(self, fn: int, x: np.ndarray) -> np.ndarray:
+        """The transport loop's quick decisions beside the exact expressions
+        (cl_debug_eval functions 7..11): x (n, inputs) -> (n, outputs), float32."""
+        x = np.ascontiguousarray(x, np.float32)
+        out = np.empty((x.shape[0], {7: 1, 8: 1, 9: 4, 10: 2, 11: 2}[fn]), np.float32)
+        self._check(self.lib.cl_debug_eval(self.handle, fn, _ptr(x), _ptr(out), x.shape[0], 0, 0))
+        return out
+
     def philox(self, ctr: np.ndarray, seed: int, use_curand: bool = False) -> np.ndarray:
         ctr = np.ascontiguousarray(ctr, dtype=np.uint32).reshape(-1, 4)
         out = np.empty_like(ctr)
