@@ -39,6 +39,8 @@ namespace cl {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int GAUSS_OFF = 1 << 24;    // sqrt(-2 log u) after the 2^24 logs
 constexpr int N_COUNTERS = 10;        // cl_counters, then the photon-steps
+constexpr int SPREAD_WARPS = 8;        // warps per SM of a launch of few photons
+constexpr size_t CTA_EXTRA_SMEM = 1024 + 8 * N_COUNTERS * 8 + 16;   // reserved and static shared memory of a CTA
 constexpr int SCTAB_BYTES = CLM_SC_N * 16;
 constexpr int LOGTAB_BYTES = ((CLM_LOG_NTAB * 16 + 127) / 128) * 128 + SCTAB_BYTES;  // both tables
 
@@ -1062,20 +1064,32 @@ static int launch_transport_spec(cl_handle* h, const KArgs& a, size_t smem, cuda
     if (h->ctas_per_sm > 0 && h->ctas_per_sm < per_sm) per_sm = h->ctas_per_sm;
     int64_t grid = (int64_t)h->num_sms * per_sm;
     KArgs b = a;
+    int threads = h->threads;
     if (b.warp_chunk <= 0) {
         // automatic: the largest chunk (fewest queue atomics) that still gives
         // every resident warp about CL_CHUNKS_PER_WARP chunks, so the end of
         // the queue stays balanced; between 32 and CL_MAX_WARP_CHUNK photons
-        const int64_t warps = grid * (h->threads / 32);
+        const int64_t warps = grid * (threads / 32);
         int64_t c = a.n / (warps * CL_CHUNKS_PER_WARP);
         c = c < 32 ? 32 : (c > CL_MAX_WARP_CHUNK ? CL_MAX_WARP_CHUNK : c);
         b.warp_chunk = (int32_t)(c & ~(int64_t)31);
+        // fewer photons than two warps per scheduler hold: spread them over that
+        // many warps, some lanes each.  The time is the longest photon's chain
+        // of steps, and a warp with few lanes runs fewer of a step's branches:
+        // CsI(Tl) 2,000 photons 271 -> 245 us, 20,000 294 -> 285 us, BGO 500
+        // photons 946 -> 849 us; with 4 warps per SM 8,000 photons take 262 us
+        // instead of 257, with 16 269 us
+        const int64_t spread = (int64_t)h->num_sms * SPREAD_WARPS;
+        if (a.n < spread * 32 && threads >= 128) {
+            b.warp_chunk = (int32_t)((a.n + spread - 1) / spread);
+            threads = 128;
+        }
     }
     // no more CTAs than warps' worth of first chunks
     const int64_t warps_needed = (b.n + b.warp_chunk - 1) / b.warp_chunk;
-    const int64_t ctas_needed = (warps_needed + (h->threads / 32) - 1) / (h->threads / 32);
+    const int64_t ctas_needed = (warps_needed + (threads / 32) - 1) / (threads / 32);
     if (grid > ctas_needed) grid = ctas_needed > 0 ? ctas_needed : 1;
-    kern<<<(unsigned)grid, h->threads, smem, st>>>(b);
+    kern<<<(unsigned)grid, threads, smem, st>>>(b);
     CK(h, cudaGetLastError(), "transport kernel launch");
     return CL_OK;
 }
@@ -1126,7 +1140,7 @@ static int enqueue_point(cl_handle* h, const Physics& P, const float* px, const 
     // costs more than the tile saves in global atomics (10^6-photon point
     // source, 8x8x81 bins: 879 M photons/s on global atomics at 4 CTAs/SM,
     // 843 M with the tile at 3)
-    const size_t per_cta = base_bytes + tile_bytes + 1024;
+    const size_t per_cta = base_bytes + tile_bytes + CTA_EXTRA_SMEM;
     const bool tile = base_bytes + tile_bytes <= (size_t)std::min(h->max_smem_optin, 160 * 1024) &&
                       4 * per_cta <= (size_t)h->max_smem_per_sm;
     const size_t smem = base_bytes + (tile ? tile_bytes : 0);
