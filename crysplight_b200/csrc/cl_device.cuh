@@ -106,6 +106,8 @@ __device__ __forceinline__ int32_t rng_level(const Rng& r)
 {
     return (int32_t)(r.block * (4u * RING_ROW) - r.pos);
 }
+// A lane without a photon: neither short of uniforms nor with room for more.
+__device__ __forceinline__ void rng_park(Rng& r) { r.pos = (r.block * 4u - 28u) * RING_ROW; }
 __device__ __forceinline__ bool rng_short(const Rng& r) { return rng_level(r) <= (DRAWS_PER_ITER - 1) * (int32_t)RING_ROW; }
 __device__ __forceinline__ bool rng_room(const Rng& r) { return rng_level(r) <= 24 * (int32_t)RING_ROW; }
 __device__ __forceinline__ bool rng_under(const Rng& r) { return rng_level(r) <= -(int32_t)RING_ROW; }
@@ -362,7 +364,7 @@ __device__ __forceinline__ float rcp_mid(float x)
 }
 
 // fresnel, src/optics.jl:10-19, where sin2t = (n1/n2)^2 (1 - cosi^2) < 1.
-__device__ __forceinline__ float fresnel_R(float n1, float n2, float sin2t, float cosi)
+static __device__ __noinline__ float fresnel_R(float n1, float n2, float sin2t, float cosi)
 {
     const float cost = sqrtf(1.0f - sin2t);
     const float a = (n1 * cosi - n2 * cost) / (n1 * cosi + n2 * cost);
@@ -430,7 +432,7 @@ __device__ __forceinline__ float axis_distance(float L, float p, float u)
 }
 
 // wall_hit, src/geometry.jl:19-32.
-__device__ __forceinline__ int32_t wall_hit(const Physics& P, float x, float y, float z,
+static __device__ __noinline__ int32_t wall_hit(const Physics& P, float x, float y, float z,
                                             float ux, float uy, float uz, float& d)
 {
     const float dx = axis_distance(P.L0, x, ux);

@@ -107,8 +107,15 @@ __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v)
     return v;
 }
 
+// The position of photon k (src/kernel.jl:171); out of line, it is a 64-bit division.
+static __device__ __noinline__ int32_t position_of(int64_t k, int32_t npos) { return (int32_t)((uint64_t)k % (uint64_t)npos); }
+
+// Rare paths of the transport kernel (these, wall_hit, fresnel_R) are functions
+// of their own: inlined, they cost the loop registers and instruction-cache
+// room.  Scan 98.0 -> 96.7 (wall_hit, fresnel_R) -> 93.5 ms (find_source),
+// 3,001 events 20.2 -> 19.9 -> 19.3 ms.
 // Galloping search: largest s >= hint with off[s] <= k (off[n_src] = total).
-__device__ __forceinline__ int64_t find_source(const int64_t* __restrict__ off, int64_t n_src,
+static __device__ __noinline__ int64_t find_source(const int64_t* __restrict__ off, int64_t n_src,
                                                int64_t hint, int64_t k)
 {
     int64_t lo = hint, step = 1;
@@ -160,12 +167,13 @@ enum : int32_t {
 // CsI(Tl)+Teflon run files; SPEC_ANY reads every flag from the parameters.
 enum : int { SPEC_ANY = 0, SPEC_ESR = 1, SPEC_TEFLON = 2 };
 
-// log of a uniform u = k 2^-24 from the table (k in 1..2^24 at [k - 1]), or
-// evaluated where there is no table.
+// log u and sqrt(-2 log u) of a uniform u = k 2^-24: from the tables, or (TAB
+// false) evaluated in place.
 __device__ __forceinline__ int uniform_index(float u) { return (int)(u * 16777216.0f) - 1; }
+template <bool TAB>
 __device__ __forceinline__ float uniform_log(const float* __restrict__ tab, float u, const double2* __restrict__ logtab)
 {
-    return tab ? __ldg(tab + uniform_index(u)) : cl_logf_u(u, logtab);
+    return TAB ? __ldg(tab + uniform_index(u)) : cl_logf_u(u, logtab);
 }
 
 // The loop computes what decides a photon's next step exactly and everything
@@ -187,7 +195,7 @@ __device__ __forceinline__ float uniform_log(const float* __restrict__ tab, floa
 // (31.2 -> 20.4 warp instructions per photon-step): BGO+ESR scan of 51.2M
 // photons 143.9 -> 100.4 ms (49 G photon-steps/s), 3,001 CsI(Tl)+Teflon events
 // 32.6 -> 20.6 ms, 10^6-photon CsI(Tl) point 1.17 -> 0.79 ms.
-template <int MODE, bool REC, bool TILE, int SPEC>
+template <int MODE, bool REC, bool TILE, int SPEC, bool TAB>
 __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(const __grid_constant__ KArgs A)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -224,7 +232,6 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
     unsigned long long* my_cnt = s_cnt[tid >> 5];
 
     const unsigned lt_mask = (1u << lane) - 1u;
-    const double2* my_tab = s_tab;
     const uint32_t sc0 = smem_addr(smem), ring0 = sc0 + LOGTAB_BYTES;
     const bool air_gap = SPEC != SPEC_ANY || P.air_gap;
     const bool uni_possible = SPEC != SPEC_ANY || (P.air_gap && P.sigma_alpha > 0.0f);
@@ -244,6 +251,7 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
     int32_t bounces = 0, nscat = 0, st = S_IDLE, face = 1, tries = 0;
     Rng rng;
     rng_init(rng, 0);
+    rng_park(rng);
     int32_t seg = 0;
     // warp-uniform work pool
     int64_t pool_lo = 0, pool_hi = 0, pool_src = 0;
@@ -327,7 +335,10 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                     if (lane == 9) add = ss;
                     my_cnt[lane] += (unsigned long long)add;
                 }
-                if (st < 0) st = S_IDLE;
+                if (st < 0) {
+                    st = S_IDLE;
+                    rng_park(rng);
+                }
             }
             if (!exhausted) {
                 const unsigned need = __ballot_sync(FULL, st == S_IDLE);
@@ -366,7 +377,7 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                 }
                 if (my_k >= 0) {
                     if (MODE == 0) {
-                        const int32_t j = A.npos == 1 ? 0 : (int32_t)((uint64_t)my_k % (uint64_t)A.npos);
+                        const int32_t j = A.npos == 1 ? 0 : position_of(my_k, A.npos);
                         x = __ldg(A.px + j); y = __ldg(A.py + j); z = __ldg(A.pz + j);
                         t = A.pt ? __ldg(A.pt + j) : 0.0f;
                     } else {
@@ -388,18 +399,18 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
         }
 
         // ---- top up the uniform ring: one Philox call site for the warp ----
-        if (__any_sync(FULL, st > 0 && rng_short(rng))) {
+        if (__any_sync(FULL, rng_short(rng))) {
             // every lane with room tops up at this convergent point, so later
             // iterations need the fill less often
             under |= rng_under(rng);
-            if (st > 0 && rng_room(rng)) rng_fill(rng, ring0, P.rk);
+            if (rng_room(rng)) rng_fill(rng, ring0, P.rk);
         }
 
         // ---- draws: this iteration's uniforms at fixed offsets ----
         const uint32_t w = ring0 + (rng.pos & RING_MASK);
         // the table lookup (tilt's gaussian, or the emission time's log) and the azimuth
         const uint32_t og = st == S_MOVE ? bulk_off : (st == S_INIT ? 2u * RING_ROW : 0u);
-        uint32_t oaz = st == S_MOVE ? bulk_off + 2u * RING_ROW : (st == S_UNI ? 2u * RING_ROW : RING_ROW);
+        uint32_t oaz = st <= S_UNI ? og + 2u * RING_ROW : RING_ROW;
         float mu = 0.0f;
         bool ray_ok = true;
         if (st == S_RAY) {
@@ -421,10 +432,10 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
         const uint32_t v = w + og;
         const float ug = ring_word(v);
         float G;                    // sqrt(-2 log u); for an emission the log itself
-        if (A.logtab) {
+        if (TAB) {
             G = __ldg(A.logtab + uniform_index(ug) + (st == S_INIT ? 0 : GAUSS_OFF));
         } else {
-            G = cl_logf_u(ug, my_tab);
+            G = cl_logf_u(ug, s_tab);
             if (st != S_INIT) G = sqrtf(-2.0f * G);
         }
         float s0, c0, s1, c1;
@@ -477,8 +488,8 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
             // -length log u is then clearly above d
             if (!((!abs_finite || u_abs < survive_below(d, P.abs_rate)) &&
                   (!ray_finite || u_ray < survive_below(d, P.ray_rate)))) {
-                const float d_abs = abs_finite ? (-P.abs_len) * uniform_log(A.logtab, u_abs, my_tab) : inf;
-                const float d_ray = ray_finite ? (-P.ray_len) * uniform_log(A.logtab, u_ray, my_tab) : inf;
+                const float d_abs = abs_finite ? (-P.abs_len) * uniform_log<TAB>(A.logtab, u_abs, s_tab) : inf;
+                const float d_ray = ray_finite ? (-P.ray_len) * uniform_log<TAB>(A.logtab, u_ray, s_tab) : inf;
                 if (d_abs < d && d_abs <= d_ray) {
                     st = -ST_ABS_BULK;
                     hit = false;
@@ -640,10 +651,9 @@ __global__ void logtab_fill(float* t)
     double2 *s_tab, *s_sctab;
     load_tables(smem, s_tab, s_sctab);
     __syncthreads();
-    const double2* my_tab = s_tab;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < (1u << 24); k += gridDim.x * blockDim.x)
     {
-        const float l = cl_logf_u(u32_to_randu(k << 8), my_tab);
+        const float l = cl_logf_u(u32_to_randu(k << 8), s_tab);
         t[k] = l;
         t[GAUSS_OFF + k] = sqrtf(-2.0f * l);
     }
@@ -835,21 +845,34 @@ static inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Allow dynamic shared memory up to the opt-in limit minus the kernel's
 // static shared memory (their sum may not exceed the limit).
-template <int MODE, bool REC, bool TILE, int SPEC>
+template <int MODE, bool REC, bool TILE, int SPEC, bool TAB>
 static void set_kernel_attrs_spec(int smem_optin)
 {
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, transport_kernel<MODE, REC, TILE, SPEC>) != cudaSuccess) return;
-    cudaFuncSetAttribute(transport_kernel<MODE, REC, TILE, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncGetAttributes(&fa, transport_kernel<MODE, REC, TILE, SPEC, TAB>) != cudaSuccess) return;
+    cudaFuncSetAttribute(transport_kernel<MODE, REC, TILE, SPEC, TAB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          smem_optin - (int)fa.sharedSizeBytes);
 }
+
+// Kernels that evaluate the logs in place serve the allocation-free entry point
+// (point mode without records) in every configuration, and a handle whose
+// tables could not be allocated in the general one.  One kernel for both carried
+// the evaluation in the loop: scan 100.4 -> 98.0 ms, 3,001 events 20.6 -> 20.2 ms
+// without it.
+template <int MODE, bool REC>
+constexpr bool spec_without_tables = MODE == 0 && !REC;
 
 template <int MODE, bool REC, bool TILE>
 static void set_kernel_attrs(int smem_optin)
 {
-    set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ANY>(smem_optin);
-    set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ESR>(smem_optin);
-    set_kernel_attrs_spec<MODE, REC, TILE, SPEC_TEFLON>(smem_optin);
+    set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ANY, true>(smem_optin);
+    set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ESR, true>(smem_optin);
+    set_kernel_attrs_spec<MODE, REC, TILE, SPEC_TEFLON, true>(smem_optin);
+    set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ANY, false>(smem_optin);
+    if constexpr (spec_without_tables<MODE, REC>) {
+        set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ESR, false>(smem_optin);
+        set_kernel_attrs_spec<MODE, REC, TILE, SPEC_TEFLON, false>(smem_optin);
+    }
 }
 
 extern "C" {
@@ -1054,10 +1077,10 @@ static int spec_of(const Physics& P)
     return P.wrap_specular ? SPEC_ESR : SPEC_TEFLON;
 }
 
-template <int MODE, bool REC, bool TILE, int SPEC>
+template <int MODE, bool REC, bool TILE, int SPEC, bool TAB>
 static int launch_transport_spec(cl_handle* h, const KArgs& a, size_t smem, cudaStream_t st)
 {
-    auto kern = transport_kernel<MODE, REC, TILE, SPEC>;
+    auto kern = transport_kernel<MODE, REC, TILE, SPEC, TAB>;
     int per_sm = 0;
     CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, h->threads, smem), "occupancy");
     if (per_sm < 1) return set_err(h, CL_ERR_ARG, "transport kernel does not fit on an SM (shared tile too large)");
@@ -1097,10 +1120,18 @@ static int launch_transport_spec(cl_handle* h, const KArgs& a, size_t smem, cuda
 template <int MODE, bool REC, bool TILE>
 static int launch_transport(cl_handle* h, const KArgs& a, size_t smem, cudaStream_t st)
 {
-    switch (spec_of(a.P)) {
-    case SPEC_ESR: return launch_transport_spec<MODE, REC, TILE, SPEC_ESR>(h, a, smem, st);
-    case SPEC_TEFLON: return launch_transport_spec<MODE, REC, TILE, SPEC_TEFLON>(h, a, smem, st);
-    default: return launch_transport_spec<MODE, REC, TILE, SPEC_ANY>(h, a, smem, st);
+    const int spec = spec_of(a.P);
+    if (!a.logtab) {
+        if constexpr (spec_without_tables<MODE, REC>) {
+            if (spec == SPEC_ESR) return launch_transport_spec<MODE, REC, TILE, SPEC_ESR, false>(h, a, smem, st);
+            if (spec == SPEC_TEFLON) return launch_transport_spec<MODE, REC, TILE, SPEC_TEFLON, false>(h, a, smem, st);
+        }
+        return launch_transport_spec<MODE, REC, TILE, SPEC_ANY, false>(h, a, smem, st);
+    }
+    switch (spec) {
+    case SPEC_ESR: return launch_transport_spec<MODE, REC, TILE, SPEC_ESR, true>(h, a, smem, st);
+    case SPEC_TEFLON: return launch_transport_spec<MODE, REC, TILE, SPEC_TEFLON, true>(h, a, smem, st);
+    default: return launch_transport_spec<MODE, REC, TILE, SPEC_ANY, true>(h, a, smem, st);
     }
 }
 
