@@ -83,7 +83,6 @@ constexpr uint32_t WAIT_BUDGET = 1u << 22;   // polls before a wait gives up
 enum Epi : int {
     EPI_F32 = 0,         // out_f[m][n] = acc
     EPI_BIAS_SILU = 1,   // z = acc + b: out_z = bf16(z), out_h = bf16(silu z)
-    EPI_BIAS_F32 = 2,    // out_f[m][n] = acc + b
     EPI_DSILU = 3,       // g = bf16(acc * silu'(zprev)): out_h, colsum += column sums of g
     EPI_PARTIAL = 4,     // out_f[split][m][n] = acc (split-K partial)
     EPI_LOSS = 5,        // o = acc + b, d = o - target: loss += scale d^2, g = bf16(2 scale d) -> out_h, colsum
@@ -102,7 +101,7 @@ struct EpiCfg {
     static constexpr int tiles = (EPI == EPI_BIAS_SILU || EPI == EPI_LOSS || EPI == EPI_DSILU) ? 2
                                  : EPI == EPI_DSILU_L1 ? 1 : 0;
     static constexpr int stages = tiles ? 3 : 4;
-    static constexpr bool bias = EPI == EPI_BIAS_SILU || EPI == EPI_BIAS_F32 || EPI == EPI_LOSS ||
+    static constexpr bool bias = EPI == EPI_BIAS_SILU || EPI == EPI_LOSS ||
                                  EPI == EPI_DSILU_L1;
     static constexpr int cst = EPI == EPI_DSILU_L1 ? 4 * 256 : (bias ? 256 : 4);
     // CTA accumulators of the column sums (bias gradient; for EPI_DSILU_L1
@@ -298,19 +297,12 @@ __device__ __forceinline__ void epilogue(const GemmArgs& G, const OutMaps& om, u
             float* o = G.out_f + (int64_t)c0 * G.ldf + row;
 #pragma unroll
             for (int i = 0; i < 32; ++i) atomicAdd(o + (int64_t)i * G.ldf, v[i]);
-        } else if (EPI == EPI_F32 || EPI == EPI_BIAS_F32 || EPI == EPI_PARTIAL) {
+        } else if (EPI == EPI_F32 || EPI == EPI_PARTIAL) {
             float* o = G.out_f + (EPI == EPI_PARTIAL ? (int64_t)blockIdx.y * G.M * G.ldf : 0) +
                        (int64_t)row * G.ldf + c0;
 #pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                float b[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                if (EPI == EPI_BIAS_F32) cst8(cst + c0 + 8 * g, b);
-                float4 q0, q1;
-                q0.x = v[8 * g] + b[0]; q0.y = v[8 * g + 1] + b[1]; q0.z = v[8 * g + 2] + b[2]; q0.w = v[8 * g + 3] + b[3];
-                q1.x = v[8 * g + 4] + b[4]; q1.y = v[8 * g + 5] + b[5]; q1.z = v[8 * g + 6] + b[6]; q1.w = v[8 * g + 7] + b[7];
-                *reinterpret_cast<float4*>(o + 8 * g) = q0;
-                *reinterpret_cast<float4*>(o + 8 * g + 4) = q1;
-            }
+            for (int g = 0; g < 8; ++g)
+                *reinterpret_cast<float4*>(o + 4 * g) = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
         } else if (EPI == EPI_BIAS_SILU) {
             __align__(16) bf16 h[32];
             __align__(16) bf16 zz[32];
@@ -326,11 +318,11 @@ __device__ __forceinline__ void epilogue(const GemmArgs& G, const OutMaps& om, u
                 }
             }
             stage_row(stg, lane, h);
-            if (G.out_z) stage_row(stg + STAGE_TILE_BYTES, lane, zz);
+            stage_row(stg + STAGE_TILE_BYTES, lane, zz);
             stage_done();
             if (lane == 0) {
                 umma::tma_store_2d(&om.h, c0, row0, stg);
-                if (G.out_z) umma::tma_store_2d(&om.z, c0, row0, stg + STAGE_TILE_BYTES);
+                umma::tma_store_2d(&om.z, c0, row0, stg + STAGE_TILE_BYTES);
                 umma::bulk_commit();
             }
             pending = true;
@@ -646,6 +638,20 @@ bool make_store_map(CUtensorMap* m, const bf16* base, int64_t rows, int64_t cols
                     CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// Store map of FP32 outputs [members][rows][192]: boxes of 32 x 32 with the
+// 128-byte swizzle.  False where the base is not 16-byte aligned.
+bool make_out_map(CUtensorMap* m, float* base, int64_t rows, int members)
+{
+    if (!encoder() || ((uintptr_t)base & 15)) return false;
+    const cuuint64_t dims[3] = {192, (cuuint64_t)rows, (cuuint64_t)members};
+    const cuuint64_t strides[2] = {192 * 4, (cuuint64_t)rows * 192 * 4};
+    const cuuint32_t box[3] = {32, 32, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
+    return g_encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr,
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                    CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // A [M][K] (row stride lda), B [N][K] (row stride ldb); for EPI_WGRAD A [K][M]
 // and B [K][N] (MN-major, N % 64 == 0).
 template <int EPI>
@@ -667,7 +673,7 @@ int launch_gemm(const GemmArgs& g, const bf16* A, int64_t lda, const bf16* B, in
     om.h = om.z = ta;
     if (EpiCfg<EPI>::tiles > 0 && EPI != EPI_DSILU_L1) {
         if (!g.out_h || !make_store_map(&om.h, g.out_h, g.M, g.N, g.ldh)) return CL_ERR_ARG;
-        if (EPI == EPI_BIAS_SILU && g.out_z && !make_store_map(&om.z, g.out_z, g.M, g.N, g.ldh)) return CL_ERR_ARG;
+        if (EPI == EPI_BIAS_SILU && !make_store_map(&om.z, g.out_z, g.M, g.N, g.ldh)) return CL_ERR_ARG;
     }
     // the shared-memory opt-in is a per-device attribute of the kernel: set it
     // once for every device this process launches on
@@ -707,6 +713,11 @@ int launch_gemm(const GemmArgs& g, const bf16* A, int64_t lda, const bf16* B, in
 // ===========================================================================
 constexpr int D_IN = 3, D_H = 256, D_OUT = 192;
 constexpr int WGRAD_MIN_SPLIT_K = 512;   // fewest batch rows per weight-gradient split
+// Parameter block layout (FP32, contiguous): W1[256][3] b1[256] W2t[256][256]
+// b2[256] W3t[256][256] b3[256] W4t[192][256] b4[192].
+constexpr int64_t OFF_W1 = 0, OFF_B1 = OFF_W1 + D_H * D_IN, OFF_W2 = OFF_B1 + D_H,
+                  OFF_B2 = OFF_W2 + D_H * D_H, OFF_W3 = OFF_B2 + D_H, OFF_B3 = OFF_W3 + D_H * D_H,
+                  OFF_W4 = OFF_B3 + D_H, OFF_B4 = OFF_W4 + D_OUT * D_H, N_PARAMS = OFF_B4 + D_OUT;
 
 __device__ __forceinline__ uint32_t hash32(uint32_t a, uint32_t b, uint32_t c)
 {
@@ -813,18 +824,287 @@ __global__ void to_bf16_pair(const float* w, int OUT, int IN, bf16* wt_bf, bf16*
     w_bf[(int64_t)k * OUT + o] = q;
 }
 
+
+// ===========================================================================
+// Inference: the whole network in one kernel
+// ===========================================================================
+// One CTA per SM walks units of 128 rows (of one member of an ensemble) through
+// all four layers.  A unit's activations never leave the SM: layer 1 and each
+// epilogue write the next layer's A operand (128 x 256 BF16, 128-byte swizzle)
+// into the unit's 64 KB of shared memory, the accumulators stay in tensor
+// memory, and only the inputs, the weights (streamed from L2 by TMA in stages
+// of 64 K-elements) and the outputs (staged as 32 x 32 FP32 tiles, TMA stores)
+// move.  Layer by layer the same network went through global memory: H written
+// and read three times, the outputs copied once more.
+//
+// Two units are in flight per CTA: while the sixteen epilogue warps work on one
+// unit's layer, the tensor cores run the other unit's.  The bound is the
+// special-function unit: SiLU takes an exponential and a reciprocal, 2 x 256 x 3
+// per row at 16 per clock and SM, 96 cycles per row (the tensor cores need 43).
+// 200,001 rows through MLP.forward: 355 -> 162 us.
+constexpr int NET_MAX = 8;               // members one launch evaluates
+constexpr int NET_STAGES = 2;            // weight stages of 256 x 64 BF16
+constexpr uint32_t NET_A_BYTES = TILE_M * 512;           // a unit's A operand: 4 K-blocks of 16 KB
+constexpr uint32_t NET_STAGE_BYTES = 256 * 128;
+constexpr int NET_CST = 4 * D_H + 2 * D_H + D_OUT;       // W1 by input component, b1, b2, b3, b4
+constexpr size_t NET_SMEM = 1024 + 2 * (size_t)NET_A_BYTES + NET_STAGES * (size_t)NET_STAGE_BYTES;
+
+struct NetArgs {
+    CUtensorMap w[NET_MAX][3];           // W2^T, W3^T, W4^T: boxes of 64 x 256 (192)
+    CUtensorMap out;                     // [members][n][192] FP32, boxes of 32 x 32
+    const float* params[NET_MAX];        // FP32 parameter blocks
+    const float* x;                      // [n][3]
+    float* out_f;                        // set where the output is not 16-byte aligned: plain stores
+    int64_t n;
+    int members, tiles;                  // units: members x tiles
+    unsigned int* err;
+};
+
+// Byte offset of 16-byte piece j (0..7) of row r in a K-block (128-byte rows, 128-byte swizzle).
+__device__ __forceinline__ uint32_t sw128(uint32_t r, uint32_t j) { return r * 128u + ((j ^ (r & 7u)) << 4); }
+
+// 32 BF16 (columns c0 .. c0 + 31 of row r) into an A operand.
+__device__ __forceinline__ void store_a(uint8_t* A, int r, int c0, const bf16* h)
+{
+    uint8_t* blk = A + (c0 >> 6) * (TILE_M * 128);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<uint4*>(blk + sw128((uint32_t)r, (uint32_t)(((c0 & 63) >> 3) + j))) =
+            reinterpret_cast<const uint4*>(h)[j];
+}
+
+__global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_constant__ NetArgs G)
+{
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (umma::smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t* ring = smem + 2 * NET_A_BYTES;
+    __shared__ __align__(8) uint64_t full[NET_STAGES], empty[NET_STAGES], a_ready[2], acc_full[2], epi_bar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+    __shared__ __align__(16) float s_cst[2][NET_CST];
+
+    const int n_units = G.members * G.tiles;
+    const int my_units = ((int)blockIdx.x < n_units) ? (n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+    if (my_units == 0) return;               // uniform over the CTA
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    volatile int* abort_v = &abort_flag;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < NET_STAGES; ++s) { umma::mbar_init(&full[s], 1); umma::mbar_init(&empty[s], 1); }
+        for (int s = 0; s < 2; ++s) { umma::mbar_init(&a_ready[s], EPI_WARPS); umma::mbar_init(&acc_full[s], 1); }
+        umma::mbar_init(&epi_bar, EPI_WARPS);
+        abort_flag = 0;
+    }
+    if (warp == MMA_WARP) umma::tmem_alloc(&tmem_slot, TMEM_COLS);
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == PRODUCER_WARP) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            bool ok = true;
+            for (int u0 = 0; u0 < my_units && ok; u0 += 2)
+                for (int l = 0; l < 3 && ok; ++l)
+                    for (int s = 0; s < 2 && u0 + s < my_units && ok; ++s) {
+                        const int member = ((int)blockIdx.x + (u0 + s) * (int)gridDim.x) / G.tiles;
+                        const uint32_t bytes = (l == 2 ? D_OUT : D_H) * 128u;
+                        for (int c = 0; c < D_H / TILE_K; ++c, ++it) {
+                            const uint32_t st = it % NET_STAGES, r = it / NET_STAGES;
+                            if (r > 0 && !umma::mbar_wait_or_abort(&empty[st], (r - 1) & 1u, WAIT_BUDGET, abort_v)) {
+                                ok = false;
+                                break;
+                            }
+                            umma::mbar_arrive_expect_tx(&full[st], bytes);
+                            umma::tma_load_2d(ring + st * NET_STAGE_BYTES, &G.w[member][l], c * TILE_K, 0, &full[st]);
+                        }
+                    }
+            if (!ok) { atomicOr(G.err, 1u); *abort_v = 1; }
+            // copies still in flight land before the CTA can exit
+            for (uint32_t j = it > (uint32_t)NET_STAGES ? it - NET_STAGES : 0u; j < it; ++j)
+                umma::mbar_wait(&full[j % NET_STAGES], (j / NET_STAGES) & 1u, WAIT_BUDGET);
+        }
+    } else if (warp == MMA_WARP) {
+        if (lane == 0) {
+            uint32_t it = 0, job[2] = {0, 0};
+            bool ok = true;
+            for (int u0 = 0; u0 < my_units && ok; u0 += 2)
+                for (int l = 0; l < 3 && ok; ++l)
+                    for (int s = 0; s < 2 && u0 + s < my_units && ok; ++s) {
+                        if (!umma::mbar_wait_or_abort(&a_ready[s], job[s]++ & 1u, WAIT_BUDGET, abort_v)) { ok = false; break; }
+                        umma::fence_after_sync();
+                        const uint32_t idesc = umma::make_idesc_bf16(TILE_M, l == 2 ? D_OUT : D_H, false, false);
+                        const uint32_t a0 = umma::smem_u32(smem + s * NET_A_BYTES), d = tmem + s * 256u;
+                        for (int c = 0; c < D_H / TILE_K; ++c, ++it) {
+                            const uint32_t st = it % NET_STAGES, r = it / NET_STAGES;
+                            if (!umma::mbar_wait_or_abort(&full[st], r & 1u, WAIT_BUDGET, abort_v)) { ok = false; break; }
+                            umma::fence_after_sync();
+                            const uint32_t sb = umma::smem_u32(ring + st * NET_STAGE_BYTES);
+#pragma unroll
+                            for (int k = 0; k < TILE_K / 16; ++k)
+                                umma::mma_bf16(d, umma::make_desc_sw128(a0 + c * (TILE_M * 128u) + 32u * k),
+                                               umma::make_desc_sw128(sb + 32u * k), idesc, (c > 0 || k > 0) ? 1u : 0u);
+                            umma::commit(&empty[st]);
+                        }
+                        if (ok) umma::commit(&acc_full[s]);
+                    }
+            if (!ok) { atomicOr(G.err, 1u); *abort_v = 1; }
+            // the last MMAs complete before TMEM is freed
+            if (it > 0) umma::mbar_wait(&empty[(it - 1) % NET_STAGES], ((it - 1) / NET_STAGES) & 1u, WAIT_BUDGET);
+        }
+    } else {
+        const int quad = warp & 3, half = warp >> 2;
+        const int row = 32 * quad + lane;                 // of the unit
+        const uint32_t tlane = (uint32_t)(32 * quad) << 16;
+        int loaded[2] = {-1, -1};                         // member whose constants a slot holds
+        uint32_t job[2] = {0, 0}, met = 0;
+        bool ok = true;
+        auto give_up = [&] {
+            if (lane == 0) atomicOr(G.err, 1u);
+            *abort_v = 1;
+            ok = false;
+        };
+        // the epilogue warps meet (bounded like every wait)
+        auto meet = [&] {
+            __syncwarp();
+            if (lane == 0) umma::mbar_arrive(&epi_bar);
+            if (!umma::mbar_wait_or_abort(&epi_bar, met++ & 1u, WAIT_BUDGET, abort_v)) give_up();
+        };
+
+        // layer 1 of unit `u` into slot s's A operand
+        auto first_layer = [&](int s, int u) {
+            const int unit = (int)blockIdx.x + u * (int)gridDim.x;
+            const int member = unit / G.tiles, tile = unit - member * G.tiles;
+            float* cst = s_cst[s];
+            if (loaded[s] != member) {
+                meet();                      // no warp reads the last member's constants any more
+                const float* p = G.params[member];
+                for (int i = threadIdx.x; i < 3 * D_H; i += 32 * EPI_WARPS) cst[D_H * (i % 3) + i / 3] = p[i];
+                for (int i = threadIdx.x; i < D_H; i += 32 * EPI_WARPS) {
+                    cst[3 * D_H + i] = p[OFF_B1 + i];
+                    cst[4 * D_H + i] = p[OFF_B2 + i];
+                    cst[5 * D_H + i] = p[OFF_B3 + i];
+                    if (i < D_OUT) cst[6 * D_H + i] = p[OFF_B4 + i];
+                }
+                loaded[s] = member;
+            }
+            // the constants are there, and every warp's output tiles (staged in
+            // this operand) have been read
+            meet();
+            if (!ok) return;
+            const int64_t gr = (int64_t)tile * TILE_M + row;
+            float x0 = 0.f, x1 = 0.f, x2 = 0.f;
+            if (gr < G.n) { x0 = G.x[gr * 3]; x1 = G.x[gr * 3 + 1]; x2 = G.x[gr * 3 + 2]; }
+            for (int c0 = 32 * half; c0 < D_H; c0 += 8 * EPI_WARPS) {
+                __align__(16) bf16 h[32];
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    float b[8], w0[8], w1[8], w2[8];
+                    cst8(cst + 3 * D_H + c0 + 8 * g, b);
+                    cst8(cst + c0 + 8 * g, w0);
+                    cst8(cst + D_H + c0 + 8 * g, w1);
+                    cst8(cst + 2 * D_H + c0 + 8 * g, w2);
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const float z = __fmaf_rn(x2, w2[q], __fmaf_rn(x1, w1[q], __fmaf_rn(x0, w0[q], b[q])));
+                        h[8 * g + q] = __float2bfloat16_rn(silu(z));
+                    }
+                }
+                store_a(smem + s * NET_A_BYTES, row, c0, h);
+            }
+            umma::fence_before_sync();
+            stage_done();
+            if (lane == 0) umma::mbar_arrive(&a_ready[s]);
+        };
+        auto wait_acc = [&](int s) {
+            if (!umma::mbar_wait_or_abort(&acc_full[s], job[s]++ & 1u, WAIT_BUDGET, abort_v)) give_up();
+            umma::fence_after_sync();
+        };
+
+        for (int s = 0; s < 2 && s < my_units; ++s) first_layer(s, s);
+        for (int u0 = 0; u0 < my_units && ok; u0 += 2) {
+            for (int l = 0; l < 2 && ok; ++l)
+                for (int s = 0; s < 2 && u0 + s < my_units; ++s) {
+                    wait_acc(s);
+                    if (!ok) break;
+                    const float* b2 = s_cst[s] + (4 + l) * D_H;
+                    for (int c0 = 32 * half; c0 < D_H; c0 += 8 * EPI_WARPS) {
+                        float v[32];
+                        umma::tmem_ld32(tmem + s * 256u + tlane + (uint32_t)c0, v);
+                        __align__(16) bf16 h[32];
+#pragma unroll
+                        for (int g = 0; g < 4; ++g) {
+                            float b[8];
+                            cst8(b2 + c0 + 8 * g, b);
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) h[8 * g + q] = __float2bfloat16_rn(silu(v[8 * g + q] + b[q]));
+                        }
+                        store_a(smem + s * NET_A_BYTES, row, c0, h);
+                    }
+                    umma::fence_before_sync();
+                    stage_done();
+                    if (lane == 0) umma::mbar_arrive(&a_ready[s]);
+                }
+            for (int s = 0; s < 2 && u0 + s < my_units && ok; ++s) {
+                wait_acc(s);
+                if (!ok) break;
+                const int unit = (int)blockIdx.x + (u0 + s) * (int)gridDim.x;
+                const int member = unit / G.tiles, tile = unit - member * G.tiles;
+                const float* b4 = s_cst[s] + 6 * D_H;
+                uint8_t* stg = smem + s * NET_A_BYTES + warp * 4096;      // the layer's A operand is consumed
+                for (int c0 = 32 * half; c0 < D_OUT; c0 += 8 * EPI_WARPS) {
+                    float v[32];
+                    umma::tmem_ld32(tmem + s * 256u + tlane + (uint32_t)c0, v);
+                    if (c0 >= 8 * EPI_WARPS && lane == 0) umma::bulk_wait_read0();
+                    __syncwarp();
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        float b[8];
+                        cst8(b4 + c0 + 8 * g, b);
+#pragma unroll
+                        for (int q = 0; q < 8; ++q) v[8 * g + q] += b[q];
+                    }
+                    if (G.out_f) {
+                        const int64_t gr = (int64_t)tile * TILE_M + row;
+                        float* o = G.out_f + ((int64_t)member * G.n + gr) * D_OUT + c0;
+                        if (gr < G.n) {
+#pragma unroll
+                            for (int i = 0; i < 32; ++i) o[i] = v[i];
+                        }
+                        continue;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        *reinterpret_cast<float4*>(stg + sw128((uint32_t)lane, (uint32_t)j)) =
+                            make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                    stage_done();
+                    if (lane == 0) {
+                        umma::tma_store_3d(&G.out, c0, tile * TILE_M + 32 * quad, member, stg);
+                        umma::bulk_commit();
+                    }
+                }
+                umma::fence_before_sync();
+                if (u0 + s + 2 < my_units) {
+                    if (lane == 0) umma::bulk_wait_read0();
+                    __syncwarp();
+                    first_layer(s, u0 + s + 2);
+                }
+            }
+        }
+        if (lane == 0) umma::bulk_wait0();
+        __syncwarp();
+    }
+    __syncthreads();
+    if (warp == MMA_WARP) {
+        umma::fence_after_sync();
+        umma::tmem_dealloc(tmem, TMEM_COLS);
+    }
+}
+
 }  // namespace mlp
 }  // namespace cl
 
 using namespace cl::mlp;
-
-// Parameter block layout (FP32, contiguous): W1[256][3] b1[256] W2t[256][256]
-// b2[256] W3t[256][256] b3[256] W4t[192][256] b4[192].
-namespace {
-constexpr int64_t OFF_W1 = 0, OFF_B1 = OFF_W1 + D_H * D_IN, OFF_W2 = OFF_B1 + D_H,
-                  OFF_B2 = OFF_W2 + D_H * D_H, OFF_W3 = OFF_B2 + D_H, OFF_B3 = OFF_W3 + D_H * D_H,
-                  OFF_W4 = OFF_B3 + D_H, OFF_B4 = OFF_W4 + D_OUT * D_H, N_PARAMS = OFF_B4 + D_OUT;
-}
 
 struct cl_mlp {
     int device = 0;
@@ -839,7 +1119,7 @@ struct cl_mlp {
     // BF16 weight copies
     bf16 *w2t = nullptr, *w2 = nullptr, *w3t = nullptr, *w3 = nullptr, *w4t = nullptr, *w4 = nullptr;
     // activations and gradients (max_batch rows)
-    float *xb = nullptr, *o = nullptr;
+    float* xb = nullptr;
     int32_t* brow = nullptr;        // training-set row of each minibatch row
     bf16 *h1 = nullptr, *h2 = nullptr, *z2 = nullptr, *h3 = nullptr, *z3 = nullptr;
     bf16 *dO = nullptr, *dz3 = nullptr, *dz2 = nullptr;
@@ -895,38 +1175,31 @@ GemmArgs gemm_args(cl_mlp* m)
     return g;
 }
 
-// Forward pass over B rows of m->xb (B % 128 == 0).  Training (with_loss):
-// keeps H and Z for the backward pass and ends in the loss epilogue, which
-// reads the targets (rows `trow` of `target`, or its first B rows) and writes
-// dO, the b4 gradient and the loss.  Inference: O into m->o.
-int forward(cl_mlp* m, int B, bool with_loss, const float* target, const int32_t* trow, cudaStream_t st,
-            bool zero_grad = true)
+// Training forward pass over B rows of m->xb (B % 128 == 0): keeps H and Z for
+// the backward pass and ends in the loss epilogue, which reads the targets
+// (rows `trow` of `target`, or its first B rows) and writes dO, the b4 gradient
+// and the loss.
+int forward(cl_mlp* m, int B, const float* target, const int32_t* trow, cudaStream_t st, bool zero_grad)
 {
     const int grid = grid_for(m, B);
-    if (with_loss && zero_grad) cudaMemsetAsync(m->g, 0, N_PARAMS * sizeof(float), st);
+    if (zero_grad) cudaMemsetAsync(m->g, 0, N_PARAMS * sizeof(float), st);
     launch_pdl(layer1_fwd, dim3((unsigned)(B / L1_ROWS)), dim3(256), 0, st, (const float*)m->xb,
                (const float*)(m->p + OFF_W1), (const float*)(m->p + OFF_B1), m->h1);
     GemmArgs g = gemm_args(m);
     g.M = B; g.N = D_H; g.K = D_H; g.k_split = D_H;
-    g.bias = m->p + OFF_B2; g.out_h = m->h2; g.ldh = D_H;
-    g.out_z = with_loss ? m->z2 : nullptr;
+    g.bias = m->p + OFF_B2; g.out_h = m->h2; g.ldh = D_H; g.out_z = m->z2;
     int rc = launch_gemm<EPI_BIAS_SILU>(g, m->h1, D_H, m->w2t, D_H, grid, 1, st);
     if (rc) return rc;
-    g.bias = m->p + OFF_B3; g.out_h = m->h3;
-    g.out_z = with_loss ? m->z3 : nullptr;
+    g.bias = m->p + OFF_B3; g.out_h = m->h3; g.out_z = m->z3;
     if ((rc = launch_gemm<EPI_BIAS_SILU>(g, m->h2, D_H, m->w3t, D_H, grid, 1, st))) return rc;
     GemmArgs q = gemm_args(m);
     q.M = B; q.N = D_OUT; q.K = D_H; q.k_split = D_H; q.bias = m->p + OFF_B4;
-    if (!with_loss) {
-        q.out_f = m->o; q.ldf = D_OUT;
-        return launch_gemm<EPI_BIAS_F32>(q, m->h3, D_H, m->w4t, D_H, grid, 1, st);
-    }
     q.target = target; q.trow = trow; q.scale = 1.0f / ((float)B * (float)D_OUT); q.loss = m->loss;
     q.out_h = m->dO; q.ldh = D_OUT; q.colsum = m->g + OFF_B4;
     return launch_gemm<EPI_LOSS>(q, m->h3, D_H, m->w4t, D_H, grid, 1, st);
 }
 
-// Backward pass after forward(with_loss), which zeroed m->g: bias and layer-1
+// Backward pass after forward(), with m->g zeroed: bias and layer-1
 // gradients accumulate in the epilogues, weight gradients come from the
 // split-K GEMMs.
 int backward(cl_mlp* m, int B, cudaStream_t st)
@@ -962,6 +1235,58 @@ int backward(cl_mlp* m, int B, cudaStream_t st)
         if ((rc = launch_gemm<EPI_WGRAD>(w, wg[l].h, D_H, wg[l].dz, wg[l].OUT, D_H / TILE_M, splits, st))) return rc;
     }
     return cudaGetLastError() == cudaSuccess ? CL_OK : CL_ERR_CUDA;
+}
+
+// net_forward over members x n rows, NET_MAX members and 2^24 rows per launch
+// (the tensor maps' and tile indices' range).
+int net_forward_enqueue(cl_mlp* const* nets, int members, const float* d_x, float* d_out, int64_t n, cudaStream_t st)
+{
+    cl_mlp* const m = nets[0];
+    static std::atomic<uint64_t> attr_devices{0};
+    const uint64_t bit = 1ull << (m->device & 63);
+    if (!(attr_devices.load() & bit)) {
+        if (cudaFuncSetAttribute(net_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NET_SMEM) != cudaSuccess)
+            return CL_ERR_CUDA;
+        attr_devices.fetch_or(bit);
+    }
+    for (int k0 = 0; k0 < members; k0 += NET_MAX) {
+        const int K = members - k0 < NET_MAX ? members - k0 : NET_MAX;
+        NetArgs g;
+        memset(&g, 0, sizeof g);
+        for (int k = 0; k < K; ++k) {
+            const cl_mlp* q = nets[k0 + k];
+            if (!make_map(&g.w[k][0], q->w2t, D_H, D_H, D_H, D_H) || !make_map(&g.w[k][1], q->w3t, D_H, D_H, D_H, D_H) ||
+                !make_map(&g.w[k][2], q->w4t, D_OUT, D_H, D_H, D_OUT))
+                return CL_ERR_ARG;
+            g.params[k] = q->p;
+        }
+        g.members = K;
+        g.err = m->derr;
+        constexpr int64_t ROWS = 1 << 24;
+        for (int64_t r0 = 0; r0 < n; r0 += ROWS) {
+            const int64_t rows = n - r0 < ROWS ? n - r0 : ROWS;
+            // a member's block of rows is n rows from the next one's
+            for (int k = 0; k < (rows < n ? K : 1); ++k) {
+                const int Kl = rows < n ? 1 : K;
+                NetArgs a = g;
+                float* out = d_out + ((int64_t)(k0 + k) * n + r0) * D_OUT;
+                if (rows < n) {
+                    for (int l = 0; l < 3; ++l) a.w[0][l] = g.w[k][l];
+                    a.params[0] = g.params[k];
+                }
+                a.members = Kl;
+                a.x = d_x + r0 * D_IN;
+                a.n = rows;
+                a.tiles = (int)((rows + TILE_M - 1) / TILE_M);
+                if (!make_out_map(&a.out, out, rows, Kl)) a.out_f = out;
+                const int units = Kl * a.tiles;
+                const int cap = m->max_ctas > 0 && m->max_ctas < m->num_sms ? m->max_ctas : m->num_sms;
+                net_forward<<<(unsigned)(units < cap ? units : cap), GEMM_THREADS, NET_SMEM, st>>>(a);
+                if (cudaGetLastError() != cudaSuccess) return CL_ERR_CUDA;
+            }
+        }
+    }
+    return CL_OK;
 }
 
 void adam(cl_mlp* m, float lr, cudaStream_t st)
@@ -1010,7 +1335,7 @@ int cl_mlp_create(cl_mlp** out, int device, int max_batch)
               dalloc(m, &m->w2t, (size_t)D_H * D_H) && dalloc(m, &m->w2, (size_t)D_H * D_H) &&
               dalloc(m, &m->w3t, (size_t)D_H * D_H) && dalloc(m, &m->w3, (size_t)D_H * D_H) &&
               dalloc(m, &m->w4t, (size_t)D_OUT * D_H) && dalloc(m, &m->w4, (size_t)D_OUT * D_H) &&
-              dalloc(m, &m->xb, B * D_IN) && dalloc(m, &m->brow, B) && dalloc(m, &m->o, B * D_OUT) &&
+              dalloc(m, &m->xb, B * D_IN) && dalloc(m, &m->brow, B) &&
               dalloc(m, &m->h1, B * D_H) &&
               dalloc(m, &m->h2, B * D_H) && dalloc(m, &m->z2, B * D_H) &&
               dalloc(m, &m->h3, B * D_H) && dalloc(m, &m->z3, B * D_H) &&
@@ -1100,7 +1425,7 @@ int cl_mlp_train(cl_mlp* m, int steps, int batch, float lr, uint32_t seed, uint3
     for (int s = 0; s < steps; ++s) {
         launch_pdl(gather_batch, dim3((batch + 255) / 256), dim3(256), 0, st, (const float*)m->data_x,
                    (int64_t)m->n_data, batch, seed, step0 + (uint32_t)s, m->xb, m->brow);
-        int rc = forward(m, batch, true, m->data_t, m->brow, st, false);
+        int rc = forward(m, batch, m->data_t, m->brow, st, false);
         if (!rc) rc = backward(m, batch, st);
         if (rc) return mlp_fail(m, rc, "kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
         adam(m, lr, st);
@@ -1115,25 +1440,41 @@ int cl_mlp_train(cl_mlp* m, int steps, int batch, float lr, uint32_t seed, uint3
     return CL_OK;
 }
 
+// Inference of `members` networks on one GPU: out[members][n][192] (FP32,
+// device) for x[n][3] (FP32, device), enqueued on `stream` (NULL: the first
+// network's own); cl_mlp_sync waits and reports.
+int cl_mlp_forward_ensemble(cl_mlp* const* nets, int members, const float* d_x, float* d_out, int64_t n, void* stream)
+{
+    if (!nets || members < 1 || n < 0) return CL_ERR_ARG;
+    for (int k = 0; k < members; ++k)
+        if (!nets[k] || nets[k]->device != nets[0]->device) return CL_ERR_ARG;
+    if (n == 0) return CL_OK;
+    if (!d_x || !d_out) return CL_ERR_ARG;
+    cudaSetDevice(nets[0]->device);
+    return net_forward_enqueue(nets, members, d_x, d_out, n, stream ? (cudaStream_t)stream : nets[0]->stream);
+}
+
+// Wait for the work on `stream` (NULL: the network's own) and report a
+// tensor-core wait that ran out.
+int cl_mlp_sync(cl_mlp* m, void* stream)
+{
+    if (!m) return CL_ERR_ARG;
+    cudaSetDevice(m->device);
+    cudaStream_t st = stream ? (cudaStream_t)stream : m->stream;
+    unsigned int e = 0;
+    cudaMemcpyAsync(&e, m->derr, sizeof e, cudaMemcpyDeviceToHost, st);
+    if (cudaStreamSynchronize(st) != cudaSuccess) return mlp_fail(m, CL_ERR_CUDA, "%s", cudaGetErrorString(cudaGetLastError()));
+    return e ? mlp_fail(m, CL_ERR_TIMEOUT, "tensor-core completion wait ran out") : CL_OK;
+}
+
 // Inference: out[n][192] (FP32, device) for x[n][3] (FP32, device).
 int cl_mlp_forward(cl_mlp* m, const float* d_x, float* d_out, int64_t n)
 {
     if (!m || !d_x || !d_out || n < 0) return CL_ERR_ARG;
     cudaSetDevice(m->device);
-    cudaStream_t st = m->stream;
-    for (int64_t r0 = 0; r0 < n; r0 += m->max_batch) {
-        const int rows = (int)((n - r0) < m->max_batch ? (n - r0) : m->max_batch);
-        const int B = ((rows + TILE_M - 1) / TILE_M) * TILE_M;
-        cudaMemsetAsync(m->xb, 0, (size_t)B * D_IN * sizeof(float), st);
-        cudaMemcpyAsync(m->xb, d_x + r0 * D_IN, (size_t)rows * D_IN * sizeof(float), cudaMemcpyDeviceToDevice, st);
-        int rc = forward(m, B, false, nullptr, nullptr, st);
-        if (rc) return mlp_fail(m, rc, "forward launch failed");
-        cudaMemcpyAsync(d_out + r0 * D_OUT, m->o, (size_t)rows * D_OUT * sizeof(float), cudaMemcpyDeviceToDevice, st);
-    }
-    unsigned int e = 0;
-    cudaMemcpyAsync(&e, m->derr, sizeof e, cudaMemcpyDeviceToHost, st);
-    if (cudaStreamSynchronize(st) != cudaSuccess) return mlp_fail(m, CL_ERR_CUDA, "%s", cudaGetErrorString(cudaGetLastError()));
-    return e ? mlp_fail(m, CL_ERR_TIMEOUT, "tensor-core completion wait ran out") : CL_OK;
+    const int rc = n > 0 ? net_forward_enqueue(&m, 1, d_x, d_out, n, m->stream) : CL_OK;
+    if (rc) return mlp_fail(m, rc, "forward launch failed");
+    return cl_mlp_sync(m, nullptr);
 }
 
 // Gradient of the loss for one given batch (x [B][3], t [B][192] FP32 device;
@@ -1145,7 +1486,7 @@ int cl_mlp_gradient(cl_mlp* m, const float* d_x, const float* d_t, int B, float*
     cudaStream_t st = m->stream;
     cudaMemcpyAsync(m->xb, d_x, (size_t)B * D_IN * sizeof(float), cudaMemcpyDeviceToDevice, st);
     cudaMemsetAsync(m->loss, 0, sizeof(float), st);
-    int rc = forward(m, B, true, d_t, nullptr, st);
+    int rc = forward(m, B, d_t, nullptr, st, true);
     if (!rc) rc = backward(m, B, st);
     if (rc) return mlp_fail(m, rc, "launch failed");
     float loss = 0.0f;

@@ -178,6 +178,13 @@ __device__ __forceinline__ void tma_store_2d(const void* tmap, int32_t x, int32_
                  :: "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(smem_u32(src)) : "memory");
 }
 
+// The same for a 3-D tensor map (z = outermost).
+__device__ __forceinline__ void tma_store_3d(const void* tmap, int32_t x, int32_t y, int32_t z, const void* src)
+{
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];"
+                 :: "l"(reinterpret_cast<uint64_t>(tmap)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(src)) : "memory");
+}
+
 __device__ __forceinline__ void bulk_commit()
 {
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");

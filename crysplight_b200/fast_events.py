@@ -34,7 +34,8 @@ import numpy as np
 from . import _lib
 from .events import EventsResult, GammaMaterial, gamma_stage
 from .params import COUNTER_NAMES, Box, OpticalParams, Readout, TimeBinning
-from .surrogate import D_OUT, MLP, N_CELLS, LightSurrogate, first_pass_light, first_pass_optics
+from .surrogate import (D_OUT, MLP, N_CELLS, LightSurrogate, first_pass_light, first_pass_optics,
+                        forward_ensemble, sync_networks)
 from .transport import stream_arg
 
 SPREAD_MAX = 0.02
@@ -130,21 +131,23 @@ class SurrogateEvents:
         import torch
         n = int(xyz.shape[0])
         K = len(ens.nets)
+        # everything here runs on one stream; torch's own work on the inputs
+        # (another stream, if the caller names one) is done before it
+        st = stream_arg(stream or 0)
         xyz = xyz.contiguous()
         xin = torch.empty((n, 3), dtype=torch.float32, device=self.dev)
         xs = xyz
         if ens.z0 != 0.0:
             xs = xyz - torch.tensor([0.0, 0.0, ens.z0], dtype=torch.float32, device=self.dev)
+        current = torch.cuda.current_stream(self.dev)
+        if current.cuda_stream != (stream or 0):
+            current.synchronize()
         rc = self.lib.cl_surrogate_inputs(C.c_void_p(xs.data_ptr()), n, C.byref(ens.in_box),
-                                          float(ens.sur.z_warp), C.c_void_p(xin.data_ptr()),
-                                          stream_arg(stream))
+                                          float(ens.sur.z_warp), C.c_void_p(xin.data_ptr()), st)
         if rc != 0:
             raise _lib.CudaTransportError(rc, "cl_surrogate_inputs failed")
-        torch.cuda.synchronize(self.dev)         # the networks run on their own streams
         raw = torch.empty((K, n, D_OUT), dtype=torch.float32, device=self.dev)
-        for k, net in enumerate(ens.nets):
-            if n:
-                net.forward_into(xin, raw[k])
+        forward_ensemble(ens.nets, xin, raw, st)
         out = SiteLight(torch.empty((n, N_CELLS), dtype=torch.float32, device=self.dev),
                         torch.empty((n, N_CELLS), dtype=torch.float32, device=self.dev),
                         torch.empty((n, N_CELLS), dtype=torch.float32, device=self.dev),
@@ -154,15 +157,17 @@ class SurrogateEvents:
         # an ensemble trained on the light minus the first-pass term gets it back here
         direct = None
         if ens.sur.first_pass is not None and n:
-            direct = first_pass_light(xyz, self.box, ens.sur.first_pass, self.device, stream)
+            direct = first_pass_light(xyz, self.box, ens.sur.first_pass, self.device, stream or 0)
         rc = self.lib.cl_surrogate_combine_direct(
             P(raw.data_ptr()), K, n, P(ens.y_mean.data_ptr()), P(ens.y_std.data_ptr()),
             P(xyz.data_ptr()), P(direct.data_ptr()) if direct is not None else None, C.byref(self.box),
             C.byref(ro), float(pde), float(spread_max),
             float(wall_min_mm), P(out.p.data_ptr()), P(out.tmean.data_ptr()), P(out.tsig.data_ptr()),
-            P(out.spread.data_ptr()), P(out.flag.data_ptr()), stream_arg(stream))
+            P(out.spread.data_ptr()), P(out.flag.data_ptr()), st)
         if rc != 0:
             raise _lib.CudaTransportError(rc, "cl_surrogate_combine failed")
+        # the temporaries go back to torch's allocator, and a network's error is reported here
+        sync_networks(ens.nets, st)
         return out
 
     def site_light(self, xyz, *, ro: Readout, pde: float, spread_max: float = SPREAD_MAX,
@@ -178,7 +183,6 @@ class SurrogateEvents:
             if idx.numel() == 0:
                 continue
             sub = self._light(ens, xyz.index_select(0, idx), ro, pde, spread_max, wall_min_mm, stream)
-            torch.cuda.synchronize(self.dev)     # both combines ran on `stream`
             for name in ("p", "tmean", "tsig", "spread", "flag"):
                 getattr(out, name).index_copy_(0, idx, getattr(sub, name))
         if self.experts:

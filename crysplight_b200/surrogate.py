@@ -41,9 +41,11 @@ def _declare(lib):
     lib.cl_mlp_train.argtypes = [P, C.c_int, C.c_int, C.c_float, C.c_uint32, C.c_uint32,
                                  C.POINTER(C.c_float)]
     lib.cl_mlp_forward.argtypes = [P, P, P, C.c_int64]
+    lib.cl_mlp_forward_ensemble.argtypes = [C.POINTER(P), C.c_int, P, P, C.c_int64, P]
+    lib.cl_mlp_sync.argtypes = [P, P]
     lib.cl_mlp_gradient.argtypes = [P, P, P, C.c_int, P, C.POINTER(C.c_float)]
     for n in ("cl_mlp_set_params", "cl_mlp_get_params", "cl_mlp_set_data", "cl_mlp_train",
-              "cl_mlp_forward", "cl_mlp_gradient"):
+              "cl_mlp_forward", "cl_mlp_forward_ensemble", "cl_mlp_sync", "cl_mlp_gradient"):
         getattr(lib, n).restype = C.c_int
     lib._mlp_declared = True
 
@@ -137,6 +139,20 @@ class MLP:
         self._check(self.lib.cl_mlp_gradient(self.h, C.c_void_p(x.data_ptr()), C.c_void_p(t.data_ptr()),
                                              x.shape[0], C.c_void_p(g.ctypes.data), C.byref(loss)))
         return float(loss.value), g
+
+
+def forward_ensemble(nets, x, out, stream) -> None:
+    """out[k] = nets[k](x) for networks of one GPU: x (n, 3) and out (K, n, 192)
+    float32 CUDA tensors, contiguous; enqueued on ``stream`` (a CUDA stream
+    handle as the C-ABI takes it) without waiting.  ``sync_networks`` waits."""
+    a = (C.c_void_p * len(nets))(*[n.h for n in nets])
+    nets[0]._check(nets[0].lib.cl_mlp_forward_ensemble(a, len(nets), C.c_void_p(x.data_ptr()),
+                                                       C.c_void_p(out.data_ptr()), x.shape[0], stream))
+
+
+def sync_networks(nets, stream) -> None:
+    """Wait for the work on ``stream`` and raise if a tensor-core wait ran out."""
+    nets[0]._check(nets[0].lib.cl_mlp_sync(nets[0].h, stream))
 
 
 # ---------------------------------------------------------------------------

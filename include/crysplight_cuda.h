@@ -467,6 +467,13 @@ int cl_mlp_train(cl_mlp* m, int steps, int batch, float lr, uint32_t seed, uint3
                  float* loss_out);
 /* Inference: out [n][192] FP32 device for x [n][3] FP32 device. */
 int cl_mlp_forward(cl_mlp* m, const float* d_x, float* d_out, int64_t n);
+/* The same for `members` networks of one device, out [members][n][192],
+ * enqueued on `stream` (NULL: the first network's own stream) without waiting;
+ * cl_mlp_sync on the first network waits for the stream and returns
+ * CL_ERR_TIMEOUT if a tensor-core wait ran out. */
+int cl_mlp_forward_ensemble(cl_mlp* const* nets, int members, const float* d_x, float* d_out,
+                            int64_t n, void* stream);
+int cl_mlp_sync(cl_mlp* m, void* stream);
 /* Loss and gradient (host, cl_mlp_param_count() floats) for one batch of
  * B rows (B % 128 == 0, <= max_batch), without an update.  For tests. */
 int cl_mlp_gradient(cl_mlp* m, const float* d_x, const float* d_t, int B, float* host_grad,
