@@ -139,7 +139,13 @@ struct GemmArgs {
 // SiLU and its derivative with the fast exponential and division (results
 // are rounded to BF16 afterwards; for z -> -inf, __fdividef by an infinite
 // denominator returns 0)
-__device__ __forceinline__ float silu(float z) { return __fdividef(z, 1.0f + __expf(-z)); }
+__device__ __forceinline__ float silu(float z)
+{
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950216293335f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return z * r;
+}
 __device__ __forceinline__ float dsilu(float z)
 {
     const float s = __fdividef(1.0f, 1.0f + __expf(-z));
@@ -638,20 +644,6 @@ bool make_store_map(CUtensorMap* m, const bf16* base, int64_t rows, int64_t cols
                     CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Store map of FP32 outputs [members][rows][192]: boxes of 32 x 32 with the
-// 128-byte swizzle.  False where the base is not 16-byte aligned.
-bool make_out_map(CUtensorMap* m, float* base, int64_t rows, int members)
-{
-    if (!encoder() || ((uintptr_t)base & 15)) return false;
-    const cuuint64_t dims[3] = {192, (cuuint64_t)rows, (cuuint64_t)members};
-    const cuuint64_t strides[2] = {192 * 4, (cuuint64_t)rows * 192 * 4};
-    const cuuint32_t box[3] = {32, 32, 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    return g_encode(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                    CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
 // A [M][K] (row stride lda), B [N][K] (row stride ldb); for EPI_WGRAD A [K][M]
 // and B [K][N] (MN-major, N % 64 == 0).
 template <int EPI>
@@ -846,15 +838,15 @@ constexpr int NET_MAX = 8;               // members one launch evaluates
 constexpr int NET_STAGES = 2;            // weight stages of 256 x 64 BF16
 constexpr uint32_t NET_A_BYTES = TILE_M * 512;           // a unit's A operand: 4 K-blocks of 16 KB
 constexpr uint32_t NET_STAGE_BYTES = 256 * 128;
-constexpr int NET_CST = 4 * D_H + 2 * D_H + D_OUT;       // W1 by input component, b1, b2, b3, b4
+constexpr int NET_CST_W1 = 2 * D_H + D_OUT;              // b2, b3, b4, then (W1 row, b1) per feature
+constexpr int NET_CST = NET_CST_W1 + 4 * D_H;
 constexpr size_t NET_SMEM = 1024 + 2 * (size_t)NET_A_BYTES + NET_STAGES * (size_t)NET_STAGE_BYTES;
 
 struct NetArgs {
     CUtensorMap w[NET_MAX][3];           // W2^T, W3^T, W4^T: boxes of 64 x 256 (192)
-    CUtensorMap out;                     // [members][n][192] FP32, boxes of 32 x 32
     const float* params[NET_MAX];        // FP32 parameter blocks
     const float* x;                      // [n][3]
-    float* out_f;                        // set where the output is not 16-byte aligned: plain stores
+    float* out;                          // [members][n][192]
     int64_t n;
     int members, tiles;                  // units: members x tiles
     unsigned int* err;
@@ -873,6 +865,21 @@ __device__ __forceinline__ void store_a(uint8_t* A, int r, int c0, const bf16* h
             reinterpret_cast<const uint4*>(h)[j];
 }
 
+// 16 consecutive floats of this lane's row: two whole 32-byte sectors.
+__device__ __forceinline__ void store_row16(float* o, const float* v, bool wide)
+{
+    if (wide) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+            asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(o + 8 * i), "f"(v[8 * i]),
+                         "f"(v[8 * i + 1]), "f"(v[8 * i + 2]), "f"(v[8 * i + 3]), "f"(v[8 * i + 4]), "f"(v[8 * i + 5]),
+                         "f"(v[8 * i + 6]), "f"(v[8 * i + 7]) : "memory");
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[i] = v[i];
+    }
+}
+
 __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_constant__ NetArgs G)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -882,6 +889,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     __shared__ __align__(16) float s_cst[2][NET_CST];
+    __shared__ float4 s_x[EPI_WARPS][16];
 
     const int n_units = G.members * G.tiles;
     const int my_units = ((int)blockIdx.x < n_units) ? (n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
@@ -890,7 +898,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
     volatile int* abort_v = &abort_flag;
     if (threadIdx.x == 0) {
         for (int s = 0; s < NET_STAGES; ++s) { umma::mbar_init(&full[s], 1); umma::mbar_init(&empty[s], 1); }
-        for (int s = 0; s < 2; ++s) { umma::mbar_init(&a_ready[s], EPI_WARPS); umma::mbar_init(&acc_full[s], 1); }
+        for (int s = 0; s < 2; ++s) {
+            umma::mbar_init(&a_ready[s], EPI_WARPS);
+            umma::mbar_init(&acc_full[s], 1);
+        }
         umma::mbar_init(&epi_bar, EPI_WARPS);
         abort_flag = 0;
     }
@@ -953,9 +964,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
             if (it > 0) umma::mbar_wait(&empty[(it - 1) % NET_STAGES], ((it - 1) / NET_STAGES) & 1u, WAIT_BUDGET);
         }
     } else {
-        const int quad = warp & 3, half = warp >> 2;
+        const int quad = warp & 3, group = warp >> 2;
         const int row = 32 * quad + lane;                 // of the unit
         const uint32_t tlane = (uint32_t)(32 * quad) << 16;
+        const bool wide = ((uintptr_t)G.out & 31) == 0;   // 32-byte stores
+        float4* const xs = s_x[warp];
         int loaded[2] = {-1, -1};                         // member whose constants a slot holds
         uint32_t job[2] = {0, 0}, met = 0;
         bool ok = true;
@@ -964,135 +977,136 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
             *abort_v = 1;
             ok = false;
         };
-        // the epilogue warps meet (bounded like every wait)
+        // the epilogue warps meet, bounded like every wait
         auto meet = [&] {
             __syncwarp();
             if (lane == 0) umma::mbar_arrive(&epi_bar);
             if (!umma::mbar_wait_or_abort(&epi_bar, met++ & 1u, WAIT_BUDGET, abort_v)) give_up();
         };
-
-        // layer 1 of unit `u` into slot s's A operand
-        auto first_layer = [&](int s, int u) {
-            const int unit = (int)blockIdx.x + u * (int)gridDim.x;
-            const int member = unit / G.tiles, tile = unit - member * G.tiles;
-            float* cst = s_cst[s];
-            if (loaded[s] != member) {
-                meet();                      // no warp reads the last member's constants any more
-                const float* p = G.params[member];
-                for (int i = threadIdx.x; i < 3 * D_H; i += 32 * EPI_WARPS) cst[D_H * (i % 3) + i / 3] = p[i];
-                for (int i = threadIdx.x; i < D_H; i += 32 * EPI_WARPS) {
-                    cst[3 * D_H + i] = p[OFF_B1 + i];
-                    cst[4 * D_H + i] = p[OFF_B2 + i];
-                    cst[5 * D_H + i] = p[OFF_B3 + i];
-                    if (i < D_OUT) cst[6 * D_H + i] = p[OFF_B4 + i];
-                }
-                loaded[s] = member;
-            }
-            // the constants are there, and every warp's output tiles (staged in
-            // this operand) have been read
-            meet();
-            if (!ok) return;
-            const int64_t gr = (int64_t)tile * TILE_M + row;
-            float x0 = 0.f, x1 = 0.f, x2 = 0.f;
-            if (gr < G.n) { x0 = G.x[gr * 3]; x1 = G.x[gr * 3 + 1]; x2 = G.x[gr * 3 + 2]; }
-            for (int c0 = 32 * half; c0 < D_H; c0 += 8 * EPI_WARPS) {
-                __align__(16) bf16 h[32];
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    float b[8], w0[8], w1[8], w2[8];
-                    cst8(cst + 3 * D_H + c0 + 8 * g, b);
-                    cst8(cst + c0 + 8 * g, w0);
-                    cst8(cst + D_H + c0 + 8 * g, w1);
-                    cst8(cst + 2 * D_H + c0 + 8 * g, w2);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const float z = __fmaf_rn(x2, w2[q], __fmaf_rn(x1, w1[q], __fmaf_rn(x0, w0[q], b[q])));
-                        h[8 * g + q] = __float2bfloat16_rn(silu(z));
-                    }
-                }
-                store_a(smem + s * NET_A_BYTES, row, c0, h);
-            }
-            umma::fence_before_sync();
-            stage_done();
-            if (lane == 0) umma::mbar_arrive(&a_ready[s]);
-        };
         auto wait_acc = [&](int s) {
             if (!umma::mbar_wait_or_abort(&acc_full[s], job[s]++ & 1u, WAIT_BUDGET, abort_v)) give_up();
             umma::fence_after_sync();
         };
+        auto operand_ready = [&](int s) {
+            umma::fence_before_sync();
+            stage_done();
+            if (lane == 0) umma::mbar_arrive(&a_ready[s]);
+        };
+        // inputs of the 16 rows whose layer 1 this warp computes, one per lane,
+        // requested a unit ahead
+        const int row1 = 16 * (warp >> 1) + (lane & 15), col1 = 128 * (warp & 1) + 4 * lane;
+        float xn[2][3];
+        auto fetch_x = [&](int s, int u) {
+            const int64_t gr = (int64_t)(((int)blockIdx.x + u * (int)gridDim.x) % G.tiles) * TILE_M + row1;
+            const bool in = u < my_units && gr < G.n;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) xn[s][k] = in ? G.x[gr * 3 + k] : 0.f;
+        };
+        // layer 1 of unit `u` into slot s's operand: 16 rows x 128 columns, four
+        // columns per lane (their weights in registers), the rows' inputs broadcast;
+        // between(k), k = 0..3, runs before each four rows
+        auto first_layer = [&](int s, int u, auto&& between) {
+            const int member = ((int)blockIdx.x + u * (int)gridDim.x) / G.tiles;
+            float* cst = s_cst[s];
+            if (loaded[s] != member) {
+                meet();                      // no warp reads the last member's constants any more
+                const float* p = G.params[member];
+                for (int i = threadIdx.x; i < D_H; i += 32 * EPI_WARPS) {
+                    cst[i] = p[OFF_B2 + i];
+                    cst[D_H + i] = p[OFF_B3 + i];
+                    if (i < D_OUT) cst[2 * D_H + i] = p[OFF_B4 + i];
+                    reinterpret_cast<float4*>(cst + NET_CST_W1)[i] =
+                        make_float4(p[OFF_W1 + 3 * i], p[OFF_W1 + 3 * i + 1], p[OFF_W1 + 3 * i + 2], p[OFF_B1 + i]);
+                }
+                loaded[s] = member;
+                meet();
+                if (!ok) return;
+            }
+            __syncwarp();
+            if (lane < 16) xs[lane] = make_float4(xn[s][0], xn[s][1], xn[s][2], 0.f);
+            __syncwarp();
+            fetch_x(s, u + 2);
+            const float4* w = reinterpret_cast<const float4*>(cst + NET_CST_W1) + col1;
+            const float4 w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
+            uint8_t* blk = smem + s * NET_A_BYTES + (col1 >> 6) * (TILE_M * 128);
+            const uint32_t j = (uint32_t)((col1 & 63) >> 3), e = (uint32_t)(col1 & 7) * 2u;
+            for (int k = 0; k < 4; ++k) {
+                between(k);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int r = 4 * k + i;
+                    const float4 x = xs[r];
+                    auto z = [&](const float4& v) { return __fmaf_rn(x.z, v.z, __fmaf_rn(x.y, v.y, __fmaf_rn(x.x, v.x, v.w))); };
+                    __nv_bfloat162 h[2] = {__floats2bfloat162_rn(silu(z(w0)), silu(z(w1))),
+                                           __floats2bfloat162_rn(silu(z(w2)), silu(z(w3)))};
+                    *reinterpret_cast<uint2*>(blk + sw128((uint32_t)(16 * (warp >> 1) + r), j) + e) =
+                        *reinterpret_cast<uint2*>(h);
+                }
+            }
+            operand_ready(s);
+        };
 
-        for (int s = 0; s < 2 && s < my_units; ++s) first_layer(s, s);
+        fetch_x(0, 0);
+        fetch_x(1, 1);
+        for (int s = 0; s < 2 && s < my_units && ok; ++s) first_layer(s, s, [](int) {});
         for (int u0 = 0; u0 < my_units && ok; u0 += 2) {
+            // layers 2 and 3: accumulator -> bias, SiLU -> next operand
             for (int l = 0; l < 2 && ok; ++l)
                 for (int s = 0; s < 2 && u0 + s < my_units; ++s) {
                     wait_acc(s);
                     if (!ok) break;
-                    const float* b2 = s_cst[s] + (4 + l) * D_H;
-                    for (int c0 = 32 * half; c0 < D_H; c0 += 8 * EPI_WARPS) {
+                    for (int c0 = 32 * group; c0 < D_H; c0 += 8 * EPI_WARPS) {
                         float v[32];
                         umma::tmem_ld32(tmem + s * 256u + tlane + (uint32_t)c0, v);
                         __align__(16) bf16 h[32];
 #pragma unroll
                         for (int g = 0; g < 4; ++g) {
                             float b[8];
-                            cst8(b2 + c0 + 8 * g, b);
+                            cst8(s_cst[s] + l * D_H + c0 + 8 * g, b);
 #pragma unroll
                             for (int q = 0; q < 8; ++q) h[8 * g + q] = __float2bfloat16_rn(silu(v[8 * g + q] + b[q]));
                         }
                         store_a(smem + s * NET_A_BYTES, row, c0, h);
                     }
-                    umma::fence_before_sync();
-                    stage_done();
-                    if (lane == 0) umma::mbar_arrive(&a_ready[s]);
+                    operand_ready(s);
                 }
+            // outputs, then layer 1 of the slot's next unit: the stores drain
+            // under its special functions
             for (int s = 0; s < 2 && u0 + s < my_units && ok; ++s) {
                 wait_acc(s);
                 if (!ok) break;
                 const int unit = (int)blockIdx.x + (u0 + s) * (int)gridDim.x;
                 const int member = unit / G.tiles, tile = unit - member * G.tiles;
-                const float* b4 = s_cst[s] + 6 * D_H;
-                uint8_t* stg = smem + s * NET_A_BYTES + warp * 4096;      // the layer's A operand is consumed
-                for (int c0 = 32 * half; c0 < D_OUT; c0 += 8 * EPI_WARPS) {
-                    float v[32];
-                    umma::tmem_ld32(tmem + s * 256u + tlane + (uint32_t)c0, v);
-                    if (c0 >= 8 * EPI_WARPS && lane == 0) umma::bulk_wait_read0();
-                    __syncwarp();
+                const int64_t gr = (int64_t)tile * TILE_M + row;
+                float* o = G.out + ((int64_t)member * G.n + gr) * D_OUT;
+                const float* b4 = s_cst[s] + 2 * D_H;
+                auto out16 = [&](int k) {
+                    const int c0 = 48 * group + 16 * k;
+                    float v[16];
+                    umma::tmem_ld16(tmem + s * 256u + tlane + (uint32_t)c0, v);
 #pragma unroll
-                    for (int g = 0; g < 4; ++g) {
+                    for (int g = 0; g < 2; ++g) {
                         float b[8];
                         cst8(b4 + c0 + 8 * g, b);
 #pragma unroll
                         for (int q = 0; q < 8; ++q) v[8 * g + q] += b[q];
                     }
-                    if (G.out_f) {
-                        const int64_t gr = (int64_t)tile * TILE_M + row;
-                        float* o = G.out_f + ((int64_t)member * G.n + gr) * D_OUT + c0;
-                        if (gr < G.n) {
-#pragma unroll
-                            for (int i = 0; i < 32; ++i) o[i] = v[i];
-                        }
-                        continue;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 8; ++j)
-                        *reinterpret_cast<float4*>(stg + sw128((uint32_t)lane, (uint32_t)j)) =
-                            make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                    stage_done();
-                    if (lane == 0) {
-                        umma::tma_store_3d(&G.out, c0, tile * TILE_M + 32 * quad, member, stg);
-                        umma::bulk_commit();
-                    }
-                }
-                umma::fence_before_sync();
-                if (u0 + s + 2 < my_units) {
-                    if (lane == 0) umma::bulk_wait_read0();
-                    __syncwarp();
-                    first_layer(s, u0 + s + 2);
+                    if (gr < G.n) store_row16(o + c0, v, wide);
+                };
+                const int nu = u0 + s + 2;
+                if (nu < my_units && ((int)blockIdx.x + nu * (int)gridDim.x) / G.tiles == member) {
+                    // every other warp starts a piece later, so that the stores
+                    // (32 bytes per clock and SM) come evenly
+                    first_layer(s, nu, [&](int k) {
+                        const int c = k - (warp & 1);
+                        if (c >= 0 && c < 3) out16(c);
+                    });
+                } else {
+                    for (int k = 0; k < 3; ++k) out16(k);
+                    if (nu < my_units) first_layer(s, nu, [](int) {});
                 }
             }
         }
-        if (lane == 0) umma::bulk_wait0();
-        __syncwarp();
     }
     __syncthreads();
     if (warp == MMA_WARP) {
@@ -1278,7 +1292,7 @@ int net_forward_enqueue(cl_mlp* const* nets, int members, const float* d_x, floa
                 a.x = d_x + r0 * D_IN;
                 a.n = rows;
                 a.tiles = (int)((rows + TILE_M - 1) / TILE_M);
-                if (!make_out_map(&a.out, out, rows, Kl)) a.out_f = out;
+                a.out = out;
                 const int units = Kl * a.tiles;
                 const int cap = m->max_ctas > 0 && m->max_ctas < m->num_sms ? m->max_ctas : m->num_sms;
                 net_forward<<<(unsigned)(units < cap ? units : cap), GEMM_THREADS, NET_SMEM, st>>>(a);
