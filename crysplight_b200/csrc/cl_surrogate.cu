@@ -325,7 +325,12 @@ __global__ void __launch_bounds__(32 * SAMPLE_WARPS, 8) surrogate_sample(const S
     if (bad) atomicOr(A.err, bad);
 }
 
-// Ensemble reduction: 64 threads per site (one per SiPM), 4 sites per CTA.
+// Ensemble reduction: one warp per site, two SiPMs per lane, all outputs of up
+// to COMBINE_BATCH members requested before the first is used (members beyond
+// them in further batches), no CTA barrier.  The bound is the members' outputs
+// from HBM or L2 (768 bytes per site and member); with 64 threads per site,
+// three loads in flight per thread and two barriers per site the kernel waited
+// on memory: 42,001 sites x 5 members 119 -> 76 us.
 struct CombineArgs {
     const float* raw;        // [K][n][3 * cells] standardised member outputs
     int32_t K;
@@ -344,63 +349,88 @@ struct CombineArgs {
     uint8_t* flag;
 };
 
-constexpr int SITES_PER_CTA = 4;
+constexpr int COMBINE_WARPS = 8;
+constexpr int COMBINE_BATCH = 5;
 
-__global__ void __launch_bounds__(CELLS * SITES_PER_CTA) surrogate_combine(const CombineArgs A)
+__global__ void __launch_bounds__(32 * COMBINE_WARPS) surrogate_combine(const CombineArgs A)
 {
-    __shared__ double red[SITES_PER_CTA][2][2];
-    const int c = threadIdx.x % CELLS;
-    const int s_loc = threadIdx.x / CELLS;
-    const int warp_in_site = c / 32;
-    const float mp = A.y_mean[c], sp = A.y_std[c];
-    const float mt = A.y_mean[CELLS + c], st = A.y_std[CELLS + c];
-    const float ml = A.y_mean[2 * CELLS + c], sl = A.y_std[2 * CELLS + c];
-    for (int64_t s0 = (int64_t)blockIdx.x * SITES_PER_CTA; s0 < A.n; s0 += (int64_t)gridDim.x * SITES_PER_CTA) {
-        const int64_t i = s0 + s_loc;
-        double sum_p = 0.0, sum_p2 = 0.0, sum_t = 0.0, sum_l = 0.0;
-        if (i < A.n) {
-            for (int k = 0; k < A.K; ++k) {
-                const float* row = A.raw + ((int64_t)k * A.n + i) * (3 * CELLS);
-                const double pk = exp((double)row[c] * sp + mp);
-                sum_p += pk;
-                sum_p2 += pk * pk;
-                sum_t += (double)row[CELLS + c] * st + mt;
-                sum_l += (double)row[2 * CELLS + c] * sl + ml;
+    const int lane = threadIdx.x & 31;
+    float mean[3][2], std[3][2];                 // per output kind and SiPM
+#pragma unroll
+    for (int o = 0; o < 3; ++o)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            mean[o][q] = A.y_mean[o * CELLS + 32 * q + lane];
+            std[o][q] = A.y_std[o * CELLS + 32 * q + lane];
+        }
+    const double invK = 1.0 / (double)A.K;
+    const int64_t stride = (int64_t)gridDim.x * COMBINE_WARPS;
+    for (int64_t i = (int64_t)blockIdx.x * COMBINE_WARPS + (threadIdx.x >> 5); i < A.n; i += stride) {
+        double sum_p[2] = {0.0, 0.0}, sum_p2[2] = {0.0, 0.0}, sum_t[2] = {0.0, 0.0}, sum_l[2] = {0.0, 0.0};
+        float dir[2] = {0.f, 0.f};
+        if (A.direct) {
+            dir[0] = A.direct[i * CELLS + lane];
+            dir[1] = A.direct[i * CELLS + 32 + lane];
+        }
+        for (int k0 = 0; k0 < A.K; k0 += COMBINE_BATCH) {
+            float v[COMBINE_BATCH][3][2];
+#pragma unroll
+            for (int k = 0; k < COMBINE_BATCH; ++k) {
+                const float* row = A.raw + ((int64_t)min(k0 + k, A.K - 1) * A.n + i) * (3 * CELLS) + lane;
+#pragma unroll
+                for (int o = 0; o < 3; ++o)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) v[k][o][q] = __ldcs(row + o * CELLS + 32 * q);
+            }
+#pragma unroll
+            for (int k = 0; k < COMBINE_BATCH; ++k) {
+                if (k0 + k >= A.K) break;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const double pk = exp((double)v[k][0][q] * std[0][q] + mean[0][q]);
+                    sum_p[q] += pk;
+                    sum_p2[q] += pk * pk;
+                    sum_t[q] += (double)v[k][1][q] * std[1][q] + mean[1][q];
+                    sum_l[q] += (double)v[k][2][q] * std[2][q] + mean[2][q];
+                }
             }
         }
-        const double invK = 1.0 / (double)A.K;
-        const double pr = sum_p * invK;
-        const double var = fmax(sum_p2 * invK - pr * pr, 0.0);
-        // the first-pass term is the same for every member: it adds to the
-        // mean and to the total the spread is relative to, not to the spread
-        const double pm = pr + (A.direct && i < A.n ? (double)A.direct[i * CELLS + c] : 0.0);
-        double a = sqrt(var), b = pm;
-        for (int o = 16; o > 0; o >>= 1) {
-            a += __shfl_down_sync(0xffffffffu, a, o);
-            b += __shfl_down_sync(0xffffffffu, b, o);
+        double a[2], b[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const double pr = sum_p[q] * invK;
+            const double var = fmax(sum_p2[q] * invK - pr * pr, 0.0);
+            // the first-pass term is the same for every member: it adds to the
+            // mean and to the total the spread is relative to, not to the spread
+            const double pm = pr + (A.direct ? (double)dir[q] : 0.0);
+            a[q] = sqrt(var);
+            b[q] = pm;
+            const int64_t at = i * CELLS + 32 * q + lane;
+            A.p[at] = (float)(pm * (double)A.pde);
+            A.tmean[at] = (float)(sum_t[q] * invK);
+            A.tsig[at] = (float)exp(sum_l[q] * invK);
         }
-        if ((c & 31) == 0) { red[s_loc][warp_in_site][0] = a; red[s_loc][warp_in_site][1] = b; }
-        __syncthreads();
-        if (i < A.n) {
-            A.p[i * CELLS + c] = (float)(pm * (double)A.pde);
-            A.tmean[i * CELLS + c] = (float)(sum_t * invK);
-            A.tsig[i * CELLS + c] = (float)exp(sum_l * invK);
-            if (c == 0) {
-                const double num = red[s_loc][0][0] + red[s_loc][1][0];
-                const double den = red[s_loc][0][1] + red[s_loc][1][1];
-                const float spr = (float)(num / fmax(den, 1e-30));
-                const float x = A.xyz[3 * i], y = A.xyz[3 * i + 1], z = A.xyz[3 * i + 2];
-                float d = fminf(fminf(x, A.L0 - x), fminf(y, A.L1 - y));
-                if (A.front_wrapped) d = fminf(d, z);
-                uint8_t f = 0;
-                if (!(spr <= A.spread_max)) f |= 1u;
-                if (d < A.wall_min_mm) f |= 2u;
-                if (!(den * (double)A.pde < 0.999)) f |= 4u;   // not a probability split: Monte Carlo
-                A.spread[i] = spr;
-                A.flag[i] = f;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                a[q] += __shfl_down_sync(0xffffffffu, a[q], o);
+                b[q] += __shfl_down_sync(0xffffffffu, b[q], o);
             }
+        if (lane == 0) {
+            const double num = a[0] + a[1];
+            const double den = b[0] + b[1];
+            const float spr = (float)(num / fmax(den, 1e-30));
+            const float x = A.xyz[3 * i], y = A.xyz[3 * i + 1], z = A.xyz[3 * i + 2];
+            float d = fminf(fminf(x, A.L0 - x), fminf(y, A.L1 - y));
+            if (A.front_wrapped) d = fminf(d, z);
+            uint8_t f = 0;
+            if (!(spr <= A.spread_max)) f |= 1u;
+            if (d < A.wall_min_mm) f |= 2u;
+            if (!(den * (double)A.pde < 0.999)) f |= 4u;   // not a probability split: Monte Carlo
+            A.spread[i] = spr;
+            A.flag[i] = f;
         }
-        __syncthreads();
     }
 }
 
@@ -423,10 +453,20 @@ __global__ void __launch_bounds__(CELLS * SITES_PER_CTA) surrogate_combine(const
 //           * (arc of the circle inside pixel c) d theta,
 // with the arcs exact (intersections of the circle with the pixel's column
 // and row strips) and theta by composite Gauss-Legendre quadrature (8 panels
-// of 8 nodes up to the critical angle; 64 threads per site, one per node).
-// The nodes' contributions are summed as 2^-40 fixed-point integers, so the
-// result does not depend on the order the threads add them in: a site's
-// term is the same bits in any batch.
+// of 8 nodes up to the critical angle).  The nodes' contributions are summed as
+// 2^-40 fixed-point integers, so the result does not depend on the order they
+// are added in: a site's term is the same bits in any batch.
+//
+// One warp per site.  First every lane takes two nodes and writes the angles at
+// which its circle crosses the edges of the pixel columns and rows it reaches
+// (arc cosines and sines: once per edge, not four per pixel).  A pixel is
+// crossed by a contiguous range of nodes, because the radii increase; the
+// (pixel, node) items of all 64 pixels are then shared out evenly over the
+// lanes (near the face one pixel has all 64 nodes).  The bound is instruction
+// issue.  A lane per pixel kept 11 of 32 lanes active and took 344 us; a thread per
+// node that evaluated four angles and one shared-memory atomic per pixel of its
+// circle's bounding box, four sites per CTA behind common barriers, issued on
+// 49% of its cycles: 42,001 sites 430 -> 204 us.
 // The rest of the light response (reflections, scattering) varies slowly
 // over the SiPM plane; a surrogate trained on it learns what the first-pass
 // term's sharp pixel edges would otherwise ask of it.
@@ -448,51 +488,46 @@ struct DirectArgs {
 
 constexpr int DIRECT_NODES = 64;
 constexpr double DIRECT_FIX = 1099511627776.0;   // 2^40
-constexpr int DIRECT_SITES_PER_CTA = 4;
+constexpr int DIRECT_WARPS = 8;
+constexpr int DIRECT_STRIDE = DIRECT_NODES + 1;  // floats per edge (odd: lanes at different edges on different banks)
 constexpr float TWO_PI_ARC = 6.283185307179586f;
 
-// Length in [0, 2pi) of the circle's azimuths phi with cos(phi) in [ca, cb]
-// and sin(phi) in [sa, sb] (bounds clamped to [-1, 1]).
-__device__ __forceinline__ float arc_in_box(float ca, float cb, float sa, float sb)
+// Shared floats of a warp: the angles of the nx + 1 column and ny + 1 row edges,
+// per node its weight (double), radius and bounding box, per pixel its sum (64
+// bits), first item and first node.
+__host__ __device__ constexpr int direct_warp_floats(int nx, int ny)
 {
-    ca = fminf(fmaxf(ca, -1.0f), 1.0f); cb = fminf(fmaxf(cb, -1.0f), 1.0f);
-    sa = fminf(fmaxf(sa, -1.0f), 1.0f); sb = fminf(fmaxf(sb, -1.0f), 1.0f);
-    const float aa = acosf(ca), ab = acosf(cb);          // ab <= aa
-    const float x1l = ab, x1h = aa, x2l = TWO_PI_ARC - aa, x2h = TWO_PI_ARC - ab;
-    const float ba = asinf(sa), bb = asinf(sb);          // in [-pi/2, pi/2]
-    float y1l, y1h, y2l = 0.0f, y2h = 0.0f;
-    if (ba >= 0.0f) { y1l = ba; y1h = bb; }
-    else if (bb < 0.0f) { y1l = ba + TWO_PI_ARC; y1h = bb + TWO_PI_ARC; }
-    else { y1l = ba + TWO_PI_ARC; y1h = TWO_PI_ARC; y2h = bb; }
-    const float pi = 0.5f * TWO_PI_ARC;
-    const float y3l = pi - bb, y3h = pi - ba;
-    float arc = 0.0f;
-    arc += fmaxf(0.0f, fminf(x1h, y1h) - fmaxf(x1l, y1l));
-    arc += fmaxf(0.0f, fminf(x1h, y2h) - fmaxf(x1l, y2l));
-    arc += fmaxf(0.0f, fminf(x1h, y3h) - fmaxf(x1l, y3l));
-    arc += fmaxf(0.0f, fminf(x2h, y1h) - fmaxf(x2l, y1l));
-    arc += fmaxf(0.0f, fminf(x2h, y2h) - fmaxf(x2l, y2l));
-    arc += fmaxf(0.0f, fminf(x2h, y3h) - fmaxf(x2l, y3l));
-    return arc;
+    return (nx + ny + 2) * DIRECT_STRIDE + (nx + ny) % 2 + 4 * DIRECT_NODES + 4 * CELLS;
 }
 
-__global__ void __launch_bounds__(DIRECT_NODES * DIRECT_SITES_PER_CTA) surrogate_direct(const DirectArgs A)
+__global__ void __launch_bounds__(32 * DIRECT_WARPS) surrogate_direct(const DirectArgs A)
 {
-    __shared__ unsigned long long acc[DIRECT_SITES_PER_CTA][CELLS];
-    const int q = threadIdx.x % DIRECT_NODES;
-    const int s_loc = threadIdx.x / DIRECT_NODES;
-    // this thread's quadrature node: panel q / 8, node q % 8 (mirror pairs)
-    const int panel = q / 8, k = q % 8;
-    const double gx = k < 4 ? -c_gl_x[3 - k] : c_gl_x[k - 4];
-    const double gw = k < 4 ? c_gl_w[3 - k] : c_gl_w[k - 4];
-    const double n1 = A.n1, n2 = A.n2;
-    const double th_max = n2 < n1 ? asin(n2 / n1) : 0.5 * 3.141592653589793;
-    const double t0 = th_max * panel / 8.0, t1 = th_max * (panel + 1) / 8.0;
-    const double th = t0 + 0.5 * (t1 - t0) * (gx + 1.0);
-    const double c = cos(th), sn = sin(th);
-    // Fresnel transmission at the readout face (as fresnel_q2, in Float64)
-    double T = 0.0;
-    {
+    extern __shared__ __align__(16) float s_direct[];
+    __shared__ double s_w[DIRECT_NODES], s_c[DIRECT_NODES];
+    __shared__ float s_tan[DIRECT_NODES];
+    const int lane = threadIdx.x & 31;
+    const int nx = A.nx, ny = A.ny;
+    float* const aa = s_direct + (threadIdx.x >> 5) * direct_warp_floats(nx, ny);   // [edge][node]
+    float* const ba = aa + (nx + 1) * DIRECT_STRIDE;
+    double* const wt = reinterpret_cast<double*>(ba + (ny + 1) * DIRECT_STRIDE + (nx + ny) % 2);   // weight x 2^40
+    unsigned long long* const acc = reinterpret_cast<unsigned long long*>(wt + DIRECT_NODES);
+    float* const rad = reinterpret_cast<float*>(acc + CELLS);
+    uint32_t* const box = reinterpret_cast<uint32_t*>(rad + DIRECT_NODES);
+    int* const item0 = reinterpret_cast<int*>(box + DIRECT_NODES);
+    int* const node0 = item0 + CELLS;
+    if (threadIdx.x < DIRECT_NODES) {
+        const int q = threadIdx.x;
+        // this quadrature node: panel q / 8, node q % 8 (mirror pairs)
+        const int panel = q / 8, k = q % 8;
+        const double gx = k < 4 ? -c_gl_x[3 - k] : c_gl_x[k - 4];
+        const double gw = k < 4 ? c_gl_w[3 - k] : c_gl_w[k - 4];
+        const double n1 = A.n1, n2 = A.n2;
+        const double th_max = n2 < n1 ? asin(n2 / n1) : 0.5 * 3.141592653589793;
+        const double t0 = th_max * panel / 8.0, t1 = th_max * (panel + 1) / 8.0;
+        const double th = t0 + 0.5 * (t1 - t0) * (gx + 1.0);
+        const double c = cos(th), sn = sin(th);
+        // Fresnel transmission at the readout face (as fresnel_R, in Float64)
+        double T = 0.0;
         const double q2 = (n1 / n2) * (n1 / n2);
         const double sin2t = q2 * (1.0 - c * c);
         if (sin2t < 1.0) {
@@ -501,44 +536,125 @@ __global__ void __launch_bounds__(DIRECT_NODES * DIRECT_SITES_PER_CTA) surrogate
             const double b = (n1 * ct - n2 * c) / (n1 * ct + n2 * c);
             T = 1.0 - 0.5 * (a * a + b * b);
         }
+        s_w[q] = 0.5 * (t1 - t0) * gw * T * sn / (4.0 * 3.141592653589793);
+        s_c[q] = c;
+        s_tan[q] = (float)(sn / c);
     }
-    const double w_node = 0.5 * (t1 - t0) * gw * T * sn / (4.0 * 3.141592653589793);
-    const float tan_th = (float)(sn / c);
-    for (int64_t s0 = (int64_t)blockIdx.x * DIRECT_SITES_PER_CTA; s0 < A.n; s0 += (int64_t)gridDim.x * DIRECT_SITES_PER_CTA) {
-        const int64_t i = s0 + s_loc;
-        for (int t = threadIdx.x; t < DIRECT_SITES_PER_CTA * CELLS; t += blockDim.x) (&acc[0][0])[t] = 0ull;
-        __syncthreads();
-        if (i < A.n) {
-            const float x0 = A.xyz[3 * i], y0 = A.xyz[3 * i + 1], z0 = A.xyz[3 * i + 2];
-            const float h = A.L2 - z0;
-            if (h > 0.0f && x0 >= 0.0f && x0 <= A.L0 && y0 >= 0.0f && y0 <= A.L1) {
-                const float wt = (float)(w_node * exp(-(double)A.mu * (double)h / c));
-                const float rho = h * tan_th;
+    __syncthreads();
+    const int64_t stride = (int64_t)gridDim.x * DIRECT_WARPS;
+    for (int64_t i = (int64_t)blockIdx.x * DIRECT_WARPS + (threadIdx.x >> 5); i < A.n; i += stride) {
+        const float x0 = A.xyz[3 * i], y0 = A.xyz[3 * i + 1], z0 = A.xyz[3 * i + 2];
+        const float h = A.L2 - z0;
+        const bool inside = h > 0.0f && x0 >= 0.0f && x0 <= A.L0 && y0 >= 0.0f && y0 <= A.L1;   // warp-uniform
+        if (inside) {
+            // ---- the crossing angles of this lane's two nodes ----
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+                const int q = lane + 32 * m;
+                const float rho = h * s_tan[q];
                 const float inv = 1.0f / rho;
                 int ilo = (int)floorf((x0 - rho) / A.pitch), ihi = (int)floorf((x0 + rho) / A.pitch);
                 int jlo = (int)floorf((y0 - rho) / A.pitch), jhi = (int)floorf((y0 + rho) / A.pitch);
-                ilo = max(ilo, 0); jlo = max(jlo, 0); ihi = min(ihi, A.nx - 1); jhi = min(jhi, A.ny - 1);
-                for (int jj = jlo; jj <= jhi; ++jj) {
-                    const float ya = fminf(jj * A.pitch, A.L1);
-                    const float yb = jj == A.ny - 1 ? A.L1 : fminf((jj + 1) * A.pitch, A.L1);
-                    for (int ii = ilo; ii <= ihi; ++ii) {
-                        const float xa = fminf(ii * A.pitch, A.L0);
-                        const float xb = ii == A.nx - 1 ? A.L0 : fminf((ii + 1) * A.pitch, A.L0);
-                        const float arc = arc_in_box((xa - x0) * inv, (xb - x0) * inv, (ya - y0) * inv,
-                                                     (yb - y0) * inv);
-                        if (arc > 0.0f)
-                            atomicAdd(&acc[s_loc][jj * A.nx + ii],
-                                      __double2ull_rn((double)wt * (double)arc * DIRECT_FIX));
-                    }
+                ilo = max(ilo, 0); jlo = max(jlo, 0); ihi = min(ihi, nx - 1); jhi = min(jhi, ny - 1);
+                for (int e = ilo; e <= ihi + 1; ++e) {
+                    const float xe = e == nx ? A.L0 : fminf(e * A.pitch, A.L0);
+                    aa[e * DIRECT_STRIDE + q] = acosf(fminf(fmaxf((xe - x0) * inv, -1.0f), 1.0f));
                 }
+                for (int e = jlo; e <= jhi + 1; ++e) {
+                    const float ye = e == ny ? A.L1 : fminf(e * A.pitch, A.L1);
+                    ba[e * DIRECT_STRIDE + q] = asinf(fminf(fmaxf((ye - y0) * inv, -1.0f), 1.0f));
+                }
+                wt[q] = (double)(float)(s_w[q] * exp(-(double)A.mu * (double)h / s_c[q])) * DIRECT_FIX;
+                rad[q] = rho;
+                // an empty range (a pixel grid smaller than the face) holds no pixel
+                box[q] = ihi < ilo || jhi < jlo ? 0x00ff00ffu
+                                                : (uint32_t)ilo | (uint32_t)ihi << 8 | (uint32_t)jlo << 16 | (uint32_t)jhi << 24;
             }
         }
-        __syncthreads();
-        for (int t = threadIdx.x; t < DIRECT_SITES_PER_CTA * CELLS; t += blockDim.x) {
-            const int64_t site = s0 + t / CELLS;
-            if (site < A.n) A.out[site * CELLS + t % CELLS] = (float)((double)(&acc[0][0])[t] / DIRECT_FIX);
+        __syncwarp();
+        // ---- the nodes whose circle crosses each pixel: [first, first + count),
+        // from the one that reaches the pixel (and whose bounding box does) to the
+        // last within its farthest corner; two pixels per lane ----
+        int total = 0;
+#pragma unroll
+        for (int m = 0; m < 2; ++m) {
+            const int c = lane + 32 * m, jj = c / nx, ii = c - jj * nx;
+            int first = 0, end = 0;
+            if (inside) {
+                const float xa = ii * A.pitch - x0, xb = (ii == nx - 1 ? A.L0 : (ii + 1) * A.pitch) - x0;
+                const float ya = jj * A.pitch - y0, yb = (jj == ny - 1 ? A.L1 : (jj + 1) * A.pitch) - y0;
+                const float nx_ = fmaxf(fmaxf(xa, -xb), 0.0f), ny_ = fmaxf(fmaxf(ya, -yb), 0.0f);
+                const float fx = fmaxf(fabsf(xa), fabsf(xb)), fy = fmaxf(fabsf(ya), fabsf(yb));
+                const float near2 = (nx_ * nx_ + ny_ * ny_) * 0.999f, far2 = (fx * fx + fy * fy) * 1.001f;
+                auto reached = [&](int q) {
+                    const uint32_t g = box[q];
+                    return rad[q] * rad[q] >= near2 && ii >= (int)(g & 255u) && ii <= (int)((g >> 8) & 255u) &&
+                           jj >= (int)((g >> 16) & 255u) && jj <= (int)(g >> 24);
+                };
+                for (int step = DIRECT_NODES / 2; step > 0; step >>= 1) {
+                    if (!reached(first + step - 1)) first += step;
+                    if (rad[end + step - 1] * rad[end + step - 1] <= far2) end += step;
+                }
+                if (!reached(first)) first = DIRECT_NODES;
+                if (end == DIRECT_NODES - 1 && rad[end] * rad[end] <= far2) end = DIRECT_NODES;
+            }
+            const int count = max(end - first, 0);
+            // items before this pixel's (pixel order)
+            int before = count;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, before, o);
+                if (lane >= o) before += up;
+            }
+            item0[c] = total + before - count;
+            node0[c] = first;
+            total += __shfl_sync(0xffffffffu, before, 31);
+            acc[c] = 0ull;
         }
-        __syncthreads();
+        __syncwarp();
+        // ---- the (pixel, node) items, an equal run of them per lane ----
+        const int per = (total + 31) >> 5;
+        int item = lane * per;
+        const int last = min(item + per, total);
+        if (item < last) {
+            int c = 0;                                // the pixel of the first item: the last one starting at or before it
+            for (int step = CELLS / 2; step > 0; step >>= 1)
+                if (item0[c + step] <= item) c += step;
+            while (item < last) {
+                const int next = c + 1 < CELLS ? item0[c + 1] : total;
+                const int jj = c / nx, ii = c - jj * nx;
+                int q = node0[c] + item - item0[c];
+                const float* pa = aa + ii * DIRECT_STRIDE;
+                const float* pb = ba + jj * DIRECT_STRIDE;
+                unsigned long long sum = 0ull;
+                for (const int stop = min(next, last); item < stop; ++item, ++q) {
+                    // azimuths with cos(phi) between the columns' edges: x1 in
+                    // [0, pi], x2 in [pi, 2 pi]
+                    const float a0 = pa[q], a1 = pa[q + DIRECT_STRIDE];             // a1 <= a0
+                    const float x1l = a1, x1h = a0, x2l = TWO_PI_ARC - a0, x2h = TWO_PI_ARC - a1;
+                    // and sin(phi) between the rows': y1 where it is positive on
+                    // [0, pi/2], y2 around pi, y3 where it is negative on [3 pi/2, 2 pi]
+                    const float b0 = pb[q], b1 = pb[q + DIRECT_STRIDE];             // in [-pi/2, pi/2]
+                    const float pi = 0.5f * TWO_PI_ARC;
+                    const float y1l = fmaxf(b0, 0.0f), y1h = fmaxf(b1, 0.0f);
+                    const float y2l = pi - b1, y2h = pi - b0;
+                    const float y3l = b0 + TWO_PI_ARC, y3h = fminf(b1, 0.0f) + TWO_PI_ARC;
+                    // x1 never meets y3, nor x2 y1
+                    float arc = fmaxf(0.0f, fminf(x1h, y1h) - fmaxf(x1l, y1l));
+                    arc += fmaxf(0.0f, fminf(x1h, y2h) - fmaxf(x1l, y2l));
+                    arc += fmaxf(0.0f, fminf(x2h, y3h) - fmaxf(x2l, y3l));
+                    arc += fmaxf(0.0f, fminf(x2h, y2h) - fmaxf(x2l, y2l));
+                    // wt * arc rounded to an integer: the low bits of the sum with 1.5 2^52
+                    sum += (unsigned long long)__double_as_longlong(fma(wt[q], (double)arc, 0x1.8p52)) -
+                           0x4338000000000000ull;
+                }
+                if (sum) atomicAdd(&acc[c], sum);
+                ++c;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int m = 0; m < 2; ++m) A.out[i * CELLS + lane + 32 * m] = (float)((double)acc[lane + 32 * m] / DIRECT_FIX);
+        __syncwarp();
     }
 }
 
@@ -619,9 +735,9 @@ int cl_surrogate_combine_direct(const float* d_raw, int32_t members, int64_t n_s
     a.front_wrapped = ro->two_sided ? 0 : 1;
     a.pde = pde; a.spread_max = spread_max; a.wall_min_mm = wall_min_mm;
     a.p = d_p; a.tmean = d_tmean; a.tsig = d_tsig; a.spread = d_spread; a.flag = d_flag;
-    const int64_t want = (n_sites + cl::sur::SITES_PER_CTA - 1) / cl::sur::SITES_PER_CTA;
-    const unsigned grid = (unsigned)(want < 148 * 64 ? want : 148 * 64);
-    cl::sur::surrogate_combine<<<grid, cl::sur::CELLS * cl::sur::SITES_PER_CTA, 0, (cudaStream_t)stream>>>(a);
+    const int64_t want = (n_sites + cl::sur::COMBINE_WARPS - 1) / cl::sur::COMBINE_WARPS;
+    const unsigned grid = (unsigned)(want < 148 * 16 ? want : 148 * 16);
+    cl::sur::surrogate_combine<<<grid, 32 * cl::sur::COMBINE_WARPS, 0, (cudaStream_t)stream>>>(a);
     return cudaGetLastError() == cudaSuccess ? CL_OK : CL_ERR_CUDA;
 }
 
@@ -643,10 +759,16 @@ int cl_surrogate_direct(const float* d_xyz, int64_t n_sites, const cl_box* box, 
     a.mu = (float)((std::isinf(op->abs_len_mm) ? 0.0 : 1.0 / (double)op->abs_len_mm) +
                    (std::isinf(op->rayleigh_mm) ? 0.0 : 1.0 / (double)op->rayleigh_mm));
     a.pitch = ro->grid.pitch_mm; a.nx = ro->grid.nx; a.ny = ro->grid.ny; a.out = d_out;
-    const int64_t want = (n_sites + cl::sur::DIRECT_SITES_PER_CTA - 1) / cl::sur::DIRECT_SITES_PER_CTA;
-    const unsigned grid = (unsigned)(want < 148 * 32 ? want : 148 * 32);
-    cl::sur::surrogate_direct<<<grid, cl::sur::DIRECT_NODES * cl::sur::DIRECT_SITES_PER_CTA, 0,
-                                (cudaStream_t)stream>>>(a);
+    const int64_t want = (n_sites + cl::sur::DIRECT_WARPS - 1) / cl::sur::DIRECT_WARPS;
+    const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
+    const size_t smem = cl::sur::DIRECT_WARPS * cl::sur::direct_warp_floats(a.nx, a.ny) * sizeof(float);
+    // 64 x 1 pixels: 144 KB (8 x 8: 46 KB); the opt-in is per device
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(cl::sur::surrogate_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        cudaGetLastError();
+        return CL_ERR_CUDA;
+    }
+    cl::sur::surrogate_direct<<<grid, 32 * cl::sur::DIRECT_WARPS, smem, (cudaStream_t)stream>>>(a);
     return cudaGetLastError() == cudaSuccess ? CL_OK : CL_ERR_CUDA;
 }
 
