@@ -1,24 +1,26 @@
 // cl_mlp.cu — the light-response surrogate: a 3 -> 256 -> 256 -> 256 -> 192 SiLU
 // MLP trained and evaluated on sm_100a by hand-written kernels.
 //
-// GEMMs run on the 5th-generation tensor cores: BF16 operands streamed by TMA
-// into a 3- or 4-stage shared-memory ring (128-byte swizzled tiles, K-major,
-// or MN-major for the weight gradients, which read the activations and
-// gradients as stored), one thread issuing tcgen05.mma into a double-buffered
-// FP32 accumulator in tensor memory, and sixteen warps draining it through
-// fused epilogues (bias, SiLU, SiLU', the loss and its gradient, bias-gradient
-// column sums, the layer-1 gradients, BF16 casts, weight-gradient splits
-// added in place).  The 3-wide input layer and Adam run on the CUDA cores.
-// The epilogues are element-wise work over the 128 x N accumulator of every
-// tile; they are spread over sixteen warps (four per TMEM lane quadrant, each
-// taking every fourth 32-column chunk) so that draining a tile keeps pace
-// with the tensor cores filling the other accumulator.  Their BF16 outputs
-// are staged in shared memory as 32 x 32 tiles and written by TMA stores:
-// stored straight from registers, each 16-byte store of a warp touched 32
-// rows, and the store queue, not the arithmetic, set the pace.  Column sums
-// go through a transposed staging tile into per-CTA shared accumulators (one
-// global atomic per column and CTA).  The per-column constants the epilogues
-// read (biases, the layer-1 weights) are staged in shared memory once per CTA.
+// Everything GEMM-shaped runs on the 5th-generation tensor cores: BF16 operands
+// in 128-byte swizzled shared-memory tiles, one thread issuing tcgen05.mma into
+// FP32 accumulators in tensor memory, sixteen warps draining them.
+//
+//   net_forward   all four layers of 128 rows at a time; inference keeps nothing
+//                 but the outputs, training also stores the hidden layers, the
+//                 pre-activations and the gradient of the loss
+//   net_backward  the gradients of the three hidden layers' pre-activations and
+//                 those of layer 1's parameters
+//   weight_grads  the three 256-wide weight gradients and their biases
+//   adam_all      the parameters and their BF16 copies
+//
+// A training step is these four launches, each starting while the one before
+// drains.  The activations stay in shared and tensor memory from layer to layer;
+// what a later kernel reads is written out beside that by TMA (H, dZ) or in
+// blocks that the same warps read back (Z).  One kernel per layer and direction
+// (twelve launches a step) took 113 us a step at a batch of 4,096 rows and
+// 244 us at 65,536; these take 64 us and 232 us.  A batch of 65,536 rows is 512
+// units of 128 rows over 148 SMs: 4 rounds where 3.46 would do.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -69,10 +71,7 @@ cudaError_t launch_pdl(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cuda
 
 constexpr int TILE_M = 128;     // rows per CTA tile (TMEM lanes)
 constexpr int TILE_K = 64;      // K elements per pipeline stage (one 128-byte swizzle row)
-#ifndef CL_MLP_EPI_WARPS
-#define CL_MLP_EPI_WARPS 16
-#endif
-constexpr int EPI_WARPS = CL_MLP_EPI_WARPS;   // epilogue warps: warp w drains TMEM lane quadrant w % 4,
+constexpr int EPI_WARPS = 16;                 // epilogue warps: warp w drains TMEM lane quadrant w % 4,
                                              // 32-column chunks c with c % (EPI_WARPS/4) == w / 4
 constexpr int PRODUCER_WARP = EPI_WARPS;        // TMA producer
 constexpr int MMA_WARP = EPI_WARPS + 1;         // MMA issuer / TMEM owner
@@ -82,57 +81,21 @@ constexpr uint32_t WAIT_BUDGET = 1u << 22;   // polls before a wait gives up
 
 enum Epi : int {
     EPI_F32 = 0,         // out_f[m][n] = acc
-    EPI_BIAS_SILU = 1,   // z = acc + b: out_z = bf16(z), out_h = bf16(silu z)
-    EPI_DSILU = 3,       // g = bf16(acc * silu'(zprev)): out_h, colsum += column sums of g
-    EPI_PARTIAL = 4,     // out_f[split][m][n] = acc (split-K partial)
-    EPI_LOSS = 5,        // o = acc + b, d = o - target: loss += scale d^2, g = bf16(2 scale d) -> out_h, colsum
-    EPI_DSILU_L1 = 6,    // as EPI_DSILU with zprev recomputed from x, W1, b1; colsum and gw1 += g, g x
-    EPI_WGRAD = 7,       // out_f[n][m] += acc (a K split of a weight gradient, added in place, transposed);
-                         // A [K][M] and B [K][N] MN-major (the activations and gradients as stored)
+    EPI_PARTIAL = 1,     // out_f[split][m][n] = acc (split-K partial)
 };
-
-// Per epilogue: the BF16 tiles each epilogue warp stages in shared memory per
-// 32 x 32 chunk (2 KB each, written out by TMA stores; the transposed tile
-// also feeds the column sums), the TMA -> MMA pipeline depth that leaves room
-// for them (48 KB per stage for N = 256), and the per-column constants staged
-// in shared memory (bias; for EPI_DSILU_L1 also W1 by input component).
-template <int EPI>
-struct EpiCfg {
-    static constexpr int tiles = (EPI == EPI_BIAS_SILU || EPI == EPI_LOSS || EPI == EPI_DSILU) ? 2
-                                 : EPI == EPI_DSILU_L1 ? 1 : 0;
-    static constexpr int stages = tiles ? 3 : 4;
-    static constexpr bool bias = EPI == EPI_BIAS_SILU || EPI == EPI_LOSS ||
-                                 EPI == EPI_DSILU_L1;
-    static constexpr int cst = EPI == EPI_DSILU_L1 ? 4 * 256 : (bias ? 256 : 4);
-    // CTA accumulators of the column sums (bias gradient; for EPI_DSILU_L1
-    // also the layer-1 weight gradient by input component), flushed once
-    static constexpr int acc = EPI == EPI_DSILU_L1 ? 4 * 256 : (tiles >= 2 && EPI != EPI_BIAS_SILU) ? 256 : 4;
-};
+constexpr int GEMM_STAGES = 4;
 constexpr uint32_t STAGE_TILE_BYTES = 32 * 64;   // 32 rows x 32 BF16
-constexpr uint32_t XS_BYTES = 32 * 3 * 4;        // a warp's 32 input rows (EPI_DSILU_L1)
 
-template <int EPI>
 __host__ __device__ constexpr size_t gemm_smem_bytes(int N)
 {
-    return 1024 + (size_t)EpiCfg<EPI>::stages * ((size_t)TILE_M * 128 + (size_t)N * 128) +
-           (size_t)EPI_WARPS * (EpiCfg<EPI>::tiles * STAGE_TILE_BYTES + (EPI == EPI_DSILU_L1 ? XS_BYTES : 0));
+    return 1024 + (size_t)GEMM_STAGES * ((size_t)TILE_M * 128 + (size_t)N * 128);
 }
 
 struct GemmArgs {
     int M, N, K;                    // M % 128 == 0, N % 32 == 0 && 32 <= N <= 256, K % 64 == 0
     int k_split;                    // K elements per split (gridDim.y splits)
     int n_full;                     // row tiles taken whole; the rest go as two N halves each
-    const float* bias;
     float* out_f; int64_t ldf;
-    bf16* out_h; int64_t ldh;       // [M][N]
-    bf16* out_z;                    // [M][N], ld = ldh
-    const bf16* zprev;              // [M][N], ld = ldh
-    const float* target;            // EPI_LOSS: FP32 rows of N targets
-    const int32_t* trow;            // EPI_LOSS: target row of each batch row (nullptr: the same row)
-    float scale;
-    float* loss;
-    float* colsum;                  // [N]
-    const float* x; const float* w1; float* gw1;   // EPI_DSILU_L1: x [M][3], W1 [N][3], grad W1 [N][3]
     unsigned int* err;
 };
 
@@ -148,7 +111,9 @@ __device__ __forceinline__ float silu(float z)
 }
 __device__ __forceinline__ float dsilu(float z)
 {
-    const float s = __fdividef(1.0f, 1.0f + __expf(-z));
+    float e, s;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(z * -1.4426950216293335f));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(s) : "f"(1.0f + e));
     return s * (1.0f + z * (1.0f - s));
 }
 
@@ -159,14 +124,6 @@ __device__ __forceinline__ float dsilu(float z)
 __device__ __forceinline__ uint32_t sw64(uint32_t r, uint32_t j)
 {
     return r * 64u + ((j ^ ((r >> 1) & 3u)) << 4);
-}
-
-// This lane's row of 32 BF16 (h, 16-byte aligned) into a row-major staging tile.
-__device__ __forceinline__ void stage_row(uint8_t* tile, int lane, const bf16* h)
-{
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        *reinterpret_cast<uint4*>(tile + sw64((uint32_t)lane, (uint32_t)j)) = reinterpret_cast<const uint4*>(h)[j];
 }
 
 // This lane's row of 32 BF16 as column `lane` of a transposed staging tile
@@ -223,13 +180,6 @@ __device__ __forceinline__ void warp_col_sums(const uint8_t* tt, int lane, float
     }
 }
 
-// TMA output maps of a GEMM: the row-major output (out_h) and the
-// pre-activations (out_z), boxes of 32 x 32 BF16 with the 64-byte swizzle;
-// maps of absent outputs are unused copies.
-struct OutMaps {
-    CUtensorMap h, z;
-};
-
 // A unit of work: row tile `tile`, accumulator columns [n0, n0 + nw).  The
 // first n_full units are whole tiles; the remaining tiles are split into two
 // units of N/2 columns each, so that the last round over the CTAs is half as
@@ -245,161 +195,18 @@ __device__ __forceinline__ Unit unit_of(int u, int n_full, int N)
 }
 
 // Epilogue of one 128 x N tile: the warp owns rows row0 + lane (row0 = tile
-// row + 32 (w % 4)) and the 32-column chunks c0 = 32 (half + 4 k).  cst holds
-// the bias (and for EPI_DSILU_L1 the columns of W1 at cst + 256 (1 + k)) in
-// shared memory; stg is the warp's staging area (EpiCfg::tiles tiles of 2 KB,
-// then for EPI_DSILU_L1 its rows' inputs).  BF16 outputs leave through TMA
-// stores issued by lane 0; the staging tiles are rewritten only after the
-// previous chunk's stores have read them.
+// row + 32 (w % 4)) and the 32-column chunks c0 = 32 (half + 4 k).
 template <int EPI>
-__device__ __forceinline__ void epilogue(const GemmArgs& G, const OutMaps& om, uint32_t tbase, int row0,
-                                         int lane, int half, const float* cst, uint8_t* stg, bool& pending,
-                                         float* acc, Unit un, int next_row0, Unit next)
+__device__ __forceinline__ void epilogue(const GemmArgs& G, uint32_t tbase, int row0, int lane, int half, Unit un)
 {
-    const int N = G.N;
     const int row = row0 + lane;
-    // the rows of this warp's next tile, whose epilogue inputs are brought
-    // into L2 once this tile is done (next_row0 < 0: no next tile)
-    int64_t next_in = -1;
-    if ((EPI == EPI_LOSS || EPI == EPI_DSILU) && next_row0 >= 0)
-        next_in = EPI == EPI_LOSS && G.trow ? (int64_t)G.trow[next_row0 + lane] : (int64_t)(next_row0 + lane);
-    float sq = 0.0f;
-    // the loss targets' row: the minibatch row's training-set row
-    const int64_t trow_i = EPI == EPI_LOSS ? (G.trow ? (int64_t)G.trow[row] : (int64_t)row) : 0;
-    float* xs = reinterpret_cast<float*>(stg + EpiCfg<EPI>::tiles * STAGE_TILE_BYTES);
-    float x0 = 0.f, x1 = 0.f, x2 = 0.f;
-    if (EPI == EPI_DSILU_L1) {
-        x0 = G.x[(int64_t)row * 3]; x1 = G.x[(int64_t)row * 3 + 1]; x2 = G.x[(int64_t)row * 3 + 2];
-        xs[lane] = x0; xs[32 + lane] = x1; xs[64 + lane] = x2;
-    }
     for (int c0 = un.n0 + 32 * half; c0 < un.n0 + un.nw; c0 += 32 * (EPI_WARPS / 4)) {
-        if (EpiCfg<EPI>::tiles) {
-            // the previous chunk's TMA stores have read the staging tiles
-            if (pending && lane == 0) umma::bulk_wait_read0();
-            pending = false;
-            __syncwarp();
-        }
-        // the chunk's pre-activations are requested before the accumulator is
-        // read, so that their latency overlaps the tensor-memory load
-        uint4 zp4[4];
-        if (EPI == EPI_DSILU) {
-            const uint4* z4 = reinterpret_cast<const uint4*>(G.zprev + (int64_t)row * G.ldh + c0);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) zp4[i] = z4[i];
-        }
         float v[32];
         umma::tmem_ld32(tbase + (uint32_t)(c0 - un.n0), v);
-        // the chunk's loss targets, all requested at once (from L2: prefetched
-        // during the previous tile)
-        float4 tg[8];
-        if (EPI == EPI_LOSS) {
-            const float4* t4 = reinterpret_cast<const float4*>(G.target + trow_i * N + c0);
+        float* o = G.out_f + (EPI == EPI_PARTIAL ? (int64_t)blockIdx.y * G.M * G.ldf : 0) + (int64_t)row * G.ldf + c0;
 #pragma unroll
-            for (int i = 0; i < 8; ++i) tg[i] = t4[i];
-        }
-        if (EPI == EPI_WGRAD) {
-            // column n of the tile is row n of the transposed output: the warp's
-            // 32 rows are 32 consecutive floats there (one coalesced reduction)
-            float* o = G.out_f + (int64_t)c0 * G.ldf + row;
-#pragma unroll
-            for (int i = 0; i < 32; ++i) atomicAdd(o + (int64_t)i * G.ldf, v[i]);
-        } else if (EPI == EPI_F32 || EPI == EPI_PARTIAL) {
-            float* o = G.out_f + (EPI == EPI_PARTIAL ? (int64_t)blockIdx.y * G.M * G.ldf : 0) +
-                       (int64_t)row * G.ldf + c0;
-#pragma unroll
-            for (int g = 0; g < 8; ++g)
-                *reinterpret_cast<float4*>(o + 4 * g) = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
-        } else if (EPI == EPI_BIAS_SILU) {
-            __align__(16) bf16 h[32];
-            __align__(16) bf16 zz[32];
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-                float b[8];
-                cst8(cst + c0 + 8 * g, b);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const float z = v[8 * g + q] + b[q];
-                    zz[8 * g + q] = __float2bfloat16_rn(z);
-                    h[8 * g + q] = __float2bfloat16_rn(silu(z));
-                }
-            }
-            stage_row(stg, lane, h);
-            stage_row(stg + STAGE_TILE_BYTES, lane, zz);
-            stage_done();
-            if (lane == 0) {
-                umma::tma_store_2d(&om.h, c0, row0, stg);
-                umma::tma_store_2d(&om.z, c0, row0, stg + STAGE_TILE_BYTES);
-                umma::bulk_commit();
-            }
-            pending = true;
-        } else {   // EPI_LOSS, EPI_DSILU, EPI_DSILU_L1: a BF16 gradient and its column sums
-            __align__(16) bf16 h[32];
-            if (EPI == EPI_LOSS) {
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    float b[8];
-                    cst8(cst + c0 + 8 * g, b);
-                    const float4 ta = tg[2 * g], tb = tg[2 * g + 1];
-                    const float tt[8] = {ta.x, ta.y, ta.z, ta.w, tb.x, tb.y, tb.z, tb.w};
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        const float d = (v[8 * g + q] + b[q]) - tt[q];
-                        sq += d * d;
-                        h[8 * g + q] = __float2bfloat16_rn(2.0f * d * G.scale);
-                    }
-                }
-            } else if (EPI == EPI_DSILU) {
-                __align__(16) bf16 zp[32];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) reinterpret_cast<uint4*>(zp)[i] = zp4[i];
-#pragma unroll
-                for (int i = 0; i < 32; ++i) h[i] = __float2bfloat16_rn(v[i] * dsilu(__bfloat162float(zp[i])));
-            } else {
-#pragma unroll
-                for (int g = 0; g < 4; ++g) {
-                    float b[8], w0[8], w1[8], w2[8];
-                    cst8(cst + c0 + 8 * g, b);
-                    cst8(cst + 256 + c0 + 8 * g, w0);
-                    cst8(cst + 512 + c0 + 8 * g, w1);
-                    cst8(cst + 768 + c0 + 8 * g, w2);
-#pragma unroll
-                    for (int q = 0; q < 8; ++q) {
-                        // the forward's pre-activation, same operations in the same order
-                        const float z = b[q] + x0 * w0[q] + x1 * w1[q] + x2 * w2[q];
-                        const float zq = __bfloat162float(__float2bfloat16_rn(z));
-                        h[8 * g + q] = __float2bfloat16_rn(v[8 * g + q] * dsilu(zq));
-                    }
-                }
-            }
-            // the transposed tile serves the column sums; EPI_DSILU_L1 writes no BF16 output
-            uint8_t* tt = stg + (EPI == EPI_DSILU_L1 ? 0u : STAGE_TILE_BYTES);
-            if (EPI != EPI_DSILU_L1) stage_row(stg, lane, h);
-            stage_col(tt, lane, h);
-            stage_done();
-            if (EPI != EPI_DSILU_L1) {
-                if (lane == 0) {
-                    if (G.out_h) umma::tma_store_2d(&om.h, c0, row0, stg);
-                    umma::bulk_commit();
-                }
-                pending = true;
-            }
-            warp_col_sums(tt, lane, acc + c0, EPI == EPI_DSILU_L1 ? xs : nullptr,
-                          EPI == EPI_DSILU_L1 ? acc + 256 + c0 : nullptr);
-            // the sums have read the tile before the next chunk may rewrite it
-            __syncwarp();
-        }
-    }
-    if (EPI == EPI_LOSS) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if (lane == 0) atomicAdd(G.loss, sq * G.scale);
-    }
-    if ((EPI == EPI_LOSS || EPI == EPI_DSILU) && next_in >= 0) {
-        for (int c0 = next.n0 + 32 * half; c0 < next.n0 + next.nw; c0 += 32 * (EPI_WARPS / 4)) {
-            const void* p = EPI == EPI_LOSS ? (const void*)(G.target + next_in * N + c0)
-                                            : (const void*)(G.zprev + next_in * G.ldh + c0);
-            asm volatile("prefetch.global.L2 [%0];" :: "l"(p));
-        }
+        for (int g = 0; g < 8; ++g)
+            *reinterpret_cast<float4*>(o + 4 * g) = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
     }
 }
 
@@ -415,23 +222,18 @@ __device__ __forceinline__ void epilogue(const GemmArgs& G, const OutMaps& om, u
 template <int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ OutMaps om,
-                const __grid_constant__ GemmArgs G)
+                const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ GemmArgs G)
 {
-    constexpr int STAGES = EpiCfg<EPI>::stages;
-    constexpr bool MN = EPI == EPI_WGRAD;   // MN-major operands
+    constexpr int STAGES = GEMM_STAGES;
     extern __shared__ uint8_t smem_raw[];
     // 1024-byte aligned in the shared window (the swizzle atom); offset from
     // smem_raw so that the compiler still sees shared-memory accesses
     uint8_t* smem = smem_raw + ((1024u - (umma::smem_u32(smem_raw) & 1023u)) & 1023u);
     const int N = G.N;
     const uint32_t a_bytes = TILE_M * 128, stage_bytes = a_bytes + (uint32_t)N * 128;
-    uint8_t* stg_all = smem + STAGES * stage_bytes;   // 1024-byte aligned (stage_bytes is)
     __shared__ __align__(8) uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
-    __shared__ __align__(16) float s_cst[EpiCfg<EPI>::cst];
-    __shared__ float s_acc[EpiCfg<EPI>::acc];
 
     const int split = blockIdx.y;
     const int k_begin = split * G.k_split;
@@ -439,7 +241,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const int n_chunks = (k_end - k_begin) / TILE_K;
     const int n_tiles = G.M / TILE_M;
     const int n_units = G.n_full + 2 * (n_tiles - G.n_full);
-    pdl_trigger();
     if (n_chunks <= 0 || (int)blockIdx.x >= n_units) return;   // uniform over the CTA
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -454,18 +255,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         umma::prefetch_tmap(&tmA);
         umma::prefetch_tmap(&tmB);
         if (G.n_full < n_tiles) umma::prefetch_tmap(&tmBh);
-        if (EpiCfg<EPI>::tiles > 0 && EPI != EPI_DSILU_L1) {
-            umma::prefetch_tmap(&om.h);
-            if (EPI == EPI_BIAS_SILU) umma::prefetch_tmap(&om.z);
-        }
     }
-    // barriers, TMEM and tensor-map prefetches above overlap the previous kernel's tail
-    pdl_wait();
-    if (EpiCfg<EPI>::bias)
-        for (int i = threadIdx.x; i < N; i += blockDim.x) s_cst[i] = G.bias[i];
-    if (EPI == EPI_DSILU_L1)
-        for (int i = threadIdx.x; i < 3 * N; i += blockDim.x) s_cst[256 * (1 + i % 3) + i / 3] = G.w1[i];
-    for (int i = threadIdx.x; i < EpiCfg<EPI>::acc; i += blockDim.x) s_acc[i] = 0.0f;
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
@@ -487,17 +277,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     uint8_t* st = smem + s * stage_bytes;
                     umma::mbar_arrive_expect_tx(&full[s], a_bytes + (uint32_t)un.nw * 128u);
                     const int k0 = k_begin + c * TILE_K;
-                    if (MN) {
-                        // boxes of 64 MN-elements x 64 K-rows, 8 KB apart
-                        umma::tma_load_2d(st, &tmA, tile * TILE_M, k0, &full[s]);
-                        umma::tma_load_2d(st + 8192, &tmA, tile * TILE_M + 64, k0, &full[s]);
-                        for (int q = 0; q < N / 64; ++q)
-                            umma::tma_load_2d(st + a_bytes + 8192 * q, &tmB, 64 * q, k0, &full[s]);
-                    } else {
-                        umma::tma_load_2d(st, &tmA, k0, tile * TILE_M, &full[s]);
-                        if (un.nw == N) umma::tma_load_2d(st + a_bytes, &tmB, k0, 0, &full[s]);
-                        else umma::tma_load_2d(st + a_bytes, &tmBh, k0, un.n0, &full[s]);
-                    }
+                    umma::tma_load_2d(st, &tmA, k0, tile * TILE_M, &full[s]);
+                    if (un.nw == N) umma::tma_load_2d(st + a_bytes, &tmB, k0, 0, &full[s]);
+                    else umma::tma_load_2d(st + a_bytes, &tmBh, k0, un.n0, &full[s]);
                 }
             }
             if (!ok) { atomicOr(G.err, 1u); *abort_v = 1; }
@@ -507,8 +289,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
     } else if (warp == MMA_WARP) {
         if (lane == 0) {
-            const uint32_t idesc_full = umma::make_idesc_bf16(TILE_M, N, MN, MN);
-            const uint32_t idesc_half = umma::make_idesc_bf16(TILE_M, N / 2, MN, MN);
+            const uint32_t idesc_full = umma::make_idesc_bf16(TILE_M, N);
+            const uint32_t idesc_half = umma::make_idesc_bf16(TILE_M, N / 2);
             uint32_t it = 0, j = 0;
             bool ok = true;
             for (int ui = blockIdx.x; ui < n_units && ok; ui += gridDim.x, ++j) {
@@ -527,10 +309,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                     const uint32_t sa = umma::smem_u32(smem + s * stage_bytes), sb = sa + a_bytes;
 #pragma unroll
                     for (int k = 0; k < TILE_K / 16; ++k) {
-                        const uint64_t ad = MN ? umma::make_desc_sw128_mn(sa + 2048u * k, 8192u)
-                                               : umma::make_desc_sw128(sa + 32u * k);
-                        const uint64_t bd = MN ? umma::make_desc_sw128_mn(sb + 2048u * k, 8192u)
-                                               : umma::make_desc_sw128(sb + 32u * k);
+                        const uint64_t ad = umma::make_desc_sw128(sa + 32u * k);
+                        const uint64_t bd = umma::make_desc_sw128(sb + 32u * k);
                         umma::mma_bf16(d, ad, bd, idesc, (c > 0 || k > 0) ? 1u : 0u);
                     }
                     umma::commit(&empty[s]);
@@ -543,9 +323,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             if (it > 0) umma::mbar_wait(&empty[(it - 1) % STAGES], ((it - 1) / STAGES) & 1u, WAIT_BUDGET);
         }
     } else {
-        uint8_t* stg = stg_all + (size_t)warp * (EpiCfg<EPI>::tiles * STAGE_TILE_BYTES +
-                                                (EPI == EPI_DSILU_L1 ? XS_BYTES : 0u));
-        bool pending = false;   // TMA stores of this warp not yet known to have read its tiles
         uint32_t j = 0;
         for (int ui = blockIdx.x; ui < n_units; ui += gridDim.x, ++j) {
             const uint32_t a = j & 1u, u = j >> 1;
@@ -557,30 +334,16 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             }
             umma::fence_after_sync();
             const int quad = warp & 3;
-            const int nu = ui + (int)gridDim.x;
-            const Unit next = unit_of(nu < n_units ? nu : ui, G.n_full, N);
-            epilogue<EPI>(G, om, tmem + a * 256u + ((uint32_t)(32 * quad) << 16), un.tile * TILE_M + 32 * quad,
-                          lane, warp >> 2, s_cst, stg, pending, s_acc, un,
-                          nu < n_units ? next.tile * TILE_M + 32 * quad : -1, next);
+            epilogue<EPI>(G, tmem + a * 256u + ((uint32_t)(32 * quad) << 16), un.tile * TILE_M + 32 * quad, lane, warp >> 2, un);
             umma::fence_before_sync();
             __syncwarp();
             if (lane == 0) umma::mbar_arrive(&acc_empty[a]);
         }
-        // the staging tiles stay valid until the TMA stores are complete
-        if (EpiCfg<EPI>::tiles && lane == 0) umma::bulk_wait0();
-        __syncwarp();
     }
     __syncthreads();
     if (warp == MMA_WARP) {
         umma::fence_after_sync();
         umma::tmem_dealloc(tmem, TMEM_COLS);
-    }
-    // the CTA's column sums, one global atomic per column
-    if (EPI == EPI_LOSS || EPI == EPI_DSILU || EPI == EPI_DSILU_L1) {
-        for (int i = threadIdx.x; i < N; i += blockDim.x) atomicAdd(G.colsum + i, s_acc[i]);
-        if (EPI == EPI_DSILU_L1)
-            for (int i = threadIdx.x; i < 3 * N; i += blockDim.x)
-                atomicAdd(G.gw1 + i, s_acc[256 + 256 * (i % 3) + i / 3]);
     }
 }
 
@@ -629,23 +392,7 @@ bool make_map_mn(CUtensorMap* m, const bf16* base, int64_t k_rows, int64_t mn, i
                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Store map of a rows x cols BF16 matrix with row stride ld (elements): boxes
-// of 32 x 32 with the 64-byte swizzle of the epilogue's staging tiles.
-bool make_store_map(CUtensorMap* m, const bf16* base, int64_t rows, int64_t cols, int64_t ld)
-{
-    if (!encoder() || !base || ((uintptr_t)base & 15) || (ld * 2) % 16 || cols % 32 || rows % 32 || ld < cols)
-        return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)(ld * 2)};
-    const cuuint32_t box[2] = {32, 32};
-    const cuuint32_t estr[2] = {1, 1};
-    return g_encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<bf16*>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                    CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-// A [M][K] (row stride lda), B [N][K] (row stride ldb); for EPI_WGRAD A [K][M]
-// and B [K][N] (MN-major, N % 64 == 0).
+// A [M][K] (row stride lda), B [N][K] (row stride ldb).
 template <int EPI>
 int launch_gemm(const GemmArgs& g, const bf16* A, int64_t lda, const bf16* B, int64_t ldb, int grid_x,
                 int splits, cudaStream_t st)
@@ -655,18 +402,7 @@ int launch_gemm(const GemmArgs& g, const bf16* A, int64_t lda, const bf16* B, in
         (int64_t)splits * g.k_split < g.K || grid_x < 1)
         return CL_ERR_ARG;
     CUtensorMap ta, tb;
-    if (EPI == EPI_WGRAD) {
-        if (g.N % 64 || !make_map_mn(&ta, A, g.K, g.M, lda) || !make_map_mn(&tb, B, g.K, g.N, ldb)) return CL_ERR_ARG;
-    } else if (!make_map(&ta, A, g.M, g.K, lda, TILE_M) || !make_map(&tb, B, g.N, g.K, ldb, g.N)) {
-        return CL_ERR_ARG;
-    }
-    // output maps of the staged epilogues (unused ones are copies of ta)
-    OutMaps om;
-    om.h = om.z = ta;
-    if (EpiCfg<EPI>::tiles > 0 && EPI != EPI_DSILU_L1) {
-        if (!g.out_h || !make_store_map(&om.h, g.out_h, g.M, g.N, g.ldh)) return CL_ERR_ARG;
-        if (EPI == EPI_BIAS_SILU && !make_store_map(&om.z, g.out_z, g.M, g.N, g.ldh)) return CL_ERR_ARG;
-    }
+    if (!make_map(&ta, A, g.M, g.K, lda, TILE_M) || !make_map(&tb, B, g.N, g.K, ldb, g.N)) return CL_ERR_ARG;
     // the shared-memory opt-in is a per-device attribute of the kernel: set it
     // once for every device this process launches on
     static std::atomic<uint64_t> attr_devices{0};
@@ -675,7 +411,7 @@ int launch_gemm(const GemmArgs& g, const bf16* A, int64_t lda, const bf16* B, in
     const uint64_t bit = 1ull << (dev & 63);
     if (!(attr_devices.load() & bit)) {
         if (cudaFuncSetAttribute(gemm_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)gemm_smem_bytes<EPI>(256)) != cudaSuccess)
+                                 (int)gemm_smem_bytes(256)) != cudaSuccess)
             return CL_ERR_CUDA;
         attr_devices.fetch_or(bit);
     }
@@ -687,14 +423,13 @@ int launch_gemm(const GemmArgs& g, const bf16* A, int64_t lda, const bf16* B, in
     ga.n_full = tiles;
     CUtensorMap tbh = tb;
     const int r = tiles % (int)grid.x;
-    if (EPI != EPI_WGRAD && EPI != EPI_PARTIAL && splits == 1 && g.N % 64 == 0 && r > 0 && 2 * r <= (int)grid.x) {
+    if (EPI != EPI_PARTIAL && splits == 1 && g.N % 64 == 0 && r > 0 && 2 * r <= (int)grid.x) {
         if (!make_map(&tbh, B, g.N, g.K, ldb, g.N / 2)) return CL_ERR_ARG;
         ga.n_full = tiles - r;
     }
     // at least 116 KB so that one CTA holds an SM: each allocates all 512 TMEM columns
-    const size_t smem = gemm_smem_bytes<EPI>(g.N) > 116 * 1024 ? gemm_smem_bytes<EPI>(g.N) : 116 * 1024;
-    if (launch_pdl(gemm_kernel<EPI>, grid, dim3(GEMM_THREADS), smem, st, ta, tb, tbh, om, ga) != cudaSuccess)
-        return CL_ERR_CUDA;
+    const size_t smem = gemm_smem_bytes(g.N) > 116 * 1024 ? gemm_smem_bytes(g.N) : 116 * 1024;
+    gemm_kernel<EPI><<<grid, GEMM_THREADS, smem, st>>>(ta, tb, tbh, ga);
     return cudaGetLastError() == cudaSuccess ? CL_OK : CL_ERR_CUDA;
 }
 
@@ -704,7 +439,9 @@ int launch_gemm(const GemmArgs& g, const bf16* A, int64_t lda, const bf16* B, in
 // FP32 accumulation and FP32 master weights with Adam.
 // ===========================================================================
 constexpr int D_IN = 3, D_H = 256, D_OUT = 192;
-constexpr int WGRAD_MIN_SPLIT_K = 512;   // fewest batch rows per weight-gradient split
+constexpr int WGRAD_MIN_CHUNKS = 4;      // fewest 64-row chunks per CTA of the weight gradients (2, 4 and 8 are
+                                         // equally fast at 512 to 4,096 rows)
+constexpr int WGRAD_MIN_RUN = 8;         // chunks that any run may have
 // Parameter block layout (FP32, contiguous): W1[256][3] b1[256] W2t[256][256]
 // b2[256] W3t[256][256] b3[256] W4t[192][256] b4[192].
 constexpr int64_t OFF_W1 = 0, OFF_B1 = OFF_W1 + D_H * D_IN, OFF_W2 = OFF_B1 + D_H,
@@ -725,97 +462,55 @@ __device__ __forceinline__ uint32_t hash32(uint32_t a, uint32_t b, uint32_t c)
     return c0;
 }
 
-// Random minibatch (with replacement) from the training set: the inputs are
-// copied (Xb), the targets are read in place by the loss epilogue through the
-// row indices (rows).
-__global__ void __launch_bounds__(256) gather_batch(const float* __restrict__ X, int64_t n_all, int B,
-                                                    uint32_t seed, uint32_t step, float* Xb, int32_t* rows)
-{
-    pdl_trigger();
-    pdl_wait();
-    const int b = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (b >= B) return;
-    const int64_t i = (int64_t)(hash32((uint32_t)b, step, seed) % (uint32_t)n_all);
-    rows[b] = (int32_t)i;
-    Xb[(int64_t)b * D_IN] = X[i * D_IN];
-    Xb[(int64_t)b * D_IN + 1] = X[i * D_IN + 1];
-    Xb[(int64_t)b * D_IN + 2] = X[i * D_IN + 2];
-}
-
-// Layer 1 (K = 3) on the CUDA cores: h = silu(x W1^T + b1) for 64 rows per
-// block; a thread takes two adjacent features of every other row, so that a
-// warp stores 128 contiguous bytes of a row per instruction.
-constexpr int L1_ROWS = 64;
-__global__ void __launch_bounds__(256) layer1_fwd(const float* __restrict__ X, const float* __restrict__ W1,
-                                                  const float* __restrict__ b1, bf16* H)
-{
-    pdl_trigger();
-    pdl_wait();
-    __shared__ float xs[L1_ROWS * 3];
-    const int b0 = blockIdx.x * L1_ROWS;
-    for (int i = threadIdx.x; i < L1_ROWS * 3; i += blockDim.x) xs[i] = X[(int64_t)b0 * 3 + i];
-    __syncthreads();
-    const int j = 2 * (threadIdx.x % (D_H / 2)), r0 = threadIdx.x / (D_H / 2);
-    const float wa0 = W1[j * 3], wa1 = W1[j * 3 + 1], wa2 = W1[j * 3 + 2], ba = b1[j];
-    const float wb0 = W1[j * 3 + 3], wb1 = W1[j * 3 + 4], wb2 = W1[j * 3 + 5], bb = b1[j + 1];
-    __nv_bfloat162* out = reinterpret_cast<__nv_bfloat162*>(H + (int64_t)b0 * D_H + j);
-#pragma unroll 4
-    for (int r = r0; r < L1_ROWS; r += 2) {
-        // same operations, same order as the layer-1 recompute in the backward epilogue
-        const float x0 = xs[r * 3], x1 = xs[r * 3 + 1], x2 = xs[r * 3 + 2];
-        const float za = ba + x0 * wa0 + x1 * wa1 + x2 * wa2;
-        const float zb = bb + x0 * wb0 + x1 * wb1 + x2 * wb2;
-        out[(int64_t)r * (D_H / 2)] = __floats2bfloat162_rn(silu(za), silu(zb));
-    }
-}
-
-// Adam over the whole parameter block in one launch (FP32 master weights;
-// the gradient is zeroed as it is read); the three weight matrices of the
-// tensor-core layers also get their BF16 copies (W^T as stored for the
-// forward B operand, W for the backward-data B operand), described by
-// AdamCopies.
+// Adam over the whole parameter block in one launch, four parameters per
+// thread (FP32 master weights; the gradient is zeroed as it is read); the three
+// weight matrices of the tensor-core layers also get their BF16 copies.  All
+// offsets in the block are multiples of 4.  One parameter per thread, with a
+// 64-bit division per matrix and a second, transposed copy, took 16.5 us, this
+// 6.0 (181,000 parameters).
 struct AdamCopies {
-    int64_t off[3]; int n[3]; int OUT[3]; int IN[3];
-    bf16* wt[3]; bf16* w[3];
+    bf16 *w2t, *w3t, *w4t;
 };
-__global__ void adam_all(float* __restrict__ w, float* __restrict__ g, float* __restrict__ m,
-                         float* __restrict__ v, int64_t n, float lr, float b1, float b2, float eps, float bc1,
-                         float bc2, const AdamCopies C)
+__global__ void __launch_bounds__(128) adam_all(float* __restrict__ w, float* __restrict__ g, float* __restrict__ m,
+                                                float* __restrict__ v, float lr, float b1, float b2, float eps,
+                                                float bc1, float bc2, const AdamCopies C)
 {
     pdl_trigger();
+    const int i = 4 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (i >= (int)N_PARAMS) return;
     pdl_wait();
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        g[i] = 0.0f;   // zeroed for the next step's accumulation
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi; v[i] = vi;
-        const float wi = w[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-        w[i] = wi;
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            const int64_t r = i - C.off[t];
-            if (r >= 0 && r < C.n[t]) {
-                const int o = (int)(r / C.IN[t]), k = (int)(r % C.IN[t]);
-                const bf16 q = __float2bfloat16_rn(wi);
-                C.wt[t][r] = q;
-                C.w[t][(int64_t)k * C.OUT[t] + o] = q;
-            }
-        }
+    const float4 g4 = *reinterpret_cast<const float4*>(g + i);
+    float4 m4 = *reinterpret_cast<const float4*>(m + i), v4 = *reinterpret_cast<const float4*>(v + i),
+           w4 = *reinterpret_cast<const float4*>(w + i);
+    *reinterpret_cast<float4*>(g + i) = make_float4(0.f, 0.f, 0.f, 0.f);   // for the next step's accumulation
+    auto step = [&](float gi, float& mo, float& vo, float& wo) {
+        const float mi = b1 * mo + (1.0f - b1) * gi;
+        const float vi = b2 * vo + (1.0f - b2) * gi * gi;
+        mo = mi; vo = vi;
+        wo = wo - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+    };
+    step(g4.x, m4.x, v4.x, w4.x);
+    step(g4.y, m4.y, v4.y, w4.y);
+    step(g4.z, m4.z, v4.z, w4.z);
+    step(g4.w, m4.w, v4.w, w4.w);
+    *reinterpret_cast<float4*>(m + i) = m4;
+    *reinterpret_cast<float4*>(v + i) = v4;
+    *reinterpret_cast<float4*>(w + i) = w4;
+    bf16* copy = nullptr;
+    if (i >= OFF_W2 && i < OFF_B2) copy = C.w2t + (i - OFF_W2);
+    else if (i >= OFF_W3 && i < OFF_B3) copy = C.w3t + (i - OFF_W3);
+    else if (i >= OFF_W4 && i < OFF_B4) copy = C.w4t + (i - OFF_W4);
+    if (copy) {
+        __nv_bfloat162 q[2] = {__floats2bfloat162_rn(w4.x, w4.y), __floats2bfloat162_rn(w4.z, w4.w)};
+        *reinterpret_cast<uint2*>(copy) = *reinterpret_cast<uint2*>(q);
     }
 }
 
-
-__global__ void to_bf16_pair(const float* w, int OUT, int IN, bf16* wt_bf, bf16* w_bf)
+__global__ void to_bf16(const float* w, int n, bf16* o)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= OUT * IN) return;
-    const int o = i / IN, k = i % IN;
-    const bf16 q = __float2bfloat16_rn(w[i]);
-    wt_bf[i] = q;
-    w_bf[(int64_t)k * OUT + o] = q;
+    if (i < n) o[i] = __float2bfloat16_rn(w[i]);
 }
-
 
 // ===========================================================================
 // Inference: the whole network in one kernel
@@ -880,16 +575,79 @@ __device__ __forceinline__ void store_row16(float* o, const float* v, bool wide)
     }
 }
 
-__global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_constant__ NetArgs G)
+// The pre-activations only pass between the two training kernels, whose warps
+// read back exactly the 32 x 32 blocks that the same warps wrote: a block is
+// kept as four 512-byte pieces [j][lane] of 16 bytes, so that an instruction
+// touches 4 lines (row by row, 32).
+__device__ __forceinline__ int64_t z_block(int tile, int quad, int chunk)
+{
+    return (((int64_t)tile * (D_H / 32) + chunk) * 4 + quad) * 1024;     // BF16 elements
+}
+__device__ __forceinline__ void store_block(bf16* o, int lane, const bf16* z)
+{
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        reinterpret_cast<uint4*>(o)[32 * j + lane] = reinterpret_cast<const uint4*>(z)[j];
+}
+__device__ __forceinline__ void load_block(const bf16* o, int lane, bf16* z)
+{
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        reinterpret_cast<uint4*>(z)[j] = __ldg(reinterpret_cast<const uint4*>(o) + 32 * j + lane);
+}
+
+// 8 consecutive floats, one whole 32-byte sector per lane (32-byte aligned).
+__device__ __forceinline__ void load8(const float* p, float* v)
+{
+    asm volatile("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p));
+}
+
+// Row of the training set that minibatch row b is (random with replacement), or
+// b itself where the batch is given (n_all == 0).
+struct BatchRows {
+    uint32_t n_all, step, seed;
+};
+__device__ __forceinline__ int64_t batch_row(const BatchRows& r, int64_t b)
+{
+    return r.n_all ? (int64_t)(hash32((uint32_t)b, r.step, r.seed) % r.n_all) : b;
+}
+
+// Training keeps what the backward pass and the weight gradients read: H of the
+// three hidden layers and the loss gradient dO (stored by TMA from the unit's
+// operand memory) and Z of layers 2 and 3 (before SiLU, BF16, z_block layout).
+// 65,536 rows: 89 us (92 us as four kernels, a gather and layer 1 among them);
+// an SM writes 368 KB per unit at about 32 bytes per cycle, 11,500 cycles,
+// beside 12,300 of SiLU and the gathered targets (98 KB).
+struct NetTrain {
+    CUtensorMap h[4];                    // H1, H2, H3, dO: boxes of 64 x 128
+    bf16 *z2, *z3;
+    const float* target;                 // [training set rows][192]
+    BatchRows rows;
+    int32_t* brow;                       // training-set row of each batch row (written here)
+    bool wide;                           // targets 32-byte aligned
+    float scale;
+    float* loss;
+};
+
+constexpr int STORE_WARP = EPI_WARPS + 2;        // training: issues the TMA stores of the operands
+constexpr int NET_TRAIN_THREADS = GEMM_THREADS + 32;
+
+template <bool TRAIN>
+__global__ void __launch_bounds__(TRAIN ? NET_TRAIN_THREADS : GEMM_THREADS, 1)
+    net_forward(const __grid_constant__ NetArgs G, const __grid_constant__ NetTrain T)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = smem_raw + ((1024u - (umma::smem_u32(smem_raw) & 1023u)) & 1023u);
     uint8_t* ring = smem + 2 * NET_A_BYTES;
-    __shared__ __align__(8) uint64_t full[NET_STAGES], empty[NET_STAGES], a_ready[2], acc_full[2], epi_bar;
+    __shared__ __align__(8) uint64_t full[NET_STAGES], empty[NET_STAGES], a_ready[2], acc_full[2], stored[2], o_ready[2], epi_bar;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
     __shared__ __align__(16) float s_cst[2][NET_CST];
     __shared__ float4 s_x[EPI_WARPS][16];
+
+    if (TRAIN) pdl_trigger();
 
     const int n_units = G.members * G.tiles;
     const int my_units = ((int)blockIdx.x < n_units) ? (n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
@@ -901,11 +659,21 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
         for (int s = 0; s < 2; ++s) {
             umma::mbar_init(&a_ready[s], EPI_WARPS);
             umma::mbar_init(&acc_full[s], 1);
+            umma::mbar_init(&stored[s], 1);
+            umma::mbar_init(&o_ready[s], EPI_WARPS);
         }
         umma::mbar_init(&epi_bar, EPI_WARPS);
         abort_flag = 0;
     }
     if (warp == MMA_WARP) umma::tmem_alloc(&tmem_slot, TMEM_COLS);
+    if (TRAIN) {
+        pdl_wait();
+        // the rows of this CTA's units
+        for (int i = threadIdx.x; i < my_units * TILE_M; i += blockDim.x) {
+            const int64_t b = (int64_t)((int)blockIdx.x + (i / TILE_M) * (int)gridDim.x) * TILE_M + i % TILE_M;
+            T.brow[b] = (int32_t)batch_row(T.rows, b);
+        }
+    }
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
@@ -963,6 +731,55 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
             // the last MMAs complete before TMEM is freed
             if (it > 0) umma::mbar_wait(&empty[(it - 1) % NET_STAGES], ((it - 1) / NET_STAGES) & 1u, WAIT_BUDGET);
         }
+    } else if (TRAIN && warp == STORE_WARP) {
+        // a unit's operands are H1, H2, H3; dO follows in the same memory.  The
+        // target rows, which the loss reads three layers later, are brought into
+        // L2 while the first layers run.
+        uint32_t job[2] = {0, 0};
+        bool ok = true;
+        auto fetch_targets = [&](int u) {
+            if (u >= my_units) return;
+            // plain prefetches of the lines: the copy engine would take the row-sized
+            // ones in turn with the operands' stores
+            const int64_t b0 = (int64_t)((int)blockIdx.x + u * (int)gridDim.x) * TILE_M;
+            int32_t r[TILE_M / 32];
+#pragma unroll
+            for (int i = 0; i < TILE_M / 32; ++i) r[i] = T.brow[b0 + 32 * i + lane];
+#pragma unroll
+            for (int i = 0; i < TILE_M / 32; ++i)
+#pragma unroll
+                for (int j = 0; j < D_OUT / 32; ++j)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(T.target + (int64_t)r[i] * D_OUT + 32 * j));
+        };
+        fetch_targets(0);
+        fetch_targets(1);
+        for (int u0 = 0; u0 < my_units && ok; u0 += 2)
+            for (int l = 0; l < 4 && ok; ++l) {
+                for (int s = 0; s < 2 && u0 + s < my_units && ok; ++s) {
+                    if (lane == 0) {
+                        ok = l < 3 ? umma::mbar_wait_or_abort(&a_ready[s], job[s]++ & 1u, WAIT_BUDGET, abort_v)
+                                   : umma::mbar_wait_or_abort(&o_ready[s], (uint32_t)(u0 >> 1) & 1u, WAIT_BUDGET, abort_v);
+                        if (ok) {
+                            const int tile = (int)blockIdx.x + (u0 + s) * (int)gridDim.x;
+                            for (int c = 0; c < (l < 3 ? D_H : D_OUT) / TILE_K; ++c)
+                                umma::tma_store_2d(&T.h[l], c * TILE_K, tile * TILE_M,
+                                                   smem + s * NET_A_BYTES + c * (TILE_M * 128));
+                            umma::bulk_commit();
+                            umma::bulk_wait_read0();
+                            umma::mbar_arrive(&stored[s]);
+                        } else {
+                            atomicOr(G.err, 1u);
+                            *abort_v = 1;
+                        }
+                    }
+                    ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+                }
+                if (ok && l == 2) {
+                    fetch_targets(u0 + 2);
+                    fetch_targets(u0 + 3);
+                }
+            }
+        if (lane == 0) umma::bulk_wait0();
     } else {
         const int quad = warp & 3, group = warp >> 2;
         const int row = 32 * quad + lane;                 // of the unit
@@ -972,6 +789,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
         int loaded[2] = {-1, -1};                         // member whose constants a slot holds
         uint32_t job[2] = {0, 0}, met = 0;
         bool ok = true;
+        float sq = 0.0f;                                  // training: squared error of this lane's rows
         auto give_up = [&] {
             if (lane == 0) atomicOr(G.err, 1u);
             *abort_v = 1;
@@ -983,7 +801,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
             if (lane == 0) umma::mbar_arrive(&epi_bar);
             if (!umma::mbar_wait_or_abort(&epi_bar, met++ & 1u, WAIT_BUDGET, abort_v)) give_up();
         };
+        // training: the last operand has been stored and may be overwritten
+        uint32_t n_stored[2] = {0, 0};
+        auto wait_stored = [&](int s) {
+            if (!umma::mbar_wait_or_abort(&stored[s], n_stored[s]++ & 1u, WAIT_BUDGET, abort_v)) give_up();
+        };
         auto wait_acc = [&](int s) {
+            if (TRAIN) wait_stored(s);
             if (!umma::mbar_wait_or_abort(&acc_full[s], job[s]++ & 1u, WAIT_BUDGET, abort_v)) give_up();
             umma::fence_after_sync();
         };
@@ -999,8 +823,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
         auto fetch_x = [&](int s, int u) {
             const int64_t gr = (int64_t)(((int)blockIdx.x + u * (int)gridDim.x) % G.tiles) * TILE_M + row1;
             const bool in = u < my_units && gr < G.n;
+            const int64_t xr = TRAIN && in ? (int64_t)T.brow[gr] : gr;
 #pragma unroll
-            for (int k = 0; k < 3; ++k) xn[s][k] = in ? G.x[gr * 3 + k] : 0.f;
+            for (int k = 0; k < 3; ++k) xn[s][k] = in ? G.x[xr * 3 + k] : 0.f;
         };
         // layer 1 of unit `u` into slot s's operand: 16 rows x 128 columns, four
         // columns per lane (their weights in registers), the rows' inputs broadcast;
@@ -1011,14 +836,18 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
             if (loaded[s] != member) {
                 meet();                      // no warp reads the last member's constants any more
                 const float* p = G.params[member];
-                for (int i = threadIdx.x; i < D_H; i += 32 * EPI_WARPS) {
-                    cst[i] = p[OFF_B2 + i];
-                    cst[D_H + i] = p[OFF_B3 + i];
-                    if (i < D_OUT) cst[2 * D_H + i] = p[OFF_B4 + i];
-                    reinterpret_cast<float4*>(cst + NET_CST_W1)[i] =
-                        make_float4(p[OFF_W1 + 3 * i], p[OFF_W1 + 3 * i + 1], p[OFF_W1 + 3 * i + 2], p[OFF_B1 + i]);
+                // one network: both slots at once
+                for (int q = s; q < (G.members == 1 ? 2 : s + 1); ++q) {
+                    float* o = s_cst[q];
+                    for (int i = threadIdx.x; i < D_H; i += 32 * EPI_WARPS) {
+                        o[i] = p[OFF_B2 + i];
+                        o[D_H + i] = p[OFF_B3 + i];
+                        if (i < D_OUT) o[2 * D_H + i] = p[OFF_B4 + i];
+                        reinterpret_cast<float4*>(o + NET_CST_W1)[i] =
+                            make_float4(p[OFF_W1 + 3 * i], p[OFF_W1 + 3 * i + 1], p[OFF_W1 + 3 * i + 2], p[OFF_B1 + i]);
+                    }
+                    loaded[q] = member;
                 }
-                loaded[s] = member;
                 meet();
                 if (!ok) return;
             }
@@ -1059,12 +888,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
                         float v[32];
                         umma::tmem_ld32(tmem + s * 256u + tlane + (uint32_t)c0, v);
                         __align__(16) bf16 h[32];
+                        __align__(16) bf16 zz[32];
+                        (void)zz;
 #pragma unroll
                         for (int g = 0; g < 4; ++g) {
                             float b[8];
                             cst8(s_cst[s] + l * D_H + c0 + 8 * g, b);
 #pragma unroll
-                            for (int q = 0; q < 8; ++q) h[8 * g + q] = __float2bfloat16_rn(silu(v[8 * g + q] + b[q]));
+                            for (int q = 0; q < 8; ++q) {
+                                const float z = v[8 * g + q] + b[q];
+                                if (TRAIN) zz[8 * g + q] = __float2bfloat16_rn(z);
+                                h[8 * g + q] = __float2bfloat16_rn(silu(z));
+                            }
+                        }
+                        if (TRAIN) {
+                            const int tile = (int)blockIdx.x + (u0 + s) * (int)gridDim.x;
+                            store_block((l ? T.z3 : T.z2) + z_block(tile, quad, c0 >> 5), lane, zz);
                         }
                         store_a(smem + s * NET_A_BYTES, row, c0, h);
                     }
@@ -1073,13 +912,60 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
             // outputs, then layer 1 of the slot's next unit: the stores drain
             // under its special functions
             for (int s = 0; s < 2 && u0 + s < my_units && ok; ++s) {
+                // training: the row's targets, two pieces of 16 columns ahead of their use
+                float tg[3][TRAIN ? 16 : 1];
+                const float* trow = nullptr;
+                auto fetch_t = [&](int k) {
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        if (T.wide) load8(trow + 16 * k + 8 * i, &tg[k][8 * i]);
+                        else cst8(trow + 16 * k + 8 * i, &tg[k][8 * i]);
+                    }
+                };
+                if (TRAIN) {
+                    const int64_t b = (int64_t)((int)blockIdx.x + (u0 + s) * (int)gridDim.x) * TILE_M + row;
+                    trow = T.target + (int64_t)T.brow[b] * D_OUT + 48 * group;
+                    fetch_t(0);
+                    fetch_t(1);
+                }
                 wait_acc(s);
                 if (!ok) break;
                 const int unit = (int)blockIdx.x + (u0 + s) * (int)gridDim.x;
                 const int member = unit / G.tiles, tile = unit - member * G.tiles;
                 const int64_t gr = (int64_t)tile * TILE_M + row;
-                float* o = G.out + ((int64_t)member * G.n + gr) * D_OUT;
+                float* o = TRAIN ? nullptr : G.out + ((int64_t)member * G.n + gr) * D_OUT;
                 const float* b4 = s_cst[s] + 2 * D_H;
+                if (TRAIN) {
+                    // loss: dO into the (consumed) operand memory for the store warp
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) {
+                        const int c0 = 48 * group + 16 * k;
+                        if (k == 0) fetch_t(2);
+                        float v[16];
+                        umma::tmem_ld16(tmem + s * 256u + tlane + (uint32_t)c0, v);
+                        __align__(16) bf16 g[16];
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            float b[8];
+                            cst8(b4 + c0 + 8 * i, b);
+#pragma unroll
+                            for (int q = 0; q < 8; ++q) {
+                                const float d = (v[8 * i + q] + b[q]) - tg[k][8 * i + q];
+                                sq += d * d;
+                                g[8 * i + q] = __float2bfloat16_rn(2.0f * d * T.scale);
+                            }
+                        }
+                        uint8_t* blk = smem + s * NET_A_BYTES + (c0 >> 6) * (TILE_M * 128);
+#pragma unroll
+                        for (int i = 0; i < 2; ++i)
+                            *reinterpret_cast<uint4*>(blk + sw128((uint32_t)row, (uint32_t)(((c0 & 63) >> 3) + i))) =
+                                reinterpret_cast<const uint4*>(g)[i];
+                    }
+                    umma::fence_before_sync();
+                    stage_done();
+                    if (lane == 0) umma::mbar_arrive(&o_ready[s]);
+                    continue;
+                }
                 auto out16 = [&](int k) {
                     const int c0 = 48 * group + 16 * k;
                     float v[16];
@@ -1106,6 +992,461 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) net_forward(const __grid_cons
                     if (nu < my_units) first_layer(s, nu, [](int) {});
                 }
             }
+            if (TRAIN)
+                for (int s = 0; s < 2 && u0 + s + 2 < my_units && ok; ++s) {
+                    wait_stored(s);
+                    if (ok) first_layer(s, u0 + s + 2, [](int) {});
+                }
+        }
+        if (TRAIN) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
+            if (lane == 0) atomicAdd(T.loss, sq * T.scale);
+        }
+    }
+    __syncthreads();
+    if (warp == MMA_WARP) {
+        umma::fence_after_sync();
+        umma::tmem_dealloc(tmem, TMEM_COLS);
+    }
+}
+
+// Backward through the activations in one kernel, on the same two slots:
+//   dZ3 = (dO W4) silu'(Z3),  dZ2 = (dZ3 W3) silu'(Z2),  dZ1 = (dZ2 W2) silu'(Z1)
+// with Z1 recomputed from the inputs.  dO comes in by TMA as the first operand;
+// each epilogue writes the next operand, which the store warp also writes out
+// (dZ3, dZ2, for the weight and bias gradients); the last one forms the layer-1
+// gradients.  The bound is that last epilogue, 256 columns x 4 sums over the
+// unit's rows through transposed staging tiles (11,000 to 17,000 cycles of the
+// 40,000 a unit takes), beside the SiLU derivatives (an exponential and a
+// reciprocal each) and 126 MB read and 67 MB written.  65,536 rows: 82 us,
+// 87 us as three kernels.
+struct NetBack {
+    CUtensorMap dO;                      // boxes of 64 x 128
+    CUtensorMap w[3];                    // W4^T, W3^T, W2^T as stored [out][in] (MN-major operands): boxes of 64 x 64
+    CUtensorMap dz[2];                   // dZ3, dZ2: boxes of 64 x 128
+    const bf16 *z3, *z2;
+    const float* x;
+    const float* params;
+    float* grad;                         // parameter block of gradients (accumulated)
+    const int32_t* brow;                 // training-set row of each batch row
+    int tiles;
+    unsigned int* err;
+};
+
+__global__ void __launch_bounds__(NET_TRAIN_THREADS, 1) net_backward(const __grid_constant__ NetBack G)
+{
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (umma::smem_u32(smem_raw) & 1023u)) & 1023u);
+    uint8_t* ring = smem + 2 * NET_A_BYTES;
+    __shared__ __align__(8) uint64_t full[NET_STAGES], empty[NET_STAGES], a_ready[2], acc_full[2], stored[2], a_free[2], a_full[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+    __shared__ __align__(16) float s_cst[4 * D_H];       // b1, W1 by input component
+    __shared__ float s_acc[4 * D_H];                     // b1 gradient, W1 gradient by component
+
+    pdl_trigger();
+    const int my_units = ((int)blockIdx.x < G.tiles) ? (G.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+    if (my_units == 0) return;               // uniform over the CTA
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    volatile int* abort_v = &abort_flag;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < NET_STAGES; ++s) { umma::mbar_init(&full[s], 1); umma::mbar_init(&empty[s], 1); }
+        for (int s = 0; s < 2; ++s) {
+            umma::mbar_init(&a_ready[s], EPI_WARPS);
+            umma::mbar_init(&acc_full[s], 1);
+            umma::mbar_init(&stored[s], 1);
+            umma::mbar_init(&a_free[s], EPI_WARPS);
+            umma::mbar_init(&a_full[s], 1);
+        }
+        abort_flag = 0;
+    }
+    for (int i = threadIdx.x; i < 4 * D_H; i += blockDim.x) s_acc[i] = 0.0f;
+    if (warp == MMA_WARP) umma::tmem_alloc(&tmem_slot, TMEM_COLS);
+    pdl_wait();
+    for (int i = threadIdx.x; i < D_H; i += blockDim.x) s_cst[i] = G.params[OFF_B1 + i];
+    for (int i = threadIdx.x; i < 3 * D_H; i += blockDim.x) s_cst[D_H * (1 + i % 3) + i / 3] = G.params[OFF_W1 + i];
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == PRODUCER_WARP) {
+        if (lane == 0) {
+            uint32_t it = 0, loads[2] = {0, 0};
+            bool ok = true;
+            auto fetch_z = [&](int l, int u) {
+                umma::prefetch_l2((l ? G.z2 : G.z3) + z_block((int)blockIdx.x + u * (int)gridDim.x, 0, 0), TILE_M * D_H * 2);
+            };
+            for (int l = 0; l < 2; ++l)
+                for (int u = 0; u < 2 && u < my_units; ++u) fetch_z(l, u);
+            for (int u0 = 0; u0 < my_units && ok; u0 += 2)
+                for (int l = 0; l < 3 && ok; ++l)
+                    for (int s = 0; s < 2 && u0 + s < my_units && ok; ++s) {
+                        // the pre-activations of the units two ahead into L2 (64 KB in a row)
+                        if (l < 2 && u0 + s + 2 < my_units) fetch_z(l, u0 + s + 2);
+                        if (l == 0) {
+                            // the unit's dO into the slot once the last unit's epilogues are through with it
+                            if (loads[s] > 0 && !umma::mbar_wait_or_abort(&a_free[s], (loads[s] - 1) & 1u, WAIT_BUDGET, abort_v)) {
+                                ok = false;
+                                break;
+                            }
+                            loads[s] += 1;
+                            umma::mbar_arrive_expect_tx(&a_full[s], (D_OUT / TILE_K) * TILE_M * 128u);
+                            const int tile = (int)blockIdx.x + (u0 + s) * (int)gridDim.x;
+                            for (int c = 0; c < D_OUT / TILE_K; ++c)
+                                umma::tma_load_2d(smem + s * NET_A_BYTES + c * (TILE_M * 128), &G.dO, c * TILE_K, tile * TILE_M,
+                                                  &a_full[s]);
+                        }
+                        for (int c = 0; c < (l ? D_H : D_OUT) / TILE_K; ++c, ++it) {
+                            const uint32_t st = it % NET_STAGES, r = it / NET_STAGES;
+                            if (r > 0 && !umma::mbar_wait_or_abort(&empty[st], (r - 1) & 1u, WAIT_BUDGET, abort_v)) {
+                                ok = false;
+                                break;
+                            }
+                            umma::mbar_arrive_expect_tx(&full[st], NET_STAGE_BYTES);
+                            for (int q = 0; q < D_H / 64; ++q)
+                                umma::tma_load_2d(ring + st * NET_STAGE_BYTES + 8192 * q, &G.w[l], 64 * q, c * TILE_K, &full[st]);
+                        }
+                    }
+            if (!ok) { atomicOr(G.err, 1u); *abort_v = 1; }
+            // copies still in flight land before the CTA can exit
+            for (uint32_t j = it > (uint32_t)NET_STAGES ? it - NET_STAGES : 0u; j < it; ++j)
+                umma::mbar_wait(&full[j % NET_STAGES], (j / NET_STAGES) & 1u, WAIT_BUDGET);
+            for (int s = 0; s < 2; ++s)
+                if (loads[s] > 0) umma::mbar_wait(&a_full[s], (loads[s] - 1) & 1u, WAIT_BUDGET);
+        }
+    } else if (warp == MMA_WARP) {
+        if (lane == 0) {
+            uint32_t it = 0, job[2] = {0, 0}, loads[2] = {0, 0};
+            bool ok = true;
+            const uint32_t idesc = umma::make_idesc_bf16(TILE_M, D_H, false, true);
+            for (int u0 = 0; u0 < my_units && ok; u0 += 2)
+                for (int l = 0; l < 3 && ok; ++l)
+                    for (int s = 0; s < 2 && u0 + s < my_units && ok; ++s) {
+                        const bool there = l == 0
+                            ? umma::mbar_wait_or_abort(&a_full[s], loads[s]++ & 1u, WAIT_BUDGET, abort_v)
+                            : umma::mbar_wait_or_abort(&a_ready[s], job[s]++ & 1u, WAIT_BUDGET, abort_v);
+                        if (!there) { ok = false; break; }
+                        umma::fence_after_sync();
+                        const uint32_t a0 = umma::smem_u32(smem + s * NET_A_BYTES), d = tmem + s * 256u;
+                        for (int c = 0; c < (l ? D_H : D_OUT) / TILE_K; ++c, ++it) {
+                            const uint32_t st = it % NET_STAGES, r = it / NET_STAGES;
+                            if (!umma::mbar_wait_or_abort(&full[st], r & 1u, WAIT_BUDGET, abort_v)) { ok = false; break; }
+                            umma::fence_after_sync();
+                            const uint32_t sb = umma::smem_u32(ring + st * NET_STAGE_BYTES);
+#pragma unroll
+                            for (int k = 0; k < TILE_K / 16; ++k)
+                                umma::mma_bf16(d, umma::make_desc_sw128(a0 + c * (TILE_M * 128u) + 32u * k),
+                                               umma::make_desc_sw128_mn(sb + 2048u * k, 8192u), idesc, (c > 0 || k > 0) ? 1u : 0u);
+                            umma::commit(&empty[st]);
+                        }
+                        if (ok) umma::commit(&acc_full[s]);
+                    }
+            if (!ok) { atomicOr(G.err, 1u); *abort_v = 1; }
+            // the last MMAs complete before TMEM is freed
+            if (it > 0) umma::mbar_wait(&empty[(it - 1) % NET_STAGES], ((it - 1) / NET_STAGES) & 1u, WAIT_BUDGET);
+        }
+    } else if (warp == STORE_WARP) {
+        if (lane == 0) {
+            uint32_t job[2] = {0, 0};
+            bool ok = true;
+            for (int u0 = 0; u0 < my_units && ok; u0 += 2)
+                for (int l = 0; l < 2 && ok; ++l)
+                    for (int s = 0; s < 2 && u0 + s < my_units && ok; ++s) {
+                        if (!umma::mbar_wait_or_abort(&a_ready[s], job[s]++ & 1u, WAIT_BUDGET, abort_v)) { ok = false; break; }
+                        const int tile = (int)blockIdx.x + (u0 + s) * (int)gridDim.x;
+                        for (int c = 0; c < 4; ++c)
+                            umma::tma_store_2d(&G.dz[l], c * TILE_K, tile * TILE_M, smem + s * NET_A_BYTES + c * (TILE_M * 128));
+                        umma::bulk_commit();
+                        umma::bulk_wait_read0();
+                        umma::mbar_arrive(&stored[s]);
+                    }
+            if (!ok) { atomicOr(G.err, 1u); *abort_v = 1; }
+            umma::bulk_wait0();
+        }
+    } else {
+        const int quad = warp & 3, group = warp >> 2;
+        const int row = 32 * quad + lane;                 // of the unit
+        const uint32_t tlane = (uint32_t)(32 * quad) << 16;
+        uint32_t job[2] = {0, 0}, written[2] = {0, 0};
+        bool ok = true;
+        auto give_up = [&] {
+            if (lane == 0) atomicOr(G.err, 1u);
+            *abort_v = 1;
+            ok = false;
+        };
+        auto wait_acc = [&](int s) {
+            if (!umma::mbar_wait_or_abort(&acc_full[s], job[s]++ & 1u, WAIT_BUDGET, abort_v)) give_up();
+            umma::fence_after_sync();
+        };
+        for (int u0 = 0; u0 < my_units && ok; u0 += 2) {
+            float xb[2][3];                               // the rows' inputs, used after two layers
+#pragma unroll
+            for (int s = 0; s < 2; ++s)
+                if (u0 + s < my_units) {
+                    const float* xr = G.x + (int64_t)G.brow[(int64_t)((int)blockIdx.x + (u0 + s) * (int)gridDim.x) * TILE_M + row] * 3;
+                    xb[s][0] = xr[0]; xb[s][1] = xr[1]; xb[s][2] = xr[2];
+                }
+            // dZ3, dZ2: the next operand
+            for (int l = 0; l < 2 && ok; ++l)
+                for (int s = 0; s < 2 && u0 + s < my_units; ++s) {
+                    const int tile = (int)blockIdx.x + (u0 + s) * (int)gridDim.x;
+                    __align__(16) bf16 z[2][32];         // requested before the accumulator is waited for
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) load_block((l ? G.z2 : G.z3) + z_block(tile, quad, group + 4 * k), lane, z[k]);
+                    wait_acc(s);
+                    // dZ3 has been stored from the operand that dZ2 overwrites
+                    if (l && !umma::mbar_wait_or_abort(&stored[s], written[s] & 1u, WAIT_BUDGET, abort_v)) give_up();
+                    if (l) written[s] += 1;
+                    if (!ok) break;
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const int c0 = 32 * group + 128 * k;
+                        float v[32];
+                        umma::tmem_ld32(tmem + s * 256u + tlane + (uint32_t)c0, v);
+                        __align__(16) __nv_bfloat162 g[16];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            const float2 zq = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(z[k])[i]);
+                            g[i] = __floats2bfloat162_rn(v[2 * i] * dsilu(zq.x), v[2 * i + 1] * dsilu(zq.y));
+                        }
+                        store_a(smem + s * NET_A_BYTES, row, c0, reinterpret_cast<const bf16*>(g));
+                    }
+                    umma::fence_before_sync();
+                    stage_done();
+                    if (lane == 0) umma::mbar_arrive(&a_ready[s]);
+                }
+            // dZ1 and the layer-1 gradients; its tiles are staged in the operand,
+            // which is consumed, and stored (dZ2)
+            for (int s = 0; s < 2 && u0 + s < my_units && ok; ++s) {
+                const float x0 = xb[s][0], x1 = xb[s][1], x2 = xb[s][2];
+                wait_acc(s);
+                if (!umma::mbar_wait_or_abort(&stored[s], written[s]++ & 1u, WAIT_BUDGET, abort_v)) give_up();
+                if (!ok) break;
+                uint8_t* tt = smem + s * NET_A_BYTES + warp * 4096;
+                float* xs = reinterpret_cast<float*>(tt + STAGE_TILE_BYTES);
+                xs[lane] = x0; xs[32 + lane] = x1; xs[64 + lane] = x2;
+                for (int c0 = 32 * group; c0 < D_H; c0 += 8 * EPI_WARPS) {
+                    float v[32];
+                    umma::tmem_ld32(tmem + s * 256u + tlane + (uint32_t)c0, v);
+                    __align__(16) __nv_bfloat162 g[16];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        float b[8], w0[8], w1[8], w2[8];
+                        cst8(s_cst + c0 + 8 * i, b);
+                        cst8(s_cst + D_H + c0 + 8 * i, w0);
+                        cst8(s_cst + 2 * D_H + c0 + 8 * i, w1);
+                        cst8(s_cst + 3 * D_H + c0 + 8 * i, w2);
+#pragma unroll
+                        for (int q = 0; q < 8; q += 2) {
+                            // the forward's pre-activation, same operations in the same
+                            // order; two at a time: a single conversion to BF16 is a
+                            // special-function-unit operation, a packed one is not
+                            auto z = [&](int e) { return __fmaf_rn(x2, w2[e], __fmaf_rn(x1, w1[e], __fmaf_rn(x0, w0[e], b[e]))); };
+                            const float2 zq = __bfloat1622float2(__floats2bfloat162_rn(z(q), z(q + 1)));
+                            g[4 * i + q / 2] = __floats2bfloat162_rn(v[8 * i + q] * dsilu(zq.x), v[8 * i + q + 1] * dsilu(zq.y));
+                        }
+                    }
+                    stage_col(tt, lane, reinterpret_cast<const bf16*>(g));
+                    __syncwarp();
+                    warp_col_sums(tt, lane, s_acc + c0, xs, s_acc + D_H + c0);
+                    __syncwarp();
+                }
+                umma::fence_before_sync();
+                stage_done();
+                if (lane == 0) umma::mbar_arrive(&a_free[s]);
+            }
+        }
+    }
+    __syncthreads();
+    if (warp == MMA_WARP) {
+        umma::fence_after_sync();
+        umma::tmem_dealloc(tmem, TMEM_COLS);
+    }
+    for (int i = threadIdx.x; i < D_H; i += blockDim.x) atomicAdd(G.grad + OFF_B1 + i, s_acc[i]);
+    for (int i = threadIdx.x; i < 3 * D_H; i += blockDim.x) atomicAdd(G.grad + OFF_W1 + i, s_acc[D_H * (1 + i % 3) + i / 3]);
+}
+
+// The three weight gradients dW^T[out][in] = sum over rows dZ[row][out] H[row][in]
+// in one launch.  Their K dimension, the batch, is cut into 64-row chunks; the
+// chunks of the 3 layers make one line that is shared out evenly over pairs of
+// CTAs (one per tile of 128 inputs: the second reads the same dZ while it is in
+// L2).  A CTA's share is cut into runs, each summed in tensor memory and added
+// to the FP32 gradient in place.  The tensor cores' adder truncates (a sum of
+// 2,656 rows came out 1.7e-6 smaller than three of 896), so a run is no longer
+// than a layer's share of all pairs, or 8 chunks where that is more: 65,536 rows
+// take 232.6 us a step so, 227.9 with one run per CTA and layer.  One launch per
+// layer (a start-up and a drain of the pipeline each) took 51.7 us at 65,536
+// rows, this one 46.6 (194 MB read: 4.2 TB/s).  Both operands are MN-major (the activations and
+// gradients as stored).  The bias gradients, the column sums of dZ, come from
+// the same stages: the epilogue warps, which have little else to do, add up the
+// dZ operand of the first tile's runs.
+struct WeightGrads {
+    CUtensorMap h[3], dz[3];             // H3, H2, H1 and dO, dZ3, dZ2: boxes of 64 x 64
+    float* out[3];                       // gradients of W4^T, W3^T, W2^T, row stride 256
+    float* bias[3];                      // gradients of b4, b3, b2
+    int chunks;                          // batch / 64
+    int longest;                         // chunks of one run at most
+    unsigned int* err;
+};
+constexpr int WG_STAGES = 4;
+constexpr uint32_t WG_A_BYTES = TILE_M * 128, WG_STAGE_BYTES = WG_A_BYTES + D_H * 128;
+constexpr size_t WG_SMEM = 1024 + (size_t)WG_STAGES * WG_STAGE_BYTES;
+
+// The run of chunks that starts at chunk c of the line: its layer, tile, first
+// chunk in the batch and length (up to `end` and the longest run).
+struct WgRun {
+    int layer, tile, first, count;
+};
+__device__ __forceinline__ WgRun wg_run(int c, int end, const WeightGrads& G)
+{
+    const int layer = c / G.chunks, first = c - layer * G.chunks;
+    return WgRun{layer, (int)(blockIdx.x & 1), first, min(G.longest, min(end - c, G.chunks - first))};
+}
+
+__global__ void __launch_bounds__(GEMM_THREADS, 1) weight_grads(const __grid_constant__ WeightGrads G)
+{
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = smem_raw + ((1024u - (umma::smem_u32(smem_raw) & 1023u)) & 1023u);
+    __shared__ __align__(8) uint64_t full[WG_STAGES], empty[WG_STAGES], acc_full[2], acc_empty[2];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int abort_flag;
+
+    pdl_trigger();
+    const int64_t line = 3 * (int64_t)G.chunks;
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int c_begin = (int)(line * pair / pairs), c_end = (int)(line * (pair + 1) / pairs);
+    if (c_begin >= c_end) return;            // uniform over the CTA
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    volatile int* abort_v = &abort_flag;
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < WG_STAGES; ++s) { umma::mbar_init(&full[s], 1); umma::mbar_init(&empty[s], 1 + EPI_WARPS); }
+        for (int a = 0; a < 2; ++a) { umma::mbar_init(&acc_full[a], 1); umma::mbar_init(&acc_empty[a], EPI_WARPS); }
+        abort_flag = 0;
+    }
+    if (warp == MMA_WARP) umma::tmem_alloc(&tmem_slot, TMEM_COLS);
+    pdl_wait();
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == PRODUCER_WARP) {
+        if (lane == 0) {
+            uint32_t it = 0;
+            bool ok = true;
+            for (int c = c_begin; c < c_end && ok;) {
+                const WgRun r = wg_run(c, c_end, G);
+                const int boxes = (r.layer ? D_H : D_OUT) / 64;
+                for (int k = 0; k < r.count; ++k, ++it) {
+                    const uint32_t s = it % WG_STAGES, n = it / WG_STAGES;
+                    if (n > 0 && !umma::mbar_wait_or_abort(&empty[s], (n - 1) & 1u, WAIT_BUDGET, abort_v)) { ok = false; break; }
+                    uint8_t* st = smem + s * WG_STAGE_BYTES;
+                    const int k0 = (r.first + k) * TILE_K;
+                    umma::mbar_arrive_expect_tx(&full[s], WG_A_BYTES + 8192u * boxes);
+                    for (int q = 0; q < 2; ++q)
+                        umma::tma_load_2d(st + 8192 * q, &G.h[r.layer], r.tile * TILE_M + 64 * q, k0, &full[s]);
+                    for (int q = 0; q < boxes; ++q)
+                        umma::tma_load_2d(st + WG_A_BYTES + 8192 * q, &G.dz[r.layer], 64 * q, k0, &full[s]);
+                }
+                c += r.count;
+            }
+            if (!ok) { atomicOr(G.err, 1u); *abort_v = 1; }
+            // copies still in flight land before the CTA can exit
+            for (uint32_t j = it > (uint32_t)WG_STAGES ? it - WG_STAGES : 0u; j < it; ++j)
+                umma::mbar_wait(&full[j % WG_STAGES], (j / WG_STAGES) & 1u, WAIT_BUDGET);
+        }
+    } else if (warp == MMA_WARP) {
+        if (lane == 0) {
+            uint32_t it = 0, j = 0;
+            bool ok = true;
+            for (int c = c_begin; c < c_end && ok; ++j) {
+                const WgRun r = wg_run(c, c_end, G);
+                const uint32_t idesc = umma::make_idesc_bf16(TILE_M, r.layer ? D_H : D_OUT, true, true);
+                const uint32_t a = j & 1u, u = j >> 1;
+                if (u > 0 && !umma::mbar_wait_or_abort(&acc_empty[a], (u - 1) & 1u, WAIT_BUDGET, abort_v)) { ok = false; break; }
+                umma::fence_after_sync();
+                const uint32_t d = tmem + a * 256u;
+                for (int k = 0; k < r.count; ++k, ++it) {
+                    const uint32_t s = it % WG_STAGES, n = it / WG_STAGES;
+                    if (!umma::mbar_wait_or_abort(&full[s], n & 1u, WAIT_BUDGET, abort_v)) { ok = false; break; }
+                    umma::fence_after_sync();
+                    const uint32_t sa = umma::smem_u32(smem + s * WG_STAGE_BYTES), sb = sa + WG_A_BYTES;
+#pragma unroll
+                    for (int q = 0; q < TILE_K / 16; ++q)
+                        umma::mma_bf16(d, umma::make_desc_sw128_mn(sa + 2048u * q, 8192u),
+                                       umma::make_desc_sw128_mn(sb + 2048u * q, 8192u), idesc, (k > 0 || q > 0) ? 1u : 0u);
+                    umma::commit(&empty[s]);
+                }
+                if (!ok) break;
+                umma::commit(&acc_full[a]);
+                c += r.count;
+            }
+            if (!ok) { atomicOr(G.err, 1u); *abort_v = 1; }
+            // the last MMAs complete before TMEM is freed
+            if (it > 0) umma::mbar_wait(&empty[(it - 1) % WG_STAGES], ((it - 1) / WG_STAGES) & 1u, WAIT_BUDGET);
+        }
+    } else {
+        const int quad = warp & 3;
+        uint32_t j = 0, it = 0;
+        bool ok = true;
+        for (int c = c_begin; c < c_end && ok; ++j) {
+            const WgRun r = wg_run(c, c_end, G);
+            const uint32_t a = j & 1u, u = j >> 1;
+            const int N = r.layer ? D_H : D_OUT;
+            // column sums of the stages' dZ (first tile): a lane takes the 8 columns
+            // of piece `piece` in every 16th row (8 lanes on 8 different bank groups)
+            const int piece = 2 * warp + (lane >> 4);
+            const bool sums = r.tile == 0 && 8 * piece < N;
+            float cs[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            for (int k = 0; k < r.count && ok; ++k, ++it) {
+                const uint32_t s = it % WG_STAGES, n = it / WG_STAGES;
+                if (!umma::mbar_wait_or_abort(&full[s], n & 1u, WAIT_BUDGET, abort_v)) { ok = false; break; }
+                if (sums) {
+                    const uint8_t* blk = smem + s * WG_STAGE_BYTES + WG_A_BYTES + 8192 * (piece >> 3);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const uint4 g4 = *reinterpret_cast<const uint4*>(blk + sw128((uint32_t)(16 * q + (lane & 15)), (uint32_t)(piece & 7)));
+                        const bf16* g8 = reinterpret_cast<const bf16*>(&g4);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) cs[e] += __bfloat162float(g8[e]);
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) umma::mbar_arrive(&empty[s]);
+            }
+            if (r.tile == 0) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+#pragma unroll
+                    for (int o = 8; o > 0; o >>= 1) cs[e] += __shfl_xor_sync(0xffffffffu, cs[e], o);
+                if (sums && (lane & 15) < 8) {
+                    float v = cs[0];
+#pragma unroll
+                    for (int e = 1; e < 8; ++e) v = (lane & 7) == e ? cs[e] : v;
+                    atomicAdd(G.bias[r.layer] + 8 * piece + (lane & 7), v);
+                }
+            }
+            if (!ok || !umma::mbar_wait_or_abort(&acc_full[a], u & 1u, WAIT_BUDGET, abort_v)) {
+                if (lane == 0) atomicOr(G.err, 1u);
+                *abort_v = 1;
+                break;
+            }
+            umma::fence_after_sync();
+            for (int c0 = 32 * (warp >> 2); c0 < N; c0 += 8 * EPI_WARPS) {
+                float v[32];
+                umma::tmem_ld32(tmem + a * 256u + ((uint32_t)(32 * quad) << 16) + (uint32_t)c0, v);
+                // column n of the tile is row n of the gradient: the warp's 32 inputs
+                // are 32 consecutive floats there (one coalesced reduction)
+                float* o = G.out[r.layer] + (int64_t)c0 * D_H + r.tile * TILE_M + 32 * quad + lane;
+#pragma unroll
+                for (int i = 0; i < 32; ++i) atomicAdd(o + i * D_H, v[i]);
+            }
+            umma::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) umma::mbar_arrive(&acc_empty[a]);
+            c += r.count;
         }
     }
     __syncthreads();
@@ -1131,9 +1472,8 @@ struct cl_mlp {
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
     int64_t adam_t = 0;
     // BF16 weight copies
-    bf16 *w2t = nullptr, *w2 = nullptr, *w3t = nullptr, *w3 = nullptr, *w4t = nullptr, *w4 = nullptr;
+    bf16 *w2t = nullptr, *w3t = nullptr, *w4t = nullptr;
     // activations and gradients (max_batch rows)
-    float* xb = nullptr;
     int32_t* brow = nullptr;        // training-set row of each minibatch row
     bf16 *h1 = nullptr, *h2 = nullptr, *z2 = nullptr, *h3 = nullptr, *z3 = nullptr;
     bf16 *dO = nullptr, *dz3 = nullptr, *dz2 = nullptr;
@@ -1169,9 +1509,9 @@ bool dalloc(cl_mlp* m, T** p, size_t count)
 
 void refresh_bf16(cl_mlp* m, cudaStream_t st)
 {
-    to_bf16_pair<<<(D_H * D_H + 255) / 256, 256, 0, st>>>(m->p + OFF_W2, D_H, D_H, m->w2t, m->w2);
-    to_bf16_pair<<<(D_H * D_H + 255) / 256, 256, 0, st>>>(m->p + OFF_W3, D_H, D_H, m->w3t, m->w3);
-    to_bf16_pair<<<(D_OUT * D_H + 255) / 256, 256, 0, st>>>(m->p + OFF_W4, D_OUT, D_H, m->w4t, m->w4);
+    to_bf16<<<(D_H * D_H + 255) / 256, 256, 0, st>>>(m->p + OFF_W2, D_H * D_H, m->w2t);
+    to_bf16<<<(D_H * D_H + 255) / 256, 256, 0, st>>>(m->p + OFF_W3, D_H * D_H, m->w3t);
+    to_bf16<<<(D_OUT * D_H + 255) / 256, 256, 0, st>>>(m->p + OFF_W4, D_OUT * D_H, m->w4t);
 }
 
 int grid_for(const cl_mlp* m, int B)
@@ -1181,74 +1521,78 @@ int grid_for(const cl_mlp* m, int B)
     return tiles < cap ? tiles : cap;
 }
 
-GemmArgs gemm_args(cl_mlp* m)
+// The shared-memory opt-in is a per-device attribute of a kernel: set once for
+// every device this process launches on.
+int net_attributes(int device)
 {
-    GemmArgs g;
-    memset(&g, 0, sizeof g);
-    g.err = m->derr;
-    return g;
+    static std::atomic<uint64_t> done{0};
+    const uint64_t bit = 1ull << (device & 63);
+    if (done.load() & bit) return CL_OK;
+    for (const void* k : {(const void*)net_forward<false>, (const void*)net_forward<true>, (const void*)net_backward,
+                          (const void*)weight_grads})
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)(k == (const void*)weight_grads ? WG_SMEM : NET_SMEM)) != cudaSuccess)
+            return CL_ERR_CUDA;
+    done.fetch_or(bit);
+    return CL_OK;
 }
 
-// Training forward pass over B rows of m->xb (B % 128 == 0): keeps H and Z for
-// the backward pass and ends in the loss epilogue, which reads the targets
-// (rows `trow` of `target`, or its first B rows) and writes dO, the b4 gradient
-// and the loss.
-int forward(cl_mlp* m, int B, const float* target, const int32_t* trow, cudaStream_t st, bool zero_grad)
+// Tensor maps of a network's W2^T, W3^T, W4^T.
+bool net_weight_maps(const cl_mlp* m, CUtensorMap* w)
 {
-    const int grid = grid_for(m, B);
-    if (zero_grad) cudaMemsetAsync(m->g, 0, N_PARAMS * sizeof(float), st);
-    launch_pdl(layer1_fwd, dim3((unsigned)(B / L1_ROWS)), dim3(256), 0, st, (const float*)m->xb,
-               (const float*)(m->p + OFF_W1), (const float*)(m->p + OFF_B1), m->h1);
-    GemmArgs g = gemm_args(m);
-    g.M = B; g.N = D_H; g.K = D_H; g.k_split = D_H;
-    g.bias = m->p + OFF_B2; g.out_h = m->h2; g.ldh = D_H; g.out_z = m->z2;
-    int rc = launch_gemm<EPI_BIAS_SILU>(g, m->h1, D_H, m->w2t, D_H, grid, 1, st);
-    if (rc) return rc;
-    g.bias = m->p + OFF_B3; g.out_h = m->h3; g.out_z = m->z3;
-    if ((rc = launch_gemm<EPI_BIAS_SILU>(g, m->h2, D_H, m->w3t, D_H, grid, 1, st))) return rc;
-    GemmArgs q = gemm_args(m);
-    q.M = B; q.N = D_OUT; q.K = D_H; q.k_split = D_H; q.bias = m->p + OFF_B4;
-    q.target = target; q.trow = trow; q.scale = 1.0f / ((float)B * (float)D_OUT); q.loss = m->loss;
-    q.out_h = m->dO; q.ldh = D_OUT; q.colsum = m->g + OFF_B4;
-    return launch_gemm<EPI_LOSS>(q, m->h3, D_H, m->w4t, D_H, grid, 1, st);
+    return make_map(&w[0], m->w2t, D_H, D_H, D_H, D_H) && make_map(&w[1], m->w3t, D_H, D_H, D_H, D_H) &&
+           make_map(&w[2], m->w4t, D_OUT, D_H, D_H, D_OUT);
 }
 
-// Backward pass after forward(), with m->g zeroed: bias and layer-1
-// gradients accumulate in the epilogues, weight gradients come from the
-// split-K GEMMs.
-int backward(cl_mlp* m, int B, cudaStream_t st)
+// Forward and backward passes over a batch of B rows (B % 128 == 0) of the
+// training set (x, target), m->g accumulating: two kernels for the activations,
+// then the weight gradients.  rows.n_all == 0: the batch is the set's first B rows.
+int forward_backward(cl_mlp* m, int B, const float* x, const float* target, const BatchRows& rows, cudaStream_t st)
 {
+    if ((uintptr_t)target & 15) return CL_ERR_ARG;       // rows of targets are read 16 bytes at a time at least
+    if (int rc = net_attributes(m->device)) return rc;
     const int grid = grid_for(m, B);
-    // backward data: dZ3 = (dO W4) * silu'(Z3), dZ2 = (dZ3 W3) * silu'(Z2), dZ1 = (dZ2 W2) * silu'(Z1)
-    GemmArgs g = gemm_args(m);
-    g.M = B; g.N = D_H; g.K = D_OUT; g.k_split = D_OUT;
-    g.out_h = m->dz3; g.ldh = D_H; g.zprev = m->z3; g.colsum = m->g + OFF_B3;
-    int rc = launch_gemm<EPI_DSILU>(g, m->dO, D_OUT, m->w4, D_OUT, grid, 1, st);
-    if (rc) return rc;
-    g.K = D_H; g.k_split = D_H;
-    g.out_h = m->dz2; g.zprev = m->z2; g.colsum = m->g + OFF_B2;
-    if ((rc = launch_gemm<EPI_DSILU>(g, m->dz3, D_H, m->w3, D_H, grid, 1, st))) return rc;
-    GemmArgs l1 = gemm_args(m);
-    l1.M = B; l1.N = D_H; l1.K = D_H; l1.k_split = D_H;
-    l1.bias = m->p + OFF_B1; l1.x = m->xb; l1.w1 = m->p + OFF_W1;
-    l1.colsum = m->g + OFF_B1; l1.gw1 = m->g + OFF_W1;
-    if ((rc = launch_gemm<EPI_DSILU_L1>(l1, m->dz2, D_H, m->w2, D_H, grid, 1, st))) return rc;
-    // weight gradients dW = H^T dZ (split-K over the batch), each split added
-    // in place into grad W^T (zeroed by the forward pass)
-    // K splits sized so that the two 128-row tiles of the 256 inputs fill every SM once
-    const int per_tile_ctas = m->num_sms / (D_H / TILE_M) > 0 ? m->num_sms / (D_H / TILE_M) : 1;
-    int k_split = ((B + per_tile_ctas - 1) / per_tile_ctas + TILE_K - 1) / TILE_K * TILE_K;
-    if (k_split < WGRAD_MIN_SPLIT_K) k_split = WGRAD_MIN_SPLIT_K;
-    const int splits = (B + k_split - 1) / k_split;
-    struct WG { const bf16* h; const bf16* dz; int OUT; int64_t off_w; };
-    const WG wg[3] = {{m->h3, m->dO, D_OUT, OFF_W4}, {m->h2, m->dz3, D_H, OFF_W3}, {m->h1, m->dz2, D_H, OFF_W2}};
+    NetArgs f;
+    NetTrain t;
+    NetBack k;
+    memset(&f, 0, sizeof f);
+    memset(&t, 0, sizeof t);
+    memset(&k, 0, sizeof k);
+    if (!net_weight_maps(m, f.w[0]) || !make_map(&t.h[0], m->h1, B, D_H, D_H, TILE_M) ||
+        !make_map(&t.h[1], m->h2, B, D_H, D_H, TILE_M) || !make_map(&t.h[2], m->h3, B, D_H, D_H, TILE_M) || !make_map(&t.h[3], m->dO, B, D_OUT, D_OUT, TILE_M) ||
+        !make_map(&k.dO, m->dO, B, D_OUT, D_OUT, TILE_M) || !make_map_mn(&k.w[0], m->w4t, D_OUT, D_H, D_H) ||
+        !make_map_mn(&k.w[1], m->w3t, D_H, D_H, D_H) || !make_map_mn(&k.w[2], m->w2t, D_H, D_H, D_H) ||
+        !make_map(&k.dz[0], m->dz3, B, D_H, D_H, TILE_M) || !make_map(&k.dz[1], m->dz2, B, D_H, D_H, TILE_M))
+        return CL_ERR_ARG;
+    f.params[0] = m->p; f.x = x; f.n = B; f.members = 1; f.tiles = B / TILE_M; f.err = m->derr;
+    t.z2 = m->z2; t.z3 = m->z3; t.target = target; t.rows = rows; t.brow = m->brow;
+    t.wide = ((uintptr_t)target & 31) == 0;
+    t.scale = 1.0f / ((float)B * (float)D_OUT); t.loss = m->loss;
+    if (launch_pdl(net_forward<true>, dim3((unsigned)grid), dim3(NET_TRAIN_THREADS), NET_SMEM, st, f, t) != cudaSuccess)
+        return CL_ERR_CUDA;
+    k.z3 = m->z3; k.z2 = m->z2; k.x = x; k.params = m->p; k.grad = m->g; k.brow = m->brow; k.tiles = B / TILE_M; k.err = m->derr;
+    if (launch_pdl(net_backward, dim3((unsigned)grid), dim3(NET_TRAIN_THREADS), NET_SMEM, st, k) != cudaSuccess)
+        return CL_ERR_CUDA;
+    WeightGrads w;
+    memset(&w, 0, sizeof w);
+    const bf16* hs[3] = {m->h3, m->h2, m->h1};
+    const bf16* dzs[3] = {m->dO, m->dz3, m->dz2};
+    const int64_t offs[3] = {OFF_W4, OFF_W3, OFF_W2};
     for (int l = 0; l < 3; ++l) {
-        GemmArgs w = gemm_args(m);
-        w.M = D_H; w.N = wg[l].OUT; w.K = B; w.k_split = k_split;
-        w.out_f = m->g + wg[l].off_w; w.ldf = D_H;
-        if ((rc = launch_gemm<EPI_WGRAD>(w, wg[l].h, D_H, wg[l].dz, wg[l].OUT, D_H / TILE_M, splits, st))) return rc;
+        const int N = l ? D_H : D_OUT;
+        if (!make_map_mn(&w.h[l], hs[l], B, D_H, D_H) || !make_map_mn(&w.dz[l], dzs[l], B, N, N)) return CL_ERR_ARG;
+        w.out[l] = m->g + offs[l];
+        w.bias[l] = m->g + offs[l] + (int64_t)N * D_H;      // b follows its W in the block
     }
-    return cudaGetLastError() == cudaSuccess ? CL_OK : CL_ERR_CUDA;
+    w.chunks = B / TILE_K;
+    w.err = m->derr;
+    // enough chunks per CTA that a run's additions (128 KB) stay small beside it
+    const int most = m->num_sms / 2, pairs = std::min(std::max(3 * w.chunks / WGRAD_MIN_CHUNKS, 3), most);
+    w.longest = std::max((w.chunks + pairs - 1) / pairs, WGRAD_MIN_RUN);
+    if (launch_pdl(weight_grads, dim3(2u * (unsigned)pairs), dim3(GEMM_THREADS),
+                   WG_SMEM, st, w) != cudaSuccess)
+        return CL_ERR_CUDA;
+    return CL_OK;
 }
 
 // net_forward over members x n rows, NET_MAX members and 2^24 rows per launch
@@ -1256,23 +1600,14 @@ int backward(cl_mlp* m, int B, cudaStream_t st)
 int net_forward_enqueue(cl_mlp* const* nets, int members, const float* d_x, float* d_out, int64_t n, cudaStream_t st)
 {
     cl_mlp* const m = nets[0];
-    static std::atomic<uint64_t> attr_devices{0};
-    const uint64_t bit = 1ull << (m->device & 63);
-    if (!(attr_devices.load() & bit)) {
-        if (cudaFuncSetAttribute(net_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NET_SMEM) != cudaSuccess)
-            return CL_ERR_CUDA;
-        attr_devices.fetch_or(bit);
-    }
+    if (int rc = net_attributes(m->device)) return rc;
     for (int k0 = 0; k0 < members; k0 += NET_MAX) {
         const int K = members - k0 < NET_MAX ? members - k0 : NET_MAX;
         NetArgs g;
         memset(&g, 0, sizeof g);
         for (int k = 0; k < K; ++k) {
-            const cl_mlp* q = nets[k0 + k];
-            if (!make_map(&g.w[k][0], q->w2t, D_H, D_H, D_H, D_H) || !make_map(&g.w[k][1], q->w3t, D_H, D_H, D_H, D_H) ||
-                !make_map(&g.w[k][2], q->w4t, D_OUT, D_H, D_H, D_OUT))
-                return CL_ERR_ARG;
-            g.params[k] = q->p;
+            if (!net_weight_maps(nets[k0 + k], g.w[k])) return CL_ERR_ARG;
+            g.params[k] = nets[k0 + k]->p;
         }
         g.members = K;
         g.err = m->derr;
@@ -1295,7 +1630,7 @@ int net_forward_enqueue(cl_mlp* const* nets, int members, const float* d_x, floa
                 a.out = out;
                 const int units = Kl * a.tiles;
                 const int cap = m->max_ctas > 0 && m->max_ctas < m->num_sms ? m->max_ctas : m->num_sms;
-                net_forward<<<(unsigned)(units < cap ? units : cap), GEMM_THREADS, NET_SMEM, st>>>(a);
+                net_forward<false><<<(unsigned)(units < cap ? units : cap), GEMM_THREADS, NET_SMEM, st>>>(a, NetTrain());
                 if (cudaGetLastError() != cudaSuccess) return CL_ERR_CUDA;
             }
         }
@@ -1308,18 +1643,9 @@ void adam(cl_mlp* m, float lr, cudaStream_t st)
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     m->adam_t += 1;
     const float bc1 = 1.0f - powf(b1, (float)m->adam_t), bc2 = 1.0f - powf(b2, (float)m->adam_t);
-    AdamCopies c;
-    const int64_t offs[3] = {OFF_W2, OFF_W3, OFF_W4};
-    const int outs[3] = {D_H, D_H, D_OUT};
-    bf16* wts[3] = {m->w2t, m->w3t, m->w4t};
-    bf16* ws[3] = {m->w2, m->w3, m->w4};
-    for (int t = 0; t < 3; ++t) {
-        c.off[t] = offs[t]; c.OUT[t] = outs[t]; c.IN[t] = D_H; c.n[t] = outs[t] * D_H;
-        c.wt[t] = wts[t]; c.w[t] = ws[t];
-    }
-    const unsigned grid = (unsigned)((N_PARAMS + 255) / 256);
-    launch_pdl(adam_all, dim3(grid), dim3(256), 0, st, m->p, m->g, m->m, m->v, (int64_t)N_PARAMS,
-               lr, b1, b2, eps, bc1, bc2, c);
+    const AdamCopies c = {m->w2t, m->w3t, m->w4t};
+    launch_pdl(adam_all, dim3((unsigned)((N_PARAMS / 4 + 127) / 128)), dim3(128), 0, st, m->p, m->g, m->m, m->v, lr, b1, b2,
+               eps, bc1, bc2, c);
 }
 
 }  // namespace
@@ -1346,10 +1672,8 @@ int cl_mlp_create(cl_mlp** out, int device, int max_batch)
     const size_t B = (size_t)max_batch;
     bool ok = dalloc(m, &m->p, N_PARAMS) && dalloc(m, &m->g, N_PARAMS) && dalloc(m, &m->m, N_PARAMS) &&
               dalloc(m, &m->v, N_PARAMS) &&
-              dalloc(m, &m->w2t, (size_t)D_H * D_H) && dalloc(m, &m->w2, (size_t)D_H * D_H) &&
-              dalloc(m, &m->w3t, (size_t)D_H * D_H) && dalloc(m, &m->w3, (size_t)D_H * D_H) &&
-              dalloc(m, &m->w4t, (size_t)D_OUT * D_H) && dalloc(m, &m->w4, (size_t)D_OUT * D_H) &&
-              dalloc(m, &m->xb, B * D_IN) && dalloc(m, &m->brow, B) &&
+              dalloc(m, &m->w2t, (size_t)D_H * D_H) && dalloc(m, &m->w3t, (size_t)D_H * D_H) &&
+              dalloc(m, &m->w4t, (size_t)D_OUT * D_H) && dalloc(m, &m->brow, B) &&
               dalloc(m, &m->h1, B * D_H) &&
               dalloc(m, &m->h2, B * D_H) && dalloc(m, &m->z2, B * D_H) &&
               dalloc(m, &m->h3, B * D_H) && dalloc(m, &m->z3, B * D_H) &&
@@ -1384,7 +1708,7 @@ void cl_mlp_destroy(cl_mlp* m)
 
 const char* cl_mlp_last_error(const cl_mlp* m) { return m ? m->err : ""; }
 
-// Cap the number of CTAs of the row-tiled GEMMs (0 = one per SM); with few
+// Cap the number of CTAs of the forward and backward passes (0 = one per SM); with few
 // CTAs each one walks many tiles (tests of the persistent pipeline).
 int cl_mlp_set_max_ctas(cl_mlp* m, int n)
 {
@@ -1437,10 +1761,8 @@ int cl_mlp_train(cl_mlp* m, int steps, int batch, float lr, uint32_t seed, uint3
     // step is an unbroken chain of kernels
     cudaMemsetAsync(m->g, 0, N_PARAMS * sizeof(float), st);
     for (int s = 0; s < steps; ++s) {
-        launch_pdl(gather_batch, dim3((batch + 255) / 256), dim3(256), 0, st, (const float*)m->data_x,
-                   (int64_t)m->n_data, batch, seed, step0 + (uint32_t)s, m->xb, m->brow);
-        int rc = forward(m, batch, m->data_t, m->brow, st, false);
-        if (!rc) rc = backward(m, batch, st);
+        const int rc = forward_backward(m, batch, m->data_x, m->data_t,
+                                        BatchRows{(uint32_t)m->n_data, step0 + (uint32_t)s, seed}, st);
         if (rc) return mlp_fail(m, rc, "kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
         adam(m, lr, st);
     }
@@ -1498,10 +1820,9 @@ int cl_mlp_gradient(cl_mlp* m, const float* d_x, const float* d_t, int B, float*
     if (!m || !d_x || !d_t || !host_grad || B < TILE_M || B % TILE_M || B > m->max_batch) return CL_ERR_ARG;
     cudaSetDevice(m->device);
     cudaStream_t st = m->stream;
-    cudaMemcpyAsync(m->xb, d_x, (size_t)B * D_IN * sizeof(float), cudaMemcpyDeviceToDevice, st);
     cudaMemsetAsync(m->loss, 0, sizeof(float), st);
-    int rc = forward(m, B, d_t, nullptr, st, true);
-    if (!rc) rc = backward(m, B, st);
+    cudaMemsetAsync(m->g, 0, N_PARAMS * sizeof(float), st);
+    const int rc = forward_backward(m, B, d_x, d_t, BatchRows{0u, 0u, 0u}, st);
     if (rc) return mlp_fail(m, rc, "launch failed");
     float loss = 0.0f;
     cudaMemcpyAsync(host_grad, m->g, N_PARAMS * sizeof(float), cudaMemcpyDeviceToHost, st);

@@ -195,6 +195,12 @@ __device__ __forceinline__ void bulk_wait0()
     asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
+// Bring `bytes` (a multiple of 16) at p (16-byte aligned) into L2.
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(p)), "r"(bytes) : "memory");
+}
+
 __device__ __forceinline__ void prefetch_tmap(const void* tmap)
 {
     asm volatile("prefetch.tensormap [%0];" :: "l"(reinterpret_cast<uint64_t>(tmap)) : "memory");

@@ -451,7 +451,7 @@ int cl_mlp_param_count(void);
 int cl_mlp_create(cl_mlp** out, int device, int max_batch);
 void cl_mlp_destroy(cl_mlp* m);
 const char* cl_mlp_last_error(const cl_mlp* m);
-/* Cap the CTAs of the batch-tiled GEMMs (0 = one per SM), for tests. */
+/* Cap the CTAs of the forward and backward passes (0 = one per SM), for tests. */
 int cl_mlp_set_max_ctas(cl_mlp* m, int n);
 /* Host buffers of cl_mlp_param_count() floats; setting resets Adam's state. */
 int cl_mlp_set_params(cl_mlp* m, const float* host);
