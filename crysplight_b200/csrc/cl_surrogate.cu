@@ -337,7 +337,8 @@ struct CombineArgs {
     int64_t n;
     const float* y_mean;     // [3 * cells]
     const float* y_std;      // [3 * cells]
-    const float* xyz;        // [n][3] mm
+    const float* xyz;        // mm, row site[i] (i where site is null)
+    const int32_t* site;     // row of the sites' arrays of each row i (may be null)
     const float* direct;     // [n][CELLS] first-pass probabilities added to the members' (may be null)
     float L0, L1, L2;
     int32_t front_wrapped;
@@ -366,6 +367,7 @@ __global__ void __launch_bounds__(32 * COMBINE_WARPS) surrogate_combine(const Co
     const double invK = 1.0 / (double)A.K;
     const int64_t stride = (int64_t)gridDim.x * COMBINE_WARPS;
     for (int64_t i = (int64_t)blockIdx.x * COMBINE_WARPS + (threadIdx.x >> 5); i < A.n; i += stride) {
+        const int64_t to = A.site ? A.site[i] : i;
         double sum_p[2] = {0.0, 0.0}, sum_p2[2] = {0.0, 0.0}, sum_t[2] = {0.0, 0.0}, sum_l[2] = {0.0, 0.0};
         float dir[2] = {0.f, 0.f};
         if (A.direct) {
@@ -405,7 +407,7 @@ __global__ void __launch_bounds__(32 * COMBINE_WARPS) surrogate_combine(const Co
             const double pm = pr + (A.direct ? (double)dir[q] : 0.0);
             a[q] = sqrt(var);
             b[q] = pm;
-            const int64_t at = i * CELLS + 32 * q + lane;
+            const int64_t at = to * CELLS + 32 * q + lane;
             A.p[at] = (float)(pm * (double)A.pde);
             A.tmean[at] = (float)(sum_t[q] * invK);
             A.tsig[at] = (float)exp(sum_l[q] * invK);
@@ -421,15 +423,15 @@ __global__ void __launch_bounds__(32 * COMBINE_WARPS) surrogate_combine(const Co
             const double num = a[0] + a[1];
             const double den = b[0] + b[1];
             const float spr = (float)(num / fmax(den, 1e-30));
-            const float x = A.xyz[3 * i], y = A.xyz[3 * i + 1], z = A.xyz[3 * i + 2];
+            const float x = A.xyz[3 * to], y = A.xyz[3 * to + 1], z = A.xyz[3 * to + 2];
             float d = fminf(fminf(x, A.L0 - x), fminf(y, A.L1 - y));
             if (A.front_wrapped) d = fminf(d, z);
             uint8_t f = 0;
             if (!(spr <= A.spread_max)) f |= 1u;
             if (d < A.wall_min_mm) f |= 2u;
             if (!(den * (double)A.pde < 0.999)) f |= 4u;   // not a probability split: Monte Carlo
-            A.spread[i] = spr;
-            A.flag[i] = f;
+            A.spread[to] = spr;
+            A.flag[to] = f;
         }
     }
 }
@@ -477,7 +479,8 @@ __constant__ double c_gl_w[4] = {0.3626837833783620, 0.3137066458778873, 0.22238
 }
 
 struct DirectArgs {
-    const float* xyz;        // [n][3] mm
+    const float* xyz;        // mm, row site[i] (i where site is null)
+    const int32_t* site;     // (may be null)
     int64_t n;
     float L0, L1, L2;
     float n1, n2, mu;        // crystal and coupling indices, attenuation 1/mm
@@ -543,7 +546,8 @@ __global__ void __launch_bounds__(32 * DIRECT_WARPS) surrogate_direct(const Dire
     __syncthreads();
     const int64_t stride = (int64_t)gridDim.x * DIRECT_WARPS;
     for (int64_t i = (int64_t)blockIdx.x * DIRECT_WARPS + (threadIdx.x >> 5); i < A.n; i += stride) {
-        const float x0 = A.xyz[3 * i], y0 = A.xyz[3 * i + 1], z0 = A.xyz[3 * i + 2];
+        const int64_t at = A.site ? A.site[i] : i;
+        const float x0 = A.xyz[3 * at], y0 = A.xyz[3 * at + 1], z0 = A.xyz[3 * at + 2];
         const float h = A.L2 - z0;
         const bool inside = h > 0.0f && x0 >= 0.0f && x0 <= A.L0 && y0 >= 0.0f && y0 <= A.L1;   // warp-uniform
         if (inside) {
@@ -659,17 +663,59 @@ __global__ void __launch_bounds__(32 * DIRECT_WARPS) surrogate_direct(const Dire
 }
 
 // Network inputs of the sites: x, y scaled to [-1, 1] and the depth through
-// w(t) = (1 - a) t + a (1 - sqrt(1 - t)), t = z / Lz clamped to [0, 1].
-__global__ void surrogate_inputs(const float* __restrict__ xyz, int64_t n, float L0, float L1, float L2,
-                                 float a, float* __restrict__ out)
+// w(t) = (1 - a) t + a (1 - sqrt(1 - t)), t = (z - z0) / Lz clamped to [0, 1].
+__global__ void surrogate_inputs(const float* __restrict__ xyz, const int32_t* __restrict__ site, int64_t n, float L0,
+                                 float L1, float L2, float z0, float a, float* __restrict__ out)
 {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const float x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
+        const int64_t at = site ? site[i] : i;
+        const float x = xyz[3 * at], y = xyz[3 * at + 1], z = xyz[3 * at + 2] - z0;
         const float t = fminf(fmaxf(z / L2, 0.0f), 1.0f);
         const float w = (1.0f - a) * t + a * (1.0f - sqrtf(1.0f - t));
         out[3 * i] = 2.0f * x / L0 - 1.0f;
         out[3 * i + 1] = 2.0f * y / L1 - 1.0f;
         out[3 * i + 2] = 2.0f * w - 1.0f;
+    }
+}
+
+// Which ensemble serves each site: the last expert whose depth range holds it,
+// else the main one (group 0; expert e is group e + 1).  Each group's sites are
+// listed in list + group * n, count[group] of them, 32 consecutive sites at a
+// time.  Evaluating the main ensemble everywhere and then the experts over it
+// cost the experts' sites twice: every network, the first-pass term and five
+// copies (42,001 sites, a third of them an expert's: 781 us, 556 so).
+constexpr int SITE_GROUPS = 257;
+struct SplitArgs {
+    const float* xyz;
+    int64_t n;
+    int32_t experts;
+    float lo[SITE_GROUPS - 1], hi[SITE_GROUPS - 1];
+    int32_t* list;
+    int32_t* count;
+};
+__global__ void __launch_bounds__(256) surrogate_split(const __grid_constant__ SplitArgs A)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); 32 * w < A.n; w += warps) {
+        const int64_t i = 32 * w + lane;
+        int group = -1;
+        if (i < A.n) {
+            const float z = A.xyz[3 * i + 2];
+            group = 0;
+            for (int e = 0; e < A.experts; ++e)
+                if (z >= A.lo[e] && z <= A.hi[e]) group = e + 1;
+        }
+        unsigned left = __ballot_sync(0xffffffffu, group >= 0);
+        while (left) {                               // one group of the warp's sites after another
+            const int g = __shfl_sync(0xffffffffu, group, __ffs(left) - 1);
+            const unsigned same = __ballot_sync(0xffffffffu, group == g);
+            int at = 0;
+            if (lane == __ffs(same) - 1) at = atomicAdd(A.count + g, __popc(same));
+            at = __shfl_sync(0xffffffffu, at, __ffs(same) - 1) + __popc(same & ((1u << lane) - 1u));
+            if (group == g) A.list[(int64_t)g * A.n + at] = (int32_t)i;
+            left &= ~same;
+        }
     }
 }
 
@@ -722,6 +768,17 @@ int cl_surrogate_combine_direct(const float* d_raw, int32_t members, int64_t n_s
                                 float* d_p, float* d_tmean, float* d_tsig, float* d_spread,
                                 uint8_t* d_flag, void* stream)
 {
+    return cl_surrogate_combine_sites(d_raw, members, n_sites, d_y_mean, d_y_std, d_xyz, nullptr, d_direct, box, ro, pde,
+                                      spread_max, wall_min_mm, d_p, d_tmean, d_tsig, d_spread, d_flag, stream);
+}
+
+int cl_surrogate_combine_sites(const float* d_raw, int32_t members, int64_t n_sites,
+                               const float* d_y_mean, const float* d_y_std, const float* d_xyz,
+                               const int32_t* d_site, const float* d_direct, const cl_box* box, const cl_readout* ro,
+                               float pde, float spread_max, float wall_min_mm,
+                               float* d_p, float* d_tmean, float* d_tsig, float* d_spread,
+                               uint8_t* d_flag, void* stream)
+{
     if (!box || !ro || members < 1 || n_sites < 0) return CL_ERR_ARG;
     if ((int64_t)ro->grid.nx * ro->grid.ny != cl::sur::CELLS) return CL_ERR_ARG;
     if (n_sites == 0) return CL_OK;
@@ -730,7 +787,7 @@ int cl_surrogate_combine_direct(const float* d_raw, int32_t members, int64_t n_s
     if (!(pde >= 0.0f && pde <= 1.0f)) return CL_ERR_ARG;
     cl::sur::CombineArgs a;
     a.raw = d_raw; a.K = members; a.n = n_sites; a.y_mean = d_y_mean; a.y_std = d_y_std; a.xyz = d_xyz;
-    a.direct = d_direct;
+    a.site = d_site; a.direct = d_direct;
     a.L0 = box->L[0]; a.L1 = box->L[1]; a.L2 = box->L[2];
     a.front_wrapped = ro->two_sided ? 0 : 1;
     a.pde = pde; a.spread_max = spread_max; a.wall_min_mm = wall_min_mm;
@@ -744,6 +801,12 @@ int cl_surrogate_combine_direct(const float* d_raw, int32_t members, int64_t n_s
 int cl_surrogate_direct(const float* d_xyz, int64_t n_sites, const cl_box* box, const cl_optical_params* op,
                         const cl_readout* ro, float* d_out, void* stream)
 {
+    return cl_surrogate_direct_sites(d_xyz, nullptr, n_sites, box, op, ro, d_out, stream);
+}
+
+int cl_surrogate_direct_sites(const float* d_xyz, const int32_t* d_site, int64_t n_sites, const cl_box* box,
+                              const cl_optical_params* op, const cl_readout* ro, float* d_out, void* stream)
+{
     if (!box || !op || !ro || n_sites < 0) return CL_ERR_ARG;
     if ((int64_t)ro->grid.nx * ro->grid.ny != cl::sur::CELLS || ro->grid.nx < 1 || !(ro->grid.pitch_mm > 0.0f))
         return CL_ERR_ARG;
@@ -754,7 +817,7 @@ int cl_surrogate_direct(const float* d_xyz, int64_t n_sites, const cl_box* box, 
     if (n_sites == 0) return CL_OK;
     if (!d_xyz || !d_out) return CL_ERR_ARG;
     cl::sur::DirectArgs a;
-    a.xyz = d_xyz; a.n = n_sites; a.L0 = box->L[0]; a.L1 = box->L[1]; a.L2 = box->L[2];
+    a.xyz = d_xyz; a.site = d_site; a.n = n_sites; a.L0 = box->L[0]; a.L1 = box->L[1]; a.L2 = box->L[2];
     a.n1 = op->n_crystal; a.n2 = op->n_coupling;
     a.mu = (float)((std::isinf(op->abs_len_mm) ? 0.0 : 1.0 / (double)op->abs_len_mm) +
                    (std::isinf(op->rayleigh_mm) ? 0.0 : 1.0 / (double)op->rayleigh_mm));
@@ -775,14 +838,40 @@ int cl_surrogate_direct(const float* d_xyz, int64_t n_sites, const cl_box* box, 
 int cl_surrogate_inputs(const float* d_xyz, int64_t n_sites, const cl_box* box, float z_warp, float* d_out,
                         void* stream)
 {
+    return cl_surrogate_inputs_sites(d_xyz, nullptr, n_sites, box, 0.0f, z_warp, d_out, stream);
+}
+
+int cl_surrogate_inputs_sites(const float* d_xyz, const int32_t* d_site, int64_t n_sites, const cl_box* box, float z0,
+                              float z_warp, float* d_out, void* stream)
+{
     if (!box || n_sites < 0 || !(z_warp >= 0.0f && z_warp <= 1.0f)) return CL_ERR_ARG;
     if (n_sites == 0) return CL_OK;
     if (!d_xyz || !d_out) return CL_ERR_ARG;
     const int64_t want = (n_sites + 255) / 256;
     const unsigned grid = (unsigned)(want < 148 * 32 ? want : 148 * 32);
-    cl::sur::surrogate_inputs<<<grid, 256, 0, (cudaStream_t)stream>>>(d_xyz, n_sites, box->L[0], box->L[1],
-                                                                      box->L[2], z_warp, d_out);
+    cl::sur::surrogate_inputs<<<grid, 256, 0, (cudaStream_t)stream>>>(d_xyz, d_site, n_sites, box->L[0], box->L[1],
+                                                                      box->L[2], z0, z_warp, d_out);
     return cudaGetLastError() == cudaSuccess ? CL_OK : CL_ERR_CUDA;
+}
+
+int cl_surrogate_split(const float* d_xyz, int64_t n_sites, int32_t experts, const float* lo, const float* hi,
+                       int32_t* d_list, int32_t* d_count, int32_t* count, void* stream)
+{
+    if (n_sites < 0 || n_sites > 0x7fffffff || experts < 0 || experts >= cl::sur::SITE_GROUPS || (experts > 0 && (!lo || !hi)) ||
+        !d_list || !d_count || !count || (n_sites > 0 && !d_xyz))
+        return CL_ERR_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
+    cl::sur::SplitArgs a;
+    a.xyz = d_xyz; a.n = n_sites; a.experts = experts; a.list = d_list; a.count = d_count;
+    for (int e = 0; e < experts; ++e) { a.lo[e] = lo[e]; a.hi[e] = hi[e]; }
+    const size_t bytes = (size_t)(experts + 1) * sizeof(int32_t);
+    if (cudaMemsetAsync(d_count, 0, bytes, st) != cudaSuccess) return CL_ERR_CUDA;
+    const int64_t want = (n_sites + 255) / 256;
+    if (want > 0) cl::sur::surrogate_split<<<(unsigned)(want < 148 * 8 ? want : 148 * 8), 256, 0, st>>>(a);
+    if (cudaGetLastError() != cudaSuccess || cudaMemcpyAsync(count, d_count, bytes, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+        cudaStreamSynchronize(st) != cudaSuccess)
+        return CL_ERR_CUDA;
+    return CL_OK;
 }
 
 int cl_debug_sampler(int fn, const double* par, int64_t n, uint64_t seed, void* d_out,

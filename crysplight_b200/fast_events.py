@@ -125,68 +125,78 @@ class SurrogateEvents:
         for r in [self.main] + self.experts:
             r.close()
 
-    def _light(self, ens: _Resident, xyz, ro: Readout, pde: float, spread_max: float,
-               wall_min_mm: float, stream) -> SiteLight:
-        """One ensemble on sites xyz ((n, 3) float32 CUDA tensor, mm)."""
+    def _light(self, ens: _Resident, xyz, site, out: SiteLight, ro: Readout, pde: float,
+               spread_max: float, wall_min_mm: float, stream):
+        """One ensemble on the sites ``site`` (int32 CUDA tensor; None: all) of
+        xyz ((n, 3) float32 CUDA tensor, mm), into their rows of ``out``:
+        enqueued; returns the temporaries, alive until the stream is waited for."""
         import torch
-        n = int(xyz.shape[0])
+        n = int((xyz if site is None else site).shape[0])
         K = len(ens.nets)
-        # everything here runs on one stream; torch's own work on the inputs
-        # (another stream, if the caller names one) is done before it
         st = stream_arg(stream or 0)
-        xyz = xyz.contiguous()
+        P = C.c_void_p
+        at = P(site.data_ptr()) if site is not None else None
         xin = torch.empty((n, 3), dtype=torch.float32, device=self.dev)
-        xs = xyz
-        if ens.z0 != 0.0:
-            xs = xyz - torch.tensor([0.0, 0.0, ens.z0], dtype=torch.float32, device=self.dev)
-        current = torch.cuda.current_stream(self.dev)
-        if current.cuda_stream != (stream or 0):
-            current.synchronize()
-        rc = self.lib.cl_surrogate_inputs(C.c_void_p(xs.data_ptr()), n, C.byref(ens.in_box),
-                                          float(ens.sur.z_warp), C.c_void_p(xin.data_ptr()), st)
+        rc = self.lib.cl_surrogate_inputs_sites(P(xyz.data_ptr()), at, n, C.byref(ens.in_box), float(ens.z0),
+                                                float(ens.sur.z_warp), P(xin.data_ptr()), st)
         if rc != 0:
             raise _lib.CudaTransportError(rc, "cl_surrogate_inputs failed")
         raw = torch.empty((K, n, D_OUT), dtype=torch.float32, device=self.dev)
         forward_ensemble(ens.nets, xin, raw, st)
-        out = SiteLight(torch.empty((n, N_CELLS), dtype=torch.float32, device=self.dev),
-                        torch.empty((n, N_CELLS), dtype=torch.float32, device=self.dev),
-                        torch.empty((n, N_CELLS), dtype=torch.float32, device=self.dev),
-                        torch.empty(n, dtype=torch.float32, device=self.dev),
-                        torch.empty(n, dtype=torch.uint8, device=self.dev))
-        P = C.c_void_p
         # an ensemble trained on the light minus the first-pass term gets it back here
         direct = None
         if ens.sur.first_pass is not None and n:
-            direct = first_pass_light(xyz, self.box, ens.sur.first_pass, self.device, stream or 0)
-        rc = self.lib.cl_surrogate_combine_direct(
-            P(raw.data_ptr()), K, n, P(ens.y_mean.data_ptr()), P(ens.y_std.data_ptr()),
-            P(xyz.data_ptr()), P(direct.data_ptr()) if direct is not None else None, C.byref(self.box),
+            direct = first_pass_light(xyz, self.box, ens.sur.first_pass, self.device, stream or 0, site)
+        rc = self.lib.cl_surrogate_combine_sites(
+            P(raw.data_ptr()), K, n, P(ens.y_mean.data_ptr()), P(ens.y_std.data_ptr()), P(xyz.data_ptr()), at,
+            P(direct.data_ptr()) if direct is not None else None, C.byref(self.box),
             C.byref(ro), float(pde), float(spread_max),
             float(wall_min_mm), P(out.p.data_ptr()), P(out.tmean.data_ptr()), P(out.tsig.data_ptr()),
             P(out.spread.data_ptr()), P(out.flag.data_ptr()), st)
         if rc != 0:
             raise _lib.CudaTransportError(rc, "cl_surrogate_combine failed")
-        # the temporaries go back to torch's allocator, and a network's error is reported here
-        sync_networks(ens.nets, st)
-        return out
+        return xin, raw, direct
+
+    def _split(self, xyz, stream):
+        """[(ensemble, its sites as int32 CUDA tensor)], main first, with the sites
+        of each: the last expert whose slab holds the site, else the main one."""
+        import torch
+        n, E = int(xyz.shape[0]), len(self.experts)
+        lo, hi, count = (C.c_float * E)(), (C.c_float * E)(), (C.c_int32 * (E + 1))()
+        for e, ens in enumerate(self.experts):
+            z0, z1 = ens.sur.depth_range()
+            lo[e], hi[e] = z0 + self.expert_margin_mm, z1
+        lists = torch.empty((E + 1, n), dtype=torch.int32, device=self.dev)
+        d_count = torch.empty(E + 1, dtype=torch.int32, device=self.dev)
+        rc = self.lib.cl_surrogate_split(C.c_void_p(xyz.data_ptr()), n, E, lo, hi, C.c_void_p(lists.data_ptr()),
+                                         C.c_void_p(d_count.data_ptr()), count, stream_arg(stream or 0))
+        if rc != 0:
+            raise _lib.CudaTransportError(rc, "cl_surrogate_split failed")
+        return [(ens, lists[g, :count[g]]) for g, ens in enumerate([self.main] + self.experts)]
 
     def site_light(self, xyz, *, ro: Readout, pde: float, spread_max: float = SPREAD_MAX,
                    wall_min_mm: float = WALL_MIN_MM, stream=None) -> SiteLight:
         """Ensemble outputs for sites xyz ((n, 3) float32 CUDA tensor, mm),
         each site from the main ensemble or the expert whose slab holds it."""
         import torch
-        out = self._light(self.main, xyz, ro, pde, spread_max, wall_min_mm, stream)
-        for ens in self.experts:
-            z0, z1 = ens.sur.depth_range()
-            z = xyz[:, 2]
-            idx = torch.nonzero((z >= z0 + self.expert_margin_mm) & (z <= z1)).flatten()
-            if idx.numel() == 0:
-                continue
-            sub = self._light(ens, xyz.index_select(0, idx), ro, pde, spread_max, wall_min_mm, stream)
-            for name in ("p", "tmean", "tsig", "spread", "flag"):
-                getattr(out, name).index_copy_(0, idx, getattr(sub, name))
-        if self.experts:
-            torch.cuda.synchronize(self.dev)
+        n = int(xyz.shape[0])
+        xyz = xyz.contiguous()
+        out = SiteLight(*(torch.empty((n, N_CELLS), dtype=torch.float32, device=self.dev) for _ in range(3)),
+                        torch.empty(n, dtype=torch.float32, device=self.dev),
+                        torch.empty(n, dtype=torch.uint8, device=self.dev))
+        # everything here runs on one stream; torch's own work on the inputs
+        # (another stream, if the caller names one) is done before it
+        current = torch.cuda.current_stream(self.dev)
+        if current.cuda_stream != (stream or 0):
+            current.synchronize()
+        parts = [(self.main, None)]
+        if self.experts and n:
+            parts = [(ens, site) for ens, site in self._split(xyz, stream) if site.numel()]
+        kept = [self._light(ens, xyz, site, out, ro, pde, spread_max, wall_min_mm, stream) for ens, site in parts]
+        # the temporaries go back to torch's allocator, and a network's error is reported here
+        for ens, _ in parts:
+            sync_networks(ens.nets, stream_arg(stream or 0))
+        del kept
         return out
 
     def transport_sites(self, box: Box, op: OpticalParams, ro: Readout, tb: TimeBinning, *,

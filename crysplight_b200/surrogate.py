@@ -349,11 +349,12 @@ def first_pass_optics(op, ro) -> tuple:
             float(ro.grid.pitch_mm), int(ro.grid.nx), int(ro.grid.ny))
 
 
-def first_pass_light(xyz, box: Box, optics: tuple, device: int = 0, stream=None):
+def first_pass_light(xyz, box: Box, optics: tuple, device: int = 0, stream=None, site=None):
     """First-pass detection probabilities (cl_surrogate_direct) of emission
     points xyz ((n, 3) float32 CUDA tensor or array, mm): torch tensor
     (n, 64) on the GPU.  A photon reaches the readout face without a bulk
-    interaction, is transmitted and lands in the SiPM's pixel; PDE 1."""
+    interaction, is transmitted and lands in the SiPM's pixel; PDE 1.  ``site``
+    (int32 CUDA tensor): row i is that of point xyz[site[i]]."""
     import torch
     from .params import OpticalParams, SipmGrid
     from .transport import stream_arg
@@ -362,10 +363,12 @@ def first_pass_light(xyz, box: Box, optics: tuple, device: int = 0, stream=None)
     n1, n2, ab, ray, pitch, nx, ny = optics
     op = OpticalParams(n1, n2, ab, ray, 1.0, True, True, 0.0, 1.0)
     ro = Readout(SipmGrid(pitch, int(nx), int(ny)))
-    out = torch.empty((x.shape[0], N_CELLS), dtype=torch.float32, device=x.device)
-    rc = _lib.load().cl_surrogate_direct(C.c_void_p(x.data_ptr()), int(x.shape[0]), C.byref(box),
-                                         C.byref(op), C.byref(ro), C.c_void_p(out.data_ptr()),
-                                         stream_arg(stream))
+    n = int((x if site is None else site).shape[0])
+    out = torch.empty((n, N_CELLS), dtype=torch.float32, device=x.device)
+    rc = _lib.load().cl_surrogate_direct_sites(C.c_void_p(x.data_ptr()),
+                                               C.c_void_p(site.data_ptr()) if site is not None else None, n,
+                                               C.byref(box), C.byref(op), C.byref(ro),
+                                               C.c_void_p(out.data_ptr()), stream_arg(stream))
     if rc != 0:
         raise _lib.CudaTransportError(rc, "cl_surrogate_direct failed")
     return out

@@ -371,6 +371,34 @@ int cl_surrogate_inputs(const float* d_xyz, int64_t n_sites, const cl_box* box, 
                         float* d_out, void* stream);
 
 /*
+ * Sites served by several ensembles (no counterpart in the reference).
+ * cl_surrogate_split lists which ensemble serves each of n_sites sites: the
+ * last expert e with lo[e] <= z <= hi[e] (host arrays; at most 256 experts),
+ * else the main ensemble.  d_list [experts + 1][n_sites] receives the sites of
+ * the main ensemble, then of each expert, d_count [experts + 1] (device) and
+ * count (host) their numbers.  Waits for `stream`.
+ *
+ * The three steps of an ensemble on such a list: as cl_surrogate_inputs (of
+ * depth z - z0), cl_surrogate_direct and cl_surrogate_combine_direct for the
+ * sites d_xyz[d_site[i]], i < n_sites; d_out, d_raw and d_direct have row i,
+ * d_p, d_tmean, d_tsig, d_spread and d_flag row d_site[i].  d_site may be NULL
+ * (site i).  Asynchronous on `stream`; nothing is allocated.
+ */
+int cl_surrogate_split(const float* d_xyz, int64_t n_sites, int32_t experts, const float* lo,
+                       const float* hi, int32_t* d_list, int32_t* d_count, int32_t* count, void* stream);
+int cl_surrogate_inputs_sites(const float* d_xyz, const int32_t* d_site, int64_t n_sites,
+                              const cl_box* box, float z0, float z_warp, float* d_out, void* stream);
+int cl_surrogate_direct_sites(const float* d_xyz, const int32_t* d_site, int64_t n_sites,
+                              const cl_box* box, const cl_optical_params* op, const cl_readout* ro,
+                              float* d_out, void* stream);
+int cl_surrogate_combine_sites(const float* d_raw, int32_t members, int64_t n_sites,
+                               const float* d_y_mean, const float* d_y_std, const float* d_xyz,
+                               const int32_t* d_site, const float* d_direct, const cl_box* box,
+                               const cl_readout* ro, float pde, float spread_max, float wall_min_mm,
+                               float* d_p, float* d_tmean, float* d_tsig, float* d_spread,
+                               uint8_t* d_flag, void* stream);
+
+/*
  * Diagnostics for tests: n draws (stream i = draw i, key = seed) of the
  * surrogate sampler's variates into device memory: fn 0 = binomial
  * (n = par[0], p = par[1]) -> int64; fn 1 = minimum of k = par[0] arrival
