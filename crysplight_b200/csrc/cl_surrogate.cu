@@ -242,8 +242,14 @@ __device__ __forceinline__ double time_uniform(int64_t i, int c, uint32_t k0, ui
 // not depend on which lane draws it.  Eight CTAs of 128 threads per SM
 // (64 registers; the Float64 special functions' latency needs the warps more
 // than the spilled registers cost).
-constexpr int SAMPLE_WARPS = 4;
-__global__ void __launch_bounds__(32 * SAMPLE_WARPS, 8) surrogate_sample(const SurSampleArgs A)
+//
+// A warp takes `sites` sites at a time, the fewest (a power of two) with which
+// all warps are resident at once: the chain is a latency of 64 dependent draws
+// however few lanes run it, and the times are shared out over all lanes anyway.
+// 2,800 sites: 1451 us with 32 per warp, 951 / 642 / 509 / 444 / 410 with 16 / 8
+// / 4 / 2 / 1; 28,000: 1725, 1545 / 1550 / 2320 (two waves) with 16 / 8 / 4.
+constexpr int SAMPLE_WARPS = 4, SAMPLE_CTAS = 8;
+__global__ void __launch_bounds__(32 * SAMPLE_WARPS, SAMPLE_CTAS) surrogate_sample(const SurSampleArgs A, int sites)
 {
     __shared__ uint16_t s_k[SAMPLE_WARPS][CELLS][32];   // hit counts of the warp's sites, by SiPM
     __shared__ uint32_t s_mask[SAMPLE_WARPS][CELLS];    // lanes whose site hit the SiPM
@@ -252,11 +258,11 @@ __global__ void __launch_bounds__(32 * SAMPLE_WARPS, 8) surrogate_sample(const S
     const int64_t nwarps = (int64_t)gridDim.x * SAMPLE_WARPS;
     unsigned bad = 0;
     unsigned long long ph = 0, det = 0;
-    for (int64_t i0 = ((int64_t)blockIdx.x * SAMPLE_WARPS + wib) * 32; i0 < A.n; i0 += nwarps * 32) {
+    for (int64_t i0 = ((int64_t)blockIdx.x * SAMPLE_WARPS + wib) * sites; i0 < A.n; i0 += nwarps * sites) {
         // ---- the binomial chain of this lane's site ----
         const int64_t i = i0 + lane;
         int64_t left = 0, base = 0;
-        if (i < A.n && !(A.flag && A.flag[i])) {
+        if (lane < sites && i < A.n && !(A.flag && A.flag[i])) {
             left = A.photons[i];
             if (left > 0) {
                 const int32_t sg = A.seg[i];
@@ -740,9 +746,11 @@ cudaError_t launch_surrogate_sample(const SurSampleArgs& a, int num_sms, cudaStr
 {
     if (a.n <= 0) return cudaSuccess;
     if (a.cells < 1 || a.cells > sur::CELLS) return cudaErrorInvalidValue;
-    const int64_t want = (a.n + 32 * sur::SAMPLE_WARPS - 1) / (32 * sur::SAMPLE_WARPS);
+    int sites = 1;
+    while (sites < 32 && a.n > (int64_t)sites * num_sms * sur::SAMPLE_CTAS * sur::SAMPLE_WARPS) sites *= 2;
+    const int64_t want = (a.n + sites * sur::SAMPLE_WARPS - 1) / (sites * sur::SAMPLE_WARPS);
     const int64_t cap = (int64_t)num_sms * 16;
-    sur::surrogate_sample<<<(unsigned)(want < cap ? want : cap), 32 * sur::SAMPLE_WARPS, 0, st>>>(a);
+    sur::surrogate_sample<<<(unsigned)(want < cap ? want : cap), 32 * sur::SAMPLE_WARPS, 0, st>>>(a, sites);
     return cudaGetLastError();
 }
 
