@@ -53,18 +53,18 @@ OPS_PER_STEP = {"scan256": 165.6, "point1m": 186.7}
 L2_FLUSH_BYTES = 256 << 20
 # DRAM bytes (read + write) per photon-step of the transport kernel, from one
 # ncu capture of each workload at a reduced size (scan: 20,000 photons per
-# point, 3.01 GB for 494.8M photon-steps; point source: the whole 10^6-photon
-# launch, 143 MB for 12.33M photon-steps, mostly the table's first touches),
-# scaled to a full launch by its photon-steps.  Almost all of it is L2 misses of the 64 MB log table (about 2
-# bytes per photon-step and lookup), which grow in proportion to the steps;
-# the sources, offsets and maps are 0.24 MB.
-TRAFFIC_PER_STEP = {"scan256": (3.003462e9 + 7.173888e6) / 494_804_727,
-                    "point1m": (139.735552e6 + 3.632384e6) / 12_332_791}
+# point, 5.14 GB for 495.9M photon-steps; point source: the whole 10^6-photon
+# launch, 540 MB for 12.31M photon-steps), scaled to a full launch by its
+# photon-steps.  Almost all of it is L2 misses of the 128 MB tables of log u and
+# sqrt(-2 log u), which grow in proportion to the steps; the sources, offsets and
+# maps are 0.24 MB.
+TRAFFIC_PER_STEP = {"scan256": (5.134535e9 + 5.811712e6) / 495_901_067,
+                    "point1m": (536.278784e6 + 3.960576e6) / 12_314_911}
 # Warp instructions the transport kernel issues per photon-step (smsp__inst_executed
-# of the same ncu captures: 15.42 G for 494.8M photon-steps on the scan, 0.80 G
-# for 12.33M on the point source); with the live steps/s this gives the
+# of the same ncu captures: 9.29 G for 495.9M photon-steps on the scan, 0.485 G
+# for 12.31M on the point source); with the live steps/s this gives the
 # kernel's issue rate against the SMs' issue slots.
-WARP_INST_PER_STEP = {"scan256": 15_422_450_065 / 494_804_727, "point1m": 804_971_827 / 12_332_791}
+WARP_INST_PER_STEP = {"scan256": 9_285_231_022 / 495_901_067, "point1m": 484_656_024 / 12_314_911}
 
 
 def events_workload(n_events: int = 50_000):
@@ -631,7 +631,7 @@ def measure_photons(eng, W, steps: int, warmup: int, dev, stream, pid_base: int 
 def roofline(W, steps_per_launch: int, launch_s: float, in_bytes: int, out_bytes: int, n_sm: int) -> dict:
     """The transport kernel against the SMs' lane-op ceiling (its bound), its
     issue rate against the issue slots, and its DRAM traffic (the L2 misses of
-    the 64 MB log table dominate it) against HBM."""
+    the 128 MB tables dominate it) against HBM."""
     peaks = measured_peaks()
     sm_mhz = peaks.get("sm_max_mhz", 1965.0)
     ops_step = OPS_PER_STEP[W["name"]]
@@ -651,7 +651,7 @@ def roofline(W, steps_per_launch: int, launch_s: float, in_bytes: int, out_bytes
                 "frac": dram / launch_s / 1e9 / hbm_peak, "dram_bytes": dram,
                 "algorithmic_bytes": in_bytes + out_bytes,
                 "note": ("DRAM bytes per launch (ncu dram__bytes read+write per photon-step x "
-                         "steps: L2 misses of the log table) over the launch time; the "
+                         "steps: L2 misses of the tables) over the launch time; the "
                          "algorithmic bytes are the sources, offsets, maps, times and counters")},
         "issue_slots": issue_slots(W["name"], steps_per_launch / launch_s, n_sm, sm_mhz),
     }
