@@ -193,8 +193,9 @@ __device__ __forceinline__ float uniform_log(const float* __restrict__ tab, floa
 //   * booking an ended photon and starting the next one wait for a few free lanes.
 // Against the same states with exact expressions and a branch per outcome
 // (31.2 -> 20.4 warp instructions per photon-step): BGO+ESR scan of 51.2M
-// photons 143.9 -> 100.4 ms (49 G photon-steps/s), 3,001 CsI(Tl)+Teflon events
-// 32.6 -> 20.6 ms, 10^6-photon CsI(Tl) point 1.17 -> 0.79 ms.
+// photons 143.9 -> 100.4 ms (49 G photon-steps/s; 93.5 ms and 18.7 instructions with
+// the rare paths out of line), 3,001 CsI(Tl)+Teflon events
+// 32.6 -> 20.6 ms (19.3), 10^6-photon CsI(Tl) point 1.17 -> 0.79 ms.
 template <int MODE, bool REC, bool TILE, int SPEC, bool TAB>
 __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(const __grid_constant__ KArgs A)
 {
