@@ -629,6 +629,7 @@ struct NetTrain {
     bool wide;                           // targets 32-byte aligned
     float scale;
     float* loss;
+    int whole;                           // tiles below this add four sums per 32 rows to the loss, the others six
 };
 
 constexpr int STORE_WARP = EPI_WARPS + 2;        // training: issues the TMA stores of the operands
@@ -646,6 +647,7 @@ __global__ void __launch_bounds__(TRAIN ? NET_TRAIN_THREADS : GEMM_THREADS, 1)
     __shared__ int abort_flag;
     __shared__ __align__(16) float s_cst[2][NET_CST];
     __shared__ float4 s_x[EPI_WARPS][16];
+    __shared__ float2 s_sq[2][4][4];         // training: squared errors by slot, 32 rows and column group
 
     if (TRAIN) pdl_trigger();
 
@@ -751,6 +753,24 @@ __global__ void __launch_bounds__(TRAIN ? NET_TRAIN_THREADS : GEMM_THREADS, 1)
                 for (int j = 0; j < D_OUT / 32; ++j)
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(T.target + (int64_t)r[i] * D_OUT + 32 * j));
         };
+        // The loss is one FP32 sum over all steps, and the rounding of its additions
+        // (about 1e-5 of it) depends on what is added at a time, not on the order.
+        // So that losses stay comparable with those of the kernel per layer, its
+        // sums are added: per 32 rows the columns 0-31 and 128-159, 32-63 and
+        // 160-191, 64-95, 96-127, and in the tiles of a short last round each 32
+        // columns by themselves.  The column groups' sums are [.x: 32 columns of
+        // one chunk, .y: 16 columns of the chunk shared with the neighbour].
+        auto add_loss = [&](int s, int tile) {
+            const int j = lane >> 2;
+            if (j >= (tile < T.whole ? 4 : 6)) return;
+            const float2* q = s_sq[s][lane & 3];
+            auto chunk = [&](int c) {
+                return c == 1 ? q[0].y + q[1].y : c == 4 ? q[2].y + q[3].y : q[(c + 1) >> 1].x;
+            };
+            float d = chunk(j);
+            if (tile < T.whole && j < 2) d += chunk(j + 4);
+            atomicAdd(T.loss, d * T.scale);
+        };
         fetch_targets(0);
         fetch_targets(1);
         for (int u0 = 0; u0 < my_units && ok; u0 += 2)
@@ -765,14 +785,22 @@ __global__ void __launch_bounds__(TRAIN ? NET_TRAIN_THREADS : GEMM_THREADS, 1)
                                 umma::tma_store_2d(&T.h[l], c * TILE_K, tile * TILE_M,
                                                    smem + s * NET_A_BYTES + c * (TILE_M * 128));
                             umma::bulk_commit();
-                            umma::bulk_wait_read0();
-                            umma::mbar_arrive(&stored[s]);
                         } else {
                             atomicOr(G.err, 1u);
                             *abort_v = 1;
                         }
                     }
                     ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+                    if (!ok) break;
+                    if (l == 3) {
+                        __syncwarp();
+                        add_loss(s, (int)blockIdx.x + (u0 + s) * (int)gridDim.x);
+                        __syncwarp();
+                    }
+                    if (lane == 0) {
+                        umma::bulk_wait_read0();
+                        umma::mbar_arrive(&stored[s]);
+                    }
                 }
                 if (ok && l == 2) {
                     fetch_targets(u0 + 2);
@@ -789,7 +817,6 @@ __global__ void __launch_bounds__(TRAIN ? NET_TRAIN_THREADS : GEMM_THREADS, 1)
         int loaded[2] = {-1, -1};                         // member whose constants a slot holds
         uint32_t job[2] = {0, 0}, met = 0;
         bool ok = true;
-        float sq = 0.0f;                                  // training: squared error of this lane's rows
         auto give_up = [&] {
             if (lane == 0) atomicOr(G.err, 1u);
             *abort_v = 1;
@@ -937,9 +964,11 @@ __global__ void __launch_bounds__(TRAIN ? NET_TRAIN_THREADS : GEMM_THREADS, 1)
                 const float* b4 = s_cst[s] + 2 * D_H;
                 if (TRAIN) {
                     // loss: dO into the (consumed) operand memory for the store warp
+                    float2 sq = make_float2(0.f, 0.f);   // squared errors, see add_loss
 #pragma unroll
                     for (int k = 0; k < 3; ++k) {
                         const int c0 = 48 * group + 16 * k;
+                        float sk = 0.0f;
                         if (k == 0) fetch_t(2);
                         float v[16];
                         umma::tmem_ld16(tmem + s * 256u + tlane + (uint32_t)c0, v);
@@ -951,7 +980,7 @@ __global__ void __launch_bounds__(TRAIN ? NET_TRAIN_THREADS : GEMM_THREADS, 1)
 #pragma unroll
                             for (int q = 0; q < 8; ++q) {
                                 const float d = (v[8 * i + q] + b[q]) - tg[k][8 * i + q];
-                                sq += d * d;
+                                sk += d * d;
                                 g[8 * i + q] = __float2bfloat16_rn(2.0f * d * T.scale);
                             }
                         }
@@ -960,7 +989,15 @@ __global__ void __launch_bounds__(TRAIN ? NET_TRAIN_THREADS : GEMM_THREADS, 1)
                         for (int i = 0; i < 2; ++i)
                             *reinterpret_cast<uint4*>(blk + sw128((uint32_t)row, (uint32_t)(((c0 & 63) >> 3) + i))) =
                                 reinterpret_cast<const uint4*>(g)[i];
+                        if (k == (group & 1 ? 0 : 2)) sq.y += sk;
+                        else sq.x += sk;
                     }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        sq.x += __shfl_xor_sync(0xffffffffu, sq.x, o);
+                        sq.y += __shfl_xor_sync(0xffffffffu, sq.y, o);
+                    }
+                    if (lane == 0) s_sq[s][quad][group] = sq;
                     umma::fence_before_sync();
                     stage_done();
                     if (lane == 0) umma::mbar_arrive(&o_ready[s]);
@@ -997,11 +1034,6 @@ __global__ void __launch_bounds__(TRAIN ? NET_TRAIN_THREADS : GEMM_THREADS, 1)
                     wait_stored(s);
                     if (ok) first_layer(s, u0 + s + 2, [](int) {});
                 }
-        }
-        if (TRAIN) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-            if (lane == 0) atomicAdd(T.loss, sq * T.scale);
         }
     }
     __syncthreads();
@@ -1568,6 +1600,8 @@ int forward_backward(cl_mlp* m, int B, const float* x, const float* target, cons
     t.z2 = m->z2; t.z3 = m->z3; t.target = target; t.rows = rows; t.brow = m->brow;
     t.wide = ((uintptr_t)target & 31) == 0;
     t.scale = 1.0f / ((float)B * (float)D_OUT); t.loss = m->loss;
+    const int tail = f.tiles % grid;
+    t.whole = 2 * tail <= grid ? f.tiles - tail : f.tiles;
     if (launch_pdl(net_forward<true>, dim3((unsigned)grid), dim3(NET_TRAIN_THREADS), NET_SMEM, st, f, t) != cudaSuccess)
         return CL_ERR_CUDA;
     k.z3 = m->z3; k.z2 = m->z2; k.x = x; k.params = m->p; k.grad = m->g; k.brow = m->brow; k.tiles = B / TILE_M; k.err = m->derr;
