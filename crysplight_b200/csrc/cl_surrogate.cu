@@ -833,9 +833,11 @@ int cl_surrogate_direct_sites(const float* d_xyz, const int32_t* d_site, int64_t
     const int64_t want = (n_sites + cl::sur::DIRECT_WARPS - 1) / cl::sur::DIRECT_WARPS;
     const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
     const size_t smem = cl::sur::DIRECT_WARPS * cl::sur::direct_warp_floats(a.nx, a.ny) * sizeof(float);
-    // 64 x 1 pixels: 144 KB (8 x 8: 46 KB); the opt-in is per device
+    // 8 x 8 pixels: 53 KB; the opt-in is per device, and for the widest grid
+    // (64 x 1: 152 KB) whatever this one is, since threads may launch different grids
+    constexpr size_t most = cl::sur::DIRECT_WARPS * cl::sur::direct_warp_floats(cl::sur::CELLS, 1) * sizeof(float);
     if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(cl::sur::surrogate_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+        cudaFuncSetAttribute(cl::sur::surrogate_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) {
         cudaGetLastError();
         return CL_ERR_CUDA;
     }
