@@ -79,6 +79,7 @@ struct KArgs {
     unsigned long long* steps;
     unsigned int* done;
     unsigned int* err;
+    unsigned long long* status;   // point: the steps and the error word, beside the outputs (or NULL)
     const float* logtab;  // log u and sqrt(-2 log u) of every uniform (logtab_fill), or NULL: compute
     unsigned long long budget_ns;   // device time budget of the launch, 0 = none
 };
@@ -626,6 +627,10 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                 const uint32_t kk = __ldcg(A.keys + i);
                 A.keys[i] = __float_as_uint(key_float(kk));
             }
+            if (tid == 0 && A.status) {
+                A.status[0] = __ldcg(A.steps);
+                A.status[1] = __ldcg(A.err);
+            }
         }
     }
 }
@@ -662,7 +667,8 @@ __global__ void logtab_fill(float* t)
 
 // Segment mode: decode tmin keys in place and sum npe per segment.
 __global__ void finalize_segments(const uint32_t* maps, uint32_t* keys, int32_t* npe,
-                                  int64_t n_seg, int32_t cells)
+                                  int64_t n_seg, int32_t cells, const unsigned long long* steps,
+                                  const unsigned int* err, unsigned long long* status)
 {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     const int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -674,6 +680,7 @@ __global__ void finalize_segments(const uint32_t* maps, uint32_t* keys, int32_t*
         for (int c = 0; c < cells; ++c) acc += m[c];
         npe[s] = (int32_t)acc;
     }
+    if (i0 == 0 && status) { status[0] = *steps; status[1] = *err; }
 }
 
 __global__ void decode_keys_kernel(uint32_t* keys, int64_t n)
@@ -785,6 +792,17 @@ struct DevBuf {
     size_t cap = 0;
 };
 
+// Calls on host arrays gather small ones in the handle's host buffer: one copy in
+// and one out, with the steps and the error word, which the kernels leave behind
+// the counters.  A copy to pageable memory waits for the stream by itself, and a
+// point source's call ended in five of them.  2,000 CsI(Tl) photons from one point
+// 237 -> 191 us a call, 10^6 784 -> 739 us (page-locked memory would save another
+// 10 us and costs 400 us per handle).  Arrays beyond the limits (4,096 positions,
+// 1,022 time bins, 507 segments), which belong to transports of milliseconds, are
+// copied one by one, straight to the caller's memory.
+constexpr size_t N_STATUS = sizeof(cl_counters) / 8, STATUS_BYTES = sizeof(cl_counters) + 16;
+constexpr size_t STAGE_IN = 64 << 10, STAGE_OUT = 256 << 10;
+
 struct cl_handle {
     int device = 0;
     int num_sms = 0;
@@ -792,6 +810,7 @@ struct cl_handle {
     DevBuf logtab;                 // the tables of the uniforms, or empty: the kernels compute them
     char err[512] = {0};
     DevBuf src, out, rec, scratch, dbg;
+    char* stage = nullptr;         // STAGE_IN + STAGE_OUT bytes, or null: host arrays are copied one by one
     int ctas_per_sm = 0;
     int threads = 256;
     int warp_chunk = CL_DEFAULT_WARP_CHUNK;   // 0: automatic per launch
@@ -930,6 +949,7 @@ int cl_create(cl_handle** out, int device)
         delete h;
         return CL_ERR_OOM;
     }
+    h->stage = (char*)malloc(STAGE_IN + STAGE_OUT);
     // 128 MB: the logs of all 2^24 uniforms and their sqrt(-2 log u); without
     // them (allocation failure) the kernels evaluate the same functions in place
     if (cudaMalloc(&h->logtab.p, sizeof(float) << 25) == cudaSuccess) {
@@ -955,6 +975,7 @@ void cl_destroy(cl_handle* h)
     if (h->stream) cudaStreamSynchronize(h->stream);
     DevBuf* bufs[] = {&h->src, &h->out, &h->rec, &h->scratch, &h->dbg, &h->logtab};
     for (DevBuf* b : bufs) if (b->p) cudaFree(b->p);
+    free(h->stage);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }
@@ -1139,7 +1160,7 @@ static int launch_transport(cl_handle* h, const KArgs& a, size_t smem, cudaStrea
 static int enqueue_point(cl_handle* h, const Physics& P, const float* px, const float* py,
                          const float* pz, const float* pt, int32_t npos, int64_t n, uint64_t pid0,
                          uint32_t* counts, uint32_t* keys, unsigned long long* counters,
-                         const cl_records* rec, cudaStream_t st)
+                         const cl_records* rec, cudaStream_t st, unsigned long long* status = nullptr)
 {
     const int cells = P.nx * P.ny;
     const int bins_total = P.nbins + 1;
@@ -1150,6 +1171,7 @@ static int enqueue_point(cl_handle* h, const Physics& P, const float* px, const 
     CK(h, cudaGetLastError(), "init kernel launch");
     if (n == 0) {
         // no photons: decode the +Inf keys into Float32 +Inf
+        if (status) CK(h, cudaMemsetAsync(status, 0, 2 * sizeof *status, st), "zero status");
         decode_keys_kernel<<<1, 256, 0, st>>>(keys, cells);
         CK(h, cudaGetLastError(), "decode launch");
         return CL_OK;
@@ -1162,7 +1184,7 @@ static int enqueue_point(cl_handle* h, const Physics& P, const float* px, const 
     a.counts = counts; a.keys = keys; a.counters = counters;
     const bool want_rec = rec && (rec->status || rec->idx || rec->t || rec->bounces);
     if (want_rec) { a.r_status = rec->status; a.r_idx = rec->idx; a.r_t = rec->t; a.r_bounces = rec->bounces; }
-    a.queue = s.queue; a.steps = s.steps; a.done = s.done; a.err = s.err;
+    a.queue = s.queue; a.steps = s.steps; a.done = s.done; a.err = s.err; a.status = status;
     a.logtab = (const float*)h->logtab.p;
     a.budget_ns = h->budget_ns;
     const size_t tile_bytes = ((size_t)n_counts + cells) * sizeof(uint32_t);
@@ -1188,7 +1210,7 @@ static int enqueue_segments(cl_handle* h, const Physics& P, const float* sx, con
                             uint32_t* maps, uint32_t* keys, int32_t* npe,
                             unsigned long long* counters, const cl_records* rec, cudaStream_t st,
                             unsigned long long* tsum = nullptr, unsigned long long* tsum2 = nullptr,
-                            const SurSampleArgs* sample = nullptr)
+                            const SurSampleArgs* sample = nullptr, unsigned long long* status = nullptr)
 {
     const int cells = P.nx * P.ny;
     const int64_t total = (int64_t)cells * n_seg;
@@ -1227,19 +1249,13 @@ static int enqueue_segments(cl_handle* h, const Physics& P, const float* sx, con
         CK(h, launch_surrogate_sample(sa, h->num_sms, st), "surrogate sampler launch");
     }
     finalize_segments<<<(unsigned)std::min<int64_t>((total + 255) / 256 + 1, 8192), 256, 0, st>>>(
-        maps, keys, npe, n_seg, cells);
+        maps, keys, npe, n_seg, cells, s.steps, s.err, status);
     CK(h, cudaGetLastError(), "finalize launch");
     return CL_OK;
 }
 
-static int collect(cl_handle* h, cudaStream_t st)
+static int report(cl_handle* h, unsigned long long steps, unsigned int err)
 {
-    Scratch s = scratch_of(h);
-    unsigned long long steps = 0;
-    unsigned int err = 0;
-    CK(h, cudaMemcpyAsync(&steps, s.steps, sizeof steps, cudaMemcpyDeviceToHost, st), "copy steps");
-    CK(h, cudaMemcpyAsync(&err, s.err, sizeof err, cudaMemcpyDeviceToHost, st), "copy status");
-    CK(h, cudaStreamSynchronize(st), "stream synchronize");
     h->last_steps = (int64_t)steps;
     if (err & 32u)
         return set_err(h, CL_ERR_TIMEOUT, "the transport ran past the handle's time budget (%.3g s); "
@@ -1250,6 +1266,14 @@ static int collect(cl_handle* h, cudaStream_t st)
     if (err & 4u) return set_err(h, CL_ERR_TIMEOUT, "a loop budget of the surrogate sampler ran out");
     if (err) return set_err(h, CL_ERR_TIMEOUT, "a device-side loop budget ran out (Rayleigh rejection sampler)");
     return CL_OK;
+}
+
+static int collect(cl_handle* h, cudaStream_t st)
+{
+    unsigned long long words[3];     // the scratch words
+    CK(h, cudaMemcpyAsync(words, h->scratch.p, sizeof words, cudaMemcpyDeviceToHost, st), "copy status");
+    CK(h, cudaStreamSynchronize(st), "stream synchronize");
+    return report(h, words[1], (unsigned int)(words[2] >> 32));
 }
 
 extern "C" {
@@ -1279,7 +1303,7 @@ int cl_run_photons(cl_handle* h, const cl_box* box, const cl_optical_params* op,
     const size_t b_src = align256(4 * (size_t)npos * sizeof(float));
     const size_t b_counts = align256(n_counts * sizeof(uint32_t));
     const size_t b_keys = align256((size_t)cells * sizeof(uint32_t));
-    const size_t b_ctr = align256(sizeof(cl_counters));
+    const size_t b_ctr = align256(STATUS_BYTES);
     if ((rc = ensure(h, h->src, b_src)) != CL_OK) return rc;
     if ((rc = ensure(h, h->out, b_counts + b_keys + b_ctr)) != CL_OK) return rc;
     float* d_px = (float*)h->src.p;
@@ -1304,19 +1328,36 @@ int cl_run_photons(cl_handle* h, const cl_box* box, const cl_optical_params* op,
         if (records->bounces) drec.bounces = (int32_t*)(base + b1 + b2 + b4);
     }
 
-    CK(h, cudaMemcpyAsync(d_px, px, npos * sizeof(float), cudaMemcpyHostToDevice, st), "copy px");
-    CK(h, cudaMemcpyAsync(d_py, py, npos * sizeof(float), cudaMemcpyHostToDevice, st), "copy py");
-    CK(h, cudaMemcpyAsync(d_pz, pz, npos * sizeof(float), cudaMemcpyHostToDevice, st), "copy pz");
-    if (pt) CK(h, cudaMemcpyAsync(d_pt, pt, npos * sizeof(float), cudaMemcpyHostToDevice, st), "copy pt");
+    const size_t fs = (size_t)npos * sizeof(float);
+    if (h->stage && 4 * fs <= STAGE_IN) {
+        char* in = h->stage;
+        memcpy(in, px, fs);
+        memcpy(in + fs, py, fs);
+        memcpy(in + 2 * fs, pz, fs);
+        if (pt) memcpy(in + 3 * fs, pt, fs);
+        CK(h, cudaMemcpyAsync(d_px, in, (pt ? 4 : 3) * fs, cudaMemcpyHostToDevice, st), "copy positions");
+    } else {
+        CK(h, cudaMemcpyAsync(d_px, px, fs, cudaMemcpyHostToDevice, st), "copy px");
+        CK(h, cudaMemcpyAsync(d_py, py, fs, cudaMemcpyHostToDevice, st), "copy py");
+        CK(h, cudaMemcpyAsync(d_pz, pz, fs, cudaMemcpyHostToDevice, st), "copy pz");
+        if (pt) CK(h, cudaMemcpyAsync(d_pt, pt, fs, cudaMemcpyHostToDevice, st), "copy pt");
+    }
 
     const Physics P = make_physics(box, op, ro, tb, tau_ns, max_bounces, seed);
     rc = enqueue_point(h, P, d_px, d_py, d_pz, pt ? d_pt : nullptr, npos, n_photons, pid_offset,
-                       d_counts, d_keys, d_ctr, want_rec ? &drec : nullptr, st);
+                       d_counts, d_keys, d_ctr, want_rec ? &drec : nullptr, st, d_ctr + N_STATUS);
     if (rc != CL_OK) return rc;
 
-    CK(h, cudaMemcpyAsync(counts, d_counts, n_counts * sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "copy counts");
-    CK(h, cudaMemcpyAsync(first_ns, d_keys, (size_t)cells * sizeof(float), cudaMemcpyDeviceToHost, st), "copy first_ns");
-    CK(h, cudaMemcpyAsync(counters, d_ctr, sizeof(cl_counters), cudaMemcpyDeviceToHost, st), "copy counters");
+    char* const back = h->stage ? h->stage + STAGE_IN : nullptr;
+    const bool gathered = h->stage && b_counts + b_keys + b_ctr <= STAGE_OUT;
+    if (gathered) {
+        CK(h, cudaMemcpyAsync(back, h->out.p, b_counts + b_keys + STATUS_BYTES, cudaMemcpyDeviceToHost, st),
+           "copy outputs");
+    } else {
+        CK(h, cudaMemcpyAsync(counts, d_counts, n_counts * sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "copy counts");
+        CK(h, cudaMemcpyAsync(first_ns, d_keys, (size_t)cells * sizeof(float), cudaMemcpyDeviceToHost, st), "copy first_ns");
+        CK(h, cudaMemcpyAsync(counters, d_ctr, sizeof(cl_counters), cudaMemcpyDeviceToHost, st), "copy counters");
+    }
     if (want_rec && n_photons > 0) {
         const size_t n = (size_t)n_photons;
         if (records->status) CK(h, cudaMemcpyAsync(records->status, drec.status, n, cudaMemcpyDeviceToHost, st), "copy status");
@@ -1324,7 +1365,14 @@ int cl_run_photons(cl_handle* h, const cl_box* box, const cl_optical_params* op,
         if (records->t) CK(h, cudaMemcpyAsync(records->t, drec.t, 4 * n, cudaMemcpyDeviceToHost, st), "copy t");
         if (records->bounces) CK(h, cudaMemcpyAsync(records->bounces, drec.bounces, 4 * n, cudaMemcpyDeviceToHost, st), "copy bounces");
     }
-    return collect(h, st);
+    if (!gathered) return collect(h, st);
+    CK(h, cudaStreamSynchronize(st), "stream synchronize");
+    unsigned long long status[2];
+    memcpy(counts, back, n_counts * sizeof(uint32_t));
+    memcpy(first_ns, back + b_counts, (size_t)cells * sizeof(float));
+    memcpy(counters, back + b_counts + b_keys, sizeof(cl_counters));
+    memcpy(status, back + b_counts + b_keys + 8 * N_STATUS, sizeof status);
+    return report(h, status[0], (unsigned int)status[1]);
 }
 
 int cl_run_photons_device(cl_handle* h, const cl_box* box, const cl_optical_params* op,
@@ -1392,7 +1440,7 @@ int cl_run_segments(cl_handle* h, const cl_box* box, const cl_optical_params* op
     const size_t b_seg = align256((size_t)n_src * sizeof(int32_t));
     const size_t b_maps = align256(total * sizeof(uint32_t));
     const size_t b_npe = align256((size_t)n_segments * sizeof(int32_t));
-    const size_t b_ctr = align256(sizeof(cl_counters));
+    const size_t b_ctr = align256(STATUS_BYTES);
     if ((rc = ensure(h, h->src, 4 * b_f + b_off + b_seg)) != CL_OK) return rc;
     if ((rc = ensure(h, h->out, 2 * b_maps + b_npe + b_ctr)) != CL_OK) return rc;
     char* sb = (char*)h->src.p;
@@ -1421,22 +1469,42 @@ int cl_run_segments(cl_handle* h, const cl_box* box, const cl_optical_params* op
         if (records->t) drec.t = (float*)(base + b1 + b2);
         if (records->bounces) drec.bounces = (int32_t*)(base + b1 + b2 + b4);
     }
-    const size_t fs = (size_t)n_src * sizeof(float);
-    CK(h, cudaMemcpyAsync(d_sx, sx, fs, cudaMemcpyHostToDevice, st), "copy sx");
-    CK(h, cudaMemcpyAsync(d_sy, sy, fs, cudaMemcpyHostToDevice, st), "copy sy");
-    CK(h, cudaMemcpyAsync(d_sz, sz, fs, cudaMemcpyHostToDevice, st), "copy sz");
-    if (st_) CK(h, cudaMemcpyAsync(d_st, st_, fs, cudaMemcpyHostToDevice, st), "copy st");
-    CK(h, cudaMemcpyAsync(d_off, src_offsets, (size_t)(n_src + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st), "copy offsets");
-    CK(h, cudaMemcpyAsync(d_seg, src_segment, (size_t)n_src * sizeof(int32_t), cudaMemcpyHostToDevice, st), "copy segments");
+    const size_t fs = (size_t)n_src * sizeof(float), os = (size_t)(n_src + 1) * sizeof(int64_t);
+    const size_t ss = (size_t)n_src * sizeof(int32_t);
+    if (h->stage && 4 * b_f + b_off + b_seg <= STAGE_IN) {
+        char* in = h->stage;              // laid out as on the device
+        memcpy(in, sx, fs);
+        memcpy(in + b_f, sy, fs);
+        memcpy(in + 2 * b_f, sz, fs);
+        if (st_) memcpy(in + 3 * b_f, st_, fs);
+        memcpy(in + 4 * b_f, src_offsets, os);
+        memcpy(in + 4 * b_f + b_off, src_segment, ss);
+        CK(h, cudaMemcpyAsync(sb, in, 4 * b_f + b_off + ss, cudaMemcpyHostToDevice, st), "copy sources");
+    } else {
+        CK(h, cudaMemcpyAsync(d_sx, sx, fs, cudaMemcpyHostToDevice, st), "copy sx");
+        CK(h, cudaMemcpyAsync(d_sy, sy, fs, cudaMemcpyHostToDevice, st), "copy sy");
+        CK(h, cudaMemcpyAsync(d_sz, sz, fs, cudaMemcpyHostToDevice, st), "copy sz");
+        if (st_) CK(h, cudaMemcpyAsync(d_st, st_, fs, cudaMemcpyHostToDevice, st), "copy st");
+        CK(h, cudaMemcpyAsync(d_off, src_offsets, os, cudaMemcpyHostToDevice, st), "copy offsets");
+        CK(h, cudaMemcpyAsync(d_seg, src_segment, ss, cudaMemcpyHostToDevice, st), "copy segments");
+    }
 
     const Physics P = make_physics(box, op, ro, tb, tau_ns, max_bounces, seed);
     rc = enqueue_segments(h, P, d_sx, d_sy, d_sz, st_ ? d_st : nullptr, d_off, d_seg, n_src, n_segments,
-                          n, pid_offset, d_maps, d_keys, d_npe, d_ctr, want_rec ? &drec : nullptr, st);
+                          n, pid_offset, d_maps, d_keys, d_npe, d_ctr, want_rec ? &drec : nullptr, st, nullptr, nullptr,
+                          nullptr, d_ctr + N_STATUS);
     if (rc != CL_OK) return rc;
-    CK(h, cudaMemcpyAsync(maps, d_maps, total * sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "copy maps");
-    CK(h, cudaMemcpyAsync(tmin, d_keys, total * sizeof(float), cudaMemcpyDeviceToHost, st), "copy tmin");
-    CK(h, cudaMemcpyAsync(npe, d_npe, (size_t)n_segments * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "copy npe");
-    CK(h, cudaMemcpyAsync(counters, d_ctr, sizeof(cl_counters), cudaMemcpyDeviceToHost, st), "copy counters");
+    char* const back = h->stage ? h->stage + STAGE_IN : nullptr;
+    const bool gathered = h->stage && 2 * b_maps + b_npe + b_ctr <= STAGE_OUT;
+    if (gathered) {
+        CK(h, cudaMemcpyAsync(back, ob, 2 * b_maps + b_npe + STATUS_BYTES, cudaMemcpyDeviceToHost, st),
+           "copy outputs");
+    } else {
+        CK(h, cudaMemcpyAsync(maps, d_maps, total * sizeof(uint32_t), cudaMemcpyDeviceToHost, st), "copy maps");
+        CK(h, cudaMemcpyAsync(tmin, d_keys, total * sizeof(float), cudaMemcpyDeviceToHost, st), "copy tmin");
+        CK(h, cudaMemcpyAsync(npe, d_npe, (size_t)n_segments * sizeof(int32_t), cudaMemcpyDeviceToHost, st), "copy npe");
+        CK(h, cudaMemcpyAsync(counters, d_ctr, sizeof(cl_counters), cudaMemcpyDeviceToHost, st), "copy counters");
+    }
     if (want_rec && n > 0) {
         const size_t m = (size_t)n;
         if (records->status) CK(h, cudaMemcpyAsync(records->status, drec.status, m, cudaMemcpyDeviceToHost, st), "copy status");
@@ -1444,7 +1512,15 @@ int cl_run_segments(cl_handle* h, const cl_box* box, const cl_optical_params* op
         if (records->t) CK(h, cudaMemcpyAsync(records->t, drec.t, 4 * m, cudaMemcpyDeviceToHost, st), "copy t");
         if (records->bounces) CK(h, cudaMemcpyAsync(records->bounces, drec.bounces, 4 * m, cudaMemcpyDeviceToHost, st), "copy bounces");
     }
-    return collect(h, st);
+    if (!gathered) return collect(h, st);
+    CK(h, cudaStreamSynchronize(st), "stream synchronize");
+    unsigned long long status[2];
+    memcpy(maps, back, total * sizeof(uint32_t));
+    memcpy(tmin, back + b_maps, total * sizeof(float));
+    memcpy(npe, back + 2 * b_maps, (size_t)n_segments * sizeof(int32_t));
+    memcpy(counters, back + 2 * b_maps + b_npe, sizeof(cl_counters));
+    memcpy(status, back + 2 * b_maps + b_npe + 8 * N_STATUS, sizeof status);
+    return report(h, status[0], (unsigned int)status[1]);
 }
 
 int cl_run_segments_device(cl_handle* h, const cl_box* box, const cl_optical_params* op,
