@@ -39,6 +39,9 @@ namespace cl {
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int GAUSS_OFF = 1 << 24;    // sqrt(-2 log u) after the 2^24 logs
 constexpr int N_COUNTERS = 10;        // cl_counters, then the photon-steps
+// Photons per slot from which a launch's detections are added slot by slot
+// (segment mode; see add_crowded): few cells, and the 64 of a full map.
+constexpr int64_t CROWDED_FEW = 1024, CROWDED = 4096;
 constexpr int SPREAD_WARPS = 8;        // warps per SM of a launch of few photons
 constexpr size_t CTA_EXTRA_SMEM = 1024 + 8 * N_COUNTERS * 8 + 16;   // reserved and static shared memory of a CTA
 constexpr int SCTAB_BYTES = CLM_SC_N * 16;
@@ -71,7 +74,7 @@ struct KArgs {
     uint32_t* counts;     // point: cells*bins_total
     uint32_t* keys;       // point: cells; segments: cells*n_seg
     uint32_t* maps;       // segments: cells*n_seg
-    unsigned long long* tsum;   // segments with moments (MODE 2): cells*n_seg
+    unsigned long long* tsum;   // segments with moments: cells*n_seg
     unsigned long long* tsum2;
     unsigned long long* counters;  // 9 x int64, cl_counters order
     uint8_t* r_status; int16_t* r_idx; float* r_t; int32_t* r_bounces;
@@ -134,6 +137,29 @@ static __device__ __noinline__ int64_t find_source(const int64_t* __restrict__ o
     }
     return lo;
 }
+
+// Adds the detections of a warp's active lanes, all lanes of a slot together:
+// one reduction per distinct slot.  Where tens of photons share a slot at any
+// time, the reductions on one address are the bound (the L2 takes about one per
+// clock); elsewhere finding the lanes out costs more than it saves.  4M photons
+// of a crystal that most leave on the first step, one 1x1 segment: 2,880 us one
+// by one, 900 so; 8x8: 1,860 and 1,700; 512 segments of 1x1: 2,230 and 930, of
+// 8x8: 985 and 1,060.  A scan of 200,000 photons per point and 8x8 map (3,125 a
+// slot) takes 93.3 ms one by one and 95.2 so; hence the two thresholds.
+static __device__ __noinline__ void add_crowded(uint32_t* maps, uint32_t* keys, unsigned long long slot, uint32_t key)
+{
+    const unsigned same = __match_any_sync(__activemask(), (uint32_t)slot);
+    key = __reduce_min_sync(same, key);
+    if ((int)(threadIdx.x & 31) == __ffs(same) - 1) {
+        atomicAdd(maps + slot, (uint32_t)__popc(same));
+        atomicMin(keys + slot, key);
+    }
+}
+
+// What a kernel instance computes: counts over the cells and time bins of one
+// readout plane; a map per segment; that with arrival-time moments; and the two
+// segment modes with crowded slots.
+enum : int { POINT = 0, SEGMENTS = 1, MOMENTS = 2, SEGMENTS_CROWDED = 3, MOMENTS_CROWDED = 4 };
 
 // Per-lane transport states of the warp loop.  One loop iteration moves each
 // active lane one state forward; a whole wall interaction (move, UNIFIED try,
@@ -284,7 +310,7 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                     const uint32_t key = float_key(t);
                     // one reduction per photon: a warp seldom detects two photons in
                     // the same slot, and finding out costs more than it saves
-                    if (MODE == 0) {
+                    if (MODE == POINT) {
                         atomicAdd(tile_counts + cell + A.cells * time_bin0(t, P), 1u);
                         // the cells' keys are hot; most photons are later than the
                         // key already there (which only ever falls)
@@ -294,9 +320,13 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                         if (seg >= 0 && (int64_t)seg < A.n_seg) {
                             const unsigned long long slot =
                                 (unsigned long long)seg * (unsigned long long)A.cells + (unsigned long long)cell;
-                            atomicAdd(A.maps + slot, 1u);
-                            atomicMin(A.keys + slot, key);
-                            if (MODE == 2) {
+                            if (MODE >= SEGMENTS_CROWDED) {
+                                add_crowded(A.maps, A.keys, slot, key);
+                            } else {
+                                atomicAdd(A.maps + slot, 1u);
+                                atomicMin(A.keys + slot, key);
+                            }
+                            if (MODE == MOMENTS || MODE == MOMENTS_CROWDED) {
                                 // fixed-point time moments (exact integer sums, order-independent)
                                 const float tc = fminf(fmaxf(t, 0.0f), CL_MOMENT_T_MAX_NS);
                                 atomicAdd(A.tsum + slot, __float2ull_rn(tc * CL_MOMENT_T_SCALE));
@@ -362,7 +392,7 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                         pool_lo = (int64_t)base;
                         pool_hi = pool_lo + A.warp_chunk;
                         if (pool_hi > A.n) pool_hi = A.n;
-                        if (MODE != 0) {
+                        if (MODE != POINT) {
                             int64_t s0 = 0;
                             if (lane == 0) s0 = find_source(A.src_off, A.n_src, pool_src, pool_lo);
                             pool_src = __shfl_sync(FULL, s0, 0);
@@ -378,7 +408,7 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                     }
                 }
                 if (my_k >= 0) {
-                    if (MODE == 0) {
+                    if (MODE == POINT) {
                         const int32_t j = A.npos == 1 ? 0 : position_of(my_k, A.npos);
                         x = __ldg(A.px + j); y = __ldg(A.py + j); z = __ldg(A.pz + j);
                         t = A.pt ? __ldg(A.pt + j) : 0.0f;
@@ -615,7 +645,7 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
         if (v) atomicAdd(tid < 9 ? A.counters + tid : A.steps, v);
     }
 
-    if (MODE == 0) {
+    if (MODE == POINT) {
         // last CTA decodes the first-time keys into Float32 in place
         __threadfence();
         __syncthreads();
@@ -880,15 +910,22 @@ static void set_kernel_attrs_spec(int smem_optin)
 // the evaluation in the loop: scan 100.4 -> 98.0 ms, 3,001 events 20.6 -> 20.2 ms
 // without it.
 template <int MODE, bool REC>
-constexpr bool spec_without_tables = MODE == 0 && !REC;
+constexpr bool spec_without_tables = MODE == POINT && !REC;
+template <int MODE>
+constexpr bool needs_tables = MODE >= SEGMENTS_CROWDED;
 
+// Of the instances that a handle with (or without) the tables launches: the
+// first call for an instance loads it.
 template <int MODE, bool REC, bool TILE>
-static void set_kernel_attrs(int smem_optin)
+static void set_kernel_attrs(int smem_optin, bool tables)
 {
-    set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ANY, true>(smem_optin);
-    set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ESR, true>(smem_optin);
-    set_kernel_attrs_spec<MODE, REC, TILE, SPEC_TEFLON, true>(smem_optin);
-    set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ANY, false>(smem_optin);
+    if (tables) {
+        set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ANY, true>(smem_optin);
+        set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ESR, true>(smem_optin);
+        set_kernel_attrs_spec<MODE, REC, TILE, SPEC_TEFLON, true>(smem_optin);
+        return;
+    }
+    if constexpr (!needs_tables<MODE>) set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ANY, false>(smem_optin);
     if constexpr (spec_without_tables<MODE, REC>) {
         set_kernel_attrs_spec<MODE, REC, TILE, SPEC_ESR, false>(smem_optin);
         set_kernel_attrs_spec<MODE, REC, TILE, SPEC_TEFLON, false>(smem_optin);
@@ -935,14 +972,6 @@ int cl_create(cl_handle** out, int device)
         delete h;
         return CL_ERR_CUDA;
     }
-    set_kernel_attrs<0, false, true>(h->max_smem_optin);
-    set_kernel_attrs<0, true, true>(h->max_smem_optin);
-    set_kernel_attrs<0, false, false>(h->max_smem_optin);
-    set_kernel_attrs<0, true, false>(h->max_smem_optin);
-    set_kernel_attrs<1, false, false>(h->max_smem_optin);
-    set_kernel_attrs<1, true, false>(h->max_smem_optin);
-    set_kernel_attrs<2, false, false>(h->max_smem_optin);
-    cudaGetLastError();
     if (ensure(h, h->scratch, 64) != CL_OK) {
         snprintf(g_create_err, sizeof g_create_err, "cl_create: %s", h->err);
         cudaStreamDestroy(h->stream);
@@ -964,6 +993,18 @@ int cl_create(cl_handle** out, int device)
         cudaGetLastError();
         h->logtab = DevBuf();
     }
+    const bool tables = h->logtab.p != nullptr;
+    set_kernel_attrs<POINT, false, true>(h->max_smem_optin, tables);
+    set_kernel_attrs<POINT, true, true>(h->max_smem_optin, tables);
+    set_kernel_attrs<POINT, false, false>(h->max_smem_optin, tables);
+    set_kernel_attrs<POINT, true, false>(h->max_smem_optin, tables);
+    set_kernel_attrs<SEGMENTS, false, false>(h->max_smem_optin, tables);
+    set_kernel_attrs<SEGMENTS, true, false>(h->max_smem_optin, tables);
+    set_kernel_attrs<MOMENTS, false, false>(h->max_smem_optin, tables);
+    set_kernel_attrs<SEGMENTS_CROWDED, false, false>(h->max_smem_optin, tables);
+    set_kernel_attrs<SEGMENTS_CROWDED, true, false>(h->max_smem_optin, tables);
+    set_kernel_attrs<MOMENTS_CROWDED, false, false>(h->max_smem_optin, tables);
+    cudaGetLastError();
     *out = h;
     return CL_OK;
 }
@@ -1143,12 +1184,14 @@ template <int MODE, bool REC, bool TILE>
 static int launch_transport(cl_handle* h, const KArgs& a, size_t smem, cudaStream_t st)
 {
     const int spec = spec_of(a.P);
-    if (!a.logtab) {
-        if constexpr (spec_without_tables<MODE, REC>) {
-            if (spec == SPEC_ESR) return launch_transport_spec<MODE, REC, TILE, SPEC_ESR, false>(h, a, smem, st);
-            if (spec == SPEC_TEFLON) return launch_transport_spec<MODE, REC, TILE, SPEC_TEFLON, false>(h, a, smem, st);
+    if constexpr (!needs_tables<MODE>) {
+        if (!a.logtab) {
+            if constexpr (spec_without_tables<MODE, REC>) {
+                if (spec == SPEC_ESR) return launch_transport_spec<MODE, REC, TILE, SPEC_ESR, false>(h, a, smem, st);
+                if (spec == SPEC_TEFLON) return launch_transport_spec<MODE, REC, TILE, SPEC_TEFLON, false>(h, a, smem, st);
+            }
+            return launch_transport_spec<MODE, REC, TILE, SPEC_ANY, false>(h, a, smem, st);
         }
-        return launch_transport_spec<MODE, REC, TILE, SPEC_ANY, false>(h, a, smem, st);
     }
     switch (spec) {
     case SPEC_ESR: return launch_transport_spec<MODE, REC, TILE, SPEC_ESR, true>(h, a, smem, st);
@@ -1198,10 +1241,10 @@ static int enqueue_point(cl_handle* h, const Physics& P, const float* px, const 
     const bool tile = base_bytes + tile_bytes <= (size_t)std::min(h->max_smem_optin, 160 * 1024) &&
                       4 * per_cta <= (size_t)h->max_smem_per_sm;
     const size_t smem = base_bytes + (tile ? tile_bytes : 0);
-    if (tile) return want_rec ? launch_transport<0, true, true>(h, a, smem, st)
-                              : launch_transport<0, false, true>(h, a, smem, st);
-    return want_rec ? launch_transport<0, true, false>(h, a, smem, st)
-                    : launch_transport<0, false, false>(h, a, smem, st);
+    if (tile) return want_rec ? launch_transport<POINT, true, true>(h, a, smem, st)
+                              : launch_transport<POINT, false, true>(h, a, smem, st);
+    return want_rec ? launch_transport<POINT, true, false>(h, a, smem, st)
+                    : launch_transport<POINT, false, false>(h, a, smem, st);
 }
 
 static int enqueue_segments(cl_handle* h, const Physics& P, const float* sx, const float* sy,
@@ -1238,9 +1281,13 @@ static int enqueue_segments(cl_handle* h, const Physics& P, const float* sx, con
         a.budget_ns = h->budget_ns;
         const size_t smem = LOGTAB_BYTES + RING_BYTES;
         a.tsum = tsum; a.tsum2 = tsum2;
-        const int rc = moments ? launch_transport<2, false, false>(h, a, smem, st)
-                     : want_rec ? launch_transport<1, true, false>(h, a, smem, st)
-                                : launch_transport<1, false, false>(h, a, smem, st);
+        const bool crowded = n / total >= (cells < 64 ? CROWDED_FEW : CROWDED) && total <= (int64_t)UINT32_MAX && a.logtab;
+        const int rc = crowded ? (moments ? launch_transport<MOMENTS_CROWDED, false, false>(h, a, smem, st)
+                                  : want_rec ? launch_transport<SEGMENTS_CROWDED, true, false>(h, a, smem, st)
+                                             : launch_transport<SEGMENTS_CROWDED, false, false>(h, a, smem, st))
+                     : moments ? launch_transport<MOMENTS, false, false>(h, a, smem, st)
+                     : want_rec ? launch_transport<SEGMENTS, true, false>(h, a, smem, st)
+                                : launch_transport<SEGMENTS, false, false>(h, a, smem, st);
         if (rc != CL_OK) return rc;
     }
     if (sample) {
@@ -1725,8 +1772,8 @@ int noalloc_setup(int dev, NoallocDevice** out)
                      dev, cudaGetErrorString(e));
             return CL_ERR_CUDA;
         }
-        set_kernel_attrs<0, false, true>(d.max_smem_optin);
-        set_kernel_attrs<0, false, false>(d.max_smem_optin);
+        set_kernel_attrs<POINT, false, true>(d.max_smem_optin, false);
+        set_kernel_attrs<POINT, false, false>(d.max_smem_optin, false);
         cudaGetLastError();
         d.base = (unsigned char*)p;
         d.ready = true;
