@@ -565,7 +565,9 @@ __global__ void __launch_bounds__(32 * DIRECT_WARPS) surrogate_direct(const Dire
                 const float inv = 1.0f / rho;
                 int ilo = (int)floorf((x0 - rho) / A.pitch), ihi = (int)floorf((x0 + rho) / A.pitch);
                 int jlo = (int)floorf((y0 - rho) / A.pitch), jhi = (int)floorf((y0 + rho) / A.pitch);
+                // the last column and row reach the face edge, beyond nx and ny pitches too
                 ilo = max(ilo, 0); jlo = max(jlo, 0); ihi = min(ihi, nx - 1); jhi = min(jhi, ny - 1);
+                ilo = min(ilo, ihi); jlo = min(jlo, jhi);
                 for (int e = ilo; e <= ihi + 1; ++e) {
                     const float xe = e == nx ? A.L0 : fminf(e * A.pitch, A.L0);
                     aa[e * DIRECT_STRIDE + q] = acosf(fminf(fmaxf((xe - x0) * inv, -1.0f), 1.0f));
@@ -576,9 +578,7 @@ __global__ void __launch_bounds__(32 * DIRECT_WARPS) surrogate_direct(const Dire
                 }
                 wt[q] = (double)(float)(s_w[q] * exp(-(double)A.mu * (double)h / s_c[q])) * DIRECT_FIX;
                 rad[q] = rho;
-                // an empty range (a pixel grid smaller than the face) holds no pixel
-                box[q] = ihi < ilo || jhi < jlo ? 0x00ff00ffu
-                                                : (uint32_t)ilo | (uint32_t)ihi << 8 | (uint32_t)jlo << 16 | (uint32_t)jhi << 24;
+                box[q] = (uint32_t)ilo | (uint32_t)ihi << 8 | (uint32_t)jlo << 16 | (uint32_t)jhi << 24;
             }
         }
         __syncwarp();
