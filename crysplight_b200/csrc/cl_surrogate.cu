@@ -467,7 +467,8 @@ __global__ void __launch_bounds__(32 * COMBINE_WARPS) surrogate_combine(const Co
 //
 // One warp per site.  First every lane takes two nodes and writes the angles at
 // which its circle crosses the edges of the pixel columns and rows it reaches
-// (arc cosines and sines: once per edge, not four per pixel).  A pixel is
+// (arc cosines and sines: once per edge, not four per pixel; for the columns or
+// rows of grids wider than DIRECT_TABULATED, at each use).  A pixel is
 // crossed by a contiguous range of nodes, because the radii increase; the
 // (pixel, node) items of all 64 pixels are then shared out evenly over the
 // lanes (near the face one pixel has all 64 nodes).  The bound is instruction
@@ -499,16 +500,29 @@ constexpr int DIRECT_NODES = 64;
 constexpr double DIRECT_FIX = 1099511627776.0;   // 2^40
 constexpr int DIRECT_WARPS = 8;
 constexpr int DIRECT_STRIDE = DIRECT_NODES + 1;  // floats per edge (odd: lanes at different edges on different banks)
+// Columns (rows) up to which their edges' angles are tabulated.  A wider grid's
+// table takes the shared memory that other warps need (64 x 1: 8 warps per SM):
+// 42,000 sites on 64 x 1 pixels 370 us tabulated and 102 with the columns' angles
+// taken per item (268 by the kernel with a thread per node), on 32 x 2 246 and 175
+// (322).  A narrower one's is read often enough: 16 x 4 209 and 256.
+constexpr int DIRECT_TABULATED = 16;
+constexpr int DIRECT_MAX_EDGES = 22;             // 16 x 4 pixels: 17 + 5
 constexpr float TWO_PI_ARC = 6.283185307179586f;
 
-// Shared floats of a warp: the angles of the nx + 1 column and ny + 1 row edges,
-// per node its weight (double), radius and bounding box, per pixel its sum (64
-// bits), first item and first node.
-__host__ __device__ constexpr int direct_warp_floats(int nx, int ny)
+// Shared floats of a warp: the angles of the tabulated edges, per node its weight
+// (double), radius, inverse radius and bounding box, per pixel its sum (64 bits),
+// first item and first node.
+__host__ __device__ constexpr int direct_warp_floats(int edges)
 {
-    return (nx + ny + 2) * DIRECT_STRIDE + (nx + ny) % 2 + 4 * DIRECT_NODES + 4 * CELLS;
+    return edges * DIRECT_STRIDE + edges % 2 + 5 * DIRECT_NODES + 4 * CELLS;
 }
 
+// The angles at which a circle crosses a column's or a row's edge, for the
+// quotient of the edge's distance from the site and the radius.
+__device__ __forceinline__ float column_angle(float v) { return acosf(fminf(fmaxf(v, -1.0f), 1.0f)); }
+__device__ __forceinline__ float row_angle(float v) { return asinf(fminf(fmaxf(v, -1.0f), 1.0f)); }
+
+template <bool XTAB, bool YTAB>
 __global__ void __launch_bounds__(32 * DIRECT_WARPS) surrogate_direct(const DirectArgs A)
 {
     extern __shared__ __align__(16) float s_direct[];
@@ -516,12 +530,14 @@ __global__ void __launch_bounds__(32 * DIRECT_WARPS) surrogate_direct(const Dire
     __shared__ float s_tan[DIRECT_NODES];
     const int lane = threadIdx.x & 31;
     const int nx = A.nx, ny = A.ny;
-    float* const aa = s_direct + (threadIdx.x >> 5) * direct_warp_floats(nx, ny);   // [edge][node]
-    float* const ba = aa + (nx + 1) * DIRECT_STRIDE;
-    double* const wt = reinterpret_cast<double*>(ba + (ny + 1) * DIRECT_STRIDE + (nx + ny) % 2);   // weight x 2^40
+    const int x_edges = XTAB ? nx + 1 : 0, edges = x_edges + (YTAB ? ny + 1 : 0);
+    float* const aa = s_direct + (threadIdx.x >> 5) * direct_warp_floats(edges);   // [edge][node]
+    float* const ba = aa + x_edges * DIRECT_STRIDE;
+    double* const wt = reinterpret_cast<double*>(aa + edges * DIRECT_STRIDE + edges % 2);   // weight x 2^40
     unsigned long long* const acc = reinterpret_cast<unsigned long long*>(wt + DIRECT_NODES);
     float* const rad = reinterpret_cast<float*>(acc + CELLS);
-    uint32_t* const box = reinterpret_cast<uint32_t*>(rad + DIRECT_NODES);
+    float* const inverse = rad + DIRECT_NODES;
+    uint32_t* const box = reinterpret_cast<uint32_t*>(inverse + DIRECT_NODES);
     int* const item0 = reinterpret_cast<int*>(box + DIRECT_NODES);
     int* const node0 = item0 + CELLS;
     if (threadIdx.x < DIRECT_NODES) {
@@ -550,6 +566,8 @@ __global__ void __launch_bounds__(32 * DIRECT_WARPS) surrogate_direct(const Dire
         s_tan[q] = (float)(sn / c);
     }
     __syncthreads();
+    auto x_edge = [&](int e) { return e == nx ? A.L0 : fminf(e * A.pitch, A.L0); };
+    auto y_edge = [&](int e) { return e == ny ? A.L1 : fminf(e * A.pitch, A.L1); };
     const int64_t stride = (int64_t)gridDim.x * DIRECT_WARPS;
     for (int64_t i = (int64_t)blockIdx.x * DIRECT_WARPS + (threadIdx.x >> 5); i < A.n; i += stride) {
         const int64_t at = A.site ? A.site[i] : i;
@@ -568,16 +586,15 @@ __global__ void __launch_bounds__(32 * DIRECT_WARPS) surrogate_direct(const Dire
                 // the last column and row reach the face edge, beyond nx and ny pitches too
                 ilo = max(ilo, 0); jlo = max(jlo, 0); ihi = min(ihi, nx - 1); jhi = min(jhi, ny - 1);
                 ilo = min(ilo, ihi); jlo = min(jlo, jhi);
-                for (int e = ilo; e <= ihi + 1; ++e) {
-                    const float xe = e == nx ? A.L0 : fminf(e * A.pitch, A.L0);
-                    aa[e * DIRECT_STRIDE + q] = acosf(fminf(fmaxf((xe - x0) * inv, -1.0f), 1.0f));
-                }
-                for (int e = jlo; e <= jhi + 1; ++e) {
-                    const float ye = e == ny ? A.L1 : fminf(e * A.pitch, A.L1);
-                    ba[e * DIRECT_STRIDE + q] = asinf(fminf(fmaxf((ye - y0) * inv, -1.0f), 1.0f));
-                }
+                if (XTAB)
+                    for (int e = ilo; e <= ihi + 1; ++e)
+                        aa[e * DIRECT_STRIDE + q] = column_angle((x_edge(e) - x0) * inv);
+                if (YTAB)
+                    for (int e = jlo; e <= jhi + 1; ++e)
+                        ba[e * DIRECT_STRIDE + q] = row_angle((y_edge(e) - y0) * inv);
                 wt[q] = (double)(float)(s_w[q] * exp(-(double)A.mu * (double)h / s_c[q])) * DIRECT_FIX;
                 rad[q] = rho;
+                inverse[q] = inv;
                 box[q] = (uint32_t)ilo | (uint32_t)ihi << 8 | (uint32_t)jlo << 16 | (uint32_t)jhi << 24;
             }
         }
@@ -635,15 +652,19 @@ __global__ void __launch_bounds__(32 * DIRECT_WARPS) surrogate_direct(const Dire
                 int q = node0[c] + item - item0[c];
                 const float* pa = aa + ii * DIRECT_STRIDE;
                 const float* pb = ba + jj * DIRECT_STRIDE;
+                const float xa = x_edge(ii) - x0, xb = x_edge(ii + 1) - x0;      // where not tabulated
+                const float ya = y_edge(jj) - y0, yb = y_edge(jj + 1) - y0;
                 unsigned long long sum = 0ull;
                 for (const int stop = min(next, last); item < stop; ++item, ++q) {
                     // azimuths with cos(phi) between the columns' edges: x1 in
                     // [0, pi], x2 in [pi, 2 pi]
-                    const float a0 = pa[q], a1 = pa[q + DIRECT_STRIDE];             // a1 <= a0
+                    const float a0 = XTAB ? pa[q] : column_angle(xa * inverse[q]);
+                    const float a1 = XTAB ? pa[q + DIRECT_STRIDE] : column_angle(xb * inverse[q]);      // a1 <= a0
                     const float x1l = a1, x1h = a0, x2l = TWO_PI_ARC - a0, x2h = TWO_PI_ARC - a1;
                     // and sin(phi) between the rows': y1 where it is positive on
                     // [0, pi/2], y2 around pi, y3 where it is negative on [3 pi/2, 2 pi]
-                    const float b0 = pb[q], b1 = pb[q + DIRECT_STRIDE];             // in [-pi/2, pi/2]
+                    const float b0 = YTAB ? pb[q] : row_angle(ya * inverse[q]);         // in [-pi/2, pi/2]
+                    const float b1 = YTAB ? pb[q + DIRECT_STRIDE] : row_angle(yb * inverse[q]);
                     const float pi = 0.5f * TWO_PI_ARC;
                     const float y1l = fmaxf(b0, 0.0f), y1h = fmaxf(b1, 0.0f);
                     const float y2l = pi - b1, y2h = pi - b0;
@@ -832,16 +853,20 @@ int cl_surrogate_direct_sites(const float* d_xyz, const int32_t* d_site, int64_t
     a.pitch = ro->grid.pitch_mm; a.nx = ro->grid.nx; a.ny = ro->grid.ny; a.out = d_out;
     const int64_t want = (n_sites + cl::sur::DIRECT_WARPS - 1) / cl::sur::DIRECT_WARPS;
     const unsigned grid = (unsigned)(want < 148 * 8 ? want : 148 * 8);
-    const size_t smem = cl::sur::DIRECT_WARPS * cl::sur::direct_warp_floats(a.nx, a.ny) * sizeof(float);
-    // 8 x 8 pixels: 53 KB; the opt-in is per device, and for the widest grid
-    // (64 x 1: 152 KB) whatever this one is, since threads may launch different grids
-    constexpr size_t most = cl::sur::DIRECT_WARPS * cl::sur::direct_warp_floats(cl::sur::CELLS, 1) * sizeof(float);
+    const bool xt = a.nx <= cl::sur::DIRECT_TABULATED, yt = a.ny <= cl::sur::DIRECT_TABULATED;
+    const int edges = (xt ? a.nx + 1 : 0) + (yt ? a.ny + 1 : 0);
+    const size_t smem = cl::sur::DIRECT_WARPS * cl::sur::direct_warp_floats(edges) * sizeof(float);
+    auto kern = !xt ? cl::sur::surrogate_direct<false, true> : !yt ? cl::sur::surrogate_direct<true, false>
+                                                                   : cl::sur::surrogate_direct<true, true>;
+    // the opt-in is per device and for the most edges tabulated, whatever this
+    // grid's are, since threads may launch different grids
+    constexpr size_t most = cl::sur::DIRECT_WARPS * cl::sur::direct_warp_floats(cl::sur::DIRECT_MAX_EDGES) * sizeof(float);
     if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(cl::sur::surrogate_direct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) {
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) != cudaSuccess) {
         cudaGetLastError();
         return CL_ERR_CUDA;
     }
-    cl::sur::surrogate_direct<<<grid, 32 * cl::sur::DIRECT_WARPS, smem, (cudaStream_t)stream>>>(a);
+    kern<<<grid, 32 * cl::sur::DIRECT_WARPS, smem, (cudaStream_t)stream>>>(a);
     return cudaGetLastError() == cudaSuccess ? CL_OK : CL_ERR_CUDA;
 }
 
