@@ -336,7 +336,9 @@ __global__ void __launch_bounds__(32 * SAMPLE_WARPS, SAMPLE_CTAS) surrogate_samp
 // them in further batches), no CTA barrier.  The bound is the members' outputs
 // from HBM or L2 (768 bytes per site and member); with 64 threads per site,
 // three loads in flight per thread and two barriers per site the kernel waited
-// on memory: 42,001 sites x 5 members 119 -> 76 us.
+// on memory: 42,000 sites x 5 members 111 -> 68 us, 1 member 45 -> 43, 7 members
+// 142 -> 88 (a batch that always loads five rows, the last one again and again:
+// 70, 47 and 98).
 struct CombineArgs {
     const float* raw;        // [K][n][3 * cells] standardised member outputs
     int32_t K;
@@ -384,7 +386,8 @@ __global__ void __launch_bounds__(32 * COMBINE_WARPS) surrogate_combine(const Co
             float v[COMBINE_BATCH][3][2];
 #pragma unroll
             for (int k = 0; k < COMBINE_BATCH; ++k) {
-                const float* row = A.raw + ((int64_t)min(k0 + k, A.K - 1) * A.n + i) * (3 * CELLS) + lane;
+                if (k0 + k >= A.K) break;
+                const float* row = A.raw + ((int64_t)(k0 + k) * A.n + i) * (3 * CELLS) + lane;
 #pragma unroll
                 for (int o = 0; o < 3; ++o)
 #pragma unroll
