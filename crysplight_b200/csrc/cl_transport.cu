@@ -30,6 +30,7 @@
 
 #include "../../include/crysplight_cuda.h"
 #include "cl_device.cuh"
+#include "cl_launch.h"
 #include "cl_surrogate.cuh"
 
 #define CL_VERSION_STRING "crysplight_b200 0.1.0 (sm_100a)"
@@ -42,7 +43,6 @@ constexpr int N_COUNTERS = 10;        // cl_counters, then the photon-steps
 // Photons per slot from which a launch's detections are added slot by slot
 // (segment mode; see add_crowded): few cells, and the 64 of a full map.
 constexpr int64_t CROWDED_FEW = 1024, CROWDED = 4096;
-constexpr int SPREAD_WARPS = 8;        // warps per SM of a launch of few photons
 constexpr size_t CTA_EXTRA_SMEM = 1024 + 8 * N_COUNTERS * 8 + 16;   // reserved and static shared memory of a CTA
 constexpr int SCTAB_BYTES = CLM_SC_N * 16;
 constexpr int LOGTAB_BYTES = ((CLM_LOG_NTAB * 16 + 127) / 128) * 128 + SCTAB_BYTES;  // both tables
@@ -174,15 +174,6 @@ enum : int32_t {
     S_LAMB = 5,   // Lambertian re-injection (src/optics.jl:118-138)
 };
 
-#ifndef CL_DEFAULT_WARP_CHUNK
-#define CL_DEFAULT_WARP_CHUNK 0
-#endif
-#ifndef CL_CHUNKS_PER_WARP
-#define CL_CHUNKS_PER_WARP 16
-#endif
-#ifndef CL_MAX_WARP_CHUNK
-#define CL_MAX_WARP_CHUNK 256
-#endif
 #ifndef CL_MIN_CTAS_PER_SM
 #define CL_MIN_CTAS_PER_SM 4
 #endif
@@ -841,9 +832,7 @@ struct cl_handle {
     char err[512] = {0};
     DevBuf src, out, rec, scratch, dbg;
     char* stage = nullptr;         // STAGE_IN + STAGE_OUT bytes, or null: host arrays are copied one by one
-    int ctas_per_sm = 0;
-    int threads = 256;
-    int warp_chunk = CL_DEFAULT_WARP_CHUNK;   // 0: automatic per launch
+    LaunchSetting launch;          // cl_set_launch
     int64_t last_steps = 0;
     int max_smem_optin = 0;
     int max_smem_per_sm = 0;
@@ -1033,9 +1022,9 @@ int cl_set_launch(cl_handle* h, int ctas_per_sm, int threads_per_cta, int warp_c
         return set_err(h, CL_ERR_ARG, "threads_per_cta must be a multiple of 32 in [32, 256]");
     if (warp_chunk != 0 && (warp_chunk < 32 || warp_chunk > (1 << 20)))
         return set_err(h, CL_ERR_ARG, "warp_chunk must be in [32, 2^20]");
-    h->ctas_per_sm = ctas_per_sm;
-    h->threads = threads_per_cta ? threads_per_cta : 256;
-    h->warp_chunk = warp_chunk ? warp_chunk : CL_DEFAULT_WARP_CHUNK;
+    h->launch.ctas_per_sm = ctas_per_sm;
+    h->launch.threads = threads_per_cta;
+    h->launch.warp_chunk = warp_chunk;
     return CL_OK;
 }
 
@@ -1145,37 +1134,13 @@ static int launch_transport_spec(cl_handle* h, const KArgs& a, size_t smem, cuda
 {
     auto kern = transport_kernel<MODE, REC, TILE, SPEC, TAB>;
     int per_sm = 0;
-    CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, h->threads, smem), "occupancy");
+    CK(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, h->launch.threads ? h->launch.threads : AUTO_THREADS,
+                                                        smem), "occupancy");
     if (per_sm < 1) return set_err(h, CL_ERR_ARG, "transport kernel does not fit on an SM (shared tile too large)");
-    if (h->ctas_per_sm > 0 && h->ctas_per_sm < per_sm) per_sm = h->ctas_per_sm;
-    int64_t grid = (int64_t)h->num_sms * per_sm;
+    const LaunchShape shape = launch_shape(a.n, h->num_sms, per_sm, h->launch);
     KArgs b = a;
-    int threads = h->threads;
-    if (b.warp_chunk <= 0) {
-        // automatic: the largest chunk (fewest queue atomics) that still gives
-        // every resident warp about CL_CHUNKS_PER_WARP chunks, so the end of
-        // the queue stays balanced; between 32 and CL_MAX_WARP_CHUNK photons
-        const int64_t warps = grid * (threads / 32);
-        int64_t c = a.n / (warps * CL_CHUNKS_PER_WARP);
-        c = c < 32 ? 32 : (c > CL_MAX_WARP_CHUNK ? CL_MAX_WARP_CHUNK : c);
-        b.warp_chunk = (int32_t)(c & ~(int64_t)31);
-        // fewer photons than two warps per scheduler hold: spread them over that
-        // many warps, some lanes each.  The time is the longest photon's chain
-        // of steps, and a warp with few lanes runs fewer of a step's branches:
-        // CsI(Tl) 2,000 photons 271 -> 245 us, 20,000 294 -> 285 us, BGO 500
-        // photons 946 -> 849 us; with 4 warps per SM 8,000 photons take 262 us
-        // instead of 257, with 16 269 us
-        const int64_t spread = (int64_t)h->num_sms * SPREAD_WARPS;
-        if (a.n < spread * 32 && threads >= 128) {
-            b.warp_chunk = (int32_t)((a.n + spread - 1) / spread);
-            threads = 128;
-        }
-    }
-    // no more CTAs than warps' worth of first chunks
-    const int64_t warps_needed = (b.n + b.warp_chunk - 1) / b.warp_chunk;
-    const int64_t ctas_needed = (warps_needed + (threads / 32) - 1) / (threads / 32);
-    if (grid > ctas_needed) grid = ctas_needed > 0 ? ctas_needed : 1;
-    kern<<<(unsigned)grid, threads, smem, st>>>(b);
+    b.warp_chunk = shape.warp_chunk;
+    kern<<<(unsigned)shape.grid, shape.threads, smem, st>>>(b);
     CK(h, cudaGetLastError(), "transport kernel launch");
     return CL_OK;
 }
@@ -1221,7 +1186,7 @@ static int enqueue_point(cl_handle* h, const Physics& P, const float* px, const 
     }
     KArgs a;
     memset(&a, 0, sizeof a);
-    a.P = P; a.pid0 = pid0; a.n = n; a.npos = npos; a.warp_chunk = h->warp_chunk;
+    a.P = P; a.pid0 = pid0; a.n = n; a.npos = npos;
     a.cells = cells; a.bins_total = bins_total;
     a.px = px; a.py = py; a.pz = pz; a.pt = pt;
     a.counts = counts; a.keys = keys; a.counters = counters;
@@ -1269,7 +1234,7 @@ static int enqueue_segments(cl_handle* h, const Physics& P, const float* sx, con
     if (n > 0) {
         KArgs a;
         memset(&a, 0, sizeof a);
-        a.P = P; a.pid0 = pid0; a.n = n; a.npos = 1; a.warp_chunk = h->warp_chunk;
+        a.P = P; a.pid0 = pid0; a.n = n; a.npos = 1;
         a.cells = cells; a.bins_total = P.nbins + 1;
         a.px = sx; a.py = sy; a.pz = sz; a.pt = sT;
         a.src_off = off; a.src_seg = segid; a.n_src = n_src; a.n_seg = n_seg;
