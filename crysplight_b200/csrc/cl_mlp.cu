@@ -1665,7 +1665,7 @@ int net_forward_enqueue(cl_mlp* const* nets, int members, const float* d_x, floa
                 const int units = Kl * a.tiles;
                 const int cap = m->max_ctas > 0 && m->max_ctas < m->num_sms ? m->max_ctas : m->num_sms;
                 net_forward<false><<<(unsigned)(units < cap ? units : cap), GEMM_THREADS, NET_SMEM, st>>>(a, NetTrain());
-                if (cudaGetLastError() != cudaSuccess) return CL_ERR_CUDA;
+                if (cudaPeekAtLastError() != cudaSuccess) return CL_ERR_CUDA;     // the caller reports it
             }
         }
     }
@@ -1815,13 +1815,18 @@ int cl_mlp_train(cl_mlp* m, int steps, int batch, float lr, uint32_t seed, uint3
 // network's own); cl_mlp_sync waits and reports.
 int cl_mlp_forward_ensemble(cl_mlp* const* nets, int members, const float* d_x, float* d_out, int64_t n, void* stream)
 {
-    if (!nets || members < 1 || n < 0) return CL_ERR_ARG;
-    for (int k = 0; k < members; ++k)
-        if (!nets[k] || nets[k]->device != nets[0]->device) return CL_ERR_ARG;
+    if (!nets || members < 1 || !nets[0]) return CL_ERR_ARG;
+    cl_mlp* const m = nets[0];
+    m->err[0] = 0;
+    if (n < 0) return mlp_fail(m, CL_ERR_ARG, "the number of rows must be >= 0");
+    for (int k = 1; k < members; ++k)
+        if (!nets[k] || nets[k]->device != m->device)
+            return mlp_fail(m, CL_ERR_ARG, "network %d of the ensemble is missing or on another device", k);
     if (n == 0) return CL_OK;
-    if (!d_x || !d_out) return CL_ERR_ARG;
-    cudaSetDevice(nets[0]->device);
-    return net_forward_enqueue(nets, members, d_x, d_out, n, stream ? (cudaStream_t)stream : nets[0]->stream);
+    if (!d_x || !d_out) return mlp_fail(m, CL_ERR_ARG, "null input or output");
+    cudaSetDevice(m->device);
+    const int rc = net_forward_enqueue(nets, members, d_x, d_out, n, stream ? (cudaStream_t)stream : m->stream);
+    return rc ? mlp_fail(m, rc, "forward launch failed: %s", cudaGetErrorString(cudaGetLastError())) : CL_OK;
 }
 
 // Wait for the work on `stream` (NULL: the network's own) and report a
@@ -1843,7 +1848,7 @@ int cl_mlp_forward(cl_mlp* m, const float* d_x, float* d_out, int64_t n)
     if (!m || !d_x || !d_out || n < 0) return CL_ERR_ARG;
     cudaSetDevice(m->device);
     const int rc = n > 0 ? net_forward_enqueue(&m, 1, d_x, d_out, n, m->stream) : CL_OK;
-    if (rc) return mlp_fail(m, rc, "forward launch failed");
+    if (rc) return mlp_fail(m, rc, "forward launch failed: %s", cudaGetErrorString(cudaGetLastError()));
     return cl_mlp_sync(m, nullptr);
 }
 
