@@ -1546,6 +1546,12 @@ void refresh_bf16(cl_mlp* m, cudaStream_t st)
     to_bf16<<<(D_OUT * D_H + 255) / 256, 256, 0, st>>>(m->p + OFF_W4, D_OUT * D_H, m->w4t);
 }
 
+// Rows of targets are read 16 bytes at a time at least.
+int check_targets(cl_mlp* m, const float* target)
+{
+    return (uintptr_t)target & 15 ? mlp_fail(m, CL_ERR_ARG, "the training targets must start on a 16-byte boundary") : CL_OK;
+}
+
 int grid_for(const cl_mlp* m, int B)
 {
     const int tiles = B / TILE_M;
@@ -1581,7 +1587,6 @@ bool net_weight_maps(const cl_mlp* m, CUtensorMap* w)
 // then the weight gradients.  rows.n_all == 0: the batch is the set's first B rows.
 int forward_backward(cl_mlp* m, int B, const float* x, const float* target, const BatchRows& rows, cudaStream_t st)
 {
-    if ((uintptr_t)target & 15) return CL_ERR_ARG;       // rows of targets are read 16 bytes at a time at least
     if (int rc = net_attributes(m->device)) return rc;
     const int grid = grid_for(m, B);
     NetArgs f;
@@ -1788,6 +1793,7 @@ int cl_mlp_train(cl_mlp* m, int steps, int batch, float lr, uint32_t seed, uint3
 {
     if (!m || steps < 0 || batch < TILE_M || batch % TILE_M || batch > m->max_batch || !m->data_x)
         return CL_ERR_ARG;
+    if (const int rc = steps > 0 ? check_targets(m, m->data_t) : CL_OK) return rc;
     cudaSetDevice(m->device);
     cudaStream_t st = m->stream;
     cudaMemsetAsync(m->loss, 0, sizeof(float), st);
@@ -1857,6 +1863,7 @@ int cl_mlp_forward(cl_mlp* m, const float* d_x, float* d_out, int64_t n)
 int cl_mlp_gradient(cl_mlp* m, const float* d_x, const float* d_t, int B, float* host_grad, float* loss_out)
 {
     if (!m || !d_x || !d_t || !host_grad || B < TILE_M || B % TILE_M || B > m->max_batch) return CL_ERR_ARG;
+    if (const int rc = check_targets(m, d_t)) return rc;
     cudaSetDevice(m->device);
     cudaStream_t st = m->stream;
     cudaMemsetAsync(m->loss, 0, sizeof(float), st);

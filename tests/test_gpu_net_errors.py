@@ -36,3 +36,18 @@ def test_a_refused_ensemble_says_why(nets):
     # a call that succeeds leaves no message of an earlier one
     assert call(both, x.data_ptr(), 128) == (_lib.CL_OK, "")
     assert lib.cl_mlp_sync(nets[0].h, C.c_void_p(1)) == _lib.CL_OK
+
+
+def test_misaligned_targets_are_refused_by_name(nets):
+    import torch
+    x = torch.rand((256, 3), device="cuda")
+    flat = torch.randn(256 * 192 + 1, device="cuda")
+    torch.cuda.synchronize()
+    t = flat[1:].view(256, 192)                  # 4 bytes past a boundary
+    nets[0].set_data(x, t)
+    with pytest.raises(_lib.CudaTransportError, match="16-byte boundary"):
+        nets[0].train(1, batch=128)
+    with pytest.raises(_lib.CudaTransportError, match="16-byte boundary"):
+        nets[0].gradient(x[:128], t[:128])
+    nets[0].set_data(x, flat[:-1].view(256, 192))
+    assert nets[0].train(1, batch=128) > 0.0
