@@ -1677,14 +1677,14 @@ int net_forward_enqueue(cl_mlp* const* nets, int members, const float* d_x, floa
     return CL_OK;
 }
 
-void adam(cl_mlp* m, float lr, cudaStream_t st)
+cudaError_t adam(cl_mlp* m, float lr, cudaStream_t st)
 {
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     m->adam_t += 1;
     const float bc1 = 1.0f - powf(b1, (float)m->adam_t), bc2 = 1.0f - powf(b2, (float)m->adam_t);
     const AdamCopies c = {m->w2t, m->w3t, m->w4t};
-    launch_pdl(adam_all, dim3((unsigned)((N_PARAMS / 4 + 127) / 128)), dim3(128), 0, st, m->p, m->g, m->m, m->v, lr, b1, b2,
-               eps, bc1, bc2, c);
+    return launch_pdl(adam_all, dim3((unsigned)((N_PARAMS / 4 + 127) / 128)), dim3(128), 0, st, m->p, m->g, m->m, m->v, lr, b1,
+                      b2, eps, bc1, bc2, c);
 }
 
 }  // namespace
@@ -1801,10 +1801,10 @@ int cl_mlp_train(cl_mlp* m, int steps, int batch, float lr, uint32_t seed, uint3
     // step is an unbroken chain of kernels
     cudaMemsetAsync(m->g, 0, N_PARAMS * sizeof(float), st);
     for (int s = 0; s < steps; ++s) {
-        const int rc = forward_backward(m, batch, m->data_x, m->data_t,
-                                        BatchRows{(uint32_t)m->n_data, step0 + (uint32_t)s, seed}, st);
+        int rc = forward_backward(m, batch, m->data_x, m->data_t,
+                                  BatchRows{(uint32_t)m->n_data, step0 + (uint32_t)s, seed}, st);
+        if (!rc && adam(m, lr, st) != cudaSuccess) rc = CL_ERR_CUDA;
         if (rc) return mlp_fail(m, rc, "kernel launch failed: %s", cudaGetErrorString(cudaGetLastError()));
-        adam(m, lr, st);
     }
     float loss = 0.0f;
     unsigned int e = 0;
