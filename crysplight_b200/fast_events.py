@@ -192,8 +192,14 @@ class SurrogateEvents:
         parts = [(self.main, None)]
         if self.experts and n:
             parts = [(ens, site) for ens, site in self._split(xyz, stream) if site.numel()]
-        kept = [self._light(ens, xyz, site, out, ro, pde, spread_max, wall_min_mm, stream) for ens, site in parts]
-        # the temporaries go back to torch's allocator, and a network's error is reported here
+        kept = []                                # of the temporaries, until the stream is through with them
+        try:
+            for ens, site in parts:
+                kept.append(self._light(ens, xyz, site, out, ro, pde, spread_max, wall_min_mm, stream))
+        except BaseException:
+            torch.cuda.synchronize(self.dev)
+            raise
+        # a network's error is reported here
         for ens, _ in parts:
             sync_networks(ens.nets, stream_arg(stream or 0))
         del kept
