@@ -157,13 +157,25 @@ class SurrogateEvents:
             raise _lib.CudaTransportError(rc, "cl_surrogate_combine failed")
         return xin, raw, direct
 
+    EXPERTS_PER_SPLIT = 256          # of one cl_surrogate_split
+
     def _split(self, xyz, stream):
-        """[(ensemble, its sites as int32 CUDA tensor)], main first, with the sites
-        of each: the last expert whose slab holds the site, else the main one."""
+        """[(ensemble, its sites as int32 CUDA tensor)] in the order of evaluation:
+        the sites of the last expert whose slab holds them, else of the main
+        ensemble.  With more experts than one split takes, the later ones take
+        their sites over from the earlier ones' outputs."""
+        parts = self._split_group([self.main] + self.experts[:self.EXPERTS_PER_SPLIT], xyz, stream)
+        for e0 in range(self.EXPERTS_PER_SPLIT, len(self.experts), self.EXPERTS_PER_SPLIT):
+            later = self.experts[e0:e0 + self.EXPERTS_PER_SPLIT]
+            parts += self._split_group([None] + later, xyz, stream)[1:]
+        return parts
+
+    def _split_group(self, group, xyz, stream):
+        """The same for group[0] and the experts group[1:]."""
         import torch
-        n, E = int(xyz.shape[0]), len(self.experts)
+        n, E = int(xyz.shape[0]), len(group) - 1
         lo, hi, count = (C.c_float * E)(), (C.c_float * E)(), (C.c_int32 * (E + 1))()
-        for e, ens in enumerate(self.experts):
+        for e, ens in enumerate(group[1:]):
             z0, z1 = ens.sur.depth_range()
             lo[e], hi[e] = z0 + self.expert_margin_mm, z1
         lists = torch.empty((E + 1, n), dtype=torch.int32, device=self.dev)
@@ -172,7 +184,7 @@ class SurrogateEvents:
                                          C.c_void_p(d_count.data_ptr()), count, stream_arg(stream or 0))
         if rc != 0:
             raise _lib.CudaTransportError(rc, "cl_surrogate_split failed")
-        return [(ens, lists[g, :count[g]]) for g, ens in enumerate([self.main] + self.experts)]
+        return [(ens, lists[g, :count[g]]) for g, ens in enumerate(group)]
 
     def site_light(self, xyz, *, ro: Readout, pde: float, spread_max: float = SPREAD_MAX,
                    wall_min_mm: float = WALL_MIN_MM, stream=None) -> SiteLight:
