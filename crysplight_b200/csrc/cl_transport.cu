@@ -508,8 +508,10 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
             rng.pos += og;
             // no bulk interaction if each uniform is clearly below its
             // survival probability exp(-d / length): the path length
-            // -length log u is then clearly above d
-            if (!((!abs_finite || u_abs < survive_below(d, P.abs_rate)) &&
+            // -length log u is then clearly above d.  (Another try moves by 0, below
+            // which no path length is but one of a negative length, SPEC_ANY's.)
+            if ((SPEC != SPEC_ANY || st == S_MOVE) &&
+                !((!abs_finite || u_abs < survive_below(d, P.abs_rate)) &&
                   (!ray_finite || u_ray < survive_below(d, P.ray_rate)))) {
                 const float d_abs = abs_finite ? (-P.abs_len) * uniform_log<TAB>(A.logtab, u_abs, s_tab) : inf;
                 const float d_ray = ray_finite ? (-P.ray_len) * uniform_log<TAB>(A.logtab, u_ray, s_tab) : inf;
@@ -1124,7 +1126,8 @@ static Scratch scratch_of(cl_handle* h)
 // The compiled configuration a launch can use (SPEC_ANY where none matches).
 static int spec_of(const Physics& P)
 {
-    if (!P.air_gap || !(P.sigma_alpha > 0.0f) || P.disc || P.two_sided || !P.abs_finite || !P.ray_finite)
+    if (!P.air_gap || !(P.sigma_alpha > 0.0f) || P.disc || P.two_sided || !P.abs_finite || !P.ray_finite ||
+        P.abs_len < 0.0f || P.ray_len < 0.0f)
         return SPEC_ANY;
     return P.wrap_specular ? SPEC_ESR : SPEC_TEFLON;
 }
