@@ -291,13 +291,11 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                 const bool det = status == ST_DETECTED;
                 int32_t idx = 0;
                 if (det) {
-                    int32_t ii = 1 + (int32_t)(x / P.pitch);
-                    int32_t jj = 1 + (int32_t)(y / P.pitch);
-                    ii = ii < P.nx ? ii : P.nx;
-                    jj = jj < P.ny ? jj : P.ny;
-                    const int32_t lin = (jj - 1) * P.nx + ii;
+                    // the conversion saturates: inside the grid whatever the pitch
+                    const int32_t ii = min((int32_t)(x / P.pitch), P.nx - 1);
+                    const int32_t jj = min((int32_t)(y / P.pitch), P.ny - 1);
+                    const int32_t cell = jj * P.nx + ii, lin = cell + 1;
                     idx = two_sided && face == FACE_FRONT ? -lin : lin;
-                    const int32_t cell = lin - 1;
                     const uint32_t key = float_key(t);
                     // one reduction per photon: a warp seldom detects two photons in
                     // the same slot, and finding out costs more than it saves
