@@ -737,6 +737,7 @@ __global__ void debug_math_kernel(int fn, const float* in, float* out, int64_t n
 //   9  (x, y, z, ux, uy, uz, Lx, Ly, Lz) -> quick distance and face (0: undecided), exact distance and face
 //  10  (n1, n2, cosi, u) -> quick and exact "reflects" (total reflection included)
 //  11  (u, d, length) -> 1 if the quick test rules a bulk event out, exact -length log u
+//  12  as 9 -> quick face (0: undecided) and incidence cosine, the exact face's |direction|
 __global__ void debug_step_kernel(int fn, const float* in, float* out, int64_t n)
 {
     __shared__ __align__(16) unsigned char tabs[LOGTAB_BYTES];
@@ -758,6 +759,18 @@ __global__ void debug_step_kernel(int fn, const float* in, float* out, int64_t n
             out[4 * i + 1] = ok ? (float)f : 0.0f;
             out[4 * i + 3] = (float)wall_hit(P, q[0], q[1], q[2], q[3], q[4], q[5], d);
             out[4 * i + 2] = d;
+        }
+        if (fn == 12) {
+            const float* q = in + 9 * i;
+            Physics P;
+            P.L0 = q[6]; P.L1 = q[7]; P.L2 = q[8];
+            float d, cosw;
+            int32_t f;
+            const bool ok = wall_hit_fast(P, q[0], q[1], q[2], q[3], q[4], q[5], d, f, cosw);
+            const int32_t g = wall_hit(P, q[0], q[1], q[2], q[3], q[4], q[5], d);
+            out[3 * i] = ok ? (float)f : 0.0f;
+            out[3 * i + 1] = cosw;
+            out[3 * i + 2] = fabsf(g <= 2 ? q[3] : (g <= 4 ? q[4] : q[5]));
         }
         if (fn == 10) {
             const float* q = in + 4 * i;
@@ -1650,7 +1663,7 @@ int cl_debug_eval(cl_handle* h, int fn, const void* in, void* out, int64_t n, ui
     if (!h) return CL_ERR_STATE;
     h->err[0] = 0;
     if (n < 0 || !out || (fn != 4 && fn != 6 && !in)) return set_err(h, CL_ERR_ARG, "bad debug arguments");
-    if (fn < 0 || fn > 11) return set_err(h, CL_ERR_ARG, "unknown debug function");
+    if (fn < 0 || fn > 12) return set_err(h, CL_ERR_ARG, "unknown debug function");
     if (fn == 4 && n_per < 1) return set_err(h, CL_ERR_ARG, "n_per must be >= 1");
     CK(h, cudaSetDevice(h->device), "cudaSetDevice");
     cudaStream_t st = h->stream;
@@ -1666,7 +1679,7 @@ int cl_debug_eval(cl_handle* h, int fn, const void* in, void* out, int64_t n, ui
     if (fn <= 2) { in_b = 4 * (size_t)n; out_b = 4 * (size_t)n; }
     else if (fn == 3 || fn == 5) { in_b = 16 * (size_t)n; out_b = 16 * (size_t)n; }
     else if (fn >= 7) {
-        constexpr size_t ni[5] = {1, 1, 9, 4, 3}, no[5] = {1, 1, 4, 2, 2};
+        constexpr size_t ni[6] = {1, 1, 9, 4, 3, 9}, no[6] = {1, 1, 4, 2, 2, 3};
         in_b = 4 * ni[fn - 7] * (size_t)n;
         out_b = 4 * no[fn - 7] * (size_t)n;
     }

@@ -253,9 +253,9 @@ class Engine:
 
     def eval_step(self, fn: int, x: np.ndarray) -> np.ndarray:
         """The transport loop's quick decisions beside the exact expressions
-        (cl_debug_eval functions 7..11): x (n, inputs) -> (n, outputs), float32."""
+        (cl_debug_eval functions 7..12): x (n, inputs) -> (n, outputs), float32."""
         x = np.ascontiguousarray(x, np.float32)
-        out = np.empty((x.shape[0], {7: 1, 8: 1, 9: 4, 10: 2, 11: 2}[fn]), np.float32)
+        out = np.empty((x.shape[0], {7: 1, 8: 1, 9: 4, 10: 2, 11: 2, 12: 3}[fn]), np.float32)
         self._check(self.lib.cl_debug_eval(self.handle, fn, _ptr(x), _ptr(out), x.shape[0], 0, 0))
         return out
 

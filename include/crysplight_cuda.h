@@ -448,12 +448,13 @@ int cl_set_time_budget(cl_handle* h, double seconds);
  * 5 = cuRAND's Philox4x32-10 on the same inputs as 3 (cross-check),
  * 6 = the first n entries of the handle's table of logs of the uniforms,
  * out_f32[k] = log((k+1) * 2^-24) as the transport uses it (in unused).
- * 7 to 11: the transport's quick decisions beside the exact expressions, n
+ * 7 to 12: the transport's quick decisions beside the exact expressions, n
  * items of float inputs -> outputs: 7 = x -> approximate square root, 8 = x ->
  * approximate reciprocal, 9 = (x, y, z, ux, uy, uz, Lx, Ly, Lz) -> quick wall
  * distance and face (0: undecided), exact distance and face, 10 = (n_crystal,
  * n_outside, cosine, u) -> quick and exact "reflects", 11 = (u, distance,
- * length) -> 1 where the quick test rules a bulk event out, exact -length log u.
+ * length) -> 1 where the quick test rules a bulk event out, exact -length log u,
+ * 12 = as 9 -> quick face and incidence cosine, exact |direction| on that axis.
  * Host buffers, synchronous.
  */
 int cl_debug_eval(cl_handle* h, int fn, const void* in, void* out, int64_t n,
