@@ -184,7 +184,6 @@ static __device__ __noinline__ float2 slow_sincosf(float x)
 // Natural log.  Table-driven (Tang 1990): x = 2^e * m, m in [sqrt(1/2), sqrt(2)),
 // m = F_j (1 + r) with F_j = 1 + j/64, ln x = e ln2 + ln F_j + log1p(r),
 // |r| < 1/90, log1p by its Taylor series to r^8.
-template <int STRIDE = 1>
 __device__ __forceinline__ float cl_logf(float x, const double2* __restrict__ tab)
 {
     const uint32_t b = __float_as_uint(x);
@@ -198,7 +197,7 @@ __device__ __forceinline__ float cl_logf(float x, const double2* __restrict__ ta
     const double m = (double)__uint_as_float(mb);
     const int j = __double2int_rn((m - 1.0) * 64.0);
     const double F = 1.0 + (double)j * 0.015625;
-    const double2 t = tab[(j - CLM_LOG_JMIN) * STRIDE];
+    const double2 t = tab[j - CLM_LOG_JMIN];
     const double r = (m - F) * t.x;            // m - F is exact
     double p = CLM_L8;
     p = fma(p, r, CLM_L7);
@@ -214,7 +213,6 @@ __device__ __forceinline__ float cl_logf(float x, const double2* __restrict__ ta
 
 // log of a uniform ((x>>8)+1)*2^-24: always a positive normal float, so the
 // domain check of cl_logf is not needed.
-template <int STRIDE = 1>
 __device__ __forceinline__ float cl_logf_u(float x, const double2* __restrict__ tab)
 {
     const uint32_t b = __float_as_uint(x);
@@ -226,7 +224,7 @@ __device__ __forceinline__ float cl_logf_u(float x, const double2* __restrict__ 
     const double m = (double)__uint_as_float(mb);
     const int j = __double2int_rn((m - 1.0) * 64.0);
     const double F = 1.0 + (double)j * 0.015625;
-    const double2 t = tab[(j - CLM_LOG_JMIN) * STRIDE];
+    const double2 t = tab[j - CLM_LOG_JMIN];
     const double r = (m - F) * t.x;
     double p = CLM_L8;
     p = fma(p, r, CLM_L7);

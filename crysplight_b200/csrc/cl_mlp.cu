@@ -94,14 +94,13 @@ __host__ __device__ constexpr size_t gemm_smem_bytes(int N)
 struct GemmArgs {
     int M, N, K;                    // M % 128 == 0, N % 32 == 0 && 32 <= N <= 256, K % 64 == 0
     int k_split;                    // K elements per split (gridDim.y splits)
-    int n_full;                     // row tiles taken whole; the rest go as two N halves each
     float* out_f; int64_t ldf;
     unsigned int* err;
 };
 
-// SiLU and its derivative with the fast exponential and division (results
-// are rounded to BF16 afterwards; for z -> -inf, __fdividef by an infinite
-// denominator returns 0)
+// SiLU and its derivative with the approximate exponential and reciprocal, results
+// below the normal range flushed to zero (they are rounded to BF16 afterwards; for
+// a large negative z the exponential is infinite and its reciprocal 0)
 __device__ __forceinline__ float silu(float z)
 {
     float e, r;
@@ -180,29 +179,15 @@ __device__ __forceinline__ void warp_col_sums(const uint8_t* tt, int lane, float
     }
 }
 
-// A unit of work: row tile `tile`, accumulator columns [n0, n0 + nw).  The
-// first n_full units are whole tiles; the remaining tiles are split into two
-// units of N/2 columns each, so that the last round over the CTAs is half as
-// long (512 tiles on 148 SMs: 3.5 tiles' time instead of 4).
-struct Unit {
-    int tile, n0, nw;
-};
-__device__ __forceinline__ Unit unit_of(int u, int n_full, int N)
-{
-    if (u < n_full) return Unit{u, 0, N};
-    const int v = u - n_full;
-    return Unit{n_full + (v >> 1), (v & 1) * (N >> 1), N >> 1};
-}
-
-// Epilogue of one 128 x N tile: the warp owns rows row0 + lane (row0 = tile
-// row + 32 (w % 4)) and the 32-column chunks c0 = 32 (half + 4 k).
+// Epilogue of one 128 x N tile of the diagnostic GEMM: the warp owns rows row0 +
+// lane (row0 = tile row + 32 (w % 4)) and the 32-column chunks c0 = 32 (half + 4 k).
 template <int EPI>
-__device__ __forceinline__ void epilogue(const GemmArgs& G, uint32_t tbase, int row0, int lane, int half, Unit un)
+__device__ __forceinline__ void epilogue(const GemmArgs& G, uint32_t tbase, int row0, int lane, int half)
 {
     const int row = row0 + lane;
-    for (int c0 = un.n0 + 32 * half; c0 < un.n0 + un.nw; c0 += 32 * (EPI_WARPS / 4)) {
+    for (int c0 = 32 * half; c0 < G.N; c0 += 32 * (EPI_WARPS / 4)) {
         float v[32];
-        umma::tmem_ld32(tbase + (uint32_t)(c0 - un.n0), v);
+        umma::tmem_ld32(tbase + (uint32_t)c0, v);
         float* o = G.out_f + (EPI == EPI_PARTIAL ? (int64_t)blockIdx.y * G.M * G.ldf : 0) + (int64_t)row * G.ldf + c0;
 #pragma unroll
         for (int g = 0; g < 8; ++g)
@@ -212,17 +197,18 @@ __device__ __forceinline__ void epilogue(const GemmArgs& G, uint32_t tbase, int 
 
 // C = A B^T on the tensor cores.  A [M][K] and B [N][K] BF16, K-major, read
 // through TMA tensor maps (128-byte swizzle, boxes of 64 x 128 rows and 64 x N
-// rows).  Persistent over 128-row tiles (blockIdx.x, stride gridDim.x), K split
-// over blockIdx.y.  Roles: warp 4 lane 0 streams A/B stages (full/empty
-// mbarriers), warp 5 lane 0 issues tcgen05.mma into one of two TMEM
-// accumulators and commits, warps 0-3 drain the other accumulator through the
-// epilogue.  Every wait is bounded; a wait that runs out sets bit 0 of *err,
+// rows).  A diagnostic (cl_umma_gemm_bf16) for the descriptors, barriers and
+// accumulators that the network kernels below use in the same way.  Persistent
+// over 128-row tiles (blockIdx.x, stride gridDim.x), K split over blockIdx.y.
+// Roles: lane 0 of warp 16 streams A/B stages (full/empty mbarriers), lane 0 of
+// warp 17 issues tcgen05.mma into one of two TMEM accumulators and commits, warps
+// 0-15 drain the other accumulator through the epilogue.  Every wait is bounded; a wait that runs out sets bit 0 of *err,
 // tells the other roles to stop, and the CTA still waits (bounded) for its
 // copies and MMAs in flight before freeing TMEM.
 template <int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ GemmArgs G)
+                const __grid_constant__ GemmArgs G)
 {
     constexpr int STAGES = GEMM_STAGES;
     extern __shared__ uint8_t smem_raw[];
@@ -240,8 +226,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const int k_end = min(G.K, k_begin + G.k_split);
     const int n_chunks = (k_end - k_begin) / TILE_K;
     const int n_tiles = G.M / TILE_M;
-    const int n_units = G.n_full + 2 * (n_tiles - G.n_full);
-    if (n_chunks <= 0 || (int)blockIdx.x >= n_units) return;   // uniform over the CTA
+    if (n_chunks <= 0 || (int)blockIdx.x >= n_tiles) return;   // uniform over the CTA
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     volatile int* abort_v = &abort_flag;
@@ -254,7 +239,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     if (warp == PRODUCER_WARP && lane == 0) {
         umma::prefetch_tmap(&tmA);
         umma::prefetch_tmap(&tmB);
-        if (G.n_full < n_tiles) umma::prefetch_tmap(&tmBh);
     }
     umma::fence_before_sync();
     __syncthreads();
@@ -265,9 +249,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         if (lane == 0) {
             uint32_t it = 0;
             bool ok = true;
-            for (int ui = blockIdx.x; ui < n_units && ok; ui += gridDim.x) {
-                const Unit un = unit_of(ui, G.n_full, N);
-                const int tile = un.tile;
+            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
                 for (int c = 0; c < n_chunks; ++c, ++it) {
                     const uint32_t s = it % STAGES, r = it / STAGES;
                     if (r > 0 && !umma::mbar_wait_or_abort(&empty[s], (r - 1) & 1u, WAIT_BUDGET, abort_v)) {
@@ -275,11 +257,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
                         break;
                     }
                     uint8_t* st = smem + s * stage_bytes;
-                    umma::mbar_arrive_expect_tx(&full[s], a_bytes + (uint32_t)un.nw * 128u);
+                    umma::mbar_arrive_expect_tx(&full[s], stage_bytes);
                     const int k0 = k_begin + c * TILE_K;
                     umma::tma_load_2d(st, &tmA, k0, tile * TILE_M, &full[s]);
-                    if (un.nw == N) umma::tma_load_2d(st + a_bytes, &tmB, k0, 0, &full[s]);
-                    else umma::tma_load_2d(st + a_bytes, &tmBh, k0, un.n0, &full[s]);
+                    umma::tma_load_2d(st + a_bytes, &tmB, k0, 0, &full[s]);
                 }
             }
             if (!ok) { atomicOr(G.err, 1u); *abort_v = 1; }
@@ -289,12 +270,10 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
     } else if (warp == MMA_WARP) {
         if (lane == 0) {
-            const uint32_t idesc_full = umma::make_idesc_bf16(TILE_M, N);
-            const uint32_t idesc_half = umma::make_idesc_bf16(TILE_M, N / 2);
+            const uint32_t idesc = umma::make_idesc_bf16(TILE_M, N);
             uint32_t it = 0, j = 0;
             bool ok = true;
-            for (int ui = blockIdx.x; ui < n_units && ok; ui += gridDim.x, ++j) {
-                const uint32_t idesc = ui < G.n_full ? idesc_full : idesc_half;
+            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++j) {
                 const uint32_t a = j & 1u, u = j >> 1;
                 if (u > 0 && !umma::mbar_wait_or_abort(&acc_empty[a], (u - 1) & 1u, WAIT_BUDGET, abort_v)) {
                     ok = false;
@@ -324,9 +303,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         }
     } else {
         uint32_t j = 0;
-        for (int ui = blockIdx.x; ui < n_units; ui += gridDim.x, ++j) {
+        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++j) {
             const uint32_t a = j & 1u, u = j >> 1;
-            const Unit un = unit_of(ui, G.n_full, N);
             if (!umma::mbar_wait_or_abort(&acc_full[a], u & 1u, WAIT_BUDGET, abort_v)) {
                 if (lane == 0) atomicOr(G.err, 1u);
                 *abort_v = 1;
@@ -334,7 +312,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
             }
             umma::fence_after_sync();
             const int quad = warp & 3;
-            epilogue<EPI>(G, tmem + a * 256u + ((uint32_t)(32 * quad) << 16), un.tile * TILE_M + 32 * quad, lane, warp >> 2, un);
+            epilogue<EPI>(G, tmem + a * 256u + ((uint32_t)(32 * quad) << 16), tile * TILE_M + 32 * quad, lane, warp >> 2);
             umma::fence_before_sync();
             __syncwarp();
             if (lane == 0) umma::mbar_arrive(&acc_empty[a]);
@@ -417,19 +395,9 @@ int launch_gemm(const GemmArgs& g, const bf16* A, int64_t lda, const bf16* B, in
     }
     const int tiles = g.M / TILE_M;
     dim3 grid((unsigned)(grid_x < tiles ? grid_x : tiles), (unsigned)splits);
-    // a last round that would occupy at most half of the CTAs runs as N halves
-    // (two units per tile) on all of them
-    GemmArgs ga = g;
-    ga.n_full = tiles;
-    CUtensorMap tbh = tb;
-    const int r = tiles % (int)grid.x;
-    if (EPI != EPI_PARTIAL && splits == 1 && g.N % 64 == 0 && r > 0 && 2 * r <= (int)grid.x) {
-        if (!make_map(&tbh, B, g.N, g.K, ldb, g.N / 2)) return CL_ERR_ARG;
-        ga.n_full = tiles - r;
-    }
     // at least 116 KB so that one CTA holds an SM: each allocates all 512 TMEM columns
     const size_t smem = gemm_smem_bytes(g.N) > 116 * 1024 ? gemm_smem_bytes(g.N) : 116 * 1024;
-    gemm_kernel<EPI><<<grid, GEMM_THREADS, smem, st>>>(ta, tb, tbh, ga);
+    gemm_kernel<EPI><<<grid, GEMM_THREADS, smem, st>>>(ta, tb, g);
     return cudaGetLastError() == cudaSuccess ? CL_OK : CL_ERR_CUDA;
 }
 

@@ -3,20 +3,16 @@
 // accumulator in tensor memory (TMEM), TMEM allocation and loads, and bounded
 // mbarrier waits.
 //
-// Operand layouts in shared memory.  (1) The canonical K-major layout without
-// swizzle (make_desc), staged by ordinary stores.  (2) The K-major layout with
-// the 128-byte swizzle (make_desc_sw128), written by TMA: a tile of R rows x
-// 64 BF16 is R rows of 128 bytes, 8-row groups 1024 bytes apart (SBO), the
-// 16-byte pieces of row r XOR-permuted by (r & 7); a K step of 16 elements
-// advances the start address by 32 bytes inside the swizzle atom.
+// Operand layouts in shared memory, both with the 128-byte swizzle and written by
+// TMA.  K-major (make_desc_sw128): a tile of R rows x 64 BF16 is R rows of 128
+// bytes, 8-row groups 1024 bytes apart (SBO), the 16-byte pieces of row r
+// XOR-permuted by (r & 7); a K step of 16 elements advances the start address by
+// 32 bytes inside the swizzle atom.  MN-major (make_desc_sw128_mn): the same with
+// rows along K.
 //
-// Layout (1) in detail: the canonical K-major layout without
-// swizzle.  A core matrix is 8 rows x 16 bytes (8 BF16 along K), its rows
-// contiguous (128 bytes).  For a tile of R rows x KC K-elements, core matrix
-// (row group g = r/8, K chunk c = k/8) sits at byte ((c * R/8) + g) * 128: row
-// groups are 128 bytes apart (stride byte offset, SBO) and K chunks R*16
-// bytes apart (leading byte offset, LBO).  One MMA instruction consumes K = 16,
-// i.e. two K chunks starting at chunk 2s.
+// A descriptor holds the start address >> 4 in bits 0-13, the leading byte offset
+// (LBO) >> 4 in bits 16-29, the stride byte offset (SBO) >> 4 in bits 32-45, its
+// version 1 in bits 46-47 and the swizzle in bits 61-63.
 #pragma once
 
 #include <cstdint>
@@ -29,26 +25,6 @@ namespace umma {
 __device__ __forceinline__ uint32_t smem_u32(const void* p)
 {
     return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-// Byte offset of element (r, k) of an R-row K-major tile in the canonical layout.
-__device__ __forceinline__ uint32_t tile_offset(uint32_t r, uint32_t k, uint32_t R)
-{
-    return (((k >> 3) * (R >> 3) + (r >> 3)) * 8u + (r & 7u)) * 16u + (k & 7u) * 2u;
-}
-
-// 64-bit shared-memory matrix descriptor (tcgen05 "matrix descriptor"):
-// start address >> 4 in bits 0-13, LBO >> 4 in bits 16-29, SBO >> 4 in bits
-// 32-45, descriptor version 1 in bits 46-47, base offset 0, no swizzle (0 in
-// bits 61-63).
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes)
-{
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
-    d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFFu) << 16;
-    d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFFu) << 32;
-    d |= (uint64_t)1 << 46;
-    return d;
 }
 
 // Descriptor of a 128-byte-swizzled K-major tile (1024-byte aligned base):
