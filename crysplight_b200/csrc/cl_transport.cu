@@ -1213,12 +1213,17 @@ static int enqueue_point(cl_handle* h, const Physics& P, const float* px, const 
     const size_t base_bytes = LOGTAB_BYTES + RING_BYTES;
     // the shared-memory histogram tile only where it still leaves room for 4
     // CTAs per SM: with fewer resident warps the loop issues less often, which
-    // costs more than the tile saves in global atomics (10^6-photon point
-    // source, 8x8x81 bins: 879 M photons/s on global atomics at 4 CTAs/SM,
-    // 843 M with the tile at 3)
+    // costs more than the tile saves in global atomics (CsI(Tl), 4M photons, 8x8x81
+    // bins: 1,867 us on global atomics at 4 CTAs/SM, 2,038 with the tile at 3; 10^6
+    // photons 728 and 751).  Room for 3 where the photons in flight (more than
+    // 2^17) share few slots, because the bins that the decay time reaches are few:
+    // there the reductions on one address are the bound (the same with no decay
+    // time: 2,040 and 1,950; a clear crystal, 41 to 81 bins: 1,865 and 860 to 910).
+    const double slots = (double)cells * (1.0 + (P.tau > 0.0f ? std::floor((double)P.tau / (double)P.bin_ns) : 0.0));
+    const int ctas = slots <= 64.0 && n >= (1 << 17) ? 3 : 4;
     const size_t per_cta = base_bytes + tile_bytes + CTA_EXTRA_SMEM;
     const bool tile = base_bytes + tile_bytes <= (size_t)std::min(h->max_smem_optin, 160 * 1024) &&
-                      4 * per_cta <= (size_t)h->max_smem_per_sm;
+                      ctas * per_cta <= (size_t)h->max_smem_per_sm;
     const size_t smem = base_bytes + (tile ? tile_bytes : 0);
     if (tile) return want_rec ? launch_transport<POINT, true, true>(h, a, smem, st)
                               : launch_transport<POINT, false, true>(h, a, smem, st);
