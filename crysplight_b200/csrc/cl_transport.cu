@@ -1218,9 +1218,11 @@ static int enqueue_point(cl_handle* h, const Physics& P, const float* px, const 
     // photons 728 and 751).  Room for 3 where the photons in flight (more than
     // 2^17) share few slots, because the bins that the decay time reaches are few:
     // there the reductions on one address are the bound (the same with no decay
-    // time: 2,040 and 1,950; a clear crystal, 41 to 81 bins: 1,865 and 860 to 910).
+    // time: 2,040 and 1,950; a clear crystal, 41 to 81 bins: 1,865 and 860 to 910;
+    // 75 to 108 slots, most photons gone after a step: 590 and 340, after twelve:
+    // 1,860 and 1,930).
     const double slots = (double)cells * (1.0 + (P.tau > 0.0f ? std::floor((double)P.tau / (double)P.bin_ns) : 0.0));
-    const int ctas = slots <= 64.0 && n >= (1 << 17) ? 3 : 4;
+    const int ctas = slots <= 128.0 && n >= (1 << 17) ? 3 : 4;
     const size_t per_cta = base_bytes + tile_bytes + CTA_EXTRA_SMEM;
     const bool tile = base_bytes + tile_bytes <= (size_t)std::min(h->max_smem_optin, 160 * 1024) &&
                       ctas * per_cta <= (size_t)h->max_smem_per_sm;

@@ -21,8 +21,8 @@ CLEAR = OpticalParams(1.79, 1.79, INF, INF, 0.99, False, True, deg2rad_f32(1.3),
     (BOX_CSI, OP_CSI_TEFLON, CENTRE_CSI, GRID, 100.0, 50, 0.0, 1 << 17),
     (BOX_CSI, OP_CSI_TEFLON, CENTRE_CSI, GRID, 0.5, 114, 0.0, 140_000),      # the largest histogram with the tile,
     (BOX_CSI, OP_CSI_TEFLON, CENTRE_CSI, GRID, 0.5, 130, 0.0, 140_000),      # one without
-    (BOX_CSI, CLEAR, CENTRE_CSI, SipmGrid(16.0, 3, 3), 10.0, 300, 69.0, 140_000),
-    (BOX_CSI, CLEAR, CENTRE_CSI, SipmGrid(16.0, 3, 3), 10.0, 300, 70.0, 140_000),
+    (BOX_CSI, CLEAR, CENTRE_CSI, SipmGrid(12.0, 4, 4), 10.0, 300, 79.0, 140_000),     # 128 slots,
+    (BOX_CSI, CLEAR, CENTRE_CSI, SipmGrid(12.0, 4, 4), 10.0, 300, 80.0, 140_000),     # 144
     (BOX_BGO, OP_BGO_ESR, CENTRE_BGO, GRID, 1.0, 80, 0.0, 135_000)])
 def test_counts_equal_the_oracle(engine, oracle, box, op, pos, grid, bin_ns, nbins, tau, n):
     tb = TimeBinning(bin_ns, nbins)
