@@ -300,7 +300,8 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
                     // one reduction per photon: a warp seldom detects two photons in
                     // the same slot, and finding out costs more than it saves
                     if (MODE == POINT) {
-                        atomicAdd(tile_counts + cell + A.cells * time_bin0(t, P), 1u);
+                        const int bin = time_bin0(t, P);       // a histogram in global memory may pass 2^31 counts
+                        atomicAdd(tile_counts + cell + (TILE ? A.cells * bin : (int64_t)A.cells * bin), 1u);
                         // the cells' keys are hot; most photons are later than the
                         // key already there (which only ever falls)
                         if (key < (TILE ? tile_keys[cell] : __ldcg(tile_keys + cell))) atomicMin(tile_keys + cell, key);
