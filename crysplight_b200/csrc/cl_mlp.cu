@@ -19,7 +19,10 @@
 // blocks that the same warps read back (Z).  One kernel per layer and direction
 // (twelve launches a step) took 113 us a step at a batch of 4,096 rows and
 // 244 us at 65,536; these take 64 us and 232 us.  A batch of 65,536 rows is 512
-// units of 128 rows over 148 SMs: 4 rounds where 3.46 would do.
+// units of 128 rows over 148 SMs: 4 rounds where 3.46 would do.  A unit that an SM
+// has left over takes 17 us forward and 20 us backward by itself, so a batch just
+// above 2 or 4 whole rounds gains nothing: 297 units 182.8 us against 181.4, 593
+// units 283 against 272 (296: 144 and 168; 592: 246 and 263).
 #include <algorithm>
 #include <cmath>
 #include <cstdarg>
@@ -488,15 +491,15 @@ __global__ void to_bf16(const float* w, int n, bf16* o)
 // epilogue write the next layer's A operand (128 x 256 BF16, 128-byte swizzle)
 // into the unit's 64 KB of shared memory, the accumulators stay in tensor
 // memory, and only the inputs, the weights (streamed from L2 by TMA in stages
-// of 64 K-elements) and the outputs (staged as 32 x 32 FP32 tiles, TMA stores)
-// move.  Layer by layer the same network went through global memory: H written
+// of 64 K-elements) and the outputs (stored from registers, 64 bytes of a row per
+// lane) move.  Layer by layer the same network went through global memory: H written
 // and read three times, the outputs copied once more.
 //
 // Two units are in flight per CTA: while the sixteen epilogue warps work on one
 // unit's layer, the tensor cores run the other unit's.  The bound is the
 // special-function unit: SiLU takes an exponential and a reciprocal, 2 x 256 x 3
 // per row at 16 per clock and SM, 96 cycles per row (the tensor cores need 43).
-// 200,001 rows through MLP.forward: 355 -> 162 us.
+// 200,001 rows through MLP.forward: 355 -> 154 us.
 constexpr int NET_MAX = 8;               // members one launch evaluates
 constexpr int NET_STAGES = 2;            // weight stages of 256 x 64 BF16
 constexpr uint32_t NET_A_BYTES = TILE_M * 512;           // a unit's A operand: 4 K-blocks of 16 KB
@@ -1019,8 +1022,9 @@ __global__ void __launch_bounds__(TRAIN ? NET_TRAIN_THREADS : GEMM_THREADS, 1)
 // gradients.  The bound is that last epilogue, 256 columns x 4 sums over the
 // unit's rows through transposed staging tiles (11,000 to 17,000 cycles of the
 // 40,000 a unit takes), beside the SiLU derivatives (an exponential and a
-// reciprocal each) and 126 MB read and 67 MB written.  65,536 rows: 82 us,
-// 87 us as three kernels.
+// reciprocal each) and, for 65,536 rows, 92 MB to read (Z3, Z2, dO) and 67 MB to
+// write (dZ3, dZ2); at DRAM 126 and 34 MB.  65,536 rows: 82 us, 87 us as three
+// kernels.
 struct NetBack {
     CUtensorMap dO;                      // boxes of 64 x 128
     CUtensorMap w[3];                    // W4^T, W3^T, W2^T as stored [out][in] (MN-major operands): boxes of 64 x 64

@@ -478,7 +478,7 @@ __global__ void __launch_bounds__(32 * COMBINE_WARPS) surrogate_combine(const Co
 // issue.  A lane per pixel kept 11 of 32 lanes active and took 344 us; a thread per
 // node that evaluated four angles and one shared-memory atomic per pixel of its
 // circle's bounding box, four sites per CTA behind common barriers, issued on
-// 49% of its cycles: 42,001 sites 430 -> 204 us.
+// 49% of its cycles: 42,000 sites 404 -> 179 us.
 // The rest of the light response (reflections, scattering) varies slowly
 // over the SiPM plane; a surrogate trained on it learns what the first-pass
 // term's sharp pixel edges would otherwise ask of it.
@@ -713,7 +713,7 @@ __global__ void surrogate_inputs(const float* __restrict__ xyz, const int32_t* _
 // listed in list + group * n, count[group] of them, 32 consecutive sites at a
 // time.  Evaluating the main ensemble everywhere and then the experts over it
 // cost the experts' sites twice: every network, the first-pass term and five
-// copies (42,001 sites, a third of them an expert's: 781 us, 556 so).
+// copies (42,001 sites, a third of them an expert's: 781 us, 549 so).
 constexpr int SITE_GROUPS = 257;
 struct SplitArgs {
     const float* xyz;

@@ -7,7 +7,7 @@
 //     chunk) and each lane refills itself with the next photon the moment
 //     its photon terminates, so long-bouncing photons never idle a warp;
 //   * parameters travel as a __grid_constant__ kernel argument (constant
-//     bank), the log table sits in shared memory;
+//     bank), the sincos and log reduction tables sit in shared memory;
 //   * point mode: where they fit, the nx*ny*(nbins+1) count tile and the nx*ny
 //     first-time tile live in shared memory; one atomic add per detection,
 //     first times by atomicMin on order-preserving uint32 keys where the
@@ -15,8 +15,9 @@
 //     coalesced global atomics and the last CTA decodes the first-time keys in
 //     place;
 //   * segment mode (scan points, 511 keV events): per-segment 8x8 maps and
-//     first-time keys are reduced with global atomics; a finalize kernel
-//     decodes keys and sums npe.
+//     first-time keys are reduced with global atomics, one of each per
+//     detection, or per distinct slot of a warp where many photons share a slot
+//     (add_crowded); a finalize kernel decodes keys and sums npe.
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -243,7 +244,10 @@ __global__ void __launch_bounds__(256, CL_MIN_CTAS_PER_SM) transport_kernel(cons
 
     // free lanes that make a turnover worth its cost: 1 / 3 / 4 lanes took 105.5 /
     // 100.5 / 101.0 ms on the scan (a photon ends every 97 steps); 1 / 4 / 8 / 10
-    // lanes 23.8 / 21.3 / 20.5 / 20.6 ms on the events (every 12 steps)
+    // lanes 23.8 / 21.3 / 20.5 / 20.6 ms on the events (every 12 steps).  The
+    // general instance serves short and long lives: 3 / 5 / 8 lanes take 1,230 /
+    // 1,170 / 1,157 us for 2M photons of 14 steps (specular paint), 1,032 / 971 /
+    // 959 of 7 (diffuse paint), 6.75 / 6.66 / 7.02 ms of 122 (polished, specular)
     constexpr int TURNOVER = SPEC == SPEC_ESR ? 3 : 8;
 
     uint32_t* tile_counts = TILE ? s_counts : A.counts;
@@ -983,7 +987,11 @@ int cl_create(cl_handle** out, int device)
     }
     h->stage = (char*)malloc(STAGE_IN + STAGE_OUT);
     // 128 MB: the logs of all 2^24 uniforms and their sqrt(-2 log u); without
-    // them (allocation failure) the kernels evaluate the same functions in place
+    // them (allocation failure) the kernels evaluate the same functions in place.
+    // The logs alone, and the root in the loop (sqrt_mid, the same bits), would fit
+    // L2 beside everything else, and cost more: scan 92.6 -> 93.9 ms, 2,000 photons
+    // 208 -> 223 us, 3,001 events 18.83 -> 18.87 ms.  A handle takes 0.8 ms to make
+    // with either.
     if (cudaMalloc(&h->logtab.p, sizeof(float) << 25) == cudaSuccess) {
         h->logtab.cap = sizeof(float) << 25;
         logtab_fill<<<h->num_sms * 4, 256, LOGTAB_BYTES, h->stream>>>((float*)h->logtab.p);

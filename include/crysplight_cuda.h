@@ -348,8 +348,8 @@ int cl_surrogate_combine_direct(const float* d_raw, int32_t members, int64_t n_s
  * (absorption or Rayleigh scattering: survival exp(-d (1/abs_len +
  * 1/rayleigh)) over the path d), is transmitted by the face (the Fresnel
  * coefficients of the transport, n_crystal -> n_coupling, total internal
- * reflection beyond the critical angle) and lands in SiPM c's pixel, at
- * PDE 1; landing points off the face count for nothing (those photons meet a
+ * reflection beyond the critical angle) and lands in SiPM c's pixel (the last
+ * column and row reach the face edge, as in the transport), at PDE 1; landing points off the face count for nothing (those photons meet a
  * side wall first).  Computed by quadrature over the polar angle (64
  * Gauss-Legendre nodes up to the critical angle) with the azimuthal arcs of
  * each pixel exact.  Requires a 64-cell grid read out on the face z = Lz
